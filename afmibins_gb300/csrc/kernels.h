@@ -214,27 +214,37 @@ template <typename T>
 PipeCfg rbgs_pipe_cfg(const Dims& d);
 
 // The V-cycle from level 0 of these levels down (smooth nu1, residual,
-// restrict, ..., the one-block CG on the last level, prolong-add, smooth nu2)
-// in one block: for the coarse levels (a few thousand cells or fewer), where
-// launches cost more than work. Equals the launch-by-launch V-cycle bit for
-// bit. For T = float the last level is solved in FP64 through cx64/cb64/cr64.
-constexpr int kMaxTailLevels = 8;
-template <typename T>
-struct TailLevels {
-    int nlev, nu1, nu2, maxit;
-    Dims d[kMaxTailLevels];
-    T* x[kMaxTailLevels];
-    T* b[kMaxTailLevels];
-    T* r[kMaxTailLevels];
-    double *cx64, *cb64, *cr64, *cw_p, *cw_q;
-    double tol;
-    int* status;
+// restrict, ..., the direct FP64 solve of the last level, prolong-add, smooth
+// nu2) in one launch on one thread-block cluster (kernels_tail.cu): for the
+// coarse levels, where launches cost more than work. Equals the
+// launch-by-launch V-cycle bit for bit. With one level it is the coarsest
+// solve alone. Only the first level's x and b are global arrays.
+constexpr int kMaxTailLevels = 12;
+constexpr long long kTailCells = 32768;  // largest level (cells) the tail takes
+constexpr int kMaxBasis = 256;           // largest coarsest-level extent of the direct solve
+// Orthonormal eigenvectors (row k: mode k, row 0 the constant) and
+// eigenvalues (of the second difference, times n^-2) of the coarsest
+// Laplacian per axis; on a 2D grid vz, lz belong to y and vy, ly are 1, 0.
+struct TailBasis {
+    const double *vx = nullptr, *vy = nullptr, *vz = nullptr, *lx = nullptr, *ly = nullptr, *lz = nullptr;
 };
 template <typename T>
-void launch_vcycle_tail(const TailLevels<T>& a, cudaStream_t s, int cluster = 1);
-// Largest thread-block cluster (16, 8 or 4 CTAs) the cluster form of the
-// V-cycle tail can be launched with on this device; 1: none.
-int vcycle_tail_cluster_max();
+struct TailLevels {
+    int nlev, flat, x_zero;  // flat: 2D grid; x_zero: x starts at zero, its contents not yet cleared
+    Dims d[kMaxTailLevels];
+    int nu1[kMaxTailLevels], nu2[kMaxTailLevels];
+    double omega;
+    T* x;
+    const T* b;
+    TailBasis basis;
+    int* status;  // receives 3 where the coarsest right-hand side is not finite
+};
+template <typename T>
+bool vcycle_tail_ok(const TailLevels<T>& a);
+template <typename T>
+void launch_vcycle_tail(const TailLevels<T>& a, cudaStream_t s);
+// the tail kernels' opt-ins on the current device (before any launch or stream capture)
+void vcycle_tail_attributes();
 template <typename T>
 void launch_rbgs_pipe(const Dims& d, const PipeCfg& c, const T* xin, T* xout, const T* b, int* err, cudaStream_t s);
 // Full-weighting restriction, src/mg/solver.h:153-181 (d = fine dims); zero
@@ -259,7 +269,8 @@ void launch_resid_restrict(const Dims& d, T* coarse_b, T* coarse_x, const T* x, 
 // Prolongation that assigns (for the op-level API).
 template <typename T>
 void launch_prolong_assign(const Dims& d, T* fine, const T* coarse, cudaStream_t s);
-// Coarsest-level solve (mean removal + CG on one block), src/mg/solver.h:264-271.
+// Coarsest-level solve (mean removal + CG on one block), src/mg/solver.h:264-271,
+// for levels the direct solve (launch_vcycle_tail with one level) does not take.
 // status[0] receives 0 or 3 (not converged).
 template <typename T>
 void launch_coarse_solve(const Dims& d, T* x, T* b, T* r, T* p, T* q, double tol, int maxit, int* status,

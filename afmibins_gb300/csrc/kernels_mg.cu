@@ -6,6 +6,7 @@
 
 #include "dfloat.cuh"
 #include "kernels.h"
+#include "mg_cells.cuh"
 
 namespace afmib {
 
@@ -725,30 +726,18 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_rbgs_pipe(Dims d, const T* 
 }
 
 // Full weighting, src/mg/solver.h:153-181: 64 taps (1,3,3,1)^3/512 around the
-// coarse cell; y clamps at the channel walls, wraps in periodic mode.
+// coarse cell (restrict_taps, mg_cells.cuh); y clamps at the channel walls,
+// wraps in periodic mode.
 template <typename T>
 __device__ __forceinline__ void restrict_cell(const Dims& d, T* coarse, const T* fine, int xc, int yc, int zc) {
     const int cx = d.nx / 2, cy = d.ny / 2;
-    if (d.nz == 1) {
-        // 2D (periodic): (1,3,3,1)^2 / 64 over 16 taps
-        const T wgt[4] = {T(1), T(3), T(3), T(1)};
-        T acc = T(0);
-#pragma unroll
-        for (int ky = 0; ky < 4; ++ky)
-#pragma unroll
-            for (int kx = 0; kx < 4; ++kx)
-                acc += (wgt[kx] * wgt[ky] / T(64)) *
-                       fine[lin(d, wrapi(2 * xc + 1 + kx - 2, d.nx), wrapi(2 * yc + 1 + ky - 2, d.ny), 0)];
-        coarse[xc + (long long)cx * yc] = acc;
-        return;
-    }
     const int xcf = 2 * xc + 1, ycf = 2 * yc + 1, zcf = 2 * zc + 1;
     int xs[4], ys[4], zs[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         const int dd = k - 2;
         xs[k] = wrapi(xcf + dd, d.nx);
-        zs[k] = wrapi(zcf + dd, d.nz);
+        zs[k] = d.nz == 1 ? 0 : wrapi(zcf + dd, d.nz);
         if (d.channel) {
             int yy = ycf + (dd > -ycf ? dd : -ycf);
             ys[k] = yy < d.ny - 1 ? yy : d.ny - 1;
@@ -756,16 +745,13 @@ __device__ __forceinline__ void restrict_cell(const Dims& d, T* coarse, const T*
             ys[k] = wrapi(ycf + dd, d.ny);
         }
     }
-    const T wgt[4] = {T(1), T(3), T(3), T(1)};
-    T acc = T(0);
-#pragma unroll
-    for (int kz = 0; kz < 4; ++kz)
-#pragma unroll
-        for (int ky = 0; ky < 4; ++ky)
-#pragma unroll
-            for (int kx = 0; kx < 4; ++kx)
-                acc += (wgt[kx] * wgt[ky] * wgt[kz] / T(512)) * fine[lin(d, xs[kx], ys[ky], zs[kz])];
-    coarse[xc + (long long)cx * (yc + (long long)cy * zc)] = acc;
+    if (d.nz == 1) {  // 2D (periodic): (1,3,3,1)^2 / 64 over 16 taps
+        coarse[xc + (long long)cx * yc] =
+            restrict_plane<T>([&](int ky, int kx) { return fine[lin(d, xs[kx], ys[ky], 0)]; }) * T(1.0 / 64.0);
+        return;
+    }
+    coarse[xc + (long long)cx * (yc + (long long)cy * zc)] =
+        restrict_taps<T>([&](int kz, int ky, int kx) { return fine[lin(d, xs[kx], ys[ky], zs[kz])]; });
 }
 
 // zero (optional): the coarse iterate, set to zero at every coarse cell
@@ -780,67 +766,64 @@ __global__ void k_restrict(Dims d, T* __restrict__ coarse, const T* __restrict__
     }
 }
 
-// Trilinear prolongation (27,9,3,1)/64, src/mg/solver.h:71-151. One thread per
-// coarse cell writes the eight fine cells between it and its +1 neighbours;
-// in channel mode the wall rows take the bilinear (9,3,1)/16 weights.
+// Trilinear prolongation (27,9,3,1)/64, src/mg/solver.h:71-151 (prolong_plane4,
+// mg_cells.cuh). One thread per coarse cell writes the eight fine cells between
+// it and its +1 neighbours; in channel mode the wall rows take the bilinear
+// (9,3,1)/16 weights. C(x, y, z): the coarse values; put(x, y, z, value,
+// scale): adds to or sets the fine cell.
 template <typename T, bool ADD>
-__device__ __forceinline__ void prolong_cell(const Dims& d, T* fine, const T* coarse, int xc, int yc, int zc) {
-    const int cx = d.nx / 2, cy = d.ny / 2, cz = d.nz / 2;
-    auto C = [&](int a, int b, int c) { return coarse[a + (long long)cx * (b + (long long)cy * c)]; };
-    auto put = [&](int a, int b, int c, T val) {
-        const long long i = lin(d, a, b, c);
-        if (ADD) fine[i] = fine[i] + val; else fine[i] = val;
-    };
-    if (d.nz == 1) {
-        // 2D (periodic): bilinear (9,3,3,1)/16 onto the four fine cells
-        auto C2 = [&](int a, int b) { return coarse[a + (long long)cx * b]; };
-        const int xn = (xc + 1) % cx, yn = (yc + 1) % cy;
-        const int xcf = 2 * xc + 1, ycf = 2 * yc + 1, xnf = (xcf + 1) % d.nx, ynf = (ycf + 1) % d.ny;
-        const T bl = C2(xc, yc), br = C2(xn, yc), ul = C2(xc, yn), ur = C2(xn, yn);
-        const T a = T(9) / T(16), b = T(3) / T(16), e = T(1) / T(16);
-        put(xcf, ycf, 0, a * bl + b * (br + ul) + e * ur);
-        put(xnf, ycf, 0, a * br + b * (bl + ur) + e * ul);
-        put(xcf, ynf, 0, a * ul + b * (ur + bl) + e * br);
-        put(xnf, ynf, 0, a * ur + b * (ul + br) + e * bl);
-        return;
-    }
-    const int xn = (xc + 1) % cx, zn = (zc + 1) % cz;
-    const int xcf = 2 * xc + 1, zcf = 2 * zc + 1;
-    const int xnf = (xcf + 1) % d.nx, znf = (zcf + 1) % d.nz;
-    const bool interior = d.channel ? (yc < cy - 1) : true;
-    if (interior) {
-        const int yn = d.channel ? yc + 1 : (yc + 1) % cy;
-        const int ycf = 2 * yc + 1, ynf = d.channel ? ycf + 1 : (ycf + 1) % d.ny;
-        const T blb = C(xc, yc, zc), brb = C(xn, yc, zc), ulb = C(xc, yn, zc), urb = C(xn, yn, zc);
-        const T blf = C(xc, yc, zn), brf = C(xn, yc, zn), ulf = C(xc, yn, zn), urf = C(xn, yn, zn);
-        const T a = T(27) / T(64), b = T(9) / T(64), c = T(3) / T(64), e = T(1) / T(64);
-        put(xcf, ycf, zcf, a * blb + b * (brb + ulb + blf) + c * (urb + ulf + brf) + e * urf);
-        put(xnf, ycf, zcf, a * brb + b * (urb + blb + brf) + c * (ulb + blf + urf) + e * ulf);
-        put(xcf, ynf, zcf, a * ulb + b * (urb + blb + ulf) + c * (brb + blf + urf) + e * brf);
-        put(xnf, ynf, zcf, a * urb + b * (brb + ulb + urf) + c * (blb + ulf + brf) + e * blf);
-        put(xcf, ycf, znf, a * blf + b * (brf + ulf + blb) + c * (urf + ulb + brb) + e * urb);
-        put(xnf, ycf, znf, a * brf + b * (urf + blf + brb) + c * (ulf + blb + urb) + e * ulb);
-        put(xcf, ynf, znf, a * ulf + b * (urf + blf + ulb) + c * (brf + blb + urb) + e * brb);
-        put(xnf, ynf, znf, a * urf + b * (brf + ulf + urb) + c * (blf + ulb + brb) + e * blb);
+__device__ __forceinline__ void prolong_put(T* fine, long long i, T val, T scale) {
+    if (ADD) fine[i] = fma_t(val, scale, fine[i]);
+    else fine[i] = val * scale;
+}
+template <typename T, typename C, typename P>
+__device__ __forceinline__ void prolong_cell_any(const Dims& d, int xc, int yc, int zc, int xn, int yn, int zn,
+                                                 const int (&xf)[2], const int (&yf)[2], const int (&zf)[2], C cv,
+                                                 P put) {
+    const int cy = d.ny / 2;
+    if (!d.channel || yc < cy - 1) {
+        const T blb = cv(xc, yc, zc), brb = cv(xn, yc, zc), ulb = cv(xc, yn, zc), urb = cv(xn, yn, zc);
+        const T blf = cv(xc, yc, zn), brf = cv(xn, yc, zn), ulf = cv(xc, yn, zn), urf = cv(xn, yn, zn);
+        prolong_plane4(blb, brb, ulb, urb, blf, brf, ulf, urf,
+                       [&](int rx, int ry, T v, T s) { put(xf[rx], yf[ry], zf[0], v, s); });
+        prolong_plane4(blf, brf, ulf, urf, blb, brb, ulb, urb,
+                       [&](int rx, int ry, T v, T s) { put(xf[rx], yf[ry], zf[1], v, s); });
     }
     if (d.channel && (yc == 0 || yc == cy - 1)) {
-        const T a = T(9) / T(16), b = T(3) / T(16), e = T(1) / T(16);
-        // a thread with cy == 1 owns both wall rows
-        for (int side = 0; side < 2; ++side) {
+        for (int side = 0; side < 2; ++side) {  // a thread with cy == 1 owns both wall rows
             if (side == 0 && yc != 0) continue;
             if (side == 1 && yc != cy - 1) continue;
-            const int ycs = side == 0 ? 0 : cy - 1, yf = side == 0 ? 0 : d.ny - 1;
-            const T bl = C(xc, ycs, zc), br = C(xn, ycs, zc), fl = C(xc, ycs, zn), fr = C(xn, ycs, zn);
-            put(xcf, yf, zcf, a * bl + b * (br + fl) + e * fr);
-            put(xnf, yf, zcf, a * br + b * (bl + fr) + e * fl);
-            put(xcf, yf, znf, a * fl + b * (fr + bl) + e * br);
-            put(xnf, yf, znf, a * fr + b * (fl + br) + e * bl);
+            const int yw = side == 0 ? 0 : d.ny - 1;
+            const T bl = cv(xc, yc, zc), br = cv(xn, yc, zc), fl = cv(xc, yc, zn), fr = cv(xn, yc, zn);
+            prolong_row2(bl, br, fl, fr, [&](int rx, T v, T s) { put(xf[rx], yw, zf[0], v, s); });
+            prolong_row2(fl, fr, bl, br, [&](int rx, T v, T s) { put(xf[rx], yw, zf[1], v, s); });
         }
     }
 }
+template <typename T, bool ADD>
+__device__ __forceinline__ void prolong_cell(const Dims& d, T* fine, const T* coarse, int xc, int yc, int zc) {
+    const int cx = d.nx / 2, cy = d.ny / 2, cz = d.nz / 2;
+    const int xn = (xc + 1) % cx, yn = (yc + 1) % cy;
+    const int xf[2] = {2 * xc + 1, (2 * xc + 2) % d.nx}, yf[2] = {2 * yc + 1, (2 * yc + 2) % d.ny};
+    if (d.nz == 1) {
+        // 2D (periodic): bilinear (9,3,3,1)/16 onto the four fine cells
+        auto C2 = [&](int a, int b) { return coarse[a + (long long)cx * b]; };
+        const T bl = C2(xc, yc), br = C2(xn, yc), ul = C2(xc, yn), ur = C2(xn, yn);
+        prolong_row2(bl, br, ul, ur,
+                     [&](int rx, T v, T s) { prolong_put<T, ADD>(fine, lin(d, xf[rx], yf[0], 0), v, s); });
+        prolong_row2(ul, ur, bl, br,
+                     [&](int rx, T v, T s) { prolong_put<T, ADD>(fine, lin(d, xf[rx], yf[1], 0), v, s); });
+        return;
+    }
+    const int zf[2] = {2 * zc + 1, (2 * zc + 2) % d.nz};
+    prolong_cell_any<T>(
+        d, xc, yc, zc, xn, yn, (zc + 1) % cz, xf, yf, zf,
+        [&](int a, int b, int c) { return coarse[a + (long long)cx * (b + (long long)cy * c)]; },
+        [&](int a, int b, int c, T v, T s) { prolong_put<T, ADD>(fine, lin(d, a, b, c), v, s); });
+}
 
 // restrict_cell / prolong_cell for 3D power-of-two levels with Ix2 indexing
-// (same taps, same weights, same summation order)
+// (the same arithmetic)
 template <typename T>
 __device__ __forceinline__ void restrict_cell2(const Dims& d, const Ix2& I, T* coarse, const T* fine, int xc, int yc,
                                                int zc) {
@@ -858,16 +841,8 @@ __device__ __forceinline__ void restrict_cell2(const Dims& d, const Ix2& I, T* c
             yo[k] = ((ycf + dd) & I.my) << I.lx;
         }
     }
-    const T wgt[4] = {T(1), T(3), T(3), T(1)};
-    T acc = T(0);
-#pragma unroll
-    for (int kz = 0; kz < 4; ++kz)
-#pragma unroll
-        for (int ky = 0; ky < 4; ++ky)
-#pragma unroll
-            for (int kx = 0; kx < 4; ++kx)
-                acc += (wgt[kx] * wgt[ky] * wgt[kz] / T(512)) * fine[xs[kx] | yo[ky] | zo[kz]];
-    coarse[xc | (yc << (I.lx - 1)) | (zc << (I.lxy - 2))] = acc;
+    coarse[xc | (yc << (I.lx - 1)) | (zc << (I.lxy - 2))] =
+        restrict_taps<T>([&](int kz, int ky, int kx) { return fine[xs[kx] | yo[ky] | zo[kz]]; });
 }
 
 template <typename T>
@@ -885,43 +860,12 @@ template <typename T, bool ADD>
 __device__ __forceinline__ void prolong_cell2(const Dims& d, const Ix2& I, T* fine, const T* coarse, int xc, int yc,
                                               int zc) {
     const int cx = d.nx / 2, cy = d.ny / 2, cz = d.nz / 2, lcx = I.lx - 1, lcxy = I.lxy - 2;
-    auto C = [&](int a, int b, int c) { return coarse[a | (b << lcx) | (c << lcxy)]; };
-    auto put = [&](int a, int b, int c, T val) {
-        const int i = I.at(a, b, c);
-        if (ADD) fine[i] = fine[i] + val; else fine[i] = val;
-    };
-    const int xn = (xc + 1) & (cx - 1), zn = (zc + 1) & (cz - 1);
-    const int xcf = 2 * xc + 1, zcf = 2 * zc + 1;
-    const int xnf = (xcf + 1) & I.mx, znf = (zcf + 1) & I.mz;
-    const bool interior = d.channel ? (yc < cy - 1) : true;
-    if (interior) {
-        const int yn = d.channel ? yc + 1 : (yc + 1) & (cy - 1);
-        const int ycf = 2 * yc + 1, ynf = d.channel ? ycf + 1 : (ycf + 1) & I.my;
-        const T blb = C(xc, yc, zc), brb = C(xn, yc, zc), ulb = C(xc, yn, zc), urb = C(xn, yn, zc);
-        const T blf = C(xc, yc, zn), brf = C(xn, yc, zn), ulf = C(xc, yn, zn), urf = C(xn, yn, zn);
-        const T a = T(27) / T(64), b = T(9) / T(64), c = T(3) / T(64), e = T(1) / T(64);
-        put(xcf, ycf, zcf, a * blb + b * (brb + ulb + blf) + c * (urb + ulf + brf) + e * urf);
-        put(xnf, ycf, zcf, a * brb + b * (urb + blb + brf) + c * (ulb + blf + urf) + e * ulf);
-        put(xcf, ynf, zcf, a * ulb + b * (urb + blb + ulf) + c * (brb + blf + urf) + e * brf);
-        put(xnf, ynf, zcf, a * urb + b * (brb + ulb + urf) + c * (blb + ulf + brf) + e * blf);
-        put(xcf, ycf, znf, a * blf + b * (brf + ulf + blb) + c * (urf + ulb + brb) + e * urb);
-        put(xnf, ycf, znf, a * brf + b * (urf + blf + brb) + c * (ulf + blb + urb) + e * ulb);
-        put(xcf, ynf, znf, a * ulf + b * (urf + blf + ulb) + c * (brf + blb + urb) + e * brb);
-        put(xnf, ynf, znf, a * urf + b * (brf + ulf + urb) + c * (blf + ulb + brb) + e * blb);
-    }
-    if (d.channel && (yc == 0 || yc == cy - 1)) {
-        const T a = T(9) / T(16), b = T(3) / T(16), e = T(1) / T(16);
-        for (int side = 0; side < 2; ++side) {
-            if (side == 0 && yc != 0) continue;
-            if (side == 1 && yc != cy - 1) continue;
-            const int ycs = side == 0 ? 0 : cy - 1, yf = side == 0 ? 0 : d.ny - 1;
-            const T bl = C(xc, ycs, zc), br = C(xn, ycs, zc), fl = C(xc, ycs, zn), fr = C(xn, ycs, zn);
-            put(xcf, yf, zcf, a * bl + b * (br + fl) + e * fr);
-            put(xnf, yf, zcf, a * br + b * (bl + fr) + e * fl);
-            put(xcf, yf, znf, a * fl + b * (fr + bl) + e * br);
-            put(xnf, yf, znf, a * fr + b * (fl + br) + e * bl);
-        }
-    }
+    const int xf[2] = {2 * xc + 1, (2 * xc + 2) & I.mx}, yf[2] = {2 * yc + 1, (2 * yc + 2) & I.my},
+              zf[2] = {2 * zc + 1, (2 * zc + 2) & I.mz};
+    prolong_cell_any<T>(
+        d, xc, yc, zc, (xc + 1) & (cx - 1), (yc + 1) & (cy - 1), (zc + 1) & (cz - 1), xf, yf, zf,
+        [&](int a, int b, int c) { return coarse[a | (b << lcx) | (c << lcxy)]; },
+        [&](int a, int b, int c, T v, T s) { prolong_put<T, ADD>(fine, I.at(a, b, c), v, s); });
 }
 
 // Fine-level residual fused with the full-weighting restriction and the
@@ -930,8 +874,8 @@ __device__ __forceinline__ void prolong_cell2(const Dims& d, const Ix2& I, T* fi
 // side: the taps reach one fine cell beyond the tile's own) is formed in
 // shared memory, one fine plane at a time, in a ring of the four planes the
 // current coarse plane reads, and every coarse cell sums its 64 taps from the
-// ring. The residual is k_residual_z2's expression and the taps are
-// restrict_cell2's in its order, so the coarse right-hand side equals the two
+// ring. The residual is k_residual_z2's expression and the sum is
+// restrict_cell2's, so the coarse right-hand side equals the two
 // kernels' bit for bit, and the fine residual is never written to memory.
 constexpr int RR_T = 16, RR_F = 2 * RR_T + 2, RR_THREADS = RR_T * RR_T;
 // ring plane layout: row stride RR_RS, even columns first and odd columns
@@ -989,23 +933,14 @@ __global__ void __launch_bounds__(RR_THREADS) k_resid_restrict2(Dims d, T* __res
         }
         row[k] = yy - yf0;
     }
-    const T wgt[4] = {T(1), T(3), T(3), T(1)};
     fill(2 * zc0 - 1);
     fill(2 * zc0);
     for (int zc = zc0; zc < zc0 + RR_CZ; ++zc) {
         fill(2 * zc + 1);
         fill(2 * zc + 2);
         __syncthreads();
-        T acc = T(0);
-#pragma unroll
-        for (int kz = 0; kz < 4; ++kz) {
-            const T* pl = ring[(2 * zc - 1 + kz) & 3];
-#pragma unroll
-            for (int ky = 0; ky < 4; ++ky)
-#pragma unroll
-                for (int kx = 0; kx < 4; ++kx)
-                    acc += (wgt[kx] * wgt[ky] * wgt[kz] / T(512)) * pl[row[ky] * RR_RS + col[kx]];
-        }
+        const T acc = restrict_taps<T>(
+            [&](int kz, int ky, int kx) { return ring[(2 * zc - 1 + kz) & 3][row[ky] * RR_RS + col[kx]]; });
         const int o = xc | (yc << (I.lx - 1)) | (zc << (I.lxy - 2));
         cb[o] = acc;
         cx[o] = T(0);
@@ -1052,13 +987,10 @@ struct Pair<double> {
     using type = double2;
 };
 
-// Full weighting with restrict_cell2's taps, weights and summation order: the
-// coarse cell's single accumulator takes its 64 terms plane by plane (kz), row
-// by row (ky), cell by cell (kx). Fine planes 2 zc + 1 and 2 zc + 2 are the
-// last two planes (kz = 2, 3) of coarse plane zc and the first two (kz = 0, 1)
-// of zc + 1, so each fine plane is read once and feeds two accumulators, the
-// second of which starts from zero with that plane's terms: the same
-// additions in the same order as the one-cell kernel, the same bits.
+// Full weighting with restrict_cell2's arithmetic (restrict_plane, full4):
+// fine planes 2 zc + 1 and 2 zc + 2 are the last two planes of coarse plane zc
+// and the first two of zc + 1, so each fine plane is read and summed once and
+// its sum serves two coarse planes: the same bits with half the sums.
 //
 // A lane reads 16 bytes of each fine tap row (CE = 4 FP32 or 2 FP64 cells)
 // and takes the cells on either side from its neighbours, so it serves CE / 2
@@ -1162,35 +1094,28 @@ __global__ void __launch_bounds__(32 * kTrBY) k_restrict_cols(Dims d, T* __restr
             e[ky][CE + 1] = r;
         }
     };
-    const T wgt[4] = {T(1), T(3), T(3), T(1)};
-    // coarse cell m of the lane: taps fine x = 2 xc - 1 .. 2 xc + 2 = e[ky][2m .. 2m + 3]
-    auto add = [&](T (&acc)[M], const T (&e)[4][CE + 2], int kz) {
+    // a plane's sum for coarse cell m of the lane: taps fine x = 2 xc - 1 ..
+    // 2 xc + 2 = e[ky][2m .. 2m + 3]
+    auto plane = [&](T (&p)[M], const T (&e)[4][CE + 2]) {
 #pragma unroll
-        for (int m = 0; m < M; ++m)
-#pragma unroll
-            for (int ky = 0; ky < 4; ++ky)
-#pragma unroll
-                for (int kx = 0; kx < 4; ++kx) acc[m] += (wgt[kx] * wgt[ky] * wgt[kz] / T(512)) * e[ky][2 * m + kx];
+        for (int m = 0; m < M; ++m) p[m] = restrict_plane<T>([&](int ky, int kx) { return e[ky][2 * m + kx]; });
     };
 #pragma unroll
     for (int i = 0; i < kTrStages - 1; ++i) issue(i);
-    T acc[M], next[M], e[4][CE + 2];
-#pragma unroll
-    for (int m = 0; m < M; ++m) acc[m] = T(0);
+    T p0[M], p1[M], p2[M], p3[M], e[4][CE + 2];
     taps(acquire(0), e);
-    add(acc, e, 0);
+    plane(p0, e);
     taps(acquire(1), e);
-    add(acc, e, 1);
+    plane(p1, e);
     const int co = (xc0 + M * lane) | ((yc0 + ty) << (I.lx - 1));
     for (int k = 0; k < CZ; ++k) {
-#pragma unroll
-        for (int m = 0; m < M; ++m) next[m] = T(0);
         taps(acquire(2 * k + 2), e);
-        add(acc, e, 2);
-        add(next, e, 0);
+        plane(p2, e);
         taps(acquire(2 * k + 3), e);
-        add(acc, e, 3);
-        add(next, e, 1);
+        plane(p3, e);
+        T acc[M];
+#pragma unroll
+        for (int m = 0; m < M; ++m) acc[m] = full4<T>(p0[m], p1[m], p2[m], p3[m]) * T(1.0 / 512.0);
         const int o = co | ((zc0 + k) << (I.lxy - 2));
         if constexpr (M == 2) {
             *reinterpret_cast<float2*>(coarse + o) = make_float2(acc[0], acc[1]);
@@ -1200,7 +1125,10 @@ __global__ void __launch_bounds__(32 * kTrBY) k_restrict_cols(Dims d, T* __restr
             if (zero) zero[o] = T(0);
         }
 #pragma unroll
-        for (int m = 0; m < M; ++m) acc[m] = next[m];
+        for (int m = 0; m < M; ++m) {
+            p0[m] = p2[m];
+            p1[m] = p3[m];
+        }
     }
     pipe::wait_pending<0>();
 }
@@ -1217,8 +1145,8 @@ __global__ void __launch_bounds__(32 * kTrBY) k_restrict_cols(Dims d, T* __restr
 // The residual plane holds 34 chunks a row (x = 2 xc0 - 4 .. 2 xc0 + 131, the
 // layout k_restrict_cols stages): each thread forms whole chunks, four cells
 // from 16-byte words and the cells on either side by single loads. Every
-// residual is k_residual_z2's expression in its order and the taps are
-// k_restrict_cols' (restrict_cell2's order), so the coarse right-hand side
+// residual is k_residual_z2's expression in its order and the sums are
+// k_restrict_cols', so the coarse right-hand side
 // equals the two kernels' bit for bit. In channel mode the rows beyond the
 // walls take the residual of the wall row, as the restriction's clamped taps
 // read it.
@@ -1357,7 +1285,6 @@ __global__ void __launch_bounds__(32 * kTrBY, 2) k_resid_restrict_cols(Dims d, f
             *reinterpret_cast<float4*>(rs + tr[u]) = o;
         }
     };
-    const float wgt[4] = {1.f, 3.f, 3.f, 1.f};
     // the restriction taps of the residual plane for this thread: e[ky][1 + q]
     // = fine x = 2 xc0 + 4 lane + q, q = -1 .. 4 (k_restrict_cols' taps)
     auto taps = [&](float (&e)[4][6]) {
@@ -1376,18 +1303,12 @@ __global__ void __launch_bounds__(32 * kTrBY, 2) k_resid_restrict_cols(Dims d, f
             e[ky][5] = r;
         }
     };
-    auto add = [&](float (&acc)[2], const float (&e)[4][6], int kz) {
+    // the last four planes' sums, oldest first
+    float p[4][2], e[4][6];
 #pragma unroll
-        for (int ky = 0; ky < 4; ++ky)
-#pragma unroll
-            for (int m = 0; m < 2; ++m)
-#pragma unroll
-                for (int kx = 0; kx < 4; ++kx)
-                    acc[m] += (wgt[kx] * wgt[ky] * wgt[kz] / 512.f) * e[ky][2 * m + kx];
-    };
+    for (int k = 0; k < 4; ++k) p[k][0] = p[k][1] = 0.f;
 #pragma unroll
     for (int k = 0; k < 4; ++k) issue(k);
-    float acc[2] = {0.f, 0.f}, next[2] = {0.f, 0.f}, e[4][6];
     const int co = (xc0 + 2 * lane) | ((yc0 + ty) << (I.lx - 1));
     for (int i = 0; i < NP; ++i) {
         pipe::wait_pending<1>();  // items <= i + 2 are in
@@ -1396,35 +1317,32 @@ __global__ void __launch_bounds__(32 * kTrBY, 2) k_resid_restrict_cols(Dims d, f
         __syncthreads();          // the residual plane is written; x item i and b item i + 1 are free
         issue(i + 4);
         taps(e);
-        if (i == 0) {
-            add(acc, e, 0);
-        } else if (i == 1) {
-            add(acc, e, 1);
-        } else if ((i & 1) == 0) {
-            add(acc, e, 2);
-            add(next, e, 0);
-        } else {
-            add(acc, e, 3);
-            add(next, e, 1);
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+            p[0][m] = p[1][m];
+            p[1][m] = p[2][m];
+            p[2][m] = p[3][m];
+            p[3][m] = restrict_plane<float>([&](int ky, int kx) { return e[ky][2 * m + kx]; });
+        }
+        if (i >= 3 && (i & 1)) {
             const int o = co | ((zc0 + (i - 3) / 2) << (I.lxy - 2));
-            *reinterpret_cast<float2*>(cb + o) = make_float2(acc[0], acc[1]);
+            const float a0 = full4<float>(p[0][0], p[1][0], p[2][0], p[3][0]) * float(1.0 / 512.0);
+            const float a1 = full4<float>(p[0][1], p[1][1], p[2][1], p[3][1]) * float(1.0 / 512.0);
+            *reinterpret_cast<float2*>(cb + o) = make_float2(a0, a1);
             *reinterpret_cast<float2*>(cxz + o) = make_float2(0.f, 0.f);
-            acc[0] = next[0];
-            acc[1] = next[1];
-            next[0] = next[1] = 0.f;
         }
     }
     pipe::wait_pending<0>();
 }
 
-// Trilinear prolongation-add with prolong_cell2's expressions. A thread owns
-// the fine pairs x = 2t, 2t+1 of rows y = 2s, 2s+1 in planes z = 2r, 2r+1:
-// fine cell 2t + 1 is the first (xcf) of coarse cell t and 2t the second
-// (xnf) of coarse cell t - 1, and likewise in y and z, so the eight cells need
-// the coarse values at t - 1 .. t + 1, s - 1 .. s + 1, r - 1 .. r + 1, kept in
-// registers as a window of three coarse planes that moves one plane per r.
-// Each fine cell takes the expression of its role (first or second in x, y
-// and z) with its terms in prolong_cell2's order, and in channel mode the wall
+// Trilinear prolongation-add with prolong_cell2's arithmetic. A thread owns
+// the fine pairs x = 2t, 2t+1 of rows y = 2s, 2s+1 in planes z = 2r, 2r+1, all
+// eight nearest to coarse cell (t, s, r): fine cell 2t + 1 is the first (xcf)
+// of coarse cell t and 2t the second (xnf) of coarse cell t - 1, and likewise
+// in y and z, so they need the coarse values at t - 1 .. t + 1, s - 1 .. s + 1,
+// r - 1 .. r + 1, kept in registers as a window of three coarse planes that
+// moves one plane per r. The sums run along z, then y, then x as in
+// prolong_plane4 and share their partial sums, and in channel mode the wall
 // rows y = 0 and ny - 1 take the wall expressions: the same bits. The block's
 // fine values of plane pair r (2 x 16 rows of 64 cells) and its tile of
 // coarse plane r + 1 arrive in shared memory by 16-byte asynchronous copies
@@ -1488,34 +1406,6 @@ __global__ void __launch_bounds__(32 * kTrBY) k_prolong_cols(Dims d, T* __restri
     };
 #pragma unroll
     for (int i = 0; i < PT::S - 1; ++i) issue(i);
-    const T a = T(27) / T(64), b = T(9) / T(64), c3 = T(3) / T(64), e = T(1) / T(64);
-    const T wa = T(9) / T(16), wb = T(3) / T(16), we = T(1) / T(16);
-    // interior cell of role (rx, ry, rz): 1 = first (xcf), 0 = second (xnf);
-    // its base coarse cell is at offset = role in the window (x, y, z alike)
-    auto cell = [&](const T (&cb)[3][3], const T (&cf)[3][3], int rx, int ry, int rz) -> T {
-        const int ox = rx, oy = ry;
-        const T blb = cb[oy][ox], brb = cb[oy][ox + 1], ulb = cb[oy + 1][ox], urb = cb[oy + 1][ox + 1];
-        const T blf = cf[oy][ox], brf = cf[oy][ox + 1], ulf = cf[oy + 1][ox], urf = cf[oy + 1][ox + 1];
-        const bool fx = rx == 1, fy = ry == 1, fz = rz == 1;
-        if (fx && fy && fz) return a * blb + b * (brb + ulb + blf) + c3 * (urb + ulf + brf) + e * urf;
-        if (!fx && fy && fz) return a * brb + b * (urb + blb + brf) + c3 * (ulb + blf + urf) + e * ulf;
-        if (fx && !fy && fz) return a * ulb + b * (urb + blb + ulf) + c3 * (brb + blf + urf) + e * brf;
-        if (!fx && !fy && fz) return a * urb + b * (brb + ulb + urf) + c3 * (blb + ulf + brf) + e * blf;
-        if (fx && fy && !fz) return a * blf + b * (brf + ulf + blb) + c3 * (urf + ulb + brb) + e * urb;
-        if (!fx && fy && !fz) return a * brf + b * (urf + blf + brb) + c3 * (ulf + blb + urb) + e * ulb;
-        if (fx && !fy && !fz) return a * ulf + b * (urf + blf + ulb) + c3 * (brf + blb + urb) + e * brb;
-        return a * urf + b * (brf + ulf + urb) + c3 * (blf + ulb + brb) + e * blb;
-    };
-    // channel wall cell of x role rx and z role rz, from coarse row s
-    auto wall = [&](const T (&cb)[3][3], const T (&cf)[3][3], int rx, int rz) -> T {
-        const int ox = rx;
-        const T bl = cb[1][ox], br = cb[1][ox + 1], fl = cf[1][ox], fr = cf[1][ox + 1];
-        const bool fx = rx == 1, fz = rz == 1;
-        if (fx && fz) return wa * bl + wb * (br + fl) + we * fr;
-        if (!fx && fz) return wa * br + wb * (bl + fr) + we * fl;
-        if (fx && !fz) return wa * fl + wb * (fr + bl) + we * br;
-        return wa * fr + wb * (fl + br) + we * bl;
-    };
     const bool wall_lo = d.channel && s == 0, wall_hi = d.channel && s == cy - 1;
     // window: coarse planes r - 1, r, r + 1 at rows s - 1 .. s + 1, cells t - 1 .. t + 1
     T w[3][3][3];
@@ -1536,25 +1426,28 @@ __global__ void __launch_bounds__(32 * kTrBY) k_prolong_cols(Dims d, T* __restri
 #pragma unroll
             for (int i = 0; i < 3; ++i) w[2][j][i] = sc[(ty + j) * PT::CW + CE + lane - 1 + i];
 #pragma unroll
-        for (int jz = 0; jz < 2; ++jz)
+        for (int jz = 0; jz < 2; ++jz) {
+            // fine plane 2r + jz: near coarse plane r, far r - 1 or r + 1 (z, then y, then x)
+            T q[3][3];
+#pragma unroll
+            for (int j = 0; j < 3; ++j)
+#pragma unroll
+                for (int i = 0; i < 3; ++i) q[j][i] = near4(w[1][j][i], w[2 * jz][j][i]);
 #pragma unroll
             for (int jy = 0; jy < 2; ++jy) {
-                const T(&cb)[3][3] = w[jz];
-                const T(&cf)[3][3] = w[jz + 1];
-                T v0, v1;  // fine x = 2t (second of t - 1), 2t + 1 (first of t)
-                if ((jy == 0 && wall_lo) || (jy == 1 && wall_hi)) {
-                    v0 = wall(cb, cf, 0, jz);
-                    v1 = wall(cb, cf, 1, jz);
-                } else {
-                    v0 = cell(cb, cf, 0, jy, jz);
-                    v1 = cell(cb, cf, 1, jy, jz);
-                }
+                const bool wl = jy == 0 ? wall_lo : wall_hi;  // a wall row has no y neighbour
+                T h[3];
+#pragma unroll
+                for (int i = 0; i < 3; ++i) h[i] = wl ? q[1][i] : near4(q[1][i], q[2 * jy][i]);
+                const T sc1 = wl ? T(1.0 / 16.0) : T(1.0 / 64.0);
+                // fine x = 2t (nearest to t, far t - 1), 2t + 1 (far t + 1)
                 const P2 old = *reinterpret_cast<const P2*>(sf + (jz * 2 * kTrBY + 2 * ty + jy) * PT::FW + 2 * lane);
                 P2 out;
-                out.x = old.x + v0;
-                out.y = old.y + v1;
+                out.x = fma_t(near4(h[1], h[0]), sc1, old.x);
+                out.y = fma_t(near4(h[1], h[2]), sc1, old.y);
                 *reinterpret_cast<P2*>(fine + ((2 * t) | ((2 * s + jy) << I.lx) | ((2 * r + jz) << I.lxy))) = out;
             }
+        }
 #pragma unroll
         for (int j = 0; j < 3; ++j)
 #pragma unroll
@@ -1567,8 +1460,8 @@ __global__ void __launch_bounds__(32 * kTrBY) k_prolong_cols(Dims d, T* __restri
 }
 
 // Coarsest level, src/mg/solver.h:264-271: remove the mean of b, then CG
-// warm-started from b with the absolute 2-norm stop. One block; the level is
-// a handful of cells (one cell for a cube).
+// warm-started from b with the absolute 2-norm stop. One block; only for
+// coarsest levels too large for the direct solve of kernels_tail.cu.
 template <typename T, int TB = kRedBlock>
 __device__ void coarse_cg_block(const Dims& d, T* xv, T* b, T* r, T* p, T* q, double tol, int maxit, int* status) {
     const long long N = d.ncell(), sxy = d.sxy();
@@ -1636,234 +1529,6 @@ __global__ void __launch_bounds__(kRedBlock) k_coarse_cg(Dims d, T* __restrict__
                                                         T* __restrict__ p, T* __restrict__ q, double tol, int maxit,
                                                         int* status) {
     coarse_cg_block(d, xv, b, r, p, q, tol, maxit, status);
-}
-
-// ---------------------------------------------------------------------------
-// Multigrid tail: the V-cycle below a level of at most 16^3 cells in one
-// block. The coarse levels are a few thousand cells or fewer, so launching
-// their ~12 kernels per level costs more than the work; here one block walks
-// the same sequence (smooth, residual, restrict, zero, ..., coarsest solve,
-// prolong-add, smooth) with block barriers between the phases. Every phase
-// runs the per-cell function of the corresponding kernel and the coarsest
-// solve is the same one-block CG, so the result equals the launch-by-launch
-// V-cycle bit for bit.
-// ---------------------------------------------------------------------------
-// threads of the one-block tail: its phases on a 16^3 level are 2048 to 4096
-// cells, so twice the reduction block size halves each phase's per-thread
-// loop (1024 threads cap the registers at 64 and spill)
-constexpr int kTailThreads = 512;
-
-// cell index -> (x, y, z) for the tail's small levels (32-bit arithmetic)
-__device__ __forceinline__ void tail_xyz(const Dims& d, int i, int& x, int& y, int& z) {
-    const int sxy = d.nx * d.ny;
-    z = i / sxy;
-    const int rem = i - z * sxy;
-    y = rem / d.nx;
-    x = rem - y * d.nx;
-}
-
-template <typename T>
-__device__ __forceinline__ void tail_sweep(const Dims& d, T* x, const T* b, int color, int t0, int ts) {
-    const int hx = d.nx / 2, total = hx * d.ny * d.nz;
-    for (int e = t0; e < total; e += ts) {
-        const int row = e / hx, t = e - row * hx;
-        const int z = row / d.ny, y = row - z * d.ny;
-        const int xx = 2 * t + ((y + z + color) & 1);
-        if (xx < d.nx) rbgs_cell(d, x, b, xx, y, z);
-    }
-}
-
-// Power-of-two 3D levels take the shift-composed forms of the same per-cell
-// functions (lap_row2, restrict_cell2, prolong_cell2: same terms, same order)
-// and decode cell indices by shifts: the one-block tail is bound by the
-// integer work of its phases, not by their few thousand cells' bytes.
-__device__ __forceinline__ bool tail_p2(const Dims& d) {
-    auto p2 = [](int v) { return (v & (v - 1)) == 0; };
-    return d.nz > 1 && p2(d.nx) && p2(d.ny) && p2(d.nz);
-}
-
-template <typename T>
-__device__ __forceinline__ void tail_sweep2(const Dims& d, const Ix2& I, T* x, const T* b, int color, int t0, int ts) {
-    const int hx = d.nx >> 1, lhx = I.lx - 1, ly = I.lxy - I.lx, total = hx * d.ny * d.nz;
-    for (int e = t0; e < total; e += ts) {
-        const int t = e & (hx - 1), row = e >> lhx;
-        const int y = row & I.my, z = row >> ly;
-        const int xx = 2 * t + ((y + z + color) & 1);
-        T S, c;
-        lap_row2(d, I, x, xx, y, z, S, c);
-        const int i = I.at(xx, y, z);
-        const T inv = T(1) / (T(d.n) * T(d.n));
-        const T rc = (c == T(6)) ? T(1.0 / 6.0) : ((c == T(5)) ? T(1.0 / 5.0) : (c == T(4) ? T(0.25) : T(1) / c));
-        x[i] = (S - b[i] * inv) * rc;
-    }
-}
-
-// With `staged`, the levels' x, b, r (and the FP64 coarsest-level vectors)
-// live in shared memory for the whole V-cycle: the top level's x and b are
-// read in, the top level's x is written back (the only result the level
-// above uses). Without it the phases work on the global arrays.
-// CL: the same phases spread over a thread-block cluster (every CTA takes a
-// share of each phase's cells; cluster barriers, whose arrive/wait release
-// and acquire the phase's global writes, separate the phases). The coarsest
-// solve runs in the cluster's first CTA, the same one-block CG, so the result
-// is the one-block tail's, bit for bit; the levels stay in global memory (L2).
-template <typename T, bool CL, int TB = kRedBlock>
-__global__ void __launch_bounds__(TB, 1) k_vcycle_tail(TailLevels<T> g, int staged) {
-    extern __shared__ __align__(16) unsigned char tsm[];
-    // the level tables in shared memory (indexed by level: a local copy
-    // would live in local memory)
-    __shared__ TailLevels<T> a;
-    if (threadIdx.x == 0) a = g;
-    __syncthreads();
-    int t0 = threadIdx.x, ts = blockDim.x;
-    bool lead = true;
-    if constexpr (CL) {
-        namespace cg = cooperative_groups;
-        const cg::cluster_group cl = cg::this_cluster();
-        t0 = (int)cl.block_rank() * blockDim.x + threadIdx.x;
-        ts = (int)cl.num_blocks() * blockDim.x;
-        lead = cl.block_rank() == 0;
-    }
-    auto sync = [&]() {
-        if constexpr (CL) cooperative_groups::this_cluster().sync();
-        else __syncthreads();
-    };
-    if (!CL && staged) {
-        // layout: per level x, b, r (T), then cx64, cb64, cr64, cw_p, cw_q (double)
-        if (threadIdx.x == 0) {
-            size_t off = 0;
-            for (int l = 0; l < a.nlev; ++l) {
-                const long long n = a.d[l].ncell();
-                a.x[l] = (T*)(tsm + off);
-                a.b[l] = a.x[l] + n;
-                a.r[l] = a.b[l] + n;
-                off += (size_t)3 * n * sizeof(T);
-                off = (off + 15) & ~(size_t)15;
-            }
-            const long long nc = a.d[a.nlev - 1].ncell();
-            double* dp = (double*)(tsm + off);
-            a.cx64 = dp;
-            a.cb64 = dp + nc;
-            a.cr64 = dp + 2 * nc;
-            a.cw_p = dp + 3 * nc;
-            a.cw_q = dp + 4 * nc;
-        }
-        __syncthreads();
-        const long long n0 = a.d[0].ncell();
-        T* const x0 = a.x[0];
-        T* const b0 = a.b[0];
-        const T* const gx = g.x[0];
-        const T* const gb = g.b[0];
-        for (long long i = threadIdx.x; i < n0; i += blockDim.x) {
-            x0[i] = gx[i];
-            b0[i] = gb[i];
-        }
-        __syncthreads();
-    }
-    // per level, the dimensions and array pointers are read once into
-    // registers: the level tables sit in local memory (indexed by level), and
-    // through a reference every access inside the cell loops was a reload
-    for (int l = 0; l + 1 < a.nlev; ++l) {
-        const Dims d = a.d[l];
-        T* const xl = a.x[l];
-        T* const bl = a.b[l];
-        T* const rl = a.r[l];
-        T* const xc = a.x[l + 1];
-        T* const bc = a.b[l + 1];
-        const bool p2 = tail_p2(d);
-        const Ix2 I(d);
-        for (int j = 0; j < a.nu1; ++j) {
-            for (int color = 0; color < 2; ++color) {
-                if (p2) tail_sweep2(d, I, xl, bl, color, t0, ts);
-                else tail_sweep(d, xl, bl, color, t0, ts);
-                sync();
-            }
-        }
-        const int n = (int)d.ncell();
-        if (p2) {
-            const T off = T(d.n) * T(d.n);
-            for (int i = t0; i < n; i += ts) {
-                const int xx = i & I.mx, yy = (i >> I.lx) & I.my, zz = i >> I.lxy;
-                T S, c;
-                lap_row2(d, I, xl, xx, yy, zz, S, c);
-                rl[i] = bl[i] - off * (S - c * xl[i]);
-            }
-        } else {
-            for (int i = t0; i < n; i += ts) {
-                int xx, yy, zz;
-                tail_xyz(d, i, xx, yy, zz);
-                residual_cell(d, rl, xl, bl, xx, yy, zz);
-            }
-        }
-        sync();
-        const Dims c = a.d[l + 1];
-        const int nc = (int)c.ncell();
-        if (p2) {
-            const int lcx = I.lx - 1, lcxy = I.lxy - 2, mcx = (d.nx >> 1) - 1, mcy = (d.ny >> 1) - 1;
-            for (int i = t0; i < nc; i += ts) {
-                restrict_cell2(d, I, bc, rl, i & mcx, (i >> lcx) & mcy, i >> lcxy);
-                xc[i] = T(0);
-            }
-        } else {
-            for (int i = t0; i < nc; i += ts) {
-                int xx, yy, zz;
-                tail_xyz(c, i, xx, yy, zz);
-                restrict_cell(d, bc, rl, xx, yy, zz);
-                xc[i] = T(0);
-            }
-        }
-        sync();
-    }
-    if (lead) {  // block-uniform: the whole first CTA (or the one block)
-        const int l = a.nlev - 1;
-        const Dims& d = a.d[l];
-        const long long n = d.ncell();
-        if constexpr (sizeof(T) == sizeof(double)) {
-            coarse_cg_block<T, TB>(d, a.x[l], a.b[l], a.r[l], a.cw_p, a.cw_q, a.tol, a.maxit, a.status);
-        } else {
-            for (long long i = threadIdx.x; i < n; i += blockDim.x) a.cb64[i] = (double)a.b[l][i];
-            __syncthreads();
-            coarse_cg_block<double, TB>(d, a.cx64, a.cb64, a.cr64, a.cw_p, a.cw_q, a.tol, a.maxit, a.status);
-            __syncthreads();
-            for (long long i = threadIdx.x; i < n; i += blockDim.x) a.x[l][i] = (T)a.cx64[i];
-        }
-    }
-    sync();
-    for (int l = a.nlev - 2; l >= 0; --l) {
-        const Dims d = a.d[l];
-        const Dims c = a.d[l + 1];
-        T* const xl = a.x[l];
-        T* const bl = a.b[l];
-        T* const xc = a.x[l + 1];
-        const bool p2 = tail_p2(d);
-        const Ix2 I(d);
-        const int nc = (int)c.ncell();
-        if (p2) {
-            const int lcx = I.lx - 1, lcxy = I.lxy - 2, mcx = (d.nx >> 1) - 1, mcy = (d.ny >> 1) - 1;
-            for (int i = t0; i < nc; i += ts)
-                prolong_cell2<T, true>(d, I, xl, xc, i & mcx, (i >> lcx) & mcy, i >> lcxy);
-        } else {
-            for (int i = t0; i < nc; i += ts) {
-                int xx, yy, zz;
-                tail_xyz(c, i, xx, yy, zz);
-                prolong_cell<T, true>(d, xl, xc, xx, yy, zz);
-            }
-        }
-        sync();
-        for (int j = 0; j < a.nu2; ++j) {
-            for (int color = 0; color < 2; ++color) {
-                if (p2) tail_sweep2(d, I, xl, bl, color, t0, ts);
-                else tail_sweep(d, xl, bl, color, t0, ts);
-                sync();
-            }
-        }
-    }
-    if (!CL && staged) {
-        const long long n0 = a.d[0].ncell();
-        T* const gx = g.x[0];
-        const T* const x0 = a.x[0];
-        for (long long i = threadIdx.x; i < n0; i += blockDim.x) gx[i] = x0[i];
-    }
 }
 
 }  // namespace
@@ -2235,94 +1900,6 @@ template void launch_lap_defect<float>(const Dims&, float*, const double*, const
                                        cudaStream_t, float*);
 
 template <typename T>
-void launch_vcycle_tail(const TailLevels<T>& a, cudaStream_t s, int cluster) {
-    if (cluster > 1) {
-        if (cluster > 8) {
-            static bool np = false;
-            if (!np)
-                np = cudaFuncSetAttribute(k_vcycle_tail<T, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
-                     cudaSuccess;
-        }
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(cluster);
-        cfg.blockDim = dim3(kRedBlock);
-        cfg.dynamicSmemBytes = 0;
-        cfg.stream = s;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = cluster;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        cudaLaunchKernelEx(&cfg, k_vcycle_tail<T, true>, a, 0);  // errors reach the caller's cudaGetLastError
-        return;
-    }
-    // shared-memory staging when the levels fit
-    size_t bytes = 0;
-    for (int l = 0; l < a.nlev; ++l) {
-        bytes += (size_t)3 * a.d[l].ncell() * sizeof(T);
-        bytes = (bytes + 15) & ~(size_t)15;
-    }
-    bytes += (size_t)5 * a.d[a.nlev - 1].ncell() * sizeof(double);
-    // one block of kTailThreads (AFMIB_TAIL_THREADS=256 or 1024 instead):
-    // the phases are per-cell and the coarsest CG sums the same cells in the
-    // same order, so the block size does not change the result
-    constexpr size_t kMax = 160 * 1024;
-    // read at every launch (graphs capture it once), so that a test can compare block sizes
-    const int threads = [] {
-        const char* e = std::getenv("AFMIB_TAIL_THREADS");
-        const int v = e ? std::atoi(e) : kTailThreads;
-        return v == 1024 || v == kRedBlock ? v : kTailThreads;
-    }();
-    static bool attr = false, attr_big = false, attr_1k = false;
-    if (threads == kTailThreads) {
-        if (!attr_big)
-            attr_big = cudaFuncSetAttribute(k_vcycle_tail<T, false, kTailThreads>,
-                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMax) == cudaSuccess;
-        if (attr_big && bytes <= kMax) k_vcycle_tail<T, false, kTailThreads><<<1, kTailThreads, bytes, s>>>(a, 1);
-        else k_vcycle_tail<T, false, kTailThreads><<<1, kTailThreads, 0, s>>>(a, 0);
-        return;
-    }
-    if (threads == 1024) {
-        if (!attr_1k)
-            attr_1k = cudaFuncSetAttribute(k_vcycle_tail<T, false, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)kMax) == cudaSuccess;
-        if (attr_1k && bytes <= kMax) k_vcycle_tail<T, false, 1024><<<1, 1024, bytes, s>>>(a, 1);
-        else k_vcycle_tail<T, false, 1024><<<1, 1024, 0, s>>>(a, 0);
-        return;
-    }
-    if (!attr)
-        attr = cudaFuncSetAttribute(k_vcycle_tail<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMax) ==
-               cudaSuccess;
-    if (attr && bytes <= kMax) k_vcycle_tail<T, false><<<1, kRedBlock, bytes, s>>>(a, 1);
-    else k_vcycle_tail<T, false><<<1, kRedBlock, 0, s>>>(a, 0);
-}
-
-int vcycle_tail_cluster_max() {
-    for (int cs : {16, 8, 4}) {
-        if (cs > 8 && cudaFuncSetAttribute(k_vcycle_tail<float, true>, cudaFuncAttributeNonPortableClusterSizeAllowed,
-                                           1) != cudaSuccess) {
-            cudaGetLastError();
-            continue;
-        }
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(cs);
-        cfg.blockDim = dim3(kRedBlock);
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = cs;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, k_vcycle_tail<float, true>, &cfg) == cudaSuccess && n > 0) return cs;
-        cudaGetLastError();
-    }
-    return 1;
-}
-template <typename T>
 void launch_coarse_solve(const Dims& d, T* x, T* b, T* r, T* p, T* q, double tol, int maxit, int* status, cudaStream_t s) {
     k_coarse_cg<T><<<1, kRedBlock, 0, s>>>(d, x, b, r, p, q, tol, maxit, status);
 }
@@ -2338,8 +1915,7 @@ void launch_coarse_solve(const Dims& d, T* x, T* b, T* r, T* p, T* q, double tol
     template void launch_prolong_add<T>(const Dims&, T*, const T*, cudaStream_t, int);                      \
     template void launch_resid_restrict<T>(const Dims&, T*, T*, const T*, const T*, cudaStream_t, int);      \
     template void launch_prolong_assign<T>(const Dims&, T*, const T*, cudaStream_t);                     \
-    template void launch_coarse_solve<T>(const Dims&, T*, T*, T*, T*, T*, double, int, int*, cudaStream_t);    \
-    template void launch_vcycle_tail<T>(const TailLevels<T>&, cudaStream_t, int);
+    template void launch_coarse_solve<T>(const Dims&, T*, T*, T*, T*, T*, double, int, int*, cudaStream_t);
 
 AFMIB_MG_INST(double)
 AFMIB_MG_INST(float)

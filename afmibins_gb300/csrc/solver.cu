@@ -170,11 +170,11 @@ struct afmib_solver {
     // FP64 kernels (opt-in, AFMIB_BFP=1: measured no faster on GB300, the
     // integer form being instruction-bound at about the FP64 kernels' time)
     bool bfp_defects = false;
-    // first multigrid level handled by the V-cycle tail (-1: none;
-    // AFMIB_MG_TAIL=0), and the thread-block cluster it runs on (1: one
-    // block)
-    int tail_level = -1;
-    int tail_cluster = 1;
+    // first multigrid level handled by the V-cycle tail of each hierarchy
+    // (-1: none; AFMIB_MG_TAIL=0), and the eigenbasis of the coarsest level's
+    // direct solve
+    int tail_level = -1, tail_level32 = -1;
+    TailBasis basis{};
     // mixed form: inner Helmholtz solves by fixed Jacobi sweeps where the
     // operator's diagonal dominance bounds them, as red-black Gauss-Seidel
     // sweeps (the default where the grid takes them: they contract as the
@@ -526,14 +526,49 @@ int smooth(afmib_solver* s, MGLevelT<T>& L, int sweeps, bool from_zero = false) 
     return AFMIB_OK;
 }
 
-// coarsest level: FP64 solve (the FP32 hierarchy hands its level to FP64)
-int coarse(afmib_solver* s, MGLevelT<double>& L) {
+// the levels from l down as the V-cycle tail takes them
+template <typename T>
+TailLevels<T> tail_levels(afmib_solver* s, size_t l, bool x_zero) {
+    auto& lv = levels<T>(s);
+    const bool f32 = sizeof(T) == sizeof(float);
+    TailLevels<T> a{};
+    a.nlev = (int)(lv.size() - l);
+    if (a.nlev > kMaxTailLevels) return a;
+    a.flat = s->d.nz == 1;
+    a.x_zero = x_zero;
+    for (int k = 0; k < a.nlev; ++k) {
+        const bool fine = l + k == 0;
+        a.d[k] = lv[l + k].d;
+        a.nu1[k] = f32 ? (fine ? s->inner_nu1 : s->inner_nu1c) : s->cfg.nu1;
+        a.nu2[k] = f32 ? (fine ? s->inner_nu2 : s->inner_nu2c) : s->cfg.nu2;
+    }
+    a.omega = f32 ? s->inner_omega : 1.0;
+    a.x = lv[l].x;
+    a.b = lv[l].b;
+    a.basis = s->basis;
+    a.status = s->dflag + 1;
+    return a;
+}
+
+// the V-cycle from level l down in one launch
+template <typename T>
+int vcycle_tail(afmib_solver* s, size_t l, bool x_zero) {
+    const TailLevels<T> a = tail_levels<T>(s, l, x_zero);
+    ProfScope ps(s, l + 1 == levels<T>(s).size() ? P_COARSE : P_TAIL, 0.0);
+    launch_vcycle_tail<T>(a, s->st);
+    CKL();
+    return AFMIB_OK;
+}
+
+// coarsest level: direct FP64 solve, or one-block FP64 CG where it is too
+// large for that (the FP32 hierarchy hands its level to FP64)
+int coarse_cg(afmib_solver* s, MGLevelT<double>& L) {
     ProfScope ps(s, P_COARSE, 3.0 * L.d.ncell() * sizeof(double));
     launch_coarse_solve<double>(L.d, L.x, L.b, L.r, s->cw_p, s->cw_q, s->cfg.tol, s->cfg.max_cg_iters, s->dflag + 1,
                                 s->st);
     return AFMIB_OK;
 }
-int coarse(afmib_solver* s, MGLevelT<float>& L) {
+int coarse_cg(afmib_solver* s, MGLevelT<float>& L) {
     const long long n = L.d.ncell();
     ProfScope ps(s, P_COARSE, 3.0 * n * sizeof(double), 3);
     launch_convert<double, float>(n, s->cb64, L.b, s->st);
@@ -542,33 +577,11 @@ int coarse(afmib_solver* s, MGLevelT<float>& L) {
     launch_convert<float, double>(n, L.x, s->cx64, s->st);
     return AFMIB_OK;
 }
-
-// the coarse V-cycle below level l in one block or one cluster (k_vcycle_tail)
 template <typename T>
-int vcycle_tail(afmib_solver* s, size_t l) {
-    auto& lv = levels<T>(s);
-    TailLevels<T> a{};
-    a.nlev = (int)(lv.size() - l);
-    a.nu1 = sizeof(T) == sizeof(float) ? s->inner_nu1c : s->cfg.nu1;
-    a.nu2 = sizeof(T) == sizeof(float) ? s->inner_nu2c : s->cfg.nu2;
-    a.maxit = s->cfg.max_cg_iters;
-    a.tol = s->cfg.tol;
-    for (int k = 0; k < a.nlev; ++k) {
-        a.d[k] = lv[l + k].d;
-        a.x[k] = lv[l + k].x;
-        a.b[k] = lv[l + k].b;
-        a.r[k] = lv[l + k].r;
-    }
-    a.cx64 = s->cx64;
-    a.cb64 = s->cb64;
-    a.cr64 = s->cr64;
-    a.cw_p = s->cw_p;
-    a.cw_q = s->cw_q;
-    a.status = s->dflag + 1;
-    ProfScope ps(s, P_TAIL, 0.0);
-    launch_vcycle_tail<T>(a, s->st, s->tail_cluster);
-    CKL();
-    return AFMIB_OK;
+int coarse(afmib_solver* s) {
+    const size_t last = levels<T>(s).size() - 1;
+    if (vcycle_tail_ok(tail_levels<T>(s, last, false))) return vcycle_tail<T>(s, last, false);
+    return coarse_cg(s, levels<T>(s)[last]);
 }
 
 // x_zero: level l's x starts at zero, its contents not yet cleared
@@ -578,11 +591,9 @@ int vcycle(afmib_solver* s, size_t l, bool x_zero = false) {
     MGLevelT<T>& L = lv[l];
     const double Ns = (double)L.d.ncell() * sizeof(T);
     const bool last = l + 1 == lv.size();
-    if (x_zero && ((s->tail_level >= 0 && l == (size_t)s->tail_level) || last))
-        CK(cudaMemsetAsync(L.x, 0, L.d.ncell() * sizeof(T), s->st));
-    if (s->tail_level >= 0 && l == (size_t)s->tail_level) return vcycle_tail<T>(s, l);
-    if (last) {
-        TRY(coarse(s, L));
+    if ((int)l == (sizeof(T) == sizeof(float) ? s->tail_level32 : s->tail_level)) return vcycle_tail<T>(s, l, x_zero);
+    if (last) {  // the coarsest solve does not read x
+        TRY(coarse<T>(s));
         CKL();
         return AFMIB_OK;
     }
@@ -1880,10 +1891,45 @@ int setup_tiles(afmib_solver* s) {
     return AFMIB_OK;
 }
 
+// Eigenvectors and eigenvalues of the coarsest level's second differences:
+// the real Fourier basis on periodic axes, cosines between walls
+int setup_basis(afmib_solver* s) {
+    const Dims& d = s->lv.back().d;
+    const bool flat = s->d.nz == 1;
+    const int ext[3] = {d.nx, flat ? 1 : d.ny, flat ? d.ny : d.nz};
+    if (std::max(ext[0], std::max(ext[1], ext[2])) > kMaxBasis || d.ncell() > kTailCells) return AFMIB_OK;
+    const double pi = std::acos(-1.0);
+    const double **v[3] = {&s->basis.vx, &s->basis.vy, &s->basis.vz}, **lam[3] = {&s->basis.lx, &s->basis.ly, &s->basis.lz};
+    for (int a = 0; a < 3; ++a) {
+        const int n = ext[a];
+        std::vector<double> V((size_t)n * n), E(n);
+        for (int k = 0; k < n; ++k) {
+            const bool wall = d.channel && a == 1;
+            const int f = wall ? k : (k + 1) / 2;  // periodic modes: 1, cos 1, sin 1, cos 2, sin 2, ...
+            const bool sine = !wall && k > 0 && k % 2 == 0;
+            const bool flat_mode = f == 0 || (!wall && 2 * f == n);  // constant, or alternating in sign
+            E[k] = 2.0 * std::cos((wall ? pi : 2 * pi) * f / n) - 2.0;
+            for (int i = 0; i < n; ++i) {
+                const double t = wall ? pi * f * (i + 0.5) / n : 2 * pi * (double)((long long)f * i % n) / n;
+                V[(size_t)k * n + i] = (sine ? std::sin(t) : std::cos(t)) * std::sqrt((flat_mode ? 1.0 : 2.0) / n);
+            }
+        }
+        double *dv = nullptr, *de = nullptr;
+        TRY(dalloc(s, &dv, V.size()));
+        TRY(dalloc(s, &de, E.size()));
+        CK(cudaMemcpy(dv, V.data(), V.size() * sizeof(double), cudaMemcpyHostToDevice));
+        CK(cudaMemcpy(de, E.data(), E.size() * sizeof(double), cudaMemcpyHostToDevice));
+        *v[a] = dv;
+        *lam[a] = de;
+    }
+    return AFMIB_OK;
+}
+
 int create(afmib_solver* s, const afmib_config* c, void* stream) {
     s->cfg = *c;
     afmib_config& g = s->cfg;
     mg_kernel_attributes();  // before any capture of the V-cycles
+    vcycle_tail_attributes();
     if (g.n <= 0) g.n = g.nx;
     if (g.nu1 <= 0) g.nu1 = 2;
     if (g.nu2 <= 0) g.nu2 = 2;
@@ -2102,28 +2148,16 @@ int create(afmib_solver* s, const afmib_config* c, void* stream) {
         TRY(dalloc(s, &s->cb64, nc));
         TRY(dalloc(s, &s->cr64, nc));
     }
-    // V-cycle tail, when it leaves at least one smoothed level above the
-    // coarsest: in one block from the first level of at most 16^3 cells, or
-    // (AFMIB_MG_TAIL_CLUSTER=n) on a cluster of n CTAs from the first level of
-    // at most 32^3
+    TRY(setup_basis(s));
+    // V-cycle tail: from the first level it takes (AFMIB_MG_TAIL=0: none)
     {
         bool tail = true;
         if (const char* e = std::getenv("AFMIB_MG_TAIL")) tail = std::string(e) != "0";
-        // the cluster form is opt-in: at 256^3 it measured 114 us per V-cycle
-        // for the levels 32^3..1 on 16 CTAs against 80 us for 16^3..1 in one
-        // block plus the 32^3 level launches, 36.2 against 36.45 IB steps/s
-        int cs = 1;
-        if (const char* e = std::getenv("AFMIB_MG_TAIL_CLUSTER")) {
-            cs = std::min(vcycle_tail_cluster_max(), std::max(1, std::atoi(e)));
-            cudaGetLastError();
+        for (size_t l = 0; tail && l + 1 < s->lv.size(); ++l) {
+            if (s->tail_level < 0 && vcycle_tail_ok(tail_levels<double>(s, l, false))) s->tail_level = (int)l;
+            if (s->mixed && s->tail_level32 < 0 && vcycle_tail_ok(tail_levels<float>(s, l, false)))
+                s->tail_level32 = (int)l;
         }
-        const long long cells = cs > 1 ? 32768 : 4096;
-        for (size_t l = 0; tail && l + 1 < s->lv.size(); ++l)
-            if (s->lv[l].d.ncell() <= cells && s->lv.size() - l <= (size_t)kMaxTailLevels) {
-                s->tail_level = (int)l;
-                s->tail_cluster = cs;
-                break;
-            }
     }
     CK(cudaStreamSynchronize(s->st));
     return AFMIB_OK;
