@@ -114,18 +114,23 @@ __device__ __forceinline__ int bid_lin() { return blockIdx.x + gridDim.x * (bloc
 __device__ __forceinline__ int nblk_lin() { return gridDim.x * gridDim.y * gridDim.z; }
 
 // Block-wide sum of NV values (TB threads per block); result valid in thread 0.
+// Through shared memory, so that the first warp alone adds (TB / 32 - 1 + 5 FP64
+// warp instructions a block; a shuffle tree in every warp took 5 per warp, and
+// the FP64 pipe issues one per 16-19 clocks).
 template <int NV, int TB = kRedBlock>
 __device__ __forceinline__ void block_sum(double (&v)[NV]) {
-    __shared__ double s[TB / 32][NV];
-    warp_sum<NV>(v);
-    const int w = tid_lin() >> 5, l = tid_lin() & 31;
-    if (l == 0)
+    __shared__ double s[NV][TB];
+    const int t = tid_lin();
 #pragma unroll
-        for (int k = 0; k < NV; ++k) s[w][k] = v[k];
+    for (int k = 0; k < NV; ++k) s[k][t] = v[k];
     __syncthreads();
-    if (w == 0) {
+    if (t < 32) {
 #pragma unroll
-        for (int k = 0; k < NV; ++k) v[k] = (l < TB / 32) ? s[l][k] : 0.0;
+        for (int k = 0; k < NV; ++k) {
+            v[k] = s[k][t];
+#pragma unroll
+            for (int j = 1; j < TB / 32; ++j) v[k] += s[k][t + 32 * j];
+        }
         warp_sum<NV>(v);
     }
     __syncthreads();
@@ -178,9 +183,12 @@ constexpr int kRBX = 32, kRBY = 8;
 // Blocks per grid: about four full waves of the 152 SMs at eight resident
 // 256-thread blocks each, so that the last wave is not a fraction.
 constexpr int kRedWaveBlocks = 152 * 8 * 4;
-inline dim3 red_grid3(int nx, int ny, int nz) {
+// FP64 reductions take a quarter of the blocks: their block sums are FP64 work
+// of a fixed size per block (12 warp instructions beside 8 per warp and cell).
+constexpr int kRedBlocks64 = 152 * 8;
+inline dim3 red_grid3(int nx, int ny, int nz, int blocks = kRedWaveBlocks) {
     const int gx = (nx + kRBX - 1) / kRBX, gy = (ny + kRBY - 1) / kRBY;
-    int gz = (kRedWaveBlocks + gx * gy - 1) / (gx * gy);
+    int gz = (blocks + gx * gy - 1) / (gx * gy);
     if (gz * gx * gy > kMaxRedBlocks) gz = kMaxRedBlocks / (gx * gy);
     if (gz > nz) gz = nz;
     if (gz < 1) gz = 1;
@@ -234,11 +242,17 @@ struct Acc {
     __device__ void add(T x) { v += x; }
 };
 
-inline int red_blocks(long long n) {
+inline int red_blocks(long long n, int blocks = kRedWaveBlocks) {
     long long b = (n + kRedBlock - 1) / kRedBlock;
-    if (b > kRedWaveBlocks) b = kRedWaveBlocks;
+    if (b > blocks) b = blocks;
     if (b < 1) b = 1;
     return (int)b;
+}
+
+// blocks of a reduction over values of type T
+template <typename T>
+constexpr int red_target() {
+    return sizeof(T) == sizeof(double) ? kRedBlocks64 : kRedWaveBlocks;
 }
 
 }  // namespace afmib

@@ -6,6 +6,7 @@
 #include "dfloat.cuh"
 #include "kernels.h"
 #include <algorithm>
+#include <cmath>
 
 namespace afmib {
 
@@ -304,58 +305,71 @@ __global__ void k_wall_update(Dims d, double* __restrict__ walls, const double* 
     }
 }
 
+// Coefficients of I + s Delta: off = s n^2, the diagonal of an interior (or 2D)
+// row and of a channel u/w wall row, the wall row's y coefficient and the
+// diagonals' reciprocals. Formed on the host and handed to the kernels: formed
+// per thread they were conversions and FP64 operations on a pipe that issues
+// one warp instruction per 16-19 clocks (cg_apply at 128^3: 84.8 -> 43.1 us with
+// the block sums and grids below).
+template <typename T>
+struct HelmK {
+    T off, diag, diagw, offw, rdiag, rdiagw;
+};
+template <typename T>
+inline HelmK<T> helm_k(const Dims& d, double scale) {
+    HelmK<T> k;
+    k.off = T(scale) * T(d.n) * T(d.n);
+    k.diag = std::fma(d.nz == 1 ? T(-4) : T(-6), k.off, T(1));
+    k.diagw = std::fma(T(-2), k.off, k.diag);
+    k.offw = k.off + k.off / T(3);
+    k.rdiag = T(1) / k.diag;
+    k.rdiagw = T(1) / k.diagw;
+    return k;
+}
+
 // (I + s Delta) applied at one point. Cell rows (u, w; all components in
 // periodic mode) carry the one-sided Dirichlet closure at the channel walls,
 // src/ns/helmholtz.h:90-104; v rows in channel mode treat the walls as zero
 // neighbours (plane 0 and its periodic image), src/ns/helmholtz.h:247-248.
 template <typename T, typename Get>
-__device__ __forceinline__ T helm_point_at(const Dims& d, int comp, T s, Get x, int xi, int yi, int zi) {
+__device__ __forceinline__ T helm_point_at(const Dims& d, int comp, const HelmK<T>& k, Get x, int xi, int yi, int zi) {
     const long long i = lin(d, xi, yi, zi);
-    const T off = s * T(d.n) * T(d.n);
     const T x0 = x(i);
     const T sx = x(lin(d, xm1(d, xi), yi, zi)) + x(lin(d, xp1(d, xi), yi, zi));
     if (d.nz == 1) {
         // 2D (periodic): the one-cell z extent folds into the diagonal,
         // src/ns/helmholtz.h:77-88
         const T sy = x(lin(d, xi, ym1(d, yi), zi)) + x(lin(d, xi, yp1(d, yi), zi));
-        return (T(1) - T(4) * off) * x0 + off * (sx + sy);
+        return k.diag * x0 + k.off * (sx + sy);
     }
     const T sz = x(lin(d, xi, yi, zm1(d, zi))) + x(lin(d, xi, yi, zp1(d, zi)));
     if (d.channel && comp != 1) {
-        T diag = T(1) - T(6) * off;
-        T sy;
-        if (yi == 0) {
-            diag -= T(2) * off;
-            sy = (off + off / T(3)) * x(lin(d, xi, 1, zi));
-        } else if (yi == d.ny - 1) {
-            diag -= T(2) * off;
-            sy = (off + off / T(3)) * x(lin(d, xi, yi - 1, zi));
-        } else {
-            sy = off * (x(lin(d, xi, yi - 1, zi)) + x(lin(d, xi, yi + 1, zi)));
-        }
-        return diag * x0 + (off * (sx + sz) + sy);
+        if (yi == 0 || yi == d.ny - 1)
+            return k.diagw * x0 + (k.off * (sx + sz) + k.offw * x(lin(d, xi, yi == 0 ? 1 : yi - 1, zi)));
+        return k.diag * x0 + (k.off * (sx + sz) + k.off * (x(lin(d, xi, yi - 1, zi)) + x(lin(d, xi, yi + 1, zi))));
     }
     if (d.channel && comp == 1 && yi == 0) return x0;
     const T sy = x(lin(d, xi, ym1(d, yi), zi)) + x(lin(d, xi, yp1(d, yi), zi));
-    return (T(1) - T(6) * off) * x0 + off * (sx + sy + sz);
+    return k.diag * x0 + k.off * (sx + sy + sz);
 }
 
 template <typename T>
-__device__ __forceinline__ T helm_point(const Dims& d, int comp, T s, const T* __restrict__ x, int xi, int yi, int zi) {
-    return helm_point_at(d, comp, s, [x](long long i) { return x[i]; }, xi, yi, zi);
+__device__ __forceinline__ T helm_point(const Dims& d, int comp, const HelmK<T>& k, const T* __restrict__ x, int xi,
+                                        int yi, int zi) {
+    return helm_point_at(d, comp, k, [x](long long i) { return x[i]; }, xi, yi, zi);
 }
 
 template <typename T>
-__global__ void k_helm_apply(Dims d, int comp, T s, T* __restrict__ out, const T* __restrict__ in) {
+__global__ void k_helm_apply(Dims d, int comp, HelmK<T> k, T* __restrict__ out, const T* __restrict__ in) {
     AFMIB_XYZ
-    out[lin(d, x, y, z)] = helm_point(d, comp, s, in, x, y, z);
+    out[lin(d, x, y, z)] = helm_point(d, comp, k, in, x, y, z);
 }
 
 // Right-hand side of the viscous solve, src/ns/solver.h:105-135.
 template <typename T, typename TF, typename TA>
 __global__ void k_helm_rhs(Dims d, int comp, int be, T* __restrict__ r, const T* __restrict__ uold,
                            const TF* __restrict__ f, const TA* __restrict__ adv, const double* __restrict__ top,
-                           const double* __restrict__ bottom, double s_plus, double s_minus, double hdt,
+                           const double* __restrict__ bottom, HelmK<T> kp, double s_plus, double s_minus, double hdt,
                            double inv_rho) {
     AFMIB_XYZ
     const long long i = lin(d, x, y, z);
@@ -375,7 +389,7 @@ __global__ void k_helm_rhs(Dims d, int comp, int be, T* __restrict__ r, const T*
     if (be) {
         r[i] = wall ? (uold[i] + T(-1) * bm) + src : uold[i] + src;
     } else {
-        const T hp = helm_point(d, comp, T(s_plus), uold, x, y, z);
+        const T hp = helm_point(d, comp, kp, uold, x, y, z);
         r[i] = wall ? (hp + (bp - bm)) + src : hp + src;
     }
 }
@@ -387,28 +401,25 @@ __global__ void k_helm_rhs(Dims d, int comp, int be, T* __restrict__ r, const T*
 // helm_point (the same expressions, so the same bits) and Q of one cell from
 // one set of neighbour loads and partial sums
 template <typename T>
-__device__ __forceinline__ void helm_point_q(const Dims& d, int comp, T s, const T* __restrict__ x, int xi, int yi,
-                                             int zi, T& hx, T& q) {
-    const T off = s * T(d.n) * T(d.n);
+__device__ __forceinline__ void helm_point_q(const Dims& d, int comp, const HelmK<T>& k, const T* __restrict__ x,
+                                             int xi, int yi, int zi, T& hx, T& q) {
     const T x0 = x[lin(d, xi, yi, zi)];
     const T sx = x[lin(d, xm1(d, xi), yi, zi)] + x[lin(d, xp1(d, xi), yi, zi)];
     if (d.nz == 1) {
         const T sy = x[lin(d, xi, ym1(d, yi), zi)] + x[lin(d, xi, yp1(d, yi), zi)];
-        hx = (T(1) - T(4) * off) * x0 + off * (sx + sy);
+        hx = k.diag * x0 + k.off * (sx + sy);
         q = (sx + sy) - T(4) * x0;
         return;
     }
     const T sz = x[lin(d, xi, yi, zm1(d, zi))] + x[lin(d, xi, yi, zp1(d, zi))];
     if (d.channel && comp != 1) {
-        T diag = T(1) - T(6) * off;
         if (yi == 0 || yi == d.ny - 1) {
-            diag -= T(2) * off;
             const T xa = x[lin(d, xi, yi == 0 ? 1 : yi - 1, zi)];
-            hx = diag * x0 + (off * (sx + sz) + (off + off / T(3)) * xa);
+            hx = k.diagw * x0 + (k.off * (sx + sz) + k.offw * xa);
             q = (sx + sz) + (T(4) / T(3)) * xa - T(8) * x0;
         } else {
             const T sy = x[lin(d, xi, yi - 1, zi)] + x[lin(d, xi, yi + 1, zi)];
-            hx = diag * x0 + (off * (sx + sz) + off * sy);
+            hx = k.diag * x0 + (k.off * (sx + sz) + k.off * sy);
             q = (sx + sz) + sy - T(6) * x0;
         }
         return;
@@ -420,7 +431,7 @@ __device__ __forceinline__ void helm_point_q(const Dims& d, int comp, T s, const
     }
     const T sy = x[lin(d, xi, ym1(d, yi), zi)] + x[lin(d, xi, yp1(d, yi), zi)];
     const T sum = sx + sy + sz;
-    hx = (T(1) - T(6) * off) * x0 + off * sum;
+    hx = k.diag * x0 + k.off * sum;
     q = sum - T(6) * x0;
 }
 
@@ -437,8 +448,9 @@ __global__ void __launch_bounds__(kRedBlock) k_helm_rhs_be_defect(Dims d, int co
                                                                  float* __restrict__ r_out, double* __restrict__ q_out,
                                                                  const double* __restrict__ uold, const TF* __restrict__ f,
                                                                  const TA* __restrict__ adv, const double* __restrict__ top,
-                                                                 const double* __restrict__ bottom, double s_minus,
-                                                                 double hdt, double inv_rho, RedScratch sc, double* out,
+                                                                 const double* __restrict__ bottom, HelmK<double> k,
+                                                                 double s_minus, double hdt, double inv_rho,
+                                                                 RedScratch sc, double* out,
                                                                  float* __restrict__ r_lo, double* __restrict__ uo_out,
                                                                  bool lo_split) {
     float acc = 0.f;
@@ -459,12 +471,11 @@ __global__ void __launch_bounds__(kRedBlock) k_helm_rhs_be_defect(Dims d, int co
             }
         }
         double hx, q;
-        helm_point_q(d, comp, s_minus, uold, xi, yi, zi, hx, q);
+        helm_point_q(d, comp, k, uold, xi, yi, zi, hx, q);
         if (!DFR) b_out[i] = b;
         q_out[i] = q;
         if (uo_out) uo_out[i] = uold[i];  // the step's start velocity, kept for the CN sub-step
-        const double off = s_minus * double(d.n) * double(d.n);  // helm_point_q's
-        const double rd = DFR ? (vwall ? -uold[i] : sb - off * q) : b - hx;
+        const double rd = DFR ? (vwall ? -uold[i] : sb - k.off * q) : b - hx;
         float lo;
         const float ri = defect_words(rd, r_lo ? &lo : nullptr, lo_split);
         r_out[i] = ri;
@@ -489,12 +500,11 @@ template <typename TF, typename TA>
 __global__ void k_helm_rhs_cn_q(Dims d, int comp, double* __restrict__ r, const double* __restrict__ uold,
                                 const double* __restrict__ q, const TF* __restrict__ f, const TA* __restrict__ adv,
                                 const double* __restrict__ top, const double* __restrict__ bottom, double s_plus,
-                                double s_minus, double hdt, double inv_rho) {
+                                double s_minus, double off, double hdt, double inv_rho) {
     AFMIB_XYZ
     const long long i = lin(d, x, y, z);
     if (d.channel && comp == 1 && y == 0) { r[i] = 0.0; return; }
     const double src = hdt * (inv_rho * cvt<double, TF>(f[i]) - cvt<double, TA>(adv[i]));
-    const double off = s_plus * double(d.n) * double(d.n);
     if (d.channel && comp != 1 && (y == 0 || y == d.ny - 1) && top) {
         const long long ixz = x + (long long)d.nx * z;
         const double wv = (y == 0) ? bottom[ixz] : top[ixz];
@@ -519,10 +529,9 @@ __global__ void __launch_bounds__(kRedBlock) k_helm_cn_first(Dims d, int comp, d
                                                             const TF* __restrict__ f, const TA* __restrict__ adv,
                                                             const double* __restrict__ top,
                                                             const double* __restrict__ bottom, double s_plus,
-                                                            double s_minus, double hdt, double inv_rho, RedScratch sc,
-                                                            double* out) {
+                                                            double s_minus, double offd, double hdt, double inv_rho,
+                                                            RedScratch sc, double* out) {
     const int xi = blockIdx.x * kRBX + threadIdx.x, yi = blockIdx.y * kRBY + threadIdx.y;
-    const double offd = (s_plus - s_minus) * double(d.n) * double(d.n);
     float acc = 0.f;
     if (xi < d.nx && yi < d.ny)
         for (int zi = blockIdx.z; zi < d.nz; zi += gridDim.z) {
@@ -695,7 +704,7 @@ __global__ void __launch_bounds__(kRedBlock) k_helm_cn_first_df(Dims d, int comp
 // test on n0 (the reference's absolute 2-norm stop, src/alg/cg.h:42).
 // ---------------------------------------------------------------------------
 template <typename T>
-__global__ void __launch_bounds__(kRedBlock) k_cg_init(Dims d, int comp, T s, const T* __restrict__ x,
+__global__ void __launch_bounds__(kRedBlock) k_cg_init(Dims d, int comp, HelmK<T> k, const T* __restrict__ x,
                                                       const T* __restrict__ b, T* __restrict__ r, T* __restrict__ p,
                                                       RedScratch sc, double* cgs) {
     const int xi = blockIdx.x * kRBX + threadIdx.x, yi = blockIdx.y * kRBY + threadIdx.y;
@@ -704,7 +713,7 @@ __global__ void __launch_bounds__(kRedBlock) k_cg_init(Dims d, int comp, T s, co
 #pragma unroll 2
         for (int zi = blockIdx.z; zi < d.nz; zi += gridDim.z) {
             const long long i = lin(d, xi, yi, zi);
-            const T ri = b[i] - helm_point(d, comp, s, x, xi, yi, zi);
+            const T ri = b[i] - helm_point(d, comp, k, x, xi, yi, zi);
             r[i] = ri;
             p[i] = ri;
             acc += ri * ri;
@@ -714,7 +723,7 @@ __global__ void __launch_bounds__(kRedBlock) k_cg_init(Dims d, int comp, T s, co
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kRedBlock) k_cg_apply(Dims d, int comp, T s, const T* __restrict__ p,
+__global__ void __launch_bounds__(kRedBlock) k_cg_apply(Dims d, int comp, HelmK<T> k, const T* __restrict__ p,
                                                        T* __restrict__ q, RedScratch sc, double* cgs) {
     const int xi = blockIdx.x * kRBX + threadIdx.x, yi = blockIdx.y * kRBY + threadIdx.y;
     T acc = T(0);
@@ -722,7 +731,7 @@ __global__ void __launch_bounds__(kRedBlock) k_cg_apply(Dims d, int comp, T s, c
 #pragma unroll 2
         for (int zi = blockIdx.z; zi < d.nz; zi += gridDim.z) {
             const long long i = lin(d, xi, yi, zi);
-            const T qi = helm_point(d, comp, s, p, xi, yi, zi);
+            const T qi = helm_point(d, comp, k, p, xi, yi, zi);
             q[i] = qi;
             acc += p[i] * qi;
         }
@@ -753,7 +762,7 @@ __global__ void __launch_bounds__(kRedBlock) k_cg_update(long long N, T* __restr
 // p' = beta p + r is formed on the fly at the seven stencil points, written
 // out of place to pn, and q = H p' with p'.q reduced; alpha in the finisher.
 template <typename T>
-__global__ void __launch_bounds__(kRedBlock) k_cg_dir_apply(Dims d, int comp, T s, const T* __restrict__ p,
+__global__ void __launch_bounds__(kRedBlock) k_cg_dir_apply(Dims d, int comp, HelmK<T> k, const T* __restrict__ p,
                                                            const T* __restrict__ r, T* __restrict__ pn,
                                                            T* __restrict__ q, RedScratch sc, double* cgs) {
     const T beta = T(cgs[3]);
@@ -765,7 +774,7 @@ __global__ void __launch_bounds__(kRedBlock) k_cg_dir_apply(Dims d, int comp, T 
         for (int zi = blockIdx.z; zi < d.nz; zi += gridDim.z) {
             const long long i = lin(d, xi, yi, zi);
             const T pi = P(i);
-            const T qi = helm_point_at(d, comp, s, P, xi, yi, zi);
+            const T qi = helm_point_at(d, comp, k, P, xi, yi, zi);
             pn[i] = pi;
             q[i] = qi;
             acc += pi * qi;
@@ -787,7 +796,8 @@ __global__ void k_cg_direction(long long N, T* __restrict__ p, const T* __restri
 // the FP64 update x += e with the FP32 correction.
 // ---------------------------------------------------------------------------
 template <typename TD, bool WALK>
-__global__ void __launch_bounds__(kRedBlock) k_helm_defect(Dims d, int comp, double s, const double* __restrict__ x,
+__global__ void __launch_bounds__(kRedBlock) k_helm_defect(Dims d, int comp, HelmK<double> k,
+                                                          const double* __restrict__ x,
                                                           const double* __restrict__ b, TD* __restrict__ r,
                                                           RedScratch sc, double* out, float* __restrict__ r_lo,
                                                           bool lo_split) {
@@ -795,7 +805,7 @@ __global__ void __launch_bounds__(kRedBlock) k_helm_defect(Dims d, int comp, dou
     auto body = [&](int xi, int yi, int zi) {
         const long long i = lin(d, xi, yi, zi);
         float lo;
-        const TD ri = defect_words(b[i] - helm_point(d, comp, s, x, xi, yi, zi), r_lo ? &lo : nullptr, lo_split);
+        const TD ri = defect_words(b[i] - helm_point(d, comp, k, x, xi, yi, zi), r_lo ? &lo : nullptr, lo_split);
         r[i] = ri;
         if (r_lo) r_lo[i] = lo;
         acc += ri * ri;
@@ -869,52 +879,43 @@ __global__ void __launch_bounds__(kRedBlock) k_helm_defect_bfp(Dims d, int comp,
 // from zero: x' = b / diag.
 // helm_point_at with Ix2 indexing (power-of-two extents): same terms, same order
 template <typename T>
-__device__ __forceinline__ T helm_point2(const Dims& d, const Ix2& I, int comp, T s, const T* __restrict__ x, int xi,
-                                         int yi, int zi) {
-    const T off = s * T(d.n) * T(d.n);
+__device__ __forceinline__ T helm_point2(const Dims& d, const Ix2& I, int comp, const HelmK<T>& k,
+                                         const T* __restrict__ x, int xi, int yi, int zi) {
     const T x0 = x[I.at(xi, yi, zi)];
     const T sx = x[I.at(I.xm(xi), yi, zi)] + x[I.at(I.xp(xi), yi, zi)];
     if (d.nz == 1) {
         const T sy = x[I.at(xi, I.ym(yi), zi)] + x[I.at(xi, I.yp(yi), zi)];
-        return (T(1) - T(4) * off) * x0 + off * (sx + sy);
+        return k.diag * x0 + k.off * (sx + sy);
     }
     const T sz = x[I.at(xi, yi, I.zm(zi))] + x[I.at(xi, yi, I.zp(zi))];
     if (d.channel && comp != 1) {
-        T diag = T(1) - T(6) * off;
-        T sy;
-        if (yi == 0) {
-            diag -= T(2) * off;
-            sy = (off + off / T(3)) * x[I.at(xi, 1, zi)];
-        } else if (yi == d.ny - 1) {
-            diag -= T(2) * off;
-            sy = (off + off / T(3)) * x[I.at(xi, yi - 1, zi)];
-        } else {
-            sy = off * (x[I.at(xi, yi - 1, zi)] + x[I.at(xi, yi + 1, zi)]);
-        }
-        return diag * x0 + (off * (sx + sz) + sy);
+        if (yi == 0 || yi == d.ny - 1)
+            return k.diagw * x0 + (k.off * (sx + sz) + k.offw * x[I.at(xi, yi == 0 ? 1 : yi - 1, zi)]);
+        return k.diag * x0 + (k.off * (sx + sz) + k.off * (x[I.at(xi, yi - 1, zi)] + x[I.at(xi, yi + 1, zi)]));
     }
     if (d.channel && comp == 1 && yi == 0) return x0;
     const T sy = x[I.at(xi, I.ym(yi), zi)] + x[I.at(xi, I.yp(yi), zi)];
-    return (T(1) - T(6) * off) * x0 + off * (sx + sy + sz);
+    return k.diag * x0 + k.off * (sx + sy + sz);
 }
 
+// reciprocal of the row's diagonal
 template <typename T>
-__device__ __forceinline__ T helm_diag(const Dims& d, int comp, T off, int y) {
-    if (d.nz == 1) return T(1) - T(4) * off;
-    if (d.channel && comp != 1 && (y == 0 || y == d.ny - 1)) return (T(1) - T(6) * off) - T(2) * off;
-    if (d.channel && comp == 1 && y == 0) return T(1);
-    return T(1) - T(6) * off;
+__device__ __forceinline__ T helm_rdiag(const Dims& d, int comp, const HelmK<T>& k, int y) {
+    if (d.channel && d.nz > 1) {
+        if (comp != 1 && (y == 0 || y == d.ny - 1)) return k.rdiagw;
+        if (comp == 1 && y == 0) return T(1);
+    }
+    return k.rdiag;
 }
 
 // ZU cells along z per thread, all computed before any is stored (the
 // sweep is out of place, so this only puts ZU cells' loads in flight at once)
 template <typename T, int ZU>
-__global__ void k_helm_jacobi(Dims d, int comp, T s, const T* __restrict__ xv, T* __restrict__ xo,
+__global__ void k_helm_jacobi(Dims d, int comp, HelmK<T> k, const T* __restrict__ xv, T* __restrict__ xo,
                               const T* __restrict__ b) {
     const int x = blockIdx.x * BX + threadIdx.x, y = blockIdx.y * BY + threadIdx.y, z0 = blockIdx.z * ZU;
     if (x >= d.nx || y >= d.ny) return;
-    const T off = s * T(d.n) * T(d.n);
-    const T rdiag = T(1) / helm_diag(d, comp, off, y);
+    const T rdiag = helm_rdiag(d, comp, k, y);
     T val[ZU];
 #pragma unroll
     for (int u = 0; u < ZU; ++u) {
@@ -922,7 +923,7 @@ __global__ void k_helm_jacobi(Dims d, int comp, T s, const T* __restrict__ xv, T
         if (!xv) {
             val[u] = b[i] * rdiag;
         } else {
-            const T hx = helm_point_at(d, comp, s, [xv](long long j) { return xv[j]; }, x, y, z0 + u);
+            const T hx = helm_point_at(d, comp, k, [xv](long long j) { return xv[j]; }, x, y, z0 + u);
             val[u] = xv[i] + (b[i] - hx) * rdiag;
         }
     }
@@ -1061,7 +1062,8 @@ void launch_wall_update(const Dims& d, double* walls, const double* wallgrad, cu
 template <typename T, typename TF, typename TA>
 void launch_helm_rhs(const Dims& d, int comp, int be, T* r, const T* uold, const TF* f, const TA* adv, const double* top,
                      const double* bottom, double s_plus, double s_minus, double dt, double inv_rho, cudaStream_t s) {
-    k_helm_rhs<T, TF, TA><<<grid3(d), block3(), 0, s>>>(d, comp, be, r, uold, f, adv, top, bottom, s_plus, s_minus,
+    k_helm_rhs<T, TF, TA><<<grid3(d), block3(), 0, s>>>(d, comp, be, r, uold, f, adv, top, bottom,
+                                                        helm_k<T>(d, s_plus), s_plus, s_minus,
                                                         be ? dt / 2 : dt, inv_rho);
 }
 template <typename TF, typename TA>
@@ -1071,7 +1073,8 @@ void launch_helm_rhs_be_defect(const Dims& d, int comp, double* b, float* r, dou
                                float* r_lo, double* uo_out) {
 #define AFMIB_BE(WALKV, DFRV, GRID)                                                                          \
     k_helm_rhs_be_defect<TF, TA, WALKV, DFRV><<<GRID, dim3(kRBX, kRBY), 0, s>>>(                             \
-        d, comp, b, r, q, uold, f, adv, top, bottom, s_minus, dt / 2, inv_rho, sc, out, r_lo, uo_out, lo_split())
+        d, comp, b, r, q, uold, f, adv, top, bottom, helm_k<double>(d, s_minus), s_minus, dt / 2, inv_rho, sc,  \
+        out, r_lo, uo_out, lo_split())
     if (walk_blocks > 0) {
         if (r_lo) AFMIB_BE(true, true, walk_grid(d, walk_blocks));
         else AFMIB_BE(true, false, walk_grid(d, walk_blocks));
@@ -1126,7 +1129,8 @@ template <typename TF, typename TA>
 void launch_helm_rhs_cn_q(const Dims& d, int comp, double* r, const double* uold, const double* q, const TF* f,
                           const TA* adv, const double* top, const double* bottom, double s_plus, double s_minus,
                           double dt, double inv_rho, cudaStream_t s) {
-    k_helm_rhs_cn_q<TF, TA><<<grid3(d), block3(), 0, s>>>(d, comp, r, uold, q, f, adv, top, bottom, s_plus, s_minus, dt,
+    k_helm_rhs_cn_q<TF, TA><<<grid3(d), block3(), 0, s>>>(d, comp, r, uold, q, f, adv, top, bottom, s_plus, s_minus,
+                                                          s_plus * double(d.n) * double(d.n), dt,
                                                           inv_rho);
 }
 template <typename TF, typename TA>
@@ -1134,7 +1138,8 @@ void launch_helm_cn_first(const Dims& d, int comp, double* x, float* rh, float* 
                           const TF* f, const TA* adv, const double* top, const double* bottom, double s_plus,
                           double s_minus, double dt, double inv_rho, RedScratch sc, double* out, cudaStream_t s) {
     k_helm_cn_first<TF, TA><<<red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s>>>(
-        d, comp, x, rh, rl, uold, q, f, adv, top, bottom, s_plus, s_minus, dt, inv_rho, sc, out);
+        d, comp, x, rh, rl, uold, q, f, adv, top, bottom, s_plus, s_minus,
+        (s_plus - s_minus) * double(d.n) * double(d.n), dt, inv_rho, sc, out);
 }
 template void launch_helm_cn_first<double, float>(const Dims&, int, double*, float*, float*, const double*,
                                                   const double*, const double*, const float*, const double*,
@@ -1163,11 +1168,11 @@ template <typename TD>
 void launch_helm_defect(const Dims& d, int comp, double scale, const double* x, const double* b, TD* r, RedScratch sc,
                         double* out, cudaStream_t s, int walk_blocks, float* r_lo) {
     if (walk_blocks > 0)
-        k_helm_defect<TD, true><<<walk_grid(d, walk_blocks), dim3(kRBX, kRBY), 0, s>>>(d, comp, scale, x, b, r, sc, out,
-                                                                                       r_lo, lo_split());
+        k_helm_defect<TD, true><<<walk_grid(d, walk_blocks), dim3(kRBX, kRBY), 0, s>>>(
+            d, comp, helm_k<double>(d, scale), x, b, r, sc, out, r_lo, lo_split());
     else
-        k_helm_defect<TD, false><<<red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s>>>(d, comp, scale, x, b, r, sc,
-                                                                                            out, r_lo, lo_split());
+        k_helm_defect<TD, false><<<red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s>>>(
+            d, comp, helm_k<double>(d, scale), x, b, r, sc, out, r_lo, lo_split());
 }
 
 // Mixed form, recursive outer residual of a viscous solve: with the FP32
@@ -1325,31 +1330,30 @@ void launch_add_correction(long long n, double* x, const TE* e, cudaStream_t s) 
 }
 template <typename T>
 void launch_helm_apply(const Dims& d, int comp, double scale, T* y, const T* x, cudaStream_t s) {
-    k_helm_apply<T><<<grid3(d), block3(), 0, s>>>(d, comp, T(scale), y, x);
+    k_helm_apply<T><<<grid3(d), block3(), 0, s>>>(d, comp, helm_k<T>(d, scale), y, x);
 }
 template <typename T>
 void launch_cg_init(const Dims& d, int comp, double scale, const T* x, const T* b, T* r, T* p, RedScratch sc,
                     double* cgs, cudaStream_t s) {
-    k_cg_init<T><<<red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s>>>(d, comp, T(scale), x, b, r, p, sc, cgs);
+    k_cg_init<T><<<red_grid3(d.nx, d.ny, d.nz, red_target<T>()), dim3(kRBX, kRBY), 0, s>>>(d, comp, helm_k<T>(d, scale), x, b, r, p, sc, cgs);
 }
 template <typename T>
 void launch_cg_apply(const Dims& d, int comp, double scale, const T* p, T* q, RedScratch sc, double* cgs, cudaStream_t s) {
-    k_cg_apply<T><<<red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s>>>(d, comp, T(scale), p, q, sc, cgs);
+    k_cg_apply<T><<<red_grid3(d.nx, d.ny, d.nz, red_target<T>()), dim3(kRBX, kRBY), 0, s>>>(d, comp, helm_k<T>(d, scale), p, q, sc, cgs);
 }
 template <typename T, int ZU>
-__global__ void k_helm_jacobi2(Dims d, int comp, T s, const T* __restrict__ xv, T* __restrict__ xo,
+__global__ void k_helm_jacobi2(Dims d, int comp, HelmK<T> k, const T* __restrict__ xv, T* __restrict__ xo,
                                const T* __restrict__ b, int rev) {
     const Ix2 I(d);
     const uint3 B = block_at(rev);
     const int x = B.x * BX + threadIdx.x, y = B.y * BY + threadIdx.y, z0 = B.z * ZU;
     if (x >= d.nx || y >= d.ny) return;
-    const T off = s * T(d.n) * T(d.n);
-    const T rdiag = T(1) / helm_diag(d, comp, off, y);
+    const T rdiag = helm_rdiag(d, comp, k, y);
     T val[ZU];
 #pragma unroll
     for (int u = 0; u < ZU; ++u) {
         const int i = I.at(x, y, z0 + u);
-        val[u] = xv ? xv[i] + (b[i] - helm_point2(d, I, comp, s, xv, x, y, z0 + u)) * rdiag : b[i] * rdiag;
+        val[u] = xv ? xv[i] + (b[i] - helm_point2(d, I, comp, k, xv, x, y, z0 + u)) * rdiag : b[i] * rdiag;
     }
 #pragma unroll
     for (int u = 0; u < ZU; ++u) xo[I.at(x, y, z0 + u)] = val[u];
@@ -1362,21 +1366,20 @@ __global__ void k_helm_jacobi2(Dims d, int comp, T s, const T* __restrict__ xv, 
 // the 7-point operator under red-black ordering the sweep contracts the
 // error as the square of the Jacobi rate.
 template <typename T, int ZU>
-__device__ __forceinline__ void helm_rbgs2_body(Dims d, int comp, T s, int color, int init, T* __restrict__ xv,
+__device__ __forceinline__ void helm_rbgs2_body(Dims d, int comp, const HelmK<T>& k, int color, int init, T* __restrict__ xv,
                                                 const T* __restrict__ b, int rev) {
     const Ix2 I(d);
     const uint3 B = block_at(rev);
     const int y = B.y * BY + threadIdx.y, t = B.x * BX + threadIdx.x, z0 = B.z * ZU;
     if (y >= d.ny || 2 * t >= d.nx) return;
-    const T off = s * T(d.n) * T(d.n);
-    const T rdiag = T(1) / helm_diag(d, comp, off, y);
+    const T rdiag = helm_rdiag(d, comp, k, y);
     T val[ZU];
     int at[ZU];
 #pragma unroll
     for (int u = 0; u < ZU; ++u) {
         const int z = z0 + u, x = 2 * t + ((y + z + color) & 1);
         const int i = I.at(x, y, z);
-        val[u] = init ? b[i] * rdiag : xv[i] + (b[i] - helm_point2(d, I, comp, s, xv, x, y, z)) * rdiag;
+        val[u] = init ? b[i] * rdiag : xv[i] + (b[i] - helm_point2(d, I, comp, k, xv, x, y, z)) * rdiag;
         at[u] = i;
     }
 #pragma unroll
@@ -1386,9 +1389,9 @@ __device__ __forceinline__ void helm_rbgs2_body(Dims d, int comp, T s, int color
     }
 }
 template <typename T, int ZU, int MINB>
-__global__ void __launch_bounds__(BX * BY, MINB) k_helm_rbgs2b(Dims d, int comp, T s, int color, int init,
+__global__ void __launch_bounds__(BX * BY, MINB) k_helm_rbgs2b(Dims d, int comp, HelmK<T> k, int color, int init,
                                                               T* __restrict__ xv, const T* __restrict__ b, int rev) {
-    helm_rbgs2_body<T, ZU>(d, comp, s, color, init, xv, b, rev);
+    helm_rbgs2_body<T, ZU>(d, comp, k, color, init, xv, b, rev);
 }
 
 template <typename T>
@@ -1398,7 +1401,7 @@ bool launch_helm_rbgs(const Dims& d, int comp, double scale, int color, int init
     const dim3 g((d.nx / 2 + BX - 1) / BX, (d.ny + BY - 1) / BY, d.nz / 8);
     // registers capped for 6 resident blocks (40 against 48): measured with the
     // multigrid smoother's cap, 50.5 against 50.0 IB steps/s at 256^3
-    k_helm_rbgs2b<T, 8, 6><<<g, dim3(BX, BY), 0, s>>>(d, comp, T(scale), color, init, x, b, rev);
+    k_helm_rbgs2b<T, 8, 6><<<g, dim3(BX, BY), 0, s>>>(d, comp, helm_k<T>(d, scale), color, init, x, b, rev);
     return true;
 }
 template bool launch_helm_rbgs<float>(const Dims&, int, double, int, int, float*, const float*, cudaStream_t, int);
@@ -1408,13 +1411,13 @@ void launch_helm_jacobi(const Dims& d, int comp, double scale, const T* x, T* xo
                         int rev) {
     const dim3 blk(BX, BY);
     if (d.nz % 8 == 0 && ix2_ok(d))
-        k_helm_jacobi2<T, 8><<<dim3((d.nx + BX - 1) / BX, (d.ny + BY - 1) / BY, d.nz / 8), blk, 0, s>>>(d, comp, T(scale),
+        k_helm_jacobi2<T, 8><<<dim3((d.nx + BX - 1) / BX, (d.ny + BY - 1) / BY, d.nz / 8), blk, 0, s>>>(d, comp, helm_k<T>(d, scale),
                                                                                                    x, xo, b, rev);
     else if (d.nz % 8 == 0)
-        k_helm_jacobi<T, 8><<<dim3((d.nx + BX - 1) / BX, (d.ny + BY - 1) / BY, d.nz / 8), blk, 0, s>>>(d, comp, T(scale), x,
+        k_helm_jacobi<T, 8><<<dim3((d.nx + BX - 1) / BX, (d.ny + BY - 1) / BY, d.nz / 8), blk, 0, s>>>(d, comp, helm_k<T>(d, scale), x,
                                                                                                   xo, b);
     else
-        k_helm_jacobi<T, 1><<<grid3(d), blk, 0, s>>>(d, comp, T(scale), x, xo, b);
+        k_helm_jacobi<T, 1><<<grid3(d), blk, 0, s>>>(d, comp, helm_k<T>(d, scale), x, xo, b);
 }
 template void launch_helm_jacobi<float>(const Dims&, int, double, const float*, float*, const float*, cudaStream_t,
                                         int);
@@ -1422,11 +1425,11 @@ template void launch_helm_jacobi<float>(const Dims&, int, double, const float*, 
 template <typename T>
 void launch_cg_dir_apply(const Dims& d, int comp, double scale, const T* p, const T* r, T* pn, T* q, RedScratch sc,
                          double* cgs, cudaStream_t s) {
-    k_cg_dir_apply<T><<<red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s>>>(d, comp, T(scale), p, r, pn, q, sc, cgs);
+    k_cg_dir_apply<T><<<red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s>>>(d, comp, helm_k<T>(d, scale), p, r, pn, q, sc, cgs);
 }
 template <typename T>
 void launch_cg_update(long long n, T* x, T* r, const T* p, const T* q, RedScratch sc, double* cgs, cudaStream_t s) {
-    k_cg_update<T><<<red_blocks(n), kRedBlock, 0, s>>>(n, x, r, p, q, sc, cgs);
+    k_cg_update<T><<<red_blocks(n, red_target<T>()), kRedBlock, 0, s>>>(n, x, r, p, q, sc, cgs);
 }
 template <typename T>
 void launch_cg_direction(long long n, T* p, const T* r, const double* cgs, cudaStream_t s) {
@@ -1434,11 +1437,11 @@ void launch_cg_direction(long long n, T* p, const T* r, const double* cgs, cudaS
 }
 template <typename T>
 void launch_sum(long long n, const T* x, RedScratch sc, double* out, cudaStream_t s) {
-    k_sum<T, false><<<red_blocks(n), kRedBlock, 0, s>>>(n, x, sc, out);
+    k_sum<T, false><<<red_blocks(n, red_target<T>()), kRedBlock, 0, s>>>(n, x, sc, out);
 }
 template <typename T>
 void launch_sumsq(long long n, const T* x, RedScratch sc, double* out, cudaStream_t s) {
-    k_sum<T, true><<<red_blocks(n), kRedBlock, 0, s>>>(n, x, sc, out);
+    k_sum<T, true><<<red_blocks(n, red_target<T>()), kRedBlock, 0, s>>>(n, x, sc, out);
 }
 template <typename T>
 void launch_sub_scalar_scaled(long long n, T* x, const double* sum, double scale, cudaStream_t s) {

@@ -15,68 +15,95 @@ namespace {
 constexpr int BX = 32, BY = 8;
 inline dim3 grid3(const Dims& d) { return dim3((d.nx + BX - 1) / BX, (d.ny + BY - 1) / BY, d.nz); }
 
+// Per-level constants and per-row coefficients of the pressure Laplacian. The
+// FP64 pipe issues one warp instruction per 16-19 clocks on an SM, conversions,
+// comparisons and divisions included, so n^2 and 1/n^2 come in as kernel
+// arguments, the neighbour count stays an integer and its coefficients are
+// selected constants (128^3 FP64 colour 24.9 -> 22.9 us, general 104^3 27.0 -> 20.8; with them formed per
+// thread a cell cost 10 FP64 instructions instead of the update's 7).
+template <typename T>
+struct LapK {
+    T off, inv;  // n^2, 1 / n^2
+};
+template <typename T>
+inline LapK<T> lap_k(const Dims& d) {
+    return LapK<T>{T(d.n) * T(d.n), T(1) / (T(d.n) * T(d.n))};
+}
+// the row's neighbour count (6; 5 or 4 at channel walls; 4 in 2D) and its reciprocal
+template <typename T>
+__device__ __forceinline__ T lap_count(int c) {
+    return c == 6 ? T(6) : (c == 5 ? T(5) : T(4));
+}
+template <typename T>
+__device__ __forceinline__ T lap_rcount(int c) {
+    return c == 6 ? T(1.0 / 6.0) : (c == 5 ? T(1.0 / 5.0) : T(0.25));
+}
+
+
 // Neighbour sum and diagonal factor of the Laplacian row at (x, y, z):
 // L x = n^2 * (S - c * x_i), c = 6 in the interior and one less per channel
 // wall (Neumann, src/mg/laplacian.h:75-82). A one-cell z extent (2D) folds
 // its two self-neighbours into the diagonal, src/mg/laplacian.h:62-73.
 template <typename T>
-__device__ __forceinline__ void lap_row(const Dims& d, const T* x, int xi, int yi, int zi, T& S, T& c) {
+__device__ __forceinline__ void lap_row(const Dims& d, const T* x, int xi, int yi, int zi, T& S, int& c) {
     if (d.nz == 1) {
         S = x[lin(d, xm1(d, xi), yi, zi)] + x[lin(d, xp1(d, xi), yi, zi)];
-        c = T(4);
+        c = 4;
     } else {
         S = (x[lin(d, xm1(d, xi), yi, zi)] + x[lin(d, xp1(d, xi), yi, zi)]) +
             (x[lin(d, xi, yi, zm1(d, zi))] + x[lin(d, xi, yi, zp1(d, zi))]);
-        c = T(6);
+        c = 6;
     }
     if (d.channel) {
-        if (yi > 0) S += x[lin(d, xi, yi - 1, zi)]; else c -= T(1);
-        if (yi < d.ny - 1) S += x[lin(d, xi, yi + 1, zi)]; else c -= T(1);
+        if (yi > 0) S += x[lin(d, xi, yi - 1, zi)]; else --c;
+        if (yi < d.ny - 1) S += x[lin(d, xi, yi + 1, zi)]; else --c;
     } else {
         S += x[lin(d, xi, ym1(d, yi), zi)] + x[lin(d, xi, yp1(d, yi), zi)];
     }
 }
 
 template <typename T>
-__global__ void k_lap(Dims d, T* __restrict__ out, const T* __restrict__ in) {
+__global__ void k_lap(Dims d, LapK<T> k, T* __restrict__ out, const T* __restrict__ in) {
     const int x = blockIdx.x * BX + threadIdx.x, y = blockIdx.y * BY + threadIdx.y, z = blockIdx.z;
     if (x >= d.nx || y >= d.ny) return;
-    T S, c;
+    T S;
+    int c;
     lap_row(d, in, x, y, z, S, c);
-    const T off = T(d.n) * T(d.n);
-    out[lin(d, x, y, z)] = off * (S - c * in[lin(d, x, y, z)]);
+    out[lin(d, x, y, z)] = k.off * (S - lap_count<T>(c) * in[lin(d, x, y, z)]);
 }
 
 // r = b - L x at one cell
 template <typename T>
-__device__ __forceinline__ void residual_cell(const Dims& d, T* r, const T* xv, const T* b, int x, int y, int z) {
-    T S, c;
+__device__ __forceinline__ void residual_cell(const Dims& d, const LapK<T>& k, T* r, const T* xv, const T* b, int x,
+                                              int y, int z) {
+    T S;
+    int c;
     lap_row(d, xv, x, y, z, S, c);
     const long long i = lin(d, x, y, z);
-    const T off = T(d.n) * T(d.n);
-    r[i] = b[i] - off * (S - c * xv[i]);
+    r[i] = b[i] - k.off * (S - lap_count<T>(c) * xv[i]);
 }
 
 template <typename T>
-__global__ void k_residual(Dims d, T* __restrict__ r, const T* __restrict__ xv, const T* __restrict__ b) {
+__global__ void k_residual(Dims d, LapK<T> k, T* __restrict__ r, const T* __restrict__ xv, const T* __restrict__ b) {
     const int x = blockIdx.x * BX + threadIdx.x, y = blockIdx.y * BY + threadIdx.y, z = blockIdx.z;
     if (x >= d.nx || y >= d.ny) return;
-    residual_cell(d, r, xv, b, x, y, z);
+    residual_cell(d, k, r, xv, b, x, y, z);
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kRedBlock) k_residual_norm(Dims d, T* __restrict__ r, const T* __restrict__ xv,
-                                                            const T* __restrict__ b, RedScratch sc, double* out) {
+__global__ void __launch_bounds__(kRedBlock) k_residual_norm(Dims d, LapK<T> k, T* __restrict__ r,
+                                                            const T* __restrict__ xv, const T* __restrict__ b,
+                                                            RedScratch sc, double* out) {
     const int xi = blockIdx.x * kRBX + threadIdx.x, yi = blockIdx.y * kRBY + threadIdx.y;
-    const T off = T(d.n) * T(d.n);
     T acc = T(0);
     if (xi < d.nx && yi < d.ny)
 #pragma unroll 2
         for (int zi = blockIdx.z; zi < d.nz; zi += gridDim.z) {
-            T S, c;
+            T S;
+            int c;
             lap_row(d, xv, xi, yi, zi, S, c);
             const long long i = lin(d, xi, yi, zi);
-            const T ri = b[i] - off * (S - c * xv[i]);
+            const T ri = b[i] - k.off * (S - lap_count<T>(c) * xv[i]);
             r[i] = ri;
             acc += ri * ri;
         }
@@ -89,20 +116,21 @@ __global__ void __launch_bounds__(kRedBlock) k_residual_norm(Dims d, T* __restri
 // r_lo: also the rest of the FP64 residual, float(r - r_float), the second
 // word of the double-float pair that k_lap_update_df updates.
 template <typename TD>
-__global__ void __launch_bounds__(kRedBlock) k_lap_defect(Dims d, TD* __restrict__ r, const double* __restrict__ xv,
+__global__ void __launch_bounds__(kRedBlock) k_lap_defect(Dims d, LapK<double> k, TD* __restrict__ r,
+                                                         const double* __restrict__ xv,
                                                          const double* __restrict__ b, RedScratch sc, double* out,
                                                          float* __restrict__ r_lo, bool lo_split) {
     const int xi = blockIdx.x * kRBX + threadIdx.x, yi = blockIdx.y * kRBY + threadIdx.y;
-    const double off = double(d.n) * double(d.n);
     TD acc = TD(0);
     if (xi < d.nx && yi < d.ny)
 #pragma unroll 2
         for (int zi = blockIdx.z; zi < d.nz; zi += gridDim.z) {
-            double S, c;
+            double S;
+            int c;
             lap_row(d, xv, xi, yi, zi, S, c);
             const long long i = lin(d, xi, yi, zi);
             float lo;
-            const TD ri = defect_words(b[i] - off * (S - c * xv[i]), r_lo ? &lo : nullptr, lo_split);
+            const TD ri = defect_words(b[i] - k.off * (S - lap_count<double>(c) * xv[i]), r_lo ? &lo : nullptr, lo_split);
             r[i] = ri;
             if (r_lo) r_lo[i] = lo;
             acc += ri * ri;
@@ -295,13 +323,13 @@ __global__ void __launch_bounds__(kRedBlock) k_lap_defect_bfp(Dims d, int k2, fl
 
 // One colour of red-black Gauss–Seidel: x_i = (b_i - n^2 S) / (-c n^2).
 template <typename T>
-__device__ __forceinline__ void rbgs_cell(const Dims& d, T* xv, const T* b, int x, int y, int z, T omega = T(1)) {
-    T S, c;
+__device__ __forceinline__ void rbgs_cell(const Dims& d, const LapK<T>& k, T* xv, const T* b, int x, int y, int z,
+                                          T omega) {
+    T S;
+    int c;
     lap_row(d, xv, x, y, z, S, c);
     const long long i = lin(d, x, y, z);
-    const T inv = T(1) / (T(d.n) * T(d.n));
-    const T rc = (c == T(6)) ? T(1.0 / 6.0) : ((c == T(5)) ? T(1.0 / 5.0) : (c == T(4) ? T(0.25) : T(1) / c));
-    T v = (S - b[i] * inv) * rc;
+    T v = (S - b[i] * k.inv) * lap_rcount<T>(c);
     if (omega != T(1)) v = v + (omega - T(1)) * (v - xv[i]);
     xv[i] = v;
 }
@@ -309,11 +337,11 @@ __device__ __forceinline__ void rbgs_cell(const Dims& d, T* xv, const T* b, int 
 // omega != 1: over-relaxed update x + omega (gs - x); omega == 1 is plain
 // Gauss-Seidel, bit for bit
 template <typename T>
-__global__ void k_rbgs(Dims d, int color, T omega, T* __restrict__ xv, const T* __restrict__ b) {
+__global__ void k_rbgs(Dims d, LapK<T> k, int color, T omega, T* __restrict__ xv, const T* __restrict__ b) {
     const int y = blockIdx.y * BY + threadIdx.y, z = blockIdx.z;
     const int x = 2 * (blockIdx.x * BX + threadIdx.x) + ((y + z + color) & 1);
     if (x >= d.nx || y >= d.ny) return;
-    rbgs_cell(d, xv, b, x, y, z, omega);
+    rbgs_cell(d, k, xv, b, x, y, z, omega);
 }
 
 // Batched forms: each thread takes ZU cells along z of its (x, y) column and
@@ -329,22 +357,21 @@ constexpr int kZU32 = 4;  // ... of the FP32 red-black colour
 constexpr int kOmegaMinNx = 64;
 
 template <typename T, int ZU>
-__global__ void k_rbgs_z(Dims d, int color, T omega, T* __restrict__ xv, const T* __restrict__ b) {
+__global__ void k_rbgs_z(Dims d, LapK<T> k, int color, T omega, T* __restrict__ xv, const T* __restrict__ b) {
     const int y = blockIdx.y * BY + threadIdx.y, t = blockIdx.x * BX + threadIdx.x, z0 = blockIdx.z * ZU;
     if (y >= d.ny) return;
     T val[ZU];
     long long at[ZU];
-    const T inv = T(1) / (T(d.n) * T(d.n));
 #pragma unroll
     for (int u = 0; u < ZU; ++u) {
         const int z = z0 + u, x = 2 * t + ((y + z + color) & 1);
         at[u] = -1;
         if (x < d.nx) {
-            T S, c;
+            T S;
+            int c;
             lap_row(d, xv, x, y, z, S, c);
             const long long i = lin(d, x, y, z);
-            const T rc = (c == T(6)) ? T(1.0 / 6.0) : ((c == T(5)) ? T(1.0 / 5.0) : (c == T(4) ? T(0.25) : T(1) / c));
-            val[u] = (S - b[i] * inv) * rc;
+            val[u] = (S - b[i] * k.inv) * lap_rcount<T>(c);
             if (omega != T(1)) val[u] = val[u] + (omega - T(1)) * (val[u] - xv[i]);
             at[u] = i;
         }
@@ -358,40 +385,39 @@ __global__ void k_rbgs_z(Dims d, int color, T omega, T* __restrict__ xv, const T
 // same order).
 template <typename T>
 __device__ __forceinline__ void lap_row2(const Dims& d, const Ix2& I, const T* x, int xi, int yi, int zi,
-                                         T& S, T& c) {
+                                         T& S, int& c) {
     if (d.nz == 1) {
         S = x[I.at(I.xm(xi), yi, zi)] + x[I.at(I.xp(xi), yi, zi)];
-        c = T(4);
+        c = 4;
     } else {
         S = (x[I.at(I.xm(xi), yi, zi)] + x[I.at(I.xp(xi), yi, zi)]) + (x[I.at(xi, yi, I.zm(zi))] + x[I.at(xi, yi, I.zp(zi))]);
-        c = T(6);
+        c = 6;
     }
     if (d.channel) {
-        if (yi > 0) S += x[I.at(xi, yi - 1, zi)]; else c -= T(1);
-        if (yi < d.ny - 1) S += x[I.at(xi, yi + 1, zi)]; else c -= T(1);
+        if (yi > 0) S += x[I.at(xi, yi - 1, zi)]; else --c;
+        if (yi < d.ny - 1) S += x[I.at(xi, yi + 1, zi)]; else --c;
     } else {
         S += x[I.at(xi, I.ym(yi), zi)] + x[I.at(xi, I.yp(yi), zi)];
     }
 }
 
 template <typename T, int ZU>
-__device__ __forceinline__ void rbgs_z2_body(Dims d, int color, T omega, T* __restrict__ xv, const T* __restrict__ b,
-                                             int rev) {
+__device__ __forceinline__ void rbgs_z2_body(Dims d, const LapK<T>& k, int color, T omega, T* __restrict__ xv,
+                                             const T* __restrict__ b, int rev) {
     const Ix2 I(d);
     const uint3 B = block_at(rev);
     const int y = B.y * BY + threadIdx.y, t = B.x * BX + threadIdx.x, z0 = B.z * ZU;
     if (y >= d.ny || 2 * t >= d.nx) return;
     T val[ZU];
     int at[ZU];
-    const T inv = T(1) / (T(d.n) * T(d.n));
 #pragma unroll
     for (int u = 0; u < ZU; ++u) {
         const int z = z0 + u, x = 2 * t + ((y + z + color) & 1);
-        T S, c;
+        T S;
+        int c;
         lap_row2(d, I, xv, x, y, z, S, c);
         const int i = I.at(x, y, z);
-        const T rc = (c == T(6)) ? T(1.0 / 6.0) : ((c == T(5)) ? T(1.0 / 5.0) : (c == T(4) ? T(0.25) : T(1) / c));
-        val[u] = (S - b[i] * inv) * rc;
+        val[u] = (S - b[i] * k.inv) * lap_rcount<T>(c);
         if (omega != T(1)) val[u] = val[u] + (omega - T(1)) * (val[u] - xv[i]);
         at[u] = i;
     }
@@ -399,8 +425,8 @@ __device__ __forceinline__ void rbgs_z2_body(Dims d, int color, T omega, T* __re
     for (int u = 0; u < ZU; ++u) xv[at[u]] = val[u];
 }
 template <typename T, int ZU>
-__global__ void k_rbgs_z2(Dims d, int color, T omega, T* __restrict__ xv, const T* __restrict__ b, int rev) {
-    rbgs_z2_body<T, ZU>(d, color, omega, xv, b, rev);
+__global__ void k_rbgs_z2(Dims d, LapK<T> k, int color, T omega, T* __restrict__ xv, const T* __restrict__ b, int rev) {
+    rbgs_z2_body<T, ZU>(d, k, color, omega, xv, b, rev);
 }
 
 // The first colour (red) of a sweep from x = 0 without reading or clearing x
@@ -410,7 +436,7 @@ __global__ void k_rbgs_z2(Dims d, int color, T omega, T* __restrict__ xv, const 
 // each pair is written as zero. The same bits as a memset of x followed by
 // the colour launch.
 template <typename T, int ZU, int MINB>
-__global__ void __launch_bounds__(BX * BY, MINB) k_rbgs_z2b_init(Dims d, T omega, T* __restrict__ xv,
+__global__ void __launch_bounds__(BX * BY, MINB) k_rbgs_z2b_init(Dims d, LapK<T> k, T omega, T* __restrict__ xv,
                                                                 const T* __restrict__ b, int rev, T zero) {
     const Ix2 I(d);
     const uint3 B = block_at(rev);
@@ -418,18 +444,16 @@ __global__ void __launch_bounds__(BX * BY, MINB) k_rbgs_z2b_init(Dims d, T omega
     if (y >= d.ny || 2 * t >= d.nx) return;
     T val[ZU];
     int at[ZU], other[ZU];
-    const T inv = T(1) / (T(d.n) * T(d.n));
 #pragma unroll
     for (int u = 0; u < ZU; ++u) {
         const int z = z0 + u, p = (y + z) & 1, x = 2 * t + p;
-        T c = d.nz == 1 ? T(4) : T(6);
+        int c = d.nz == 1 ? 4 : 6;
         if (d.channel) {
-            if (!(y > 0)) c -= T(1);
-            if (!(y < d.ny - 1)) c -= T(1);
+            if (!(y > 0)) --c;
+            if (!(y < d.ny - 1)) --c;
         }
         const int i = I.at(x, y, z);
-        const T rc = (c == T(6)) ? T(1.0 / 6.0) : ((c == T(5)) ? T(1.0 / 5.0) : (c == T(4) ? T(0.25) : T(1) / c));
-        val[u] = (zero - b[i] * inv) * rc;
+        val[u] = (zero - b[i] * k.inv) * lap_rcount<T>(c);
         if (omega != T(1)) val[u] = val[u] + (omega - T(1)) * (val[u] - zero);
         at[u] = i;
         other[u] = I.at(2 * t + 1 - p, y, z);
@@ -441,9 +465,9 @@ __global__ void __launch_bounds__(BX * BY, MINB) k_rbgs_z2b_init(Dims d, T omega
     }
 }
 template <typename T, int ZU, int MINB>
-__global__ void __launch_bounds__(BX * BY, MINB) k_rbgs_z2b(Dims d, int color, T omega, T* __restrict__ xv,
+__global__ void __launch_bounds__(BX * BY, MINB) k_rbgs_z2b(Dims d, LapK<T> k, int color, T omega, T* __restrict__ xv,
                                                            const T* __restrict__ b, int rev) {
-    rbgs_z2_body<T, ZU>(d, color, omega, xv, b, rev);
+    rbgs_z2_body<T, ZU>(d, k, color, omega, xv, b, rev);
 }
 
 // The FP32 colour on float pairs: a thread owns the pairs (2t, 2t+1) of its
@@ -516,36 +540,37 @@ __global__ void __launch_bounds__(BX * BY, MINB) k_rbgs_pair(Dims d, int color, 
 }
 
 template <typename T, int ZU>
-__global__ void k_residual_z2(Dims d, T* __restrict__ r, const T* __restrict__ xv, const T* __restrict__ b, int rev) {
+__global__ void k_residual_z2(Dims d, LapK<T> k, T* __restrict__ r, const T* __restrict__ xv, const T* __restrict__ b,
+                              int rev) {
     const Ix2 I(d);
     const uint3 B = block_at(rev);
     const int x = B.x * BX + threadIdx.x, y = B.y * BY + threadIdx.y, z0 = B.z * ZU;
     if (x >= d.nx || y >= d.ny) return;
-    const T off = T(d.n) * T(d.n);
     T val[ZU];
 #pragma unroll
     for (int u = 0; u < ZU; ++u) {
-        T S, c;
+        T S;
+        int c;
         lap_row2(d, I, xv, x, y, z0 + u, S, c);
         const int i = I.at(x, y, z0 + u);
-        val[u] = b[i] - off * (S - c * xv[i]);
+        val[u] = b[i] - k.off * (S - lap_count<T>(c) * xv[i]);
     }
 #pragma unroll
     for (int u = 0; u < ZU; ++u) r[I.at(x, y, z0 + u)] = val[u];
 }
 
 template <typename T, int ZU>
-__global__ void k_residual_z(Dims d, T* __restrict__ r, const T* __restrict__ xv, const T* __restrict__ b) {
+__global__ void k_residual_z(Dims d, LapK<T> k, T* __restrict__ r, const T* __restrict__ xv, const T* __restrict__ b) {
     const int x = blockIdx.x * BX + threadIdx.x, y = blockIdx.y * BY + threadIdx.y, z0 = blockIdx.z * ZU;
     if (x >= d.nx || y >= d.ny) return;
-    const T off = T(d.n) * T(d.n);
     T val[ZU];
 #pragma unroll
     for (int u = 0; u < ZU; ++u) {
-        T S, c;
+        T S;
+        int c;
         lap_row(d, xv, x, y, z0 + u, S, c);
         const long long i = lin(d, x, y, z0 + u);
-        val[u] = b[i] - off * (S - c * xv[i]);
+        val[u] = b[i] - k.off * (S - lap_count<T>(c) * xv[i]);
     }
 #pragma unroll
     for (int u = 0; u < ZU; ++u) r[lin(d, x, y, z0 + u)] = val[u];
@@ -910,10 +935,11 @@ __global__ void __launch_bounds__(RR_THREADS) k_resid_restrict2(Dims d, T* __res
                 y &= I.my;
             }
             const int x = (xf0 + jx) & I.mx;
-            T S, c;
+            T S;
+            int c;
             lap_row2(d, I, xv, x, y, z, S, c);
             const int i = I.at(x, y, z);
-            dst[rr_at(jy, jx)] = b[i] - off * (S - c * xv[i]);
+            dst[rr_at(jy, jx)] = b[i] - off * (S - lap_count<T>(c) * xv[i]);
         }
     };
     const int cxl = tid % RR_T, cyl = tid / RR_T;
@@ -1476,10 +1502,11 @@ __device__ void coarse_cg_block(const Dims& d, T* xv, T* b, T* r, T* p, T* q, do
     };
     auto apply = [&](const T* in, long long i) {
         const int xi = (int)(i % d.nx), yi = (int)((i % sxy) / d.nx), zi = (int)(i / sxy);
-        T S, c;
+        T S;
+        int c;
         // the one-cell (or one-row) levels fold self-neighbours into the diagonal
         lap_row(d, in, xi, yi, zi, S, c);
-        return off * (S - c * in[i]);
+        return off * (S - lap_count<T>(c) * in[i]);
     };
     double m = 0.0;
     for (long long i = threadIdx.x; i < N; i += blockDim.x) m += (double)b[i];
@@ -1547,19 +1574,20 @@ int batch_min_nx() {
 
 template <typename T>
 void launch_lap_apply(const Dims& d, T* y, const T* x, cudaStream_t s) {
-    k_lap<T><<<grid3(d), dim3(BX, BY), 0, s>>>(d, y, x);
+    k_lap<T><<<grid3(d), dim3(BX, BY), 0, s>>>(d, lap_k<T>(d), y, x);
 }
 template <typename T>
 void launch_residual(const Dims& d, T* r, const T* x, const T* b, RedScratch* sc, double* out, cudaStream_t s, int rev) {
     if (sc && out)
-        k_residual_norm<T><<<red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s>>>(d, r, x, b, *sc, out);
+        k_residual_norm<T><<<red_grid3(d.nx, d.ny, d.nz, red_target<T>()), dim3(kRBX, kRBY), 0, s>>>(d, lap_k<T>(d), r, x, b, *sc, out);
     else if (d.nz % kZU == 0 && d.nx >= batch_min_nx() && ix2_ok(d))
-        k_residual_z2<T, kZU><<<dim3((d.nx + BX - 1) / BX, (d.ny + BY - 1) / BY, d.nz / kZU), dim3(BX, BY), 0, s>>>(d, r, x, b,
-                                                                                                          rev);
+        k_residual_z2<T, kZU><<<dim3((d.nx + BX - 1) / BX, (d.ny + BY - 1) / BY, d.nz / kZU), dim3(BX, BY), 0, s>>>(
+            d, lap_k<T>(d), r, x, b, rev);
     else if (d.nz % kZU == 0 && d.nx >= batch_min_nx())
-        k_residual_z<T, kZU><<<dim3((d.nx + BX - 1) / BX, (d.ny + BY - 1) / BY, d.nz / kZU), dim3(BX, BY), 0, s>>>(d, r, x, b);
+        k_residual_z<T, kZU><<<dim3((d.nx + BX - 1) / BX, (d.ny + BY - 1) / BY, d.nz / kZU), dim3(BX, BY), 0, s>>>(
+            d, lap_k<T>(d), r, x, b);
     else
-        k_residual<T><<<grid3(d), dim3(BX, BY), 0, s>>>(d, r, x, b);
+        k_residual<T><<<grid3(d), dim3(BX, BY), 0, s>>>(d, lap_k<T>(d), r, x, b);
 }
 // The pair kernel is opt-in (AFMIB_RBGS_PAIR=1, read at every launch): at
 // 256^3 its colour launches took 39.5 us against 29.9 for the scalar kernel
@@ -1586,7 +1614,7 @@ void launch_rbgs_from_zero(const Dims& d, T* x, const T* b, cudaStream_t s, doub
     if (!off && sizeof(T) == sizeof(float) && d.nz % kZU == 0 && d.nz % kZU32 == 0 && d.nx >= batch_min_nx() &&
         ix2_ok(d) && !rbgs_pair_ok(d)) {
         const dim3 g((d.nx / 2 + BX - 1) / BX, (d.ny + BY - 1) / BY, d.nz / kZU32);
-        k_rbgs_z2b_init<T, kZU32, 6><<<g, dim3(BX, BY), 0, s>>>(d, T(omega), x, b, rev, T(0));
+        k_rbgs_z2b_init<T, kZU32, 6><<<g, dim3(BX, BY), 0, s>>>(d, lap_k<T>(d), T(omega), x, b, rev, T(0));
         return;
     }
     cudaMemsetAsync(x, 0, (size_t)d.ncell() * sizeof(T), s);
@@ -1613,16 +1641,16 @@ void launch_rbgs(const Dims& d, int color, T* x, const T* b, cudaStream_t s, dou
             // 32.7 us; four cells with 8 blocks: the same as 6)
             if (sizeof(T) == sizeof(float) && d.nz % kZU32 == 0) {
                 const dim3 g4(g.x, g.y, d.nz / kZU32);
-                k_rbgs_z2b<T, kZU32, 6><<<g4, dim3(BX, BY), 0, s>>>(d, color, T(omega), x, b, rev);
+                k_rbgs_z2b<T, kZU32, 6><<<g4, dim3(BX, BY), 0, s>>>(d, lap_k<T>(d), color, T(omega), x, b, rev);
             }
             else
-                k_rbgs_z2<T, kZU><<<g, dim3(BX, BY), 0, s>>>(d, color, T(omega), x, b, rev);
+                k_rbgs_z2<T, kZU><<<g, dim3(BX, BY), 0, s>>>(d, lap_k<T>(d), color, T(omega), x, b, rev);
         }
-        else k_rbgs_z<T, kZU><<<g, dim3(BX, BY), 0, s>>>(d, color, T(omega), x, b);
+        else k_rbgs_z<T, kZU><<<g, dim3(BX, BY), 0, s>>>(d, lap_k<T>(d), color, T(omega), x, b);
         return;
     }
     dim3 g((d.nx / 2 + BX - 1) / BX, (d.ny + BY - 1) / BY, d.nz);
-    k_rbgs<T><<<g, dim3(BX, BY), 0, s>>>(d, color, T(omega), x, b);
+    k_rbgs<T><<<g, dim3(BX, BY), 0, s>>>(d, lap_k<T>(d), color, T(omega), x, b);
 }
 namespace {
 int log2_exact(int v) {
@@ -1869,7 +1897,8 @@ void launch_prolong_assign(const Dims& d, T* fine, const T* coarse, cudaStream_t
 template <typename TD>
 void launch_lap_defect(const Dims& d, TD* r, const double* x, const double* b, RedScratch sc, double* out, cudaStream_t s,
                        float* r_lo) {
-    k_lap_defect<TD><<<red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s>>>(d, r, x, b, sc, out, r_lo, lo_split());
+    k_lap_defect<TD><<<red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s>>>(d, lap_k<double>(d), r, x, b, sc, out, r_lo,
+                                                                              lo_split());
 }
 void launch_lap_defect_df(const Dims& d, float* rh, float* rl, const double* x, const double* b, const double* sum,
                           double scale, RedScratch sc, double* out, cudaStream_t s) {
