@@ -250,10 +250,17 @@ void launch_rbgs_pipe(const Dims& d, const PipeCfg& c, const T* xin, T* xout, co
 // Full-weighting restriction, src/mg/solver.h:153-181 (d = fine dims); zero
 // (optional): the coarse iterate, set to zero in the same pass.
 template <typename T>
-void launch_restrict(const Dims& d, T* coarse, const T* fine, cudaStream_t s, int rev = 0, T* zero = nullptr);
-// fine += P coarse (trilinear), src/mg/solver.h:71-151 and :211-212.
+void launch_restrict(const Dims& d, T* coarse, const T* fine, cudaStream_t s, int rev = 0, T* zero = nullptr,
+                     bool red = false);
+// r = b - L x on the red cells only; launch_restrict with red reads those and
+// takes the black ones as zero (restrict_after_sweep, mg_cells.cuh)
 template <typename T>
-void launch_prolong_add(const Dims& d, T* fine, const T* coarse, cudaStream_t s, int rev = 0);
+void launch_residual_red(const Dims& d, T* r, const T* x, const T* b, cudaStream_t s, int rev = 0);
+// fine += P coarse (trilinear), src/mg/solver.h:71-151 and :211-212. black: on
+// the black cells only, where the kernel can leave the others out
+// (prolong_before_sweep)
+template <typename T>
+void launch_prolong_add(const Dims& d, T* fine, const T* coarse, cudaStream_t s, int rev = 0, bool black = false);
 // coarse_b = restriction of (b - L x), coarse_x = 0, in one pass (the
 // residual stays in shared memory), for the levels resid_restrict_fused_ok
 // takes: by default FP32 3D power-of-two levels with nx >= 256 (the column
@@ -265,7 +272,7 @@ bool resid_restrict_fused_ok(const Dims& d, size_t elem, const void* x, const vo
 void mg_kernel_attributes();
 template <typename T>
 void launch_resid_restrict(const Dims& d, T* coarse_b, T* coarse_x, const T* x, const T* b, cudaStream_t s,
-                           int rev = 0);
+                           int rev = 0, bool red = false);
 // Prolongation that assigns (for the op-level API).
 template <typename T>
 void launch_prolong_assign(const Dims& d, T* fine, const T* coarse, cudaStream_t s);

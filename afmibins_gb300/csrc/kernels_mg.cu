@@ -352,9 +352,6 @@ __global__ void k_rbgs(Dims d, LapK<T> k, int color, T omega, T* __restrict__ xv
 // one-cell kernels.
 constexpr int kZU = 8;  // z cells per thread of the batched stencil kernels
 constexpr int kZU32 = 4;  // ... of the FP32 red-black colour
-// smallest level (x extent) on which a requested over-relaxation applies;
-// the coarser levels, the one-block tail among them, stay Gauss-Seidel
-constexpr int kOmegaMinNx = 64;
 
 template <typename T, int ZU>
 __global__ void k_rbgs_z(Dims d, LapK<T> k, int color, T omega, T* __restrict__ xv, const T* __restrict__ b) {
@@ -576,6 +573,32 @@ __global__ void k_residual_z(Dims d, LapK<T> k, T* __restrict__ r, const T* __re
     for (int u = 0; u < ZU; ++u) r[lin(d, x, y, z0 + u)] = val[u];
 }
 
+// The residual on the red cells alone (restrict_after_sweep): the same
+// expression; the black cells of r are not written. ZU cells along z per thread.
+template <typename T, int ZU, bool P2>
+__global__ void k_residual_red(Dims d, LapK<T> k, T* __restrict__ r, const T* __restrict__ xv, const T* __restrict__ b,
+                               int rev) {
+    const Ix2 I(d);
+    const uint3 B = block_at(rev);
+    const int t = B.x * BX + threadIdx.x, y = B.y * BY + threadIdx.y, z0 = B.z * ZU;
+    if (2 * t >= d.nx || y >= d.ny) return;
+    T val[ZU];
+    long long at[ZU];
+#pragma unroll
+    for (int u = 0; u < ZU; ++u) {
+        const int z = z0 + u, x = 2 * t + ((y + z) & 1);
+        T S;
+        int c;
+        if (P2) lap_row2(d, I, xv, x, y, z, S, c);
+        else lap_row(d, xv, x, y, z, S, c);
+        const long long i = P2 ? (long long)I.at(x, y, z) : lin(d, x, y, z);
+        val[u] = b[i] - k.off * (S - lap_count<T>(c) * xv[i]);
+        at[u] = i;
+    }
+#pragma unroll
+    for (int u = 0; u < ZU; ++u) r[at[u]] = val[u];
+}
+
 // ---------------------------------------------------------------------------
 // Pipelined red-black sweep: one full sweep (red, then black) per launch, out
 // of place (xin -> xout). A block owns FY full-width rows (every x of the row,
@@ -753,7 +776,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_rbgs_pipe(Dims d, const T* 
 // Full weighting, src/mg/solver.h:153-181: 64 taps (1,3,3,1)^3/512 around the
 // coarse cell (restrict_taps, mg_cells.cuh); y clamps at the channel walls,
 // wraps in periodic mode.
-template <typename T>
+template <typename T, bool RED>
 __device__ __forceinline__ void restrict_cell(const Dims& d, T* coarse, const T* fine, int xc, int yc, int zc) {
     const int cx = d.nx / 2, cy = d.ny / 2;
     const int xcf = 2 * xc + 1, ycf = 2 * yc + 1, zcf = 2 * zc + 1;
@@ -771,20 +794,30 @@ __device__ __forceinline__ void restrict_cell(const Dims& d, T* coarse, const T*
         }
     }
     if (d.nz == 1) {  // 2D (periodic): (1,3,3,1)^2 / 64 over 16 taps
+        auto row = [&](int ky) {
+            return red_row<T>(ys[ky] & 1, [&](int kx) { return fine[lin(d, xs[kx], ys[ky], 0)]; });
+        };
         coarse[xc + (long long)cx * yc] =
-            restrict_plane<T>([&](int ky, int kx) { return fine[lin(d, xs[kx], ys[ky], 0)]; }) * T(1.0 / 64.0);
+            (RED ? full4<T>(row(0), row(1), row(2), row(3))
+                 : restrict_plane<T>([&](int ky, int kx) { return fine[lin(d, xs[kx], ys[ky], 0)]; })) *
+            T(1.0 / 64.0);
         return;
     }
-    coarse[xc + (long long)cx * (yc + (long long)cy * zc)] =
-        restrict_taps<T>([&](int kz, int ky, int kx) { return fine[lin(d, xs[kx], ys[ky], zs[kz])]; });
+    const long long o = xc + (long long)cx * (yc + (long long)cy * zc);
+    if (RED)
+        coarse[o] = restrict_rows<T>([&](int kz, int ky) {
+            return red_row<T>((ys[ky] + zs[kz]) & 1, [&](int kx) { return fine[lin(d, xs[kx], ys[ky], zs[kz])]; });
+        });
+    else
+        coarse[o] = restrict_taps<T>([&](int kz, int ky, int kx) { return fine[lin(d, xs[kx], ys[ky], zs[kz])]; });
 }
 
 // zero (optional): the coarse iterate, set to zero at every coarse cell
-template <typename T>
+template <typename T, bool RED>
 __global__ void k_restrict(Dims d, T* __restrict__ coarse, const T* __restrict__ fine, T* __restrict__ zero) {
     const int xc = blockIdx.x * BX + threadIdx.x, yc = blockIdx.y * BY + threadIdx.y, zc = blockIdx.z;
     if (xc >= d.nx / 2 || yc >= d.ny / 2) return;
-    restrict_cell(d, coarse, fine, xc, yc, zc);
+    restrict_cell<T, RED>(d, coarse, fine, xc, yc, zc);
     if (zero) {
         const long long cx = d.nx / 2, cy = d.ny / 2;
         zero[d.nz == 1 ? xc + cx * yc : xc + cx * (yc + cy * zc)] = T(0);
@@ -801,7 +834,8 @@ __device__ __forceinline__ void prolong_put(T* fine, long long i, T val, T scale
     if (ADD) fine[i] = fma_t(val, scale, fine[i]);
     else fine[i] = val * scale;
 }
-template <typename T, typename C, typename P>
+// BLACK: on the black cells only (prolong_before_sweep)
+template <typename T, bool BLACK, typename C, typename P>
 __device__ __forceinline__ void prolong_cell_any(const Dims& d, int xc, int yc, int zc, int xn, int yn, int zn,
                                                  const int (&xf)[2], const int (&yf)[2], const int (&zf)[2], C cv,
                                                  P put) {
@@ -809,23 +843,23 @@ __device__ __forceinline__ void prolong_cell_any(const Dims& d, int xc, int yc, 
     if (!d.channel || yc < cy - 1) {
         const T blb = cv(xc, yc, zc), brb = cv(xn, yc, zc), ulb = cv(xc, yn, zc), urb = cv(xn, yn, zc);
         const T blf = cv(xc, yc, zn), brf = cv(xn, yc, zn), ulf = cv(xc, yn, zn), urf = cv(xn, yn, zn);
-        prolong_plane4(blb, brb, ulb, urb, blf, brf, ulf, urf,
+        prolong_plane4(blb, brb, ulb, urb, blf, brf, ulf, urf, BLACK, 0,
                        [&](int rx, int ry, T v, T s) { put(xf[rx], yf[ry], zf[0], v, s); });
-        prolong_plane4(blf, brf, ulf, urf, blb, brb, ulb, urb,
+        prolong_plane4(blf, brf, ulf, urf, blb, brb, ulb, urb, BLACK, 1,
                        [&](int rx, int ry, T v, T s) { put(xf[rx], yf[ry], zf[1], v, s); });
     }
     if (d.channel && (yc == 0 || yc == cy - 1)) {
         for (int side = 0; side < 2; ++side) {  // a thread with cy == 1 owns both wall rows
             if (side == 0 && yc != 0) continue;
             if (side == 1 && yc != cy - 1) continue;
-            const int yw = side == 0 ? 0 : d.ny - 1;
+            const int yw = side == 0 ? 0 : d.ny - 1, ry = 1 - side;  // row 0 is even, ny - 1 odd
             const T bl = cv(xc, yc, zc), br = cv(xn, yc, zc), fl = cv(xc, yc, zn), fr = cv(xn, yc, zn);
-            prolong_row2(bl, br, fl, fr, [&](int rx, T v, T s) { put(xf[rx], yw, zf[0], v, s); });
-            prolong_row2(fl, fr, bl, br, [&](int rx, T v, T s) { put(xf[rx], yw, zf[1], v, s); });
+            prolong_row2(bl, br, fl, fr, black_col(BLACK, ry, 0), [&](int rx, T v, T s) { put(xf[rx], yw, zf[0], v, s); });
+            prolong_row2(fl, fr, bl, br, black_col(BLACK, ry, 1), [&](int rx, T v, T s) { put(xf[rx], yw, zf[1], v, s); });
         }
     }
 }
-template <typename T, bool ADD>
+template <typename T, bool ADD, bool BLACK>
 __device__ __forceinline__ void prolong_cell(const Dims& d, T* fine, const T* coarse, int xc, int yc, int zc) {
     const int cx = d.nx / 2, cy = d.ny / 2, cz = d.nz / 2;
     const int xn = (xc + 1) % cx, yn = (yc + 1) % cy;
@@ -834,14 +868,14 @@ __device__ __forceinline__ void prolong_cell(const Dims& d, T* fine, const T* co
         // 2D (periodic): bilinear (9,3,3,1)/16 onto the four fine cells
         auto C2 = [&](int a, int b) { return coarse[a + (long long)cx * b]; };
         const T bl = C2(xc, yc), br = C2(xn, yc), ul = C2(xc, yn), ur = C2(xn, yn);
-        prolong_row2(bl, br, ul, ur,
+        prolong_row2(bl, br, ul, ur, black_col(BLACK, 0, 1),
                      [&](int rx, T v, T s) { prolong_put<T, ADD>(fine, lin(d, xf[rx], yf[0], 0), v, s); });
-        prolong_row2(ul, ur, bl, br,
+        prolong_row2(ul, ur, bl, br, black_col(BLACK, 1, 1),
                      [&](int rx, T v, T s) { prolong_put<T, ADD>(fine, lin(d, xf[rx], yf[1], 0), v, s); });
         return;
     }
     const int zf[2] = {2 * zc + 1, (2 * zc + 2) % d.nz};
-    prolong_cell_any<T>(
+    prolong_cell_any<T, BLACK>(
         d, xc, yc, zc, xn, yn, (zc + 1) % cz, xf, yf, zf,
         [&](int a, int b, int c) { return coarse[a + (long long)cx * (b + (long long)cy * c)]; },
         [&](int a, int b, int c, T v, T s) { prolong_put<T, ADD>(fine, lin(d, a, b, c), v, s); });
@@ -849,11 +883,13 @@ __device__ __forceinline__ void prolong_cell(const Dims& d, T* fine, const T* co
 
 // restrict_cell / prolong_cell for 3D power-of-two levels with Ix2 indexing
 // (the same arithmetic)
-template <typename T>
+template <typename T, bool RED>
 __device__ __forceinline__ void restrict_cell2(const Dims& d, const Ix2& I, T* coarse, const T* fine, int xc, int yc,
                                                int zc) {
     const int xcf = 2 * xc + 1, ycf = 2 * yc + 1, zcf = 2 * zc + 1;
     int xs[4], yo[4], zo[4];
+    // parity of row ky's y (clamped at channel walls) plus plane kz's z
+    auto odd = [&](int kz, int ky) { return (((yo[ky] >> I.lx) + (zo[kz] >> I.lxy)) & 1) != 0; };
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         const int dd = k - 2;
@@ -866,28 +902,33 @@ __device__ __forceinline__ void restrict_cell2(const Dims& d, const Ix2& I, T* c
             yo[k] = ((ycf + dd) & I.my) << I.lx;
         }
     }
-    coarse[xc | (yc << (I.lx - 1)) | (zc << (I.lxy - 2))] =
-        restrict_taps<T>([&](int kz, int ky, int kx) { return fine[xs[kx] | yo[ky] | zo[kz]]; });
+    const int o = xc | (yc << (I.lx - 1)) | (zc << (I.lxy - 2));
+    if (RED)
+        coarse[o] = restrict_rows<T>([&](int kz, int ky) {
+            return red_row<T>(odd(kz, ky), [&](int kx) { return fine[xs[kx] | yo[ky] | zo[kz]]; });
+        });
+    else
+        coarse[o] = restrict_taps<T>([&](int kz, int ky, int kx) { return fine[xs[kx] | yo[ky] | zo[kz]]; });
 }
 
-template <typename T>
+template <typename T, bool RED>
 __global__ void k_restrict2(Dims d, T* __restrict__ coarse, const T* __restrict__ fine, int rev,
                             T* __restrict__ zero) {
     const Ix2 I(d);
     const uint3 B = block_at(rev);
     const int xc = B.x * BX + threadIdx.x, yc = B.y * BY + threadIdx.y, zc = B.z;
     if (xc >= d.nx / 2 || yc >= d.ny / 2) return;
-    restrict_cell2(d, I, coarse, fine, xc, yc, zc);
+    restrict_cell2<T, RED>(d, I, coarse, fine, xc, yc, zc);
     if (zero) zero[xc | (yc << (I.lx - 1)) | (zc << (I.lxy - 2))] = T(0);
 }
 
-template <typename T, bool ADD>
+template <typename T, bool ADD, bool BLACK>
 __device__ __forceinline__ void prolong_cell2(const Dims& d, const Ix2& I, T* fine, const T* coarse, int xc, int yc,
                                               int zc) {
     const int cx = d.nx / 2, cy = d.ny / 2, cz = d.nz / 2, lcx = I.lx - 1, lcxy = I.lxy - 2;
     const int xf[2] = {2 * xc + 1, (2 * xc + 2) & I.mx}, yf[2] = {2 * yc + 1, (2 * yc + 2) & I.my},
               zf[2] = {2 * zc + 1, (2 * zc + 2) & I.mz};
-    prolong_cell_any<T>(
+    prolong_cell_any<T, BLACK>(
         d, xc, yc, zc, (xc + 1) & (cx - 1), (yc + 1) & (cy - 1), (zc + 1) & (cz - 1), xf, yf, zf,
         [&](int a, int b, int c) { return coarse[a | (b << lcx) | (c << lcxy)]; },
         [&](int a, int b, int c, T v, T s) { prolong_put<T, ADD>(fine, I.at(a, b, c), v, s); });
@@ -913,7 +954,7 @@ __device__ __forceinline__ int rr_at(int jy, int jx) { return jy * RR_RS + (jx &
 template <typename T, int RR_CZ>
 __global__ void __launch_bounds__(RR_THREADS) k_resid_restrict2(Dims d, T* __restrict__ cb, T* __restrict__ cx,
                                                                const T* __restrict__ xv, const T* __restrict__ b,
-                                                               int rev) {
+                                                               int rev, bool red) {
     __shared__ T ring[4][RR_F * RR_RS];
     const Ix2 I(d);
     const uint3 B = block_at(rev);
@@ -935,6 +976,10 @@ __global__ void __launch_bounds__(RR_THREADS) k_resid_restrict2(Dims d, T* __res
                 y &= I.my;
             }
             const int x = (xf0 + jx) & I.mx;
+            if (red && ((x + y + z) & 1)) {  // restrict_after_sweep
+                dst[rr_at(jy, jx)] = T(0);
+                continue;
+            }
             T S;
             int c;
             lap_row2(d, I, xv, x, y, z, S, c);
@@ -974,20 +1019,20 @@ __global__ void __launch_bounds__(RR_THREADS) k_resid_restrict2(Dims d, T* __res
     }
 }
 
-template <typename T, bool ADD>
+template <typename T, bool ADD, bool BLACK>
 __global__ void k_prolong2(Dims d, T* __restrict__ fine, const T* __restrict__ coarse, int rev) {
     const Ix2 I(d);
     const uint3 B = block_at(rev);
     const int xc = B.x * BX + threadIdx.x, yc = B.y * BY + threadIdx.y, zc = B.z;
     if (xc >= d.nx / 2 || yc >= d.ny / 2) return;
-    prolong_cell2<T, ADD>(d, I, fine, coarse, xc, yc, zc);
+    prolong_cell2<T, ADD, BLACK>(d, I, fine, coarse, xc, yc, zc);
 }
 
-template <typename T, bool ADD>
+template <typename T, bool ADD, bool BLACK>
 __global__ void k_prolong(Dims d, T* __restrict__ fine, const T* __restrict__ coarse) {
     const int xc = blockIdx.x * BX + threadIdx.x, yc = blockIdx.y * BY + threadIdx.y, zc = blockIdx.z;
     if (xc >= d.nx / 2 || yc >= d.ny / 2) return;
-    prolong_cell<T, ADD>(d, fine, coarse, xc, yc, zc);
+    prolong_cell<T, ADD, BLACK>(d, fine, coarse, xc, yc, zc);
 }
 
 // Column-marching transfers for 3D power-of-two levels whose coarse x extent
@@ -1589,6 +1634,17 @@ void launch_residual(const Dims& d, T* r, const T* x, const T* b, RedScratch* sc
     else
         k_residual<T><<<grid3(d), dim3(BX, BY), 0, s>>>(d, lap_k<T>(d), r, x, b);
 }
+template <typename T>
+void launch_residual_red(const Dims& d, T* r, const T* x, const T* b, cudaStream_t s, int rev) {
+    constexpr int ZU = 4;
+    const int gx = (d.nx / 2 + BX - 1) / BX, gy = (d.ny + BY - 1) / BY;
+    const LapK<T> k = lap_k<T>(d);
+    const bool batch = d.nz % ZU == 0 && d.nx >= batch_min_nx(), p2 = ix2_ok(d);
+    if (batch && p2) k_residual_red<T, ZU, true><<<dim3(gx, gy, d.nz / ZU), dim3(BX, BY), 0, s>>>(d, k, r, x, b, rev);
+    else if (batch) k_residual_red<T, ZU, false><<<dim3(gx, gy, d.nz / ZU), dim3(BX, BY), 0, s>>>(d, k, r, x, b, rev);
+    else if (p2) k_residual_red<T, 1, true><<<dim3(gx, gy, d.nz), dim3(BX, BY), 0, s>>>(d, k, r, x, b, rev);
+    else k_residual_red<T, 1, false><<<dim3(gx, gy, d.nz), dim3(BX, BY), 0, s>>>(d, k, r, x, b, rev);
+}
 // The pair kernel is opt-in (AFMIB_RBGS_PAIR=1, read at every launch): at
 // 256^3 its colour launches took 39.5 us against 29.9 for the scalar kernel
 // (53.7 against 56.5 IB steps/s): 60 registers hold it to 4 resident blocks
@@ -1763,9 +1819,9 @@ inline dim3 transfer_grid(const Dims& d, int planes, int bx = 32) {
 }
 
 template <typename T>
-void launch_restrict(const Dims& d, T* coarse, const T* fine, cudaStream_t s, int rev, T* zero) {
+void launch_restrict(const Dims& d, T* coarse, const T* fine, cudaStream_t s, int rev, T* zero, bool red) {
     if constexpr (sizeof(T) == sizeof(float)) {
-        if (transfer_cols_ok(d, fine, coarse) && (d.nx / 2) % TrTile<T>::CX == 0 &&
+        if (!red && transfer_cols_ok(d, fine, coarse) && (d.nx / 2) % TrTile<T>::CX == 0 &&
             (reinterpret_cast<uintptr_t>(zero) & 15) == 0) {
             const int z = transfer_planes(d, TrTile<T>::CX);
             const dim3 g = transfer_grid(d, z, TrTile<T>::CX), b(32, kTrBY);
@@ -1778,8 +1834,11 @@ void launch_restrict(const Dims& d, T* coarse, const T* fine, cudaStream_t s, in
     }
     dim3 g((d.nx / 2 + BX - 1) / BX, (d.ny / 2 + BY - 1) / BY, d.nz == 1 ? 1 : d.nz / 2);
     if (d.nz > 1 && d.nx >= 2 && d.ny >= 2 && ix2_ok(d))
-        k_restrict2<T><<<g, dim3(BX, BY), 0, s>>>(d, coarse, fine, rev, zero);
-    else k_restrict<T><<<g, dim3(BX, BY), 0, s>>>(d, coarse, fine, zero);
+        red ? k_restrict2<T, true><<<g, dim3(BX, BY), 0, s>>>(d, coarse, fine, rev, zero)
+            : k_restrict2<T, false><<<g, dim3(BX, BY), 0, s>>>(d, coarse, fine, rev, zero);
+    else
+        red ? k_restrict<T, true><<<g, dim3(BX, BY), 0, s>>>(d, coarse, fine, zero)
+            : k_restrict<T, false><<<g, dim3(BX, BY), 0, s>>>(d, coarse, fine, zero);
 }
 // Fine-level residual and restriction in one pass. AFMIB_RESID_RESTRICT
 // (read at every call, so that a test can compare the paths in one process):
@@ -1824,7 +1883,8 @@ void mg_kernel_attributes() {
 }
 
 template <typename T>
-void launch_resid_restrict(const Dims& d, T* coarse_b, T* coarse_x, const T* x, const T* b, cudaStream_t s, int rev) {
+void launch_resid_restrict(const Dims& d, T* coarse_b, T* coarse_x, const T* x, const T* b, cudaStream_t s, int rev,
+                           bool red) {
     if constexpr (sizeof(T) == sizeof(float)) {
         if (rr_mode(d, sizeof(T), x, b, coarse_b, coarse_x) == 2) {
             // coarse planes per block: the largest of 8, 4, 2 that leaves at least
@@ -1862,14 +1922,14 @@ void launch_resid_restrict(const Dims& d, T* coarse_b, T* coarse_x, const T* x, 
     const int cols = (d.nx / 2 / RR_T) * (d.ny / 2 / RR_T), cz = d.nz / 2;
     if (cz % 8 == 0 && cols * (cz / 8) >= 2 * 152)
         k_resid_restrict2<T, 8><<<dim3(d.nx / 2 / RR_T, d.ny / 2 / RR_T, cz / 8), RR_THREADS, 0, s>>>(
-            d, coarse_b, coarse_x, x, b, rev);
+            d, coarse_b, coarse_x, x, b, rev, red);
     else
         k_resid_restrict2<T, 2><<<dim3(d.nx / 2 / RR_T, d.ny / 2 / RR_T, cz / 2), RR_THREADS, 0, s>>>(
-            d, coarse_b, coarse_x, x, b, rev);
+            d, coarse_b, coarse_x, x, b, rev, red);
 }
 
 template <typename T>
-void launch_prolong_add(const Dims& d, T* fine, const T* coarse, cudaStream_t s, int rev) {
+void launch_prolong_add(const Dims& d, T* fine, const T* coarse, cudaStream_t s, int rev, bool black) {
     if constexpr (sizeof(T) == sizeof(float)) {
         if (transfer_cols_ok(d, fine, coarse)) {
             // AFMIB_PROLONG_MAX_PLANES caps the planes per block (a sweep knob)
@@ -1886,13 +1946,16 @@ void launch_prolong_add(const Dims& d, T* fine, const T* coarse, cudaStream_t s,
     }
     dim3 g((d.nx / 2 + BX - 1) / BX, (d.ny / 2 + BY - 1) / BY, d.nz == 1 ? 1 : d.nz / 2);
     if (d.nz > 1 && d.nx >= 2 && d.ny >= 2 && ix2_ok(d))
-        k_prolong2<T, true><<<g, dim3(BX, BY), 0, s>>>(d, fine, coarse, rev);
-    else k_prolong<T, true><<<g, dim3(BX, BY), 0, s>>>(d, fine, coarse);
+        black ? k_prolong2<T, true, true><<<g, dim3(BX, BY), 0, s>>>(d, fine, coarse, rev)
+              : k_prolong2<T, true, false><<<g, dim3(BX, BY), 0, s>>>(d, fine, coarse, rev);
+    else
+        black ? k_prolong<T, true, true><<<g, dim3(BX, BY), 0, s>>>(d, fine, coarse)
+              : k_prolong<T, true, false><<<g, dim3(BX, BY), 0, s>>>(d, fine, coarse);
 }
 template <typename T>
 void launch_prolong_assign(const Dims& d, T* fine, const T* coarse, cudaStream_t s) {
     dim3 g((d.nx / 2 + BX - 1) / BX, (d.ny / 2 + BY - 1) / BY, d.nz == 1 ? 1 : d.nz / 2);
-    k_prolong<T, false><<<g, dim3(BX, BY), 0, s>>>(d, fine, coarse);
+    k_prolong<T, false, false><<<g, dim3(BX, BY), 0, s>>>(d, fine, coarse);
 }
 template <typename TD>
 void launch_lap_defect(const Dims& d, TD* r, const double* x, const double* b, RedScratch sc, double* out, cudaStream_t s,
@@ -1936,13 +1999,14 @@ void launch_coarse_solve(const Dims& d, T* x, T* b, T* r, T* p, T* q, double tol
 #define AFMIB_MG_INST(T)                                                                                 \
     template void launch_lap_apply<T>(const Dims&, T*, const T*, cudaStream_t);                          \
     template void launch_residual<T>(const Dims&, T*, const T*, const T*, RedScratch*, double*, cudaStream_t, int); \
+    template void launch_residual_red<T>(const Dims&, T*, const T*, const T*, cudaStream_t, int);                  \
     template void launch_rbgs<T>(const Dims&, int, T*, const T*, cudaStream_t, double, int);                        \
     template void launch_rbgs_from_zero<T>(const Dims&, T*, const T*, cudaStream_t, double, int);                  \
     template PipeCfg rbgs_pipe_cfg<T>(const Dims&);                                                      \
     template void launch_rbgs_pipe<T>(const Dims&, const PipeCfg&, const T*, T*, const T*, int*, cudaStream_t); \
-    template void launch_restrict<T>(const Dims&, T*, const T*, cudaStream_t, int, T*);                     \
-    template void launch_prolong_add<T>(const Dims&, T*, const T*, cudaStream_t, int);                      \
-    template void launch_resid_restrict<T>(const Dims&, T*, T*, const T*, const T*, cudaStream_t, int);      \
+    template void launch_restrict<T>(const Dims&, T*, const T*, cudaStream_t, int, T*, bool);               \
+    template void launch_prolong_add<T>(const Dims&, T*, const T*, cudaStream_t, int, bool);                \
+    template void launch_resid_restrict<T>(const Dims&, T*, T*, const T*, const T*, cudaStream_t, int, bool); \
     template void launch_prolong_assign<T>(const Dims&, T*, const T*, cudaStream_t);                     \
     template void launch_coarse_solve<T>(const Dims&, T*, T*, T*, T*, T*, double, int, int*, cudaStream_t);
 

@@ -42,7 +42,6 @@ namespace {
 constexpr int kTailThreads = 512;
 constexpr size_t kTailSmem = 200 * 1024;
 constexpr int kLaneCells = 64;   // coarse cells per CTA up to which the restriction takes a half warp per cell
-constexpr int kOmegaMinNx = 64;  // kernels_mg.cu: over-relaxation on levels at least this wide
 
 // One level of the tail. On a 2D grid the slabs are rows: ny = 1 and nz is the
 // grid's y extent (flat).
@@ -52,7 +51,7 @@ struct TailLv {
     int P, nc;                        // planes per CTA (1, even, or all), CTAs that own any
     unsigned mP, mhx, mny, mcy;       // division by P, nx/2, ny and ny/2 (fdiv)
     int ox, ob, orr;                  // offsets of x, b, r in every CTA's shared memory, in T
-    int nu1, nu2;
+    int nu1, nu2, red, black;         // restrict_after_sweep, prolong_before_sweep
     T omega, inv, off;                // off = n^2 and inv = 1 / n^2, as the level kernels round them
 };
 template <typename T>
@@ -243,7 +242,13 @@ __device__ __noinline__ void smooth(const TailLv<T>& L, unsigned x0, int z0, int
         }
         if (res) {
             resid(red, nr);
-            resid(black, nb);
+            if (L.red) {
+#pragma unroll
+                for (int k = 0; k < kCells; ++k)
+                    if (k < nb) sts(black[k].c + dr, T(0));
+            } else {
+                resid(black, nb);
+            }
             barrier();
         }
         return;
@@ -255,7 +260,16 @@ __device__ __noinline__ void smooth(const TailLv<T>& L, unsigned x0, int z0, int
     }
     if (res) {
         for (int color = 0; color < 2; ++color)
-            for (int e = tid; e < total; e += kCells * bd) resid(q, decode(q, color, e));
+            for (int e = tid; e < total; e += kCells * bd) {
+                const int n = decode(q, color, e);
+                if (color == 0 || !L.red) {
+                    resid(q, n);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < kCells; ++k)
+                        if (k < n) sts(q[k].c + dr, T(0));
+                }
+            }
         barrier();
     }
 }
@@ -310,7 +324,7 @@ __device__ __noinline__ void restrict_share(const TailLv<T>& L, const TailLv<T>&
             if (e < total) {
                 where(e, xc, yc, zc, p);
                 const T* q = plane(zc, kz) + rowof(yc, ky);
-                rs = full4<T>(q[col(xc, 0)], q[col(xc, 1)], q[col(xc, 2)], q[col(xc, 3)]);
+                rs = full4<T>(q[col(xc, 0)], q[col(xc, 1)], q[col(xc, 2)], q[col(xc, 3)]);  // black taps are zeros
             }
             T s[4];
 #pragma unroll
@@ -327,14 +341,22 @@ __device__ __noinline__ void restrict_share(const TailLv<T>& L, const TailLv<T>&
         where(e, xc, yc, zc, p);
         const T* rp[4];
         int xs[4], ys[4];
+        unsigned odd = 0;  // parity of row ky (clamped at channel walls)
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             rp[k] = plane(zc, k);
             xs[k] = col(xc, k);
             ys[k] = rowof(yc, k);
+            odd |= (unsigned)((fdiv(ys[k], L.mhx) >> 1) & 1) << k;  // ys = nx y
         }
         T acc;
-        if (FLAT) acc = restrict_plane<T>([&](int ky, int kx) { return rp[ky][xs[kx]]; }) * T(1.0 / 64.0);
+        if (!FLAT && L.red)
+            acc = restrict_rows<T>([&](int kz, int ky) {
+                // plane 2 zc - 1 + kz: the parity of kz + 1
+                return red_row<T>((((odd >> ky) + kz + 1) & 1) != 0,
+                                  [&](int kx) { return rp[kz][xs[kx] + ys[ky]]; });
+            });
+        else if (FLAT) acc = restrict_plane<T>([&](int ky, int kx) { return rp[ky][xs[kx]]; }) * T(1.0 / 64.0);
         else acc = restrict_taps<T>([&](int kz, int ky, int kx) { return rp[kz][xs[kx] + ys[ky]]; });
         store(zc, p, acc);
     }
@@ -361,8 +383,10 @@ __device__ __noinline__ void prolong_share(const TailLv<T>& L, const TailLv<T>& 
             const int i = x + nx * y;
             Xp[i] = fma_t(v, s, Xp[i]);
         };
+        const bool black = L.black;
+        const int rz = (z & 1) ? 0 : 1;  // on a 2D grid z is y
         if (FLAT) {
-            prolong_row2(near[xc], near[xn], far[xc], far[xn], [&](int rx, T v, T s) { put(xf[rx], 0, v, s); });
+            prolong_row2(near[xc], near[xn], far[xc], far[xn], black_col(black, rz, 1), [&](int rx, T v, T s) { put(xf[rx], 0, v, s); });
             continue;
         }
         const int a = hx * yc;
@@ -370,13 +394,13 @@ __device__ __noinline__ void prolong_share(const TailLv<T>& L, const TailLv<T>& 
             const int b = yc + 1 == cy ? 0 : a + hx;
             const int yf[2] = {2 * yc + 1, 2 * yc + 2 == ny ? 0 : 2 * yc + 2};
             prolong_plane4(near[xc + a], near[xn + a], near[xc + b], near[xn + b], far[xc + a], far[xn + a],
-                           far[xc + b], far[xn + b], [&](int rx, int ry, T v, T s) { put(xf[rx], yf[ry], v, s); });
+                           far[xc + b], far[xn + b], black, rz, [&](int rx, int ry, T v, T s) { put(xf[rx], yf[ry], v, s); });
         }
         if (CH && yc == 0)
-            prolong_row2(near[xc + a], near[xn + a], far[xc + a], far[xn + a],
+            prolong_row2(near[xc + a], near[xn + a], far[xc + a], far[xn + a], black_col(black, 1, rz),
                          [&](int rx, T v, T s) { put(xf[rx], 0, v, s); });
         if (CH && yc == cy - 1)
-            prolong_row2(near[xc + a], near[xn + a], far[xc + a], far[xn + a],
+            prolong_row2(near[xc + a], near[xn + a], far[xc + a], far[xn + a], black_col(black, 0, rz),
                          [&](int rx, T v, T s) { put(xf[rx], ny - 1, v, s); });
     }
 }
@@ -624,6 +648,8 @@ size_t tail_layout(const TailLevels<T>& a, int cs, TailArgs<T>* g) {
         off = (off + 3) & ~(size_t)3;
         L.nu1 = a.nu1[l];
         L.nu2 = a.nu2[l];
+        L.red = restrict_after_sweep(d, sizeof(T), L.nu1);
+        L.black = prolong_before_sweep(d, sizeof(T), L.nu2);
         L.omega = d.nx < kOmegaMinNx ? T(1) : T(a.omega);
         if (l + 1 < a.nlev && (d.nx & 1)) return 0;
     }

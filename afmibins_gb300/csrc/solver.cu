@@ -18,6 +18,7 @@
 #include "kernels.h"
 #include "kernels_ib.h"
 #include "kernels_adjoint.h"
+#include "mg_cells.cuh"
 #include "snapshot_io.h"
 
 using namespace afmib;
@@ -598,30 +599,35 @@ int vcycle(afmib_solver* s, size_t l, bool x_zero = false) {
         return AFMIB_OK;
     }
     const bool fine = l == 0;
-    TRY(smooth(s, L, sizeof(T) == sizeof(float) ? (fine ? s->inner_nu1 : s->inner_nu1c) : s->cfg.nu1, x_zero));
+    const int nu1 = sizeof(T) == sizeof(float) ? (fine ? s->inner_nu1 : s->inner_nu1c) : s->cfg.nu1;
+    const int nu2 = sizeof(T) == sizeof(float) ? (fine ? s->inner_nu2 : s->inner_nu2c) : s->cfg.nu2;
+    const bool red = restrict_after_sweep(L.d, sizeof(T), nu1);
+    TRY(smooth(s, L, nu1, x_zero));
     MGLevelT<T>& C = lv[l + 1];
     if (resid_restrict_fused_ok(L.d, sizeof(T), L.x, L.b, C.b, C.x)) {
         // x, b read; coarse b and x written (the fine residual stays on chip)
         ProfScope ps(s, fine ? P_RESID_RESTRICT0 : P_RESID_RESTRICT, 2 * Ns + 2 * Ns / 8);
-        launch_resid_restrict<T>(L.d, C.b, C.x, L.x, L.b, s->st, pass_dir(s, L.d, sizeof(T)));
+        launch_resid_restrict<T>(L.d, C.b, C.x, L.x, L.b, s->st, pass_dir(s, L.d, sizeof(T)), red);
     } else {
         {
             ProfScope ps(s, fine ? P_RESID0 : P_RESID, 3 * Ns);
-            launch_residual<T>(L.d, L.r, L.x, L.b, nullptr, nullptr, s->st, pass_dir(s, L.d, sizeof(T)));
+            if (red) launch_residual_red<T>(L.d, L.r, L.x, L.b, s->st, pass_dir(s, L.d, sizeof(T)));
+            else launch_residual<T>(L.d, L.r, L.x, L.b, nullptr, nullptr, s->st, pass_dir(s, L.d, sizeof(T)));
         }
         {
             // the coarse iterate starts from zero: set in the same pass
             ProfScope ps(s, fine ? P_RESTRICT0 : P_RESTRICT, Ns + Ns / 8 + Ns / 8);
-            launch_restrict<T>(L.d, C.b, L.r, s->st, pass_dir(s, L.d, sizeof(T)), C.x);
+            launch_restrict<T>(L.d, C.b, L.r, s->st, pass_dir(s, L.d, sizeof(T)), C.x, red);
         }
     }
     CKL();
     TRY(vcycle<T>(s, l + 1));
     {
         ProfScope ps(s, fine ? P_PROLONG0 : P_PROLONG, 2 * Ns + Ns / 8);
-        launch_prolong_add<T>(L.d, L.x, C.x, s->st, pass_dir(s, L.d, sizeof(T)));
+        launch_prolong_add<T>(L.d, L.x, C.x, s->st, pass_dir(s, L.d, sizeof(T)),
+                              prolong_before_sweep(L.d, sizeof(T), nu2));
     }
-    TRY(smooth(s, L, sizeof(T) == sizeof(float) ? (fine ? s->inner_nu2 : s->inner_nu2c) : s->cfg.nu2));
+    TRY(smooth(s, L, nu2));
     return AFMIB_OK;
 }
 
