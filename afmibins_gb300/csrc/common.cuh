@@ -96,7 +96,7 @@ constexpr int kMaxRedBlocks = 8192;
 
 struct RedScratch {
     double* partial;     // [kMaxRedBlocks * kMaxRedVals]
-    unsigned* ticket;    // [1]
+    unsigned* ticket;    // [1], or one per reduction of a launch that makes several (at most kMaxRedVals)
 };
 constexpr int kMaxRedVals = 4;
 
@@ -140,14 +140,15 @@ __device__ __forceinline__ void block_sum(double (&v)[NV]) {
 // thread of every block exactly once. Returns true in exactly one thread (the
 // finisher: thread 0 of the last block), where v then holds the totals, so
 // that a caller can derive further scalars (CG coefficients) in place.
+// (bid of nb: the block among those that reduce together.)
 template <int NV>
-__device__ __forceinline__ bool grid_sum(double (&v)[NV], RedScratch sc, double* out) {
+__device__ __forceinline__ bool grid_sum(double (&v)[NV], RedScratch sc, double* out, int bid, int nb) {
     __shared__ bool last;
     block_sum<NV>(v);
-    const int tid = tid_lin(), nb = nblk_lin();
+    const int tid = tid_lin();
     if (tid == 0) {
 #pragma unroll
-        for (int k = 0; k < NV; ++k) sc.partial[(size_t)k * kMaxRedBlocks + bid_lin()] = v[k];
+        for (int k = 0; k < NV; ++k) sc.partial[(size_t)k * kMaxRedBlocks + bid] = v[k];
         __threadfence();
         unsigned t = atomicAdd(sc.ticket, 1u);
         last = (t == (unsigned)nb - 1);
@@ -173,6 +174,11 @@ __device__ __forceinline__ bool grid_sum(double (&v)[NV], RedScratch sc, double*
         }
     }
     return false;
+}
+
+template <int NV>
+__device__ __forceinline__ bool grid_sum(double (&v)[NV], RedScratch sc, double* out) {
+    return grid_sum<NV>(v, sc, out, bid_lin(), nblk_lin());
 }
 
 // Stencil reductions run on (32 x 8)-thread blocks over (x, y) tiles with

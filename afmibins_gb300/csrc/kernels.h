@@ -125,6 +125,23 @@ void launch_cg_apply(const Dims& d, int comp, double scale, const T* p, T* q, Re
 // update:    x += alpha p, r -= alpha q, n1 = r.r, beta = n1 / n0, n0 = n1
 template <typename T>
 void launch_cg_update(long long n, T* x, T* r, const T* p, const T* q, RedScratch sc, double* cgs, cudaStream_t s);
+// FP64 CG on up to three independent viscous systems at once (one component
+// each, same scale): a launch serves every system, so small grids fill the GPU
+// and pay a third of the launches. System c's scalars are cgs[8 c + {0: n0 = r.r,
+// 1: p.q, 2: n1, 3: beta, 4: alpha, 5: done, 6: iterations}]. A system is done
+// once !(sqrt(n0) > tol) (NaN included); its blocks then return at once, so that
+// the host may launch the next iteration before it has read this one's norm.
+struct CgBatch {
+    int n;
+    int comp[3];
+    double *x[3], *r[3], *p[3], *q[3];
+    const double* b[3];
+};
+constexpr int kCgScalars = 8;
+void launch_cgb_init(const Dims& d, double scale, const CgBatch& g, double tol, RedScratch sc, double* cgs, cudaStream_t s);
+void launch_cgb_apply(const Dims& d, double scale, const CgBatch& g, RedScratch sc, double* cgs, cudaStream_t s);
+void launch_cgb_update(const Dims& d, const CgBatch& g, double tol, RedScratch sc, double* cgs, cudaStream_t s);
+void launch_cgb_direction(const Dims& d, const CgBatch& g, const double* cgs, cudaStream_t s);
 // one Jacobi sweep x' = x + (b - H x) / diag(H) (x == nullptr: from zero)
 template <typename T>
 void launch_helm_jacobi(const Dims& d, int comp, double scale, const T* x, T* xo, const T* b, cudaStream_t s,

@@ -791,6 +791,125 @@ __global__ void k_cg_direction(long long N, T* __restrict__ p, const T* __restri
 }
 
 // ---------------------------------------------------------------------------
+// Batched FP64 CG (CgBatch, kernels.h). The arithmetic per system is that of
+// the kernels above. Grids: gz blocks along z per system; the vector kernels
+// take a system per blockIdx.y and two cells per 16-byte access.
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(kRedBlock) k_cgb_init(Dims d, CgBatch g, HelmK<double> k, int gz, double tol,
+                                                       RedScratch sc, double* cgs) {
+    const int c = blockIdx.z / gz, zb = blockIdx.z - c * gz;
+    const int xi = blockIdx.x * kRBX + threadIdx.x, yi = blockIdx.y * kRBY + threadIdx.y;
+    const double *x = g.x[c], *b = g.b[c];
+    double *r = g.r[c], *p = g.p[c];
+    double acc = 0.0;
+    if (xi < d.nx && yi < d.ny)
+#pragma unroll 2
+        for (int zi = zb; zi < d.nz; zi += gz) {
+            const long long i = lin(d, xi, yi, zi);
+            const double ri = b[i] - helm_point(d, g.comp[c], k, x, xi, yi, zi);
+            r[i] = ri;
+            p[i] = ri;
+            acc += ri * ri;
+        }
+    double a[1] = {acc};
+    double* s = cgs + kCgScalars * c;
+    sc.partial += (size_t)c * kMaxRedBlocks;
+    sc.ticket += c;
+    if (grid_sum<1>(a, sc, s, blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * zb), gridDim.x * gridDim.y * gz)) {
+        s[5] = sqrt(a[0]) > tol ? 0.0 : 1.0;
+        s[6] = 0.0;
+    }
+}
+
+__global__ void __launch_bounds__(kRedBlock) k_cgb_apply(Dims d, CgBatch g, HelmK<double> k, int gz, RedScratch sc,
+                                                        double* cgs) {
+    const int c = blockIdx.z / gz, zb = blockIdx.z - c * gz;
+    double* s = cgs + kCgScalars * c;
+    if (s[5] != 0.0) return;
+    const int xi = blockIdx.x * kRBX + threadIdx.x, yi = blockIdx.y * kRBY + threadIdx.y;
+    const double* __restrict__ p = g.p[c];
+    double* __restrict__ q = g.q[c];
+    double acc = 0.0;
+    if (xi < d.nx && yi < d.ny)
+#pragma unroll 2
+        for (int zi = zb; zi < d.nz; zi += gz) {
+            const long long i = lin(d, xi, yi, zi);
+            const double qi = helm_point(d, g.comp[c], k, p, xi, yi, zi);
+            q[i] = qi;
+            acc += p[i] * qi;
+        }
+    double a[1] = {acc};
+    sc.partial += (size_t)c * kMaxRedBlocks;
+    sc.ticket += c;
+    if (grid_sum<1>(a, sc, s + 1, blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * zb), gridDim.x * gridDim.y * gz))
+        s[4] = s[0] / a[0];  // alpha = n0 / (p.Ap)
+}
+
+template <bool VEC>
+__global__ void __launch_bounds__(kRedBlock) k_cgb_update(long long N, CgBatch g, double tol, RedScratch sc, double* cgs) {
+    const int c = blockIdx.y;
+    double* s = cgs + kCgScalars * c;
+    if (s[5] != 0.0) return;  // set below only once every block of the system has passed here
+    const double alpha = s[4];
+    double *x = g.x[c], *r = g.r[c];
+    const double *p = g.p[c], *q = g.q[c];
+    double part = 0.0;
+    const long long st = (long long)gridDim.x * blockDim.x, i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (VEC) {
+        for (long long j = i0; j < N / 2; j += st) {
+            const double2 pv = reinterpret_cast<const double2*>(p)[j], qv = reinterpret_cast<const double2*>(q)[j];
+            double2 xv = reinterpret_cast<double2*>(x)[j], rv = reinterpret_cast<double2*>(r)[j];
+            xv.x = xv.x + alpha * pv.x;
+            xv.y = xv.y + alpha * pv.y;
+            rv.x = rv.x - qv.x * alpha;
+            rv.y = rv.y - qv.y * alpha;
+            reinterpret_cast<double2*>(x)[j] = xv;
+            reinterpret_cast<double2*>(r)[j] = rv;
+            part += rv.x * rv.x;
+            part += rv.y * rv.y;
+        }
+    } else {
+        for (long long i = i0; i < N; i += st) {
+            x[i] = x[i] + alpha * p[i];
+            const double ri = r[i] - q[i] * alpha;
+            r[i] = ri;
+            part += ri * ri;
+        }
+    }
+    double acc[1] = {part};
+    sc.partial += (size_t)c * kMaxRedBlocks;
+    sc.ticket += c;
+    if (grid_sum<1>(acc, sc, s + 2, blockIdx.x, gridDim.x)) {
+        s[3] = acc[0] / s[0];  // beta = n1 / n0
+        s[0] = acc[0];
+        s[5] = sqrt(acc[0]) > tol ? 0.0 : 1.0;
+        s[6] += 1.0;
+    }
+}
+
+template <bool VEC>
+__global__ void __launch_bounds__(kRedBlock) k_cgb_direction(long long N, CgBatch g, const double* cgs) {
+    const int c = blockIdx.y;
+    const double* s = cgs + kCgScalars * c;
+    if (s[5] != 0.0) return;
+    const double beta = s[3];
+    double* p = g.p[c];
+    const double* r = g.r[c];
+    const long long st = (long long)gridDim.x * blockDim.x, i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (VEC) {
+        for (long long j = i0; j < N / 2; j += st) {
+            double2 pv = reinterpret_cast<double2*>(p)[j];
+            const double2 rv = reinterpret_cast<const double2*>(r)[j];
+            pv.x = pv.x * beta + rv.x;
+            pv.y = pv.y * beta + rv.y;
+            reinterpret_cast<double2*>(p)[j] = pv;
+        }
+    } else {
+        for (long long i = i0; i < N; i += st) p[i] = p[i] * beta + r[i];
+    }
+}
+
+// ---------------------------------------------------------------------------
 // Defect-correction pieces of the mixed form: the residual of the FP64 state
 // evaluated in FP64 and handed to the FP32 inner solve as an FP32 defect, and
 // the FP64 update x += e with the FP32 correction.
@@ -1340,6 +1459,43 @@ void launch_cg_init(const Dims& d, int comp, double scale, const T* x, const T* 
 template <typename T>
 void launch_cg_apply(const Dims& d, int comp, double scale, const T* p, T* q, RedScratch sc, double* cgs, cudaStream_t s) {
     k_cg_apply<T><<<red_grid3(d.nx, d.ny, d.nz, red_target<T>()), dim3(kRBX, kRBY), 0, s>>>(d, comp, helm_k<T>(d, scale), p, q, sc, cgs);
+}
+// the grid of one system, times the systems along z
+static dim3 cgb_grid(const Dims& d, int n, int* gz) {
+    const dim3 g = red_grid3(d.nx, d.ny, d.nz, std::max(1, kRedBlocks64 / n));
+    *gz = (int)g.z;
+    return dim3(g.x, g.y, g.z * n);
+}
+static bool cgb_vec(long long N, const CgBatch& g) {
+    uintptr_t a = 0;
+    for (int c = 0; c < g.n; ++c)
+        a |= (uintptr_t)g.x[c] | (uintptr_t)g.r[c] | (uintptr_t)g.p[c] | (uintptr_t)g.q[c];
+    return N % 2 == 0 && a % 16 == 0;
+}
+void launch_cgb_init(const Dims& d, double scale, const CgBatch& g, double tol, RedScratch sc, double* cgs,
+                     cudaStream_t s) {
+    int gz;
+    const dim3 grid = cgb_grid(d, g.n, &gz);
+    k_cgb_init<<<grid, dim3(kRBX, kRBY), 0, s>>>(d, g, helm_k<double>(d, scale), gz, tol, sc, cgs);
+}
+void launch_cgb_apply(const Dims& d, double scale, const CgBatch& g, RedScratch sc, double* cgs, cudaStream_t s) {
+    int gz;
+    const dim3 grid = cgb_grid(d, g.n, &gz);
+    k_cgb_apply<<<grid, dim3(kRBX, kRBY), 0, s>>>(d, g, helm_k<double>(d, scale), gz, sc, cgs);
+}
+void launch_cgb_update(const Dims& d, const CgBatch& g, double tol, RedScratch sc, double* cgs, cudaStream_t s) {
+    const long long N = d.ncell();
+    const bool vec = cgb_vec(N, g);
+    const dim3 grid(red_blocks(vec ? N / 2 : N, std::max(1, kRedBlocks64 / g.n)), g.n);
+    if (vec) k_cgb_update<true><<<grid, kRedBlock, 0, s>>>(N, g, tol, sc, cgs);
+    else k_cgb_update<false><<<grid, kRedBlock, 0, s>>>(N, g, tol, sc, cgs);
+}
+void launch_cgb_direction(const Dims& d, const CgBatch& g, const double* cgs, cudaStream_t s) {
+    const long long N = d.ncell();
+    const bool vec = cgb_vec(N, g);
+    const dim3 grid(red_blocks(vec ? N / 2 : N, std::max(1, kRedWaveBlocks / g.n)), g.n);
+    if (vec) k_cgb_direction<true><<<grid, kRedBlock, 0, s>>>(N, g, cgs);
+    else k_cgb_direction<false><<<grid, kRedBlock, 0, s>>>(N, g, cgs);
 }
 template <typename T, int ZU>
 __global__ void k_helm_jacobi2(Dims d, int comp, HelmK<T> k, const T* __restrict__ xv, T* __restrict__ xo,

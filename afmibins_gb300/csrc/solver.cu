@@ -127,7 +127,11 @@ struct afmib_solver {
     // (AFMIB_CN_START_OLD=0: the current velocity and an FP64 stencil)
     bool cn_start_old = true;
     double *divb = nullptr, *walls = nullptr, *wallgrad = nullptr;
-    double *cg_r = nullptr, *cg_p = nullptr, *cg_q = nullptr;
+    // CG vectors (the mixed form solves one system at a time with them), the
+    // batched solve's scalars, their two pinned copies and the copies' events
+    double *cg_r[3] = {}, *cg_p[3] = {}, *cg_q[3] = {};
+    double *cgs = nullptr, *hcg = nullptr;
+    cudaEvent_t ev_cg[2] = {};
     double *tmp[3] = {};
     std::vector<MGLevel> lv;
     double *cw_p = nullptr, *cw_q = nullptr;
@@ -416,45 +420,81 @@ int read_scalars(afmib_solver* s, int first, int n) {
 }
 
 // ---------------------------------------------------------------------------
-// CG, src/alg/cg.h:32-56 (absolute 2-norm stop, warm start from x), bounded.
-// Algorithmic bytes per launch (s = 8): init 4N s, apply 2N s, update 6N s,
-// direction 3N s.
+// CG, src/alg/cg.h:32-56 (absolute 2-norm stop, warm start from x), bounded,
+// on n independent systems at once (CgBatch). The host launches each iteration
+// before it has read the previous one's norms (a system that has stopped
+// returns at once from every later launch), so the GPU does not wait for the
+// host: one iteration of empty launches at the end instead of a round trip of
+// about 12 us per iteration and system.
+// Algorithmic bytes per launch and system (s = 8): init 4N s, apply 2N s,
+// update 6N s, direction 3N s.
 // ---------------------------------------------------------------------------
-int cg_solve(afmib_solver* s, int comp, double scale, double* x, const double* b, int* iters) {
+int cg_solve_batch(afmib_solver* s, int n, const int* comp, double scale, double* const* x, const double* const* b,
+                   int* iters) {
     const Dims& d = s->d;
-    const long long N = s->N();
-    const double Ns = (double)N * sizeof(double);
+    const double Ns = (double)s->N() * sizeof(double) * n;
+    CgBatch g{};
+    g.n = n;
+    for (int c = 0; c < n; ++c) {
+        g.comp[c] = comp[c];
+        g.x[c] = x[c];
+        g.b[c] = b[c];
+        g.r[c] = s->cg_r[c];
+        g.p[c] = s->cg_p[c];
+        g.q[c] = s->cg_q[c];
+    }
+    const size_t sb = sizeof(double) * kCgScalars * n;
+    // the scalars after each iteration in one of two pinned blocks
+    auto post = [&](int slot) -> int {
+        CK(cudaMemcpyAsync(s->hcg + slot * 3 * kCgScalars, s->cgs, sb, cudaMemcpyDeviceToHost, s->st));
+        CK(cudaEventRecord(s->ev_cg[slot], s->st));
+        return AFMIB_OK;
+    };
     {
         ProfScope ps(s, P_CG_INIT, 4 * Ns);
-        launch_cg_init<double>(d, comp, scale, x, b, s->cg_r, s->cg_p, s->red, s->scal, s->st);
+        launch_cgb_init(d, scale, g, s->cfg.tol, s->red, s->cgs, s->st);
     }
     CKL();
-    TRY(read_scalars(s, 0, 1));
-    int it = 0;
-    int status = AFMIB_OK;
-    while (std::sqrt(s->hscal[0]) > s->cfg.tol) {
-        if (!std::isfinite(s->hscal[0])) { status = s->fail(AFMIB_ERR_NAN, "CG residual is not finite"); break; }
-        if (it >= s->cfg.max_cg_iters) { status = s->fail(AFMIB_ERR_NOCONV, "CG iteration cap reached"); break; }
-        {
-            ProfScope ps(s, P_CG_APPLY, 2 * Ns);
-            launch_cg_apply<double>(d, comp, scale, s->cg_p, s->cg_q, s->red, s->scal, s->st);
+    TRY(post(0));
+    const double* h = nullptr;
+    bool done = false;
+    for (int it = 0;; ++it) {
+        // iteration it is launched while the state before it, in slot it % 2, is still on its way
+        const bool more = it < s->cfg.max_cg_iters;
+        if (more) {
+            {
+                ProfScope ps(s, P_CG_APPLY, 2 * Ns);
+                launch_cgb_apply(d, scale, g, s->red, s->cgs, s->st);
+            }
+            {
+                ProfScope ps(s, P_CG_UPDATE, 6 * Ns);
+                launch_cgb_update(d, g, s->cfg.tol, s->red, s->cgs, s->st);
+            }
+            TRY(post((it + 1) % 2));
+            {
+                ProfScope ps(s, P_CG_DIR, 3 * Ns);
+                launch_cgb_direction(d, g, s->cgs, s->st);
+            }
+            CKL();
         }
-        {
-            ProfScope ps(s, P_CG_UPDATE, 6 * Ns);
-            launch_cg_update<double>(N, x, s->cg_r, s->cg_p, s->cg_q, s->red, s->scal, s->st);
-        }
-        CK(cudaMemcpyAsync(s->hscal, s->scal, sizeof(double), cudaMemcpyDeviceToHost, s->st));
-        {
-            ProfScope ps(s, P_CG_DIR, 3 * Ns);
-            launch_cg_direction<double>(N, s->cg_p, s->cg_r, s->scal, s->st);
-        }
-        CKL();
-        TRY(sync(s));
-        ++it;
+        CK(cudaEventSynchronize(s->ev_cg[it % 2]));
+        h = s->hcg + (it % 2) * 3 * kCgScalars;
+        done = true;
+        for (int c = 0; c < n; ++c) done = done && h[c * kCgScalars + 5] != 0.0;
+        if (done || !more) break;
     }
-    s->stats.cg_iters += it;
-    s->stats.last_cg_norm = std::sqrt(s->hscal[0]);
-    if (iters) *iters = it;
+    int status = AFMIB_OK;
+    for (int c = 0; c < n; ++c) {
+        const double n0 = h[c * kCgScalars];
+        const int it = (int)h[c * kCgScalars + 6];
+        s->stats.cg_iters += it;
+        s->stats.last_cg_norm = std::sqrt(n0);
+        if (iters) iters[c] = it;
+        if (status != AFMIB_OK) continue;
+        if (!std::isfinite(n0)) status = s->fail(AFMIB_ERR_NAN, "CG residual is not finite");
+        else if (h[c * kCgScalars + 5] == 0.0) status = s->fail(AFMIB_ERR_NOCONV, "CG iteration cap reached");
+    }
+    if (status != AFMIB_OK || s->prof) TRY(sync(s));
     return status;
 }
 
@@ -1285,9 +1325,11 @@ int substep(afmib_solver* s) {
         }
     }
     CKL();
-    for (int c = 0; c < 3; ++c) {
-        if (s->mixed) TRY(helm_solve_mixed(s, c, s->s_minus(), vel[c], s->rhs[c]));
-        else TRY(cg_solve(s, c, s->s_minus(), vel[c], s->rhs[c], nullptr));
+    if (s->mixed) {
+        for (int c = 0; c < 3; ++c) TRY(helm_solve_mixed(s, c, s->s_minus(), vel[c], s->rhs[c]));
+    } else {
+        const int comp[3] = {0, 1, 2};
+        TRY(cg_solve_batch(s, 3, comp, s->s_minus(), vel, s->rhs, nullptr));
     }
     s->proj_phase = be ? 0 : 1;
     const int prc = project(s);
@@ -1623,9 +1665,14 @@ int project_fields(afmib_solver* s, double* u, double* v, double* w) {
 int helm_inverse(afmib_solver* s, double* x, const double* b) {
     const long long N = s->N();
     CK(cudaMemsetAsync(x, 0, 3 * N * sizeof(double), s->st));
+    if (!s->mixed) {
+        const int comp[3] = {0, 1, 2};
+        double* const xs[3] = {x, x + N, x + 2 * N};
+        const double* const bs[3] = {b, b + N, b + 2 * N};
+        return cg_solve_batch(s, 3, comp, s->s_minus(), xs, bs, nullptr);
+    }
     for (int c = 0; c < 3; ++c) {
-        if (s->mixed) TRY(helm_solve_mixed(s, c, s->s_minus(), x + c * N, b + c * N));
-        else TRY(cg_solve(s, c, s->s_minus(), x + c * N, b + c * N, nullptr));
+        TRY(helm_solve_mixed(s, c, s->s_minus(), x + c * N, b + c * N));
     }
     return AFMIB_OK;
 }
@@ -2028,16 +2075,21 @@ int create(afmib_solver* s, const afmib_config* c, void* stream) {
     }
     TRY(dalloc(s, &s->walls, 4 * s->nxz()));
     TRY(dalloc(s, &s->wallgrad, 8 * s->nxz()));
-    TRY(dalloc(s, &s->cg_r, N));
-    TRY(dalloc(s, &s->cg_p, N));
-    TRY(dalloc(s, &s->cg_q, N));
+    for (int c = 0; c < (s->mixed ? 1 : 3); ++c) {
+        TRY(dalloc(s, &s->cg_r[c], N));
+        TRY(dalloc(s, &s->cg_p[c], N));
+        TRY(dalloc(s, &s->cg_q[c], N));
+    }
+    TRY(dalloc(s, &s->cgs, 3 * kCgScalars));
+    CK(cudaMallocHost((void**)&s->hcg, 2 * 3 * kCgScalars * sizeof(double)));
+    for (auto& e : s->ev_cg) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     TRY(dalloc(s, &s->red.partial, (size_t)kMaxRedBlocks * kMaxRedVals));
-    TRY(dalloc(s, &s->red.ticket, 1));
+    TRY(dalloc(s, &s->red.ticket, kMaxRedVals));
     TRY(dalloc(s, &s->scal, 24));
     TRY(dalloc(s, &s->dflag, 4));
     CK(cudaMallocHost((void**)&s->hscal, 24 * sizeof(double)));
     CK(cudaMallocHost((void**)&s->hflag, 4 * sizeof(int)));
-    CK(cudaMemsetAsync(s->red.ticket, 0, sizeof(unsigned), s->st));
+    CK(cudaMemsetAsync(s->red.ticket, 0, kMaxRedVals * sizeof(unsigned), s->st));
     CK(cudaMemsetAsync(s->dflag, 0, 4 * sizeof(int), s->st));
     CK(cudaMemsetAsync(s->walls, 0, 4 * s->nxz() * sizeof(double), s->st));
     CK(cudaMemsetAsync(s->wallgrad, 0, 8 * s->nxz() * sizeof(double), s->st));
@@ -2235,6 +2287,9 @@ int afmib_destroy(afmib_solver* s) {
     for (auto e : s->prof_pool) cudaEventDestroy(e);
     if (s->hscal) cudaFreeHost(s->hscal);
     if (s->hflag) cudaFreeHost(s->hflag);
+    if (s->hcg) cudaFreeHost(s->hcg);
+    for (auto e : s->ev_cg)
+        if (e) cudaEventDestroy(e);
     for (cudaStream_t q : {s->aux, s->hi})
         if (q) {
             cudaStreamSynchronize(q);
@@ -2623,7 +2678,7 @@ int afmib_helmholtz_cg(afmib_solver* s, int comp, double scale, double* x, const
         TRY(copy_in(s, s->tmp[0], x, s->N()));
         TRY(copy_in(s, s->tmp[1], b, s->N()));
     }
-    const int rc = cg_solve(s, comp, scale, s->tmp[0], s->tmp[1], iters);
+    const int rc = cg_solve_batch(s, 1, &comp, scale, &s->tmp[0], &s->tmp[1], iters);
     if (comp == 1) TRY(v_out(s, x, s->tmp[0]));
     else TRY(copy_out(s, x, s->tmp[0], s->N()));
     TRY(sync(s));
