@@ -57,7 +57,7 @@ AFMIB_HD TO cvt(TI v) { return TO(v); }
 template <>
 AFMIB_HD double cvt<double, float>(float v) { return f32_to_f64(v); }
 
-struct df2 {
+struct alignas(8) df2 {
     float hi, lo;
 };
 

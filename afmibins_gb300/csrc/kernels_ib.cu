@@ -16,6 +16,7 @@
 // and with t = frac(s - off), S = sin(pi t / 2), C = cos(pi t / 2):
 //   phi/n = (1 - S)/4, (1 + C)/4, (1 + S)/4, (1 - C)/4      (sum = 1)
 // (cos(pi r/2) at r = -1-t, -t, 1-t, 2-t). One sincospi per axis and offset.
+#include <algorithm>
 #include <type_traits>
 
 #include "dfloat.cuh"
@@ -335,212 +336,301 @@ __device__ __forceinline__ T tc_to(TC v) { return T(v); }
 template <>
 __device__ __forceinline__ double tc_to<double, dfl>(dfl v) { return f32_to_f64(v.v.hi) + f32_to_f64(v.v.lo); }
 
+// Running sum of double-float products: an exact two-sum of the leading words and
+// a plain sum of the trailing ones.
+struct alignas(8) DfAcc {
+    float s, e;  // leading sum (two-summed), trailing sum
+};
+__device__ __forceinline__ void dfacc_add(DfAcc& a, float p, float pe) {
+    const float s = a.s + p;
+    const float v = s - a.s;
+    a.e += ((a.s - (s - v)) + (p - v)) + pe;
+    a.s = s;
+}
+__device__ __forceinline__ void dfacc_mul_add(DfAcc& a, df2 x, df2 y) {
+    const float p = x.hi * y.hi;
+    float e = fmaf(x.hi, y.hi, -p);
+    e = fmaf(x.hi, y.lo, fmaf(x.lo, y.hi, e));
+    dfacc_add(a, p, e);
+}
+__device__ __forceinline__ df2 dfacc_pair(DfAcc a) {
+    df2 r;
+    r.hi = a.s + a.e;
+    r.lo = a.e - (r.hi - a.s);
+    return r;
+}
+
 // ---------------------------------------------------------------------------
-// Gather spreading. One block (TS^3 threads, one face per component each) per
-// active output tile. The markers binned in E = the tile grown by two cells
-// per side are staged in shared memory in E-cell order (x fastest): every E
-// row (ey, ez) is cut into at most three tile segments, each a contiguous run
-// of the sorted markers, and one block scan of the segment lengths places the
-// runs. A face at E-local J gathers cells [J-2, J+1] along its own axis and
-// [J-2, J+2] along the other two, i.e. at most 25 contiguous runs, in a fixed
-// order: no float atomics, bitwise repeatable.
-// A tile whose neighbourhood holds more than `cap` markers is either left to
-// a second, larger-capacity launch (ovf_list given) or, in that launch,
-// spread in chunks of `cap` staged markers. A face visits its runs in
-// increasing staged order (rows ascend in E-linear order), so cutting that
-// order into chunks leaves every face's summation order, and its result bits,
-// unchanged: there is no marker-density limit.
+// Spreading. One block per active output tile of TS x TS x TZ faces and
+// component (taken from a counter: their costs differ widely near a membrane).
+// The markers binned in E = the tile grown by two cells per side are staged in
+// shared memory in E-cell order (x fastest): every E row (ey, ez) is at most
+// three contiguous runs of the sorted markers, one per x tile, and one block
+// scan of the run lengths places them. The face planes of the tile each walk
+// the staged markers whose cells lie within reach, a contiguous range; the
+// ranges of all planes laid end to end are cut into equal shares for the warps.
+// A warp walks its part of a plane with a half warp per marker and a lane per
+// face of the marker's 4 x 4 footprint in the plane, into sums in shared
+// memory (one copy per half warp), and leaves them in the slot of (plane,
+// warp); after a barrier each plane's slots are added in warp order. No float
+// atomics and a fixed order: bitwise repeatable. More markers than `cap` are
+// taken in chunks of cap, the later ones added to the tile's faces in global
+// memory: there is no marker-density limit.
+//
+// Bound by issue and shared-memory latency of the walks (FP64: by the FP64
+// pipe as well, one instruction per marker, plane and half of the staged
+// products). The form before gave each face a thread that searched the runs
+// within its reach: 25 rows per face and component, a few markers each, most of
+// them out of its support, so its lanes diverged. One warp per plane without
+// the equal shares waited at the barrier for half its time (ncu). Measured at
+// 256^3, 200,000 markers on shells: FP64 1397 -> 448 us, double-float
+// 980 -> 497 us.
 // ---------------------------------------------------------------------------
+constexpr int kSpreadWarps = 8;
+constexpr int kSpreadCap = 192;  // FP64 or double-float markers staged at once
+constexpr int kSpreadBlocks = 5;  // blocks per SM
+// values staged per marker: 4 x weights, and the products of 4 z and 4 y weights
+// with the force
+constexpr int kSpreadVals = 4 + 16;
+
+// face sums of the compute type TC: acc += a b, and the value of two of them
+template <typename TC>
+struct FaceSum {
+    typedef TC type;
+    static __device__ __forceinline__ type zero() { return TC(0); }
+    static __device__ __forceinline__ void madd(type& s, TC a, TC b) { s += a * b; }
+    static __device__ __forceinline__ TC total(type a, type b) { return a + b; }
+    static __device__ __forceinline__ TC add(TC a, TC b) { return a + b; }
+};
+template <>
+struct FaceSum<dfl> {
+    typedef DfAcc type;
+    static __device__ __forceinline__ type zero() { return DfAcc{0.f, 0.f}; }
+    static __device__ __forceinline__ void madd(type& s, dfl a, dfl b) { dfacc_mul_add(s, a.v, b.v); }
+    static __device__ __forceinline__ dfl total(type a, type b) { return dfl{df_add(dfacc_pair(a), dfacc_pair(b))}; }
+    static __device__ __forceinline__ dfl add(dfl a, dfl b) { return dfl{df_add(a.v, b.v)}; }
+};
+
 template <typename T, int TS, int TZ, typename TC = T>
-__global__ void __launch_bounds__(TS * TS * TZ) k_spread_gather(Dims d, int M, const int* __restrict__ perm,
-                                                                MarkerW<T> mw, const T* __restrict__ G,
-                                                                const double* __restrict__ vol, double scale,
-                                                                const int* __restrict__ slot, const int* __restrict__ ctab,
-                                                                const int* __restrict__ list, const int* __restrict__ count,
-                                                                int cap, T* __restrict__ fu, T* __restrict__ fv,
-                                                                T* __restrict__ fw,
-                                                                int* __restrict__ ovf_list, int* __restrict__ ovf_count,
-                                                                int* __restrict__ next_tile) {
+__global__ void __launch_bounds__(32 * kSpreadWarps, kSpreadBlocks)
+    k_spread_tiles(Dims d, int M, const int* __restrict__ perm, MarkerW<T> mw, const T* __restrict__ G,
+                   const double* __restrict__ vol, double scale, const int* __restrict__ slot,
+                   const int* __restrict__ ctab, const int* __restrict__ list, const int* __restrict__ count, int cap,
+                   T* __restrict__ fu, T* __restrict__ fv, T* __restrict__ fw, int* __restrict__ next_item) {
     // 3D: TZ == TS, the neighbourhood grows by 2 cells per side along every
     // axis. 2D (TZ == 1, nz == 1): one plane, no z halo.
-    constexpr int NT = TS * TS * TZ, E = TS + 4, EZ = TZ == 1 ? 1 : TS + 4, HZ = TZ == 1 ? 0 : 2;
-    constexpr int E2 = E * E, E3 = E2 * EZ, C = TS * TS * TZ;
-    constexpr int CPT = (E3 + NT - 1) / NT;  // consecutive E cells per thread
+    constexpr int NW = kSpreadWarps, NT = 32 * NW, E = TS + 4, EZ = TZ == 1 ? 1 : TS + 4, HZ = TZ == 1 ? 0 : 2;
+    constexpr int C = TS * TS * TZ, PL = TS * TS, SLOTS = NW + TZ - 1;
+    constexpr int NSEG = 3 * E * EZ, SPT = (NSEG + NT - 1) / NT;  // runs, consecutive runs per thread
+    typedef FaceSum<TC> FS;
+    typedef typename FS::type Sum;
     extern __shared__ __align__(16) unsigned char smem[];
-    int* s_estart = (int*)smem;          // E3 + 1: first staged slot of each E cell
-    int* s_scan = s_estart + (E3 + 1);   // NT / 32: warp totals of the block scan
-    int* s_k = s_scan + NT;              // cap: marker index of each staged slot
-    int* s_base = s_k + cap;             // cap: packed E-local first faces
-    // cap * 12: x weights, y weights, z weights times the marker's force
-    TC* s_w = (TC*)(((uintptr_t)(s_base + cap) + 15) & ~(uintptr_t)15);
-
+    TC* const s_w = (TC*)smem;                                   // [cap][kSpreadVals]
+    Sum* const s_acc = (Sum*)(s_w + (size_t)cap * kSpreadVals);  // [warps][2][PL]
+    TC* const s_part = (TC*)(s_acc + NW * 2 * PL);               // [SLOTS][PL]: sums of (plane, warp) at plane + warp
+    int* const s_k = (int*)(s_part + SLOTS * PL);                // [cap]: marker of each staged slot
+    unsigned* const s_b = (unsigned*)(s_k + cap);                // [cap]: packed footprint of each staged marker
+    __shared__ int s_warp[NW], s_z[EZ + 1], s_li;
     const int ntx = d.nx / TS, nty = d.ny / TS;
-    const int ncount = *count;
+    const int nitem = 3 * *count;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int lx = tid % TS, ly = (tid / TS) % TS, lz = tid / (TS * TS);
     auto wrap1 = [](int v, int n) { return v < 0 ? v + n : (v >= n ? v - n : v); };
-    // tiles are taken from a shared counter (their costs differ widely near a
-    // membrane); each tile is still computed by one block, in a fixed order
-    __shared__ int s_li;
     for (;;) {
         __syncthreads();
-        if (tid == 0) s_li = atomicAdd(next_tile, 1);
+        if (tid == 0) s_li = atomicAdd(next_item, 1);
         __syncthreads();
         const int li = s_li;
-        if (li >= ncount) break;
-        const int t = list[li];
+        if (li >= nitem) break;
+        const int t = list[li / 3], comp = li % 3;
         const int tx = t % ntx, ty = (t / ntx) % nty, tz = t / (ntx * nty);
         const int ox = tx * TS - 2, oy = ty * TS - 2, oz = tz * TZ - HZ;  // E origin (unwrapped cells)
-        // sorted run [p0, p0 + cnt) of the markers binned in E cell e
-        auto run_of = [&](int e, int& p0, int& cnt) {
-            p0 = 0;
-            cnt = 0;
-            const int ex = e % E, ey = (e / E) % E, ez = e / E2;
-            const int gy = oy + ey;
-            if (d.channel && (gy < 0 || gy >= d.ny)) return;
-            const int gx = wrap1(ox + ex, d.nx), gyw = wrap1(gy, d.ny), gz = wrap1(oz + ez, d.nz);
-            const int sl = slot[gx / TS + ntx * (gyw / TS + nty * (gz / TZ))];
-            if (sl < 0) return;
-            const int lc = (gx % TS) + TS * ((gyw % TS) + TS * (gz % TZ));
-            const int* row = ctab + (size_t)sl * (C + 1) + lc;
-            p0 = row[0];
-            cnt = row[1] - p0;
-        };
-        // ---- markers of each E cell (E-linear order e = ex + E (ey + E ez)):
-        //      thread tid takes cells [tid * CPT, tid * CPT + CPT), whose
-        //      cell-table loads are independent of one another
-        int cnt[CPT], p0[CPT];
-        int tot = 0;
+        // ---- this thread's runs: sorted positions [p0, p0 + cnt)
+        int p0[SPT], cnt[SPT], tot = 0;
 #pragma unroll
-        for (int k = 0; k < CPT; ++k) {
-            const int e = tid * CPT + k;
-            cnt[k] = 0;
-            p0[k] = 0;
-            if (e < E3) run_of(e, p0[k], cnt[k]);
+        for (int k = 0; k < SPT; ++k) {
+            const int sg = tid * SPT + k;
+            p0[k] = cnt[k] = 0;
+            if (sg < NSEG) {
+                const int part = sg % 3, row = sg / 3, ey = row % E, ez = row / E;
+                const int gy = oy + ey;
+                if (!(d.channel && (gy < 0 || gy >= d.ny))) {
+                    const int gyw = wrap1(gy, d.ny), gz = wrap1(oz + ez, d.nz);
+                    const int txs = wrap1(tx + part - 1, ntx);
+                    const int sl = slot[txs + ntx * (gyw / TS + nty * (gz / TZ))];
+                    if (sl >= 0) {
+                        const int x0 = part == 0 ? TS - 2 : 0, len = part == 1 ? TS : 2;
+                        const int* r = ctab + (size_t)sl * (C + 1) + x0 + TS * ((gyw % TS) + TS * (gz % TZ));
+                        p0[k] = r[0];
+                        cnt[k] = r[len] - p0[k];
+                    }
+                }
+            }
             tot += cnt[k];
         }
-        // ---- block exclusive scan of the per-thread totals (thread order = E order);
-        //      NT < 32 (4 x 4 x 1 tiles) is one partial warp
-        constexpr int NW = (NT + 31) / 32;
-        constexpr unsigned WMASK = NT >= 32 ? 0xffffffffu : ((1u << NT) - 1u);
-        constexpr int WLAST = NT >= 32 ? 31 : NT - 1;
+        // ---- block exclusive scan of the totals (thread order = E order)
         int inc = tot;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(WMASK, inc, o);
+            const int v = __shfl_up_sync(0xffffffffu, inc, o);
             if (lane >= o) inc += v;
         }
-        if (lane == WLAST) s_scan[warp] = inc;
+        if (lane == 31) s_warp[warp] = inc;
         __syncthreads();
-        if (warp == 0) {
-            int w = lane < NW ? s_scan[lane] : 0;
+        int off = inc - tot, nall = 0;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(WMASK, w, o);
-                if (lane >= o) w += v;
-            }
-            if (lane < NW) s_scan[lane] = w;  // inclusive warp prefix
+        for (int w = 0; w < NW; ++w) {
+            if (w < warp) off += s_warp[w];
+            nall += s_warp[w];
         }
-        __syncthreads();
-        const int nc_all = s_scan[NW - 1];
-        int off = inc - tot + (warp > 0 ? s_scan[warp - 1] : 0);
         // an active tile whose neighbourhood holds no marker (its occupied
         // neighbour tiles' markers lie beyond the 2-cell halo) adds nothing:
         // its faces keep the zeros the callers wrote (block-uniform)
-        if (nc_all == 0) continue;
-        const bool chunked = nc_all > cap;  // block-uniform
-        if (chunked && ovf_list) {           // left to the large-capacity pass
-            if (tid == 0) ovf_list[atomicAdd(ovf_count, 1)] = t;
-            continue;
+        if (nall == 0) continue;
+        {
+            int o = off;
+#pragma unroll
+            for (int k = 0; k < SPT; ++k) {
+                const int sg = tid * SPT + k;
+                if (sg < NSEG && sg % (3 * E) == 0) s_z[sg / (3 * E)] = o;  // first staged marker of E plane ez
+                o += cnt[k];
+            }
+            if (tid == 0) s_z[EZ] = nall;
         }
-        // ---- E-cell starts and, in one pass, the staged marker indices
+        const int vx = comp == 0 ? 0 : 1, vy = comp == 1 ? 0 : 1, vz = comp == 2 ? 0 : 1;  // face offsets
+        for (int lo = 0; lo < nall; lo += cap) {
+            const int nc = nall - lo < cap ? nall - lo : cap;
+            __syncthreads();  // s_z is written; the previous chunk is done with the staged markers
+            {
+                int o = off - lo;  // this thread's first run, relative to the chunk
 #pragma unroll
-        for (int k = 0; k < CPT; ++k) {
-            const int e = tid * CPT + k;
-            if (e < E3) {
-                s_estart[e] = off;
-                if (!chunked)
-                    for (int m = 0; m < cnt[k]; ++m) s_k[off + m] = perm[p0[k] + m];
-                off += cnt[k];
-            }
-        }
-        if (tid == 0) s_estart[E3] = nc_all;
-        const int nchunk = chunked ? (nc_all + cap - 1) / cap : 1;
-        // chunked: marker indices of staged slots [lo, lo + cap) from this
-        // thread's E cells (runs looked up again: nothing held across chunks)
-        auto stage_ids = [&](int lo) {
-            for (int k = 0; k < CPT; ++k) {
-                const int e = tid * CPT + k;
-                if (e >= E3) break;
-                const int o = s_estart[e], n = s_estart[e + 1] - o;
-                if (n == 0 || o + n <= lo || o >= lo + cap) continue;
-                int q0, qn;
-                run_of(e, q0, qn);
-                const int a = lo - o > 0 ? lo - o : 0, b = lo + cap - o < n ? lo + cap - o : n;
-                for (int m = a; m < b; ++m) s_k[o + m - lo] = perm[q0 + m];
-            }
-        };
-        __syncthreads();
-        // ---- one component at a time (and, past the capacity, one chunk at a time)
-        const int J[3] = {lx + 2, ly + 2, lz + HZ};
-        for (int comp = 0; comp < 3; ++comp) {
-            TC acc = tc_from<TC>(0.0);
-            const unsigned jp = 0x00808080u | (unsigned)(J[0] + 8) | ((unsigned)(J[1] + 8) << 8) |
-                                ((unsigned)(J[2] + 8) << 16);
-            const int hx = (comp == 0) ? J[0] + 1 : J[0] + 2;
-            const int hy = (comp == 1) ? J[1] + 1 : J[1] + 2;
-            const int hz = TZ == 1 ? J[2] : ((comp == 2) ? J[2] + 1 : J[2] + 2);
-            for (int ch = 0; ch < nchunk; ++ch) {
-                const int lo = ch * cap, nc = nc_all - lo < cap ? nc_all - lo : cap;
-                if (chunked) {
-                    __syncthreads();  // the previous chunk's gather is done with s_k, s_base, s_w
-                    stage_ids(lo);
-                    __syncthreads();
+                for (int k = 0; k < SPT; ++k) {
+                    const int m0 = o < 0 ? -o : 0, m1 = cnt[k] < nc - o ? cnt[k] : nc - o;
+                    for (int m = m0; m < m1; ++m) s_k[o + m] = perm[p0[k] + m];
+                    o += cnt[k];
                 }
-                for (int sl = tid; sl < nc; sl += NT) {
-                    const int k = s_k[sl];
-                    const TC g = tc_from<TC>((double)G[(size_t)comp * M + k] * (vol ? vol[k] : 1.0) * scale);
-                    int packed = 0;
-#pragma unroll
-                    for (int a = 0; a < 3; ++a) {
-                        const int v = (a == comp) ? 0 : 1;
-                        const int o = a == 0 ? ox : (a == 1 ? oy : oz);
-                        const int n_a = a == 0 ? d.nx : (a == 1 ? d.ny : d.nz);
-                        // E-local first face: cell relative to the E origin + offset
-                        int ec = mw.cell[3 * k + a] - o;
-                        if (!(a == 1 && d.channel)) ec = wrapi(ec, n_a);
-                        const int b = ec + mw.dbase[(k * 3 + a) * 2 + v];
-                        packed |= (b + 8) << (8 * a);
-                        const T* w = mw.w + (((size_t)k * 3 + a) * 2 + v) * 4;
-#pragma unroll
-                        for (int m = 0; m < 4; ++m)
-                            s_w[(size_t)sl * 12 + a * 4 + m] = a == 2 ? tc_from<TC>(w[m]) * g : tc_from<TC>(w[m]);
-                    }
-                    s_base[sl] = packed;
-                }
-                __syncthreads();
-                for (int ez = J[2] - HZ; ez <= hz; ++ez)
-                    for (int ey = J[1] - 2; ey <= hy; ++ey) {
-                        const int row = E * (ey + E * ez);
-                        int s0 = s_estart[row + J[0] - 2] - lo, s1 = s_estart[row + hx + 1] - lo;
-                        s0 = s0 > 0 ? s0 : 0;
-                        s1 = s1 < nc ? s1 : nc;
-                        for (int sl = s0; sl < s1; ++sl) {
-                            // per byte (0x80 + J + 8) - (b + 8): no borrow crosses a
-                            // byte (all fields < 0x80); the face is in the marker's
-                            // support iff every byte is 0x80 + {0..3}
-                            const unsigned t = jp - (unsigned)s_base[sl];
-                            if ((t & 0x00FCFCFCu) == 0x00808080u) {
-                                const TC* w = s_w + (size_t)sl * 12;
-                                acc += (w[t & 3u] * w[4 + ((t >> 8) & 3u)]) * w[8 + ((t >> 16) & 3u)];
-                            }
-                        }
-                    }
             }
-            T* f = comp == 0 ? fu : (comp == 1 ? fv : fw);
-            const int gx = tx * TS + lx, gy = ty * TS + ly, gz = tz * TZ + lz;
-            if (!(d.channel && comp == 1 && gy == 0)) f[lin(d, gx, gy, gz)] = tc_to<T, TC>(acc);
             __syncthreads();
+            // ---- the chunk's products, a marker's values on consecutive threads
+            for (int i = tid; i < nc * 4; i += NT) {
+                const int m = i >> 2, j = i & 3, k = s_k[m];
+                const T* w = mw.w + (size_t)k * 24;
+                TC* o = s_w + (size_t)m * kSpreadVals;
+                double g = (double)G[(size_t)comp * M + k];
+                if (vol) g *= vol[k];
+                const TC wz = tc_from<TC>(w[16 + 4 * vz + j]) * tc_from<TC>(g);
+                o[j] = tc_from<TC>(w[4 * vx + j]);
+#pragma unroll
+                for (int y = 0; y < 4; ++y) o[4 + 4 * j + y] = tc_from<TC>(w[8 + 4 * vy + y]) * wz;
+            }
+            // ---- and footprints: the lanes (4 iy + ix) whose faces lie in the tile, the face of lane 0
+            //      within the plane (36 added) and the first face plane (8 added)
+            for (int m = tid; m < nc; m += NT) {
+                const int k = s_k[m];
+                int f[3];
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    const int o = a == 0 ? ox : (a == 1 ? oy : oz);
+                    const int n_a = a == 0 ? d.nx : (a == 1 ? d.ny : d.nz);
+                    int ec = mw.cell[3 * k + a] - o;  // E-local cell
+                    if (!(a == 1 && d.channel)) ec = wrapi(ec, n_a);
+                    f[a] = ec + mw.dbase[(k * 3 + a) * 2 + (a == comp ? 0 : 1)];  // E-local first face
+                }
+                unsigned mx = 0, mask = 0;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) mx |= (unsigned)(f[0] + i - 2) < (unsigned)TS ? 1u << i : 0u;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) mask |= (unsigned)(f[1] + i - 2) < (unsigned)TS ? mx << (4 * i) : 0u;
+                s_b[m] = mask | (unsigned)(f[0] - 2 + TS * (f[1] - 2) + 36) << 16 | (unsigned)(f[2] + 8) << 24;
+            }
+            __syncthreads();
+            // ---- walks: E planes of cells within reach of face plane J = lz + HZ are [J - 2, J + 2]
+            //      ([J - 2, J + 1] where the faces sit on integer z), the only one in 2D
+            auto range = [&](int lz, int& m0, int& m1) {
+                const int J = lz + HZ, e0 = TZ == 1 ? 0 : J - 2, e1 = TZ == 1 ? 0 : (comp == 2 ? J + 1 : J + 2);
+                m0 = s_z[e0] - lo;
+                m1 = s_z[e1 + 1] - lo;
+                m0 = m0 > 0 ? m0 : 0;
+                m1 = m1 < nc ? m1 : nc;
+                if (m1 < m0) m1 = m0;
+            };
+            int visits = 0;
+#pragma unroll
+            for (int lz = 0; lz < TZ; ++lz) {
+                int m0, m1;
+                range(lz, m0, m1);
+                visits += m1 - m0;
+            }
+            // warp w takes visits [share(w), share(w + 1)), even shares so that both halves work
+            const int per = ((visits + 2 * NW - 1) / (2 * NW)) * 2;
+            auto part_of = [&](int w, int first, int m0, int m1, int& a, int& b) {
+                a = w * per - first;
+                b = a + per;
+                a = m0 + (a > 0 ? a : 0);
+                b = m0 + (b < m1 - m0 ? b : m1 - m0);
+                return a < b;
+            };
+            {
+                Sum* const acc = s_acc + warp * 2 * PL;
+                const int half = lane >> 4, l16 = lane & 15;
+                Sum* const mine = acc + half * PL + (l16 & 3) + TS * (l16 >> 2) - 36;
+                const TC* const wx0 = s_w + (l16 & 3);
+                const TC* const wyz0 = s_w + 4 + (l16 >> 2);
+                int first = 0;
+                for (int lz = 0; lz < TZ; ++lz) {
+                    int m0, m1, a, b;
+                    range(lz, m0, m1);
+                    if (part_of(warp, first, m0, m1, a, b)) {
+                        for (int i = lane; i < 2 * PL; i += 32) acc[i] = FS::zero();
+                        __syncwarp();
+                        // this lane's term of marker m: its face sum, or null outside the plane or the tile
+                        auto term = [&](int m, TC& x, TC& yz) -> Sum* {
+                            if (m >= b) return nullptr;
+                            const unsigned pk = s_b[m];
+                            const unsigned kz = (unsigned)(lz + HZ + 8) - (pk >> 24);
+                            if (kz >= 4u || !((pk >> l16) & 1u)) return nullptr;
+                            x = wx0[m * kSpreadVals];
+                            yz = wyz0[m * kSpreadVals + 4 * kz];
+                            return mine + ((pk >> 16) & 255u);
+                        };
+                        // two markers of the half warp in flight: the second's loads do
+                        // not wait for the first's sum
+                        for (int m = a + half; m - half < b; m += 4) {
+                            TC x0, y0, x1, y1;
+                            Sum* const f0 = term(m, x0, y0);
+                            Sum* const f1 = term(m + 2, x1, y1);
+                            if (f0) FS::madd(*f0, x0, y0);
+                            __syncwarp();
+                            if (f1) FS::madd(*f1, x1, y1);
+                            __syncwarp();
+                        }
+                        for (int i = lane; i < PL; i += 32) s_part[(lz + warp) * PL + i] = FS::total(acc[i], acc[PL + i]);
+                        __syncwarp();
+                    }
+                    first += m1 - m0;
+                }
+            }
+            __syncthreads();
+            // ---- a plane's parts in warp order
+            T* const out = comp == 0 ? fu : (comp == 1 ? fv : fw);
+            int first = 0;
+            for (int lz = 0; lz < TZ; ++lz) {
+                int m0, m1;
+                range(lz, m0, m1);
+                if (lz % NW == warp)
+                    for (int i = lane; i < PL; i += 32) {
+                        TC v = tc_from<TC>(0.0);
+                        for (int w = 0; w < NW; ++w) {
+                            int a, b;
+                            if (part_of(w, first, m0, m1, a, b)) v = FS::add(v, s_part[(lz + w) * PL + i]);
+                        }
+                        const int gx = tx * TS + i % TS, gy = ty * TS + i / TS, gz = tz * TZ + lz;
+                        if (d.channel && comp == 1 && gy == 0) continue;  // the wall plane
+                        const T r = T((double)tc_to<T, TC>(v) * scale);
+                        T* const o = out + lin(d, gx, gy, gz);
+                        *o = lo == 0 ? r : *o + r;
+                    }
+                first += m1 - m0;
+            }
         }
     }
 }
@@ -596,28 +686,6 @@ __global__ void k_interp(Dims d, int M, const int* __restrict__ perm, MarkerW<T>
 // the result is within a few units of 2^-46 of the largest term times the 4
 // to 16 terms of a sum. One FP64 addition per component turns the pair back
 // into FP64.
-struct DfAcc {
-    float s, e;  // leading sum (two-summed), trailing sum
-};
-__device__ __forceinline__ void dfacc_add(DfAcc& a, float p, float pe) {
-    const float s = a.s + p;
-    const float v = s - a.s;
-    a.e += ((a.s - (s - v)) + (p - v)) + pe;
-    a.s = s;
-}
-__device__ __forceinline__ void dfacc_mul_add(DfAcc& a, df2 x, df2 y) {
-    const float p = x.hi * y.hi;
-    float e = fmaf(x.hi, y.hi, -p);
-    e = fmaf(x.hi, y.lo, fmaf(x.lo, y.hi, e));
-    dfacc_add(a, p, e);
-}
-__device__ __forceinline__ df2 dfacc_pair(DfAcc a) {
-    df2 r;
-    r.hi = a.s + a.e;
-    r.lo = a.e - (r.hi - a.s);
-    return r;
-}
-
 constexpr int kInterpDfBlock = 128;
 
 template <bool PAIRS>
@@ -781,54 +849,31 @@ void launch_cell_table(int TS, int TZ, const unsigned* keys, const int* tstart, 
     else k_cell_table<4, 1><<<blocks, 16, 0, s>>>(keys, tstart, tend, occ, occ_count, ctab);
 }
 
-template <typename T>
-size_t spread_smem_bytes(int TS, int TZ, int cap) {
-    const int E = TS + 4, EZ = TZ == 1 ? 1 : TS + 4, E3 = E * E * EZ, NT = TS * TS * TZ;
-    size_t ints = (size_t)(E3 + 1) + NT + 2 * (size_t)cap;
-    size_t bytes = ints * sizeof(int);
-    bytes = (bytes + 15) & ~(size_t)15;
-    bytes += (size_t)cap * 12 * sizeof(T);
-    return bytes;
-}
-
 template <typename T, int TS, int TZ, typename TC>
 static void spread_launch(const Dims& d, int M, const int* perm, MarkerW<T> mw, const T* G, const double* vol,
                           double scale, const int* slot, const int* ctab, const int* list, const int* count,
-                          int max_tiles, int cap, T* fu, T* fv, T* fw, int* ovf_list, int* ovf_count,
-                          int* next_tile, cudaStream_t s) {
-    static_assert(sizeof(TC) == sizeof(T), "the staged weights take the input type's size");
-    const size_t smem = spread_smem_bytes<T>(TS, TZ, cap);
-    // opt in to exactly the dynamic shared memory this launch uses (the
-    // kernel's static shared memory counts against the same 227 KB)
-    static size_t configured = 0;  // the largest capacity asked for so far
-    if (configured < smem) {
-        if (cudaFuncSetAttribute(k_spread_gather<T, TS, TZ, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem) != cudaSuccess)
-            return;  // the launch error is reported by the caller's cudaGetLastError
-        configured = smem;
-    }
-    int blocks = max_tiles < 152 * 4 ? max_tiles : 152 * 4;
-    if (blocks < 1) blocks = 1;
-    k_spread_gather<T, TS, TZ, TC><<<blocks, TS * TS * TZ, smem, s>>>(d, M, perm, mw, G, vol, scale, slot, ctab,
-                                                                      list, count, cap, fu, fv, fw, ovf_list,
-                                                                      ovf_count, next_tile);
+                          int max_tiles, T* fu, T* fv, T* fw, int* next_tile, cudaStream_t s) {
+    const int cap = kSpreadCap * 8 / (int)sizeof(TC);
+    const size_t smem = sizeof(TC) * ((size_t)cap * kSpreadVals + (3 * kSpreadWarps + TZ - 1) * TS * TS) + 8 * (size_t)cap;
+    cudaFuncSetAttribute(k_spread_tiles<T, TS, TZ, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const int blocks = std::max(1, std::min(3 * max_tiles, 152 * kSpreadBlocks));
+    k_spread_tiles<T, TS, TZ, TC><<<blocks, 32 * kSpreadWarps, smem, s>>>(d, M, perm, mw, G, vol, scale, slot, ctab,
+                                                                         list, count, cap, fu, fv, fw, next_tile);
 }
 
 template <typename T>
-void launch_spread_gather(const Dims& d, int TS, int M, const int* perm, MarkerW<T> mw, const T* G, const double* vol,
-                          double scale, const int* slot, const int* ctab, const int* list, const int* count,
-                          int max_tiles, int cap, T* fu, T* fv, T* fw, int* ovf_list, int* ovf_count,
-                          int* next_tile, cudaStream_t s, bool dfloat) {
+void launch_spread(const Dims& d, int TS, int M, const int* perm, MarkerW<T> mw, const T* G, const double* vol,
+                   double scale, const int* slot, const int* ctab, const int* list, const int* count, int max_tiles,
+                   T* fu, T* fv, T* fw, int* next_tile, cudaStream_t s, bool dfloat) {
     const bool flat = d.nz == 1;
 #define AFMIB_SPREAD(TSV, TZV)                                                                                     \
     do {                                                                                                           \
         if (dfloat && sizeof(T) == sizeof(double))                                                                 \
             spread_launch<T, TSV, TZV, std::conditional_t<sizeof(T) == sizeof(double), dfl, T>>(                   \
-                d, M, perm, mw, G, vol, scale, slot, ctab, list, count, max_tiles, cap, fu, fv, fw, ovf_list,      \
-                ovf_count, next_tile, s);                                                                          \
+                d, M, perm, mw, G, vol, scale, slot, ctab, list, count, max_tiles, fu, fv, fw, next_tile, s);      \
         else                                                                                                       \
-            spread_launch<T, TSV, TZV, T>(d, M, perm, mw, G, vol, scale, slot, ctab, list, count, max_tiles, cap, \
-                                          fu, fv, fw, ovf_list, ovf_count, next_tile, s);                         \
+            spread_launch<T, TSV, TZV, T>(d, M, perm, mw, G, vol, scale, slot, ctab, list, count, max_tiles, fu,   \
+                                          fv, fw, next_tile, s);                                                   \
     } while (0)
     if (TS == 8 && !flat) AFMIB_SPREAD(8, 8);
     else if (TS == 4 && !flat) AFMIB_SPREAD(4, 4);
@@ -865,10 +910,9 @@ void launch_marker_axpy(int M, double* Xo, const double* Xi, const double* U, do
                                             cudaStream_t);                                                         \
     template void launch_marker_prep<T>(const Dims&, int, int, const double*, unsigned*, int*, MarkerW<T>, int*, \
                                         cudaStream_t, bool);                                                     \
-    template size_t spread_smem_bytes<T>(int, int, int);                                                             \
-    template void launch_spread_gather<T>(const Dims&, int, int, const int*, MarkerW<T>, const T*, const double*, \
-                                          double, const int*, const int*, const int*, const int*, int, int, T*,  \
-                                          T*, T*, int*, int*, int*, cudaStream_t, bool);                        \
+    template void launch_spread<T>(const Dims&, int, int, const int*, MarkerW<T>, const T*, const double*, double,  \
+                                   const int*, const int*, const int*, const int*, int, T*, T*, T*, int*,           \
+                                   cudaStream_t, bool);                                                             \
     template void launch_interp<T, double>(const Dims&, int, const int*, MarkerW<T>, const double*, const double*, \
                                            const double*, double*, cudaStream_t);                               \
     template void launch_interp<T, float>(const Dims&, int, const int*, MarkerW<T>, const float*, const float*,  \

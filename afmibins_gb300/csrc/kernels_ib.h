@@ -49,21 +49,16 @@ void launch_active_tiles(int ntx, int nty, int ntz, int channel, const int* tsta
 void launch_cell_table(int TS, int TZ, const unsigned* keys, const int* tstart, const int* tend, const int* occ,
                        const int* occ_count, int max_occ, int* ctab, cudaStream_t s);
 
-template <typename T>
-size_t spread_smem_bytes(int TS, int TZ, int cap);
 // f_c(face) = scale * sum_k (phi/n)^3 * vol_k * G_c,k over the active tiles
 // (faces of the other tiles, and of active tiles whose neighbourhood holds no
-// marker, are left untouched: the callers zero the fields first). A tile whose neighbourhood
-// holds more than `cap` markers is appended to ovf_list (and left untouched)
-// when ovf_list is given, else spread in chunks of `cap` markers (same
-// result bits as one pass). Blocks take tiles from *next_tile, which must be
-// zero at launch. dfloat (FP64 inputs): weight products and face sums in
-// double-float on the FP32 pipe (relative 2^-44) instead of FP64.
+// marker, are left untouched: the callers zero the fields first). Blocks take
+// tiles from *next_tile, which must be zero at launch. dfloat (FP64 inputs):
+// weight products and face sums in double-float on the FP32 pipe (relative
+// 2^-44) instead of FP64.
 template <typename T>
-void launch_spread_gather(const Dims& d, int TS, int M, const int* perm, MarkerW<T> mw, const T* G, const double* vol,
-                          double scale, const int* slot, const int* ctab, const int* list, const int* count,
-                          int max_tiles, int cap, T* fu, T* fv, T* fw, int* ovf_list, int* ovf_count,
-                          int* next_tile, cudaStream_t s, bool dfloat = false);
+void launch_spread(const Dims& d, int TS, int M, const int* perm, MarkerW<T> mw, const T* G, const double* vol,
+                   double scale, const int* slot, const int* ctab, const int* list, const int* count, int max_tiles,
+                   T* fu, T* fv, T* fw, int* next_tile, cudaStream_t s, bool dfloat = false);
 
 // U[c*M + k] = sum (phi/n)^3 u_c(face); perm (may be null) orders the threads.
 // T: weight and arithmetic type, TF: field storage type

@@ -226,9 +226,8 @@ struct afmib_solver {
     int *vals = nullptr, *vals2 = nullptr, *perm = nullptr;
     int TS = 0, TZ = 0, ntx = 0, nty = 0, ntz = 0, ntiles = 0;  // TZ: tile depth (TS; 1 on a 2D grid)
     int tile_cells() const { return TS * TS * TZ; }
-    // tcount: [0] active output tiles, [1] occupied tiles, [2] tiles left to the large-capacity spreading pass,
-    // [3], [4] the two passes' tile counters
-    int *tstart = nullptr, *tend = nullptr, *tlist = nullptr, *tcount = nullptr, *tovf = nullptr;
+    // tcount: [0] active output tiles, [1] occupied tiles, [2] the spreading's tile counter
+    int *tstart = nullptr, *tend = nullptr, *tlist = nullptr, *tcount = nullptr;
     int *tslot = nullptr, *tocc = nullptr, *ctab = nullptr;
     int ctab_cap = 0;  // occupied tiles the cell table can hold
     MarkerW<double> mw{};
@@ -1443,18 +1442,13 @@ int bin_markers(afmib_solver* s, const double* P, bool fp32 = false, bool df_wei
     return AFMIB_OK;
 }
 
-// Spreading in two passes: blocks sized for `cap_small` neighbourhood markers
-// (two blocks per SM) take every active tile whose neighbourhood fits and list
-// the others, which a second pass with `cap_large` handles. Each tile is
-// computed once, by one of the passes, with the same arithmetic.
+// the faces of the active tiles (launch_spread)
 template <typename T>
-int spread_two_pass(afmib_solver* s, MarkerW<T> mw, const T* G, const double* vol, double scale, T* fu, T* fv, T* fw,
-                    int cap_small, int cap_large, bool dfloat = false) {
-    CK(cudaMemsetAsync(s->tcount + 2, 0, 3 * sizeof(int), s->st));  // overflow count and the two tile counters
-    launch_spread_gather<T>(s->d, s->TS, s->M, s->perm, mw, G, vol, scale, s->tslot, s->ctab, s->tlist, s->tcount,
-                            s->ntiles, cap_small, fu, fv, fw, s->tovf, s->tcount + 2, s->tcount + 3, s->st, dfloat);
-    launch_spread_gather<T>(s->d, s->TS, s->M, s->perm, mw, G, vol, scale, s->tslot, s->ctab, s->tovf, s->tcount + 2,
-                            s->ntiles, cap_large, fu, fv, fw, nullptr, nullptr, s->tcount + 4, s->st, dfloat);
+int spread_tiles(afmib_solver* s, MarkerW<T> mw, const T* G, const double* vol, double scale, T* fu, T* fv, T* fw,
+                 bool dfloat = false) {
+    CK(cudaMemsetAsync(s->tcount + 2, 0, sizeof(int), s->st));  // the tile counter
+    launch_spread<T>(s->d, s->TS, s->M, s->perm, mw, G, vol, scale, s->tslot, s->ctab, s->tlist, s->tcount, s->ntiles,
+                     fu, fv, fw, s->tcount + 2, s->st, dfloat);
     return AFMIB_OK;
 }
 
@@ -1468,7 +1462,7 @@ int spread_generic(afmib_solver* s, const double* G, const double* vol, double s
     const double touched = (double)s->stats.spread_tiles * s->tile_cells();
     {
         ProfScope ps(s, P_SPREAD, (double)s->M * (24 + 3 * 8 + 8 + 8) + 3 * touched * 8);
-        TRY(spread_two_pass<double>(s, s->mw, G, vol, scale, fu, fv, fw, 896, 1536));
+        TRY(spread_tiles<double>(s, s->mw, G, vol, scale, fu, fv, fw));
     }
     CKL();
     return AFMIB_OK;
@@ -1489,11 +1483,10 @@ int spread_forces(afmib_solver* s, const double* vol, double* fu, double* fv, do
     CK(cudaMemsetAsync(fv, 0, N * sizeof(double), s->st));
     CK(cudaMemsetAsync(fw, 0, N * sizeof(double), s->st));
     const double n3 = spread_scale(s->d);
-    const int cap = 1536;
     const double touched = (double)s->stats.spread_tiles * s->tile_cells();
     {
         ProfScope ps(s, P_SPREAD, (double)s->M * (24 + 3 * 8 + 8 + 8) + 3 * touched * 8);
-        TRY(spread_two_pass<double>(s, s->mw, s->G, vol, n3, fu, fv, fw, 896, cap, dfloat));
+        TRY(spread_tiles<double>(s, s->mw, s->G, vol, n3, fu, fv, fw, dfloat));
     }
     CKL();
     return AFMIB_OK;
@@ -1503,11 +1496,10 @@ int spread_forces32(afmib_solver* s, const double* vol) {
     const long long N = s->N();
     for (int c = 0; c < 3; ++c) CK(cudaMemsetAsync(s->f32[c], 0, N * sizeof(float), s->st));
     const double n3 = spread_scale(s->d);
-    const int cap = 3072;
     const double touched = (double)s->stats.spread_tiles * s->tile_cells();
     {
         ProfScope ps(s, P_SPREAD, (double)s->M * (24 + 3 * 4 + 8 + 8) + 3 * touched * 4);
-        TRY(spread_two_pass<float>(s, s->mw32, s->G32, vol, n3, s->f32[0], s->f32[1], s->f32[2], 1792, cap));
+        TRY(spread_tiles<float>(s, s->mw32, s->G32, vol, n3, s->f32[0], s->f32[1], s->f32[2]));
     }
     CKL();
     return AFMIB_OK;
@@ -1937,8 +1929,7 @@ int setup_tiles(afmib_solver* s) {
     TRY(dalloc(s, &s->tstart, s->ntiles));
     TRY(dalloc(s, &s->tend, s->ntiles));
     TRY(dalloc(s, &s->tlist, s->ntiles));
-    TRY(dalloc(s, &s->tcount, 5));
-    TRY(dalloc(s, &s->tovf, s->ntiles));
+    TRY(dalloc(s, &s->tcount, 3));
     TRY(dalloc(s, &s->tslot, s->ntiles));
     TRY(dalloc(s, &s->tocc, s->ntiles));
     return AFMIB_OK;
