@@ -90,6 +90,126 @@ __global__ void __launch_bounds__(BX * BY, P2 ? 6 : 4) k_advect(Dims d, T* __res
     }
 }
 
+// The FP64 advection of 3D grids without repeated fluxes. GB300's FP64 pipe
+// bounds it, and k_advect forms every flux two or three times (81 FP64
+// instructions per cell). Here a thread walks ZC planes along z with two rows of
+// y: it forms its cells' six fluxes once (unscaled sums and products: the 1/4 of
+// the averages joins the factor n at the end, exactly), takes the fluxes at
+// x + 1 from its neighbours through shared memory, those at z + 1 from its next
+// step, and forms again only the three at y + 1 above its second row: 37 FP64
+// instructions per cell. A block spans whole rows of x (the wrap in x is then
+// another thread of the block) and as many row pairs as make about 256 threads.
+// Measured: a call on 192 x 160 x 128 device fields 641 -> 311 us (copies left out
+// as well), the 128^3 FP64 IB step 14.06 -> 13.82 ms (two launches).
+constexpr int kAdvRows = 2, kAdvMaxNx = 512;
+__global__ void __launch_bounds__(kAdvMaxNx) k_advect_rows(Dims d, int by, int zc, double n4, double* __restrict__ ua,
+                                                          double* __restrict__ va, double* __restrict__ wa,
+                                                          const double* __restrict__ u, const double* __restrict__ v,
+                                                          const double* __restrict__ w) {
+    extern __shared__ double sh[];  // [2][3][kAdvRows][threads]: uu, uv, uw of every thread's cells
+    const int nt = blockDim.x, t = threadIdx.x;
+    const int x = t % d.nx, ty = t / d.nx;
+    const int y0 = (blockIdx.x * by + ty) * kAdvRows, z0 = blockIdx.y * zc;
+    const int nz = min(zc, d.nz - z0);
+    const bool lane_ok = ty < by && y0 < d.ny;
+    const int tr = ty >= by ? t : (x == d.nx - 1 ? t - x : t + 1);  // the thread of x + 1
+    // rows y0 - 1 .. y0 + 2 of a plane at x and x - 1
+    long long row[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        int y = y0 - 1 + j;
+        y = y < 0 ? y + d.ny : (y >= d.ny ? y - d.ny : y);
+        y = y >= d.ny ? y - d.ny : y;  // y0 + 2 on the last odd row, or beyond it on an idle thread
+        row[j] = (long long)d.nx * (lane_ok ? y : 0);
+    }
+    const int xm = x == 0 ? d.nx - 1 : x - 1;
+    const long long sxy = d.sxy();
+    double uz[2], vz[3], wz[2];  // the plane below: u, w at rows 1, 2 and v at rows 1, 2, 3
+    double au[2], av[2], aw[2], fu[2], fv[2], fw[2];  // plane z: x and y parts, z fluxes
+    {
+        const long long pz = sxy * (z0 == 0 ? d.nz - 1 : z0 - 1);
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            if (r < 2) {
+                uz[r] = u[pz + row[r + 1] + x];
+                wz[r] = w[pz + row[r + 1] + x];
+            }
+            vz[r] = v[pz + row[r + 1] + x];
+        }
+    }
+    for (int k = 0; k <= nz; ++k) {
+        const int z = z0 + k;
+        const long long pz = sxy * (z >= d.nz ? z - d.nz : z);
+        double uc[4], vc[4], wc[4], ul[2], vl[3], wl[2];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            uc[j] = u[pz + row[j] + x];
+            vc[j] = v[pz + row[j] + x];
+            wc[j] = w[pz + row[j] + x];
+        }
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            if (r < 2) {
+                ul[r] = u[pz + row[r + 1] + xm];
+                wl[r] = w[pz + row[r + 1] + xm];
+            }
+            vl[r] = v[pz + row[r + 1] + xm];
+        }
+        // four times the fluxes at the cells' own corners, and uv, vv, vw of the row above
+        double uu[2], uv[3], uw[2], vv[3], vw[3], ww[2];
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            double q = uc[r + 1] + uc[r];
+            uv[r] = q * (vc[r + 1] + vl[r]);
+            q = vc[r + 1] + vc[r];
+            vv[r] = q * q;
+            vw[r] = (vz[r] + vc[r + 1]) * (wc[r + 1] + wc[r]);
+            if (r < 2) {
+                q = uc[r + 1] + ul[r];
+                uu[r] = q * q;
+                uw[r] = (uz[r] + uc[r + 1]) * (wl[r] + wc[r + 1]);
+                q = wc[r + 1] + wz[r];
+                ww[r] = q * q;
+            }
+        }
+        if (k > 0 && lane_ok) {  // plane z - 1 is complete
+            const long long po = sxy * (z - 1);
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+                if (y0 + r < d.ny) {
+                    const long long i = po + row[r + 1] + x;
+                    ua[i] = n4 * (au[r] + (uw[r] - fu[r]));
+                    va[i] = d.channel && y0 + r == 0 ? 0.0 : n4 * (av[r] + (vw[r] - fv[r]));
+                    wa[i] = n4 * (aw[r] + (ww[r] - fw[r]));
+                }
+        }
+        if (k == nz) break;
+        double* const s = sh + (size_t)(k & 1) * 3 * kAdvRows * nt;
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            s[(0 * kAdvRows + r) * nt + t] = uu[r];
+            s[(1 * kAdvRows + r) * nt + t] = uv[r];
+            s[(2 * kAdvRows + r) * nt + t] = uw[r];
+        }
+        __syncthreads();  // (two buffers: the previous step's reads are done before this one's second writes)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const double uup = s[(0 * kAdvRows + r) * nt + tr], uvp = s[(1 * kAdvRows + r) * nt + tr],
+                         uwp = s[(2 * kAdvRows + r) * nt + tr];
+            au[r] = (uup - uu[r]) + (uv[r + 1] - uv[r]);
+            av[r] = (uvp - uv[r]) + (vv[r + 1] - vv[r]);
+            aw[r] = (uwp - uw[r]) + (vw[r + 1] - vw[r]);
+            fu[r] = uw[r];
+            fv[r] = vw[r];
+            fw[r] = ww[r];
+            uz[r] = uc[r + 1];
+            wz[r] = wc[r + 1];
+        }
+#pragma unroll
+        for (int r = 0; r < 3; ++r) vz[r] = vc[r + 1];
+    }
+}
+
 // The mixed form's advection of the FP64 velocity, in FP32 from its pairs of
 // floats (h: the nearest float, l: the rest, written by the projection; plane
 // 0 of v is the zero wall in channel mode as above). The fluxes are those of
@@ -1149,6 +1269,30 @@ inline int ew_blocks(long long n) {
 
 template <typename TI, typename T>
 void launch_advect(const Dims& d, T* ua, T* va, T* wa, const TI* u, const TI* v, const TI* w, cudaStream_t s) {
+    if constexpr (sizeof(TI) == sizeof(double) && sizeof(T) == sizeof(double)) {
+        // 3D rows that fit a block; 2D grids (a plane of latency) and longer rows keep the one-cell kernel
+        if (d.nz > 1 && d.ny > 1 && d.nx <= kAdvMaxNx) {
+            const int by = std::max(1, std::min(256 / d.nx, (d.ny + kAdvRows - 1) / kAdvRows));
+            const int nt = (by * d.nx + 31) / 32 * 32;
+            const int gy = (d.ny + by * kAdvRows - 1) / (by * kAdvRows);
+            // planes per block: the fewest waves times steps (zc + 1) at about 512 threads per SM
+            const int wave = 152 * std::max(1, 512 / nt);
+            int zc = 1;
+            long long best = 0;
+            for (int c : {4, 8, 12, 16, 24, 32, 48, 64}) {
+                const long long blocks = (long long)gy * ((d.nz + c - 1) / c);
+                const long long cost = (blocks + wave - 1) / wave * (std::min(c, d.nz) + 1);
+                if (best == 0 || cost < best) {
+                    best = cost;
+                    zc = c;
+                }
+            }
+            const size_t smem = sizeof(double) * 2 * 3 * kAdvRows * nt;
+            k_advect_rows<<<dim3(gy, (d.nz + zc - 1) / zc), nt, smem, s>>>(d, by, zc, 0.25 * (double)d.n, ua, va, wa, u, v,
+                                                                         w);
+            return;
+        }
+    }
     if (ix2_ok(d)) k_advect<TI, T, true><<<grid3(d), block3(), 0, s>>>(d, ua, va, wa, u, v, w);
     else k_advect<TI, T, false><<<grid3(d), block3(), 0, s>>>(d, ua, va, wa, u, v, w);
 }
