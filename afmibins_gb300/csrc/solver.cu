@@ -40,6 +40,9 @@ struct afmib_solver {
     cudaStream_t st = nullptr;
     bool own_stream = false;
     std::vector<void*> allocs;
+    bool creating = false;  // dalloc cuts small buffers from the arena
+    char* arena = nullptr;
+    size_t arena_left = 0;
     std::string err;
     afmib_stats stats{};
 
@@ -269,6 +272,8 @@ struct afmib_solver {
 
 namespace {
 
+constexpr size_t kArenaMost = 64 << 10, kArenaChunk = 1 << 20;
+
 #define CK(call)                                                                              \
     do {                                                                                      \
         cudaError_t e_ = (call);                                                              \
@@ -287,10 +292,26 @@ namespace {
         if (rc_ != AFMIB_OK) return rc_; \
     } while (0)
 
+// Device memory freed with the solver. While it is created, small buffers are
+// cut from chunks: each cudaMalloc takes about 10 us, and there are dozens.
 template <typename T>
 int dalloc(afmib_solver* s, T** p, size_t count) {
     void* q = nullptr;
-    CK(cudaMalloc(&q, (count > 0 ? count : 1) * sizeof(T)));
+    const size_t bytes = (count > 0 ? count : 1) * sizeof(T);
+    if (s->creating && bytes <= kArenaMost) {
+        const size_t need = (bytes + 255) & ~(size_t)255;
+        if (s->arena_left < need) {
+            CK(cudaMalloc(&q, kArenaChunk));
+            s->allocs.push_back(q);
+            s->arena = (char*)q;
+            s->arena_left = kArenaChunk;
+        }
+        *p = (T*)s->arena;
+        s->arena += need;
+        s->arena_left -= need;
+        return AFMIB_OK;
+    }
+    CK(cudaMalloc(&q, bytes));
     s->allocs.push_back(q);
     *p = (T*)q;
     return AFMIB_OK;
@@ -335,6 +356,65 @@ int copy_out(afmib_solver* s, double* dst, const double* src, long long n) {
     if (dst) CK(cudaMemcpyAsync(dst, src, n * sizeof(double), cudaMemcpyDefault, s->st));
     return AFMIB_OK;
 }
+
+// The caller's buffers of a single-operator call: the kernels read and write
+// them in place where they are memory of this device, aligned, and no output
+// overlaps another buffer of the call (then the copies that every other pointer
+// needs would be most of the call: 12 of them for a spread and an
+// interpolation, 500 MB each way at 256^3); host, managed and other devices'
+// memory goes through the solver's own buffers.
+struct CallBufs {
+    afmib_solver* s;
+    struct Range { uintptr_t a, b; bool out; };
+    std::vector<Range> all;
+    std::vector<std::pair<double*, std::pair<const double*, long long>>> back;  // copies to make at the end
+
+    explicit CallBufs(afmib_solver* s_) : s(s_) {}
+    // every buffer first, so that in() and out() know the overlaps
+    void reads(const void* p, long long n) { if (p) all.push_back({(uintptr_t)p, (uintptr_t)p + n * sizeof(double), false}); }
+    void writes(const void* p, long long n) { if (p) all.push_back({(uintptr_t)p, (uintptr_t)p + n * sizeof(double), true}); }
+    bool direct(const void* p, long long n, bool out) const {
+        const uintptr_t a = (uintptr_t)p, b = a + n * sizeof(double);
+        if (a % sizeof(double)) return false;
+        int self = 0;
+        for (const Range& r : all)
+            if (r.a < b && a < r.b) {
+                if (r.a == a && r.b == b && r.out == out && self++ == 0) continue;  // the buffer itself
+                if (out || r.out) return false;
+            }
+        cudaPointerAttributes at{};
+        if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        int dev = -1;
+        return at.type == cudaMemoryTypeDevice && cudaGetDevice(&dev) == cudaSuccess && at.device == dev;
+    }
+    // p itself, or its values in own
+    int in(const double* p, long long n, double* own, const double** use) {
+        if (direct(p, n, false)) {
+            *use = p;
+            return AFMIB_OK;
+        }
+        CK(cudaMemcpyAsync(own, p, n * sizeof(double), cudaMemcpyDefault, s->st));
+        *use = own;
+        return AFMIB_OK;
+    }
+    // p itself, or own, copied to p by finish()
+    void out(double* p, long long n, double* own, double** use) {
+        if (direct(p, n, true)) {
+            *use = p;
+            return;
+        }
+        *use = own;
+        back.push_back({p, {own, n}});
+    }
+    int finish() {
+        for (const auto& c : back)
+            CK(cudaMemcpyAsync(c.first, c.second.first, c.second.second * sizeof(double), cudaMemcpyDefault, s->st));
+        return AFMIB_OK;
+    }
+};
 
 void prof_flush(afmib_solver* s);
 
@@ -1943,6 +2023,8 @@ int setup_basis(afmib_solver* s) {
     const int ext[3] = {d.nx, flat ? 1 : d.ny, flat ? d.ny : d.nz};
     if (std::max(ext[0], std::max(ext[1], ext[2])) > kMaxBasis || d.ncell() > kTailCells) return AFMIB_OK;
     const double pi = std::acos(-1.0);
+    std::vector<double> all;  // per axis: eigenvectors, eigenvalues
+    size_t off[3];
     const double **v[3] = {&s->basis.vx, &s->basis.vy, &s->basis.vz}, **lam[3] = {&s->basis.lx, &s->basis.ly, &s->basis.lz};
     for (int a = 0; a < 3; ++a) {
         const int n = ext[a];
@@ -1958,19 +2040,25 @@ int setup_basis(afmib_solver* s) {
                 V[(size_t)k * n + i] = (sine ? std::sin(t) : std::cos(t)) * std::sqrt((flat_mode ? 1.0 : 2.0) / n);
             }
         }
-        double *dv = nullptr, *de = nullptr;
-        TRY(dalloc(s, &dv, V.size()));
-        TRY(dalloc(s, &de, E.size()));
-        CK(cudaMemcpy(dv, V.data(), V.size() * sizeof(double), cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(de, E.data(), E.size() * sizeof(double), cudaMemcpyHostToDevice));
-        *v[a] = dv;
-        *lam[a] = de;
+        off[a] = all.size();
+        all.insert(all.end(), V.begin(), V.end());
+        all.insert(all.end(), E.begin(), E.end());
+    }
+    double* dev = nullptr;
+    TRY(dalloc(s, &dev, all.size()));
+    CK(cudaMemcpyAsync(dev, all.data(), all.size() * sizeof(double), cudaMemcpyHostToDevice, s->st));
+    CK(cudaStreamSynchronize(s->st));  // the host copy goes
+    for (int a = 0; a < 3; ++a) {
+        *v[a] = dev + off[a];
+        *lam[a] = dev + off[a] + (size_t)ext[a] * ext[a];
     }
     return AFMIB_OK;
 }
 
 int create(afmib_solver* s, const afmib_config* c, void* stream) {
     s->cfg = *c;
+    s->creating = true;
+    struct Created { afmib_solver* s; ~Created() { s->creating = false; } } created{s};
     afmib_config& g = s->cfg;
     mg_kernel_attributes();  // before any capture of the V-cycles
     vcycle_tail_attributes();
@@ -2072,14 +2160,16 @@ int create(afmib_solver* s, const afmib_config* c, void* stream) {
         TRY(dalloc(s, &s->cg_q[c], N));
     }
     TRY(dalloc(s, &s->cgs, 3 * kCgScalars));
-    CK(cudaMallocHost((void**)&s->hcg, 2 * 3 * kCgScalars * sizeof(double)));
     for (auto& e : s->ev_cg) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     TRY(dalloc(s, &s->red.partial, (size_t)kMaxRedBlocks * kMaxRedVals));
     TRY(dalloc(s, &s->red.ticket, kMaxRedVals));
     TRY(dalloc(s, &s->scal, 24));
     TRY(dalloc(s, &s->dflag, 4));
-    CK(cudaMallocHost((void**)&s->hscal, 24 * sizeof(double)));
-    CK(cudaMallocHost((void**)&s->hflag, 4 * sizeof(int)));
+    // one pinned block (an allocation takes about 100 us): scalars, the CG's scalars, flags
+    constexpr int kHostScal = 24, kHostCg = 2 * 3 * kCgScalars;
+    CK(cudaMallocHost((void**)&s->hscal, (kHostScal + kHostCg) * sizeof(double) + 4 * sizeof(int)));
+    s->hcg = s->hscal + kHostScal;
+    s->hflag = (int*)(s->hcg + kHostCg);
     CK(cudaMemsetAsync(s->red.ticket, 0, kMaxRedVals * sizeof(unsigned), s->st));
     CK(cudaMemsetAsync(s->dflag, 0, 4 * sizeof(int), s->st));
     CK(cudaMemsetAsync(s->walls, 0, 4 * s->nxz() * sizeof(double), s->st));
@@ -2277,8 +2367,6 @@ int afmib_destroy(afmib_solver* s) {
     for (auto& p : s->prof_pend) { cudaEventDestroy(p.a); cudaEventDestroy(p.b); }
     for (auto e : s->prof_pool) cudaEventDestroy(e);
     if (s->hscal) cudaFreeHost(s->hscal);
-    if (s->hflag) cudaFreeHost(s->hflag);
-    if (s->hcg) cudaFreeHost(s->hcg);
     for (auto e : s->ev_cg)
         if (e) cudaEventDestroy(e);
     for (cudaStream_t q : {s->aux, s->hi})
@@ -2342,9 +2430,13 @@ int afmib_get_velocity(afmib_solver* s, double* u, double* v, double* w) {
 
 int afmib_get_pressure(afmib_solver* s, double* p) {
     if (!s || !p) return AFMIB_ERR_ARG;
-    launch_helm_apply<double>(s->d, 0, s->s_minus(), s->tmp[0], s->lv[0].x, s->st);
+    CallBufs cb(s);
+    cb.writes(p, s->N());
+    double* y;
+    cb.out(p, s->N(), s->tmp[0], &y);
+    launch_helm_apply<double>(s->d, 0, s->s_minus(), y, s->lv[0].x, s->st);
     CKL();
-    TRY(copy_out(s, p, s->tmp[0], s->N()));
+    TRY(cb.finish());
     return sync(s);
 }
 
@@ -2592,27 +2684,46 @@ int afmib_div(afmib_solver* s, double* dout, const double* u, const double* v, c
               const double* bottom) {
     if (!s || !dout || !u || !v || !w) return AFMIB_ERR_ARG;
     const long long N = s->N(), nxz = s->nxz();
-    TRY(copy_in(s, s->tmp[0], u, N));
-    TRY(v_in(s, s->tmp[1], v));
-    TRY(copy_in(s, s->tmp[2], w, N));
-    TRY(copy_in(s, s->adv[0], top, nxz));
-    TRY(copy_in(s, s->adv[1], bottom, nxz));
-    launch_div<double>(s->d, s->divb, s->tmp[0], s->tmp[1], s->tmp[2], s->adv[0], s->adv[1], s->st);
+    CallBufs cb(s);
+    cb.writes(dout, N);
+    cb.reads(u, N);
+    cb.reads(v, s->nv_user());
+    cb.reads(w, N);
+    cb.reads(top, nxz);
+    cb.reads(bottom, nxz);
+    const double *pu, *pv = s->tmp[1], *pw, *pt = nullptr, *pb = nullptr;
+    double* pd;
+    TRY(cb.in(u, N, s->tmp[0], &pu));
+    if (s->d.channel) TRY(v_in(s, s->tmp[1], v));  // gains its wall plane
+    else TRY(cb.in(v, N, s->tmp[1], &pv));
+    TRY(cb.in(w, N, s->tmp[2], &pw));
+    if (top) TRY(cb.in(top, nxz, s->adv[0], &pt));
+    if (bottom) TRY(cb.in(bottom, nxz, s->adv[1], &pb));
+    cb.out(dout, N, s->divb, &pd);
+    launch_div<double>(s->d, pd, pu, pv, pw, pt, pb, s->st);
     CKL();
-    TRY(copy_out(s, dout, s->divb, N));
+    TRY(cb.finish());
     return sync(s);
 }
 
 int afmib_grad(afmib_solver* s, double* px, double* py, double* pz, const double* p) {
     if (!s || !px || !py || !pz || !p) return AFMIB_ERR_ARG;
     const long long N = s->N();
-    TRY(copy_in(s, s->divb, p, N));
-    CK(cudaMemsetAsync(s->tmp[1], 0, N * sizeof(double), s->st));
-    launch_grad<double>(s->d, s->tmp[0], s->tmp[1], s->tmp[2], s->divb, s->st);
+    CallBufs cb(s);
+    cb.writes(px, N);
+    cb.writes(py, s->nv_user());
+    cb.writes(pz, N);
+    cb.reads(p, N);
+    const double* in;
+    double *gx, *gy = s->tmp[1], *gz;
+    TRY(cb.in(p, N, s->divb, &in));
+    cb.out(px, N, s->tmp[0], &gx);
+    if (!s->d.channel) cb.out(py, N, s->tmp[1], &gy);
+    cb.out(pz, N, s->tmp[2], &gz);
+    launch_grad<double>(s->d, gx, gy, gz, in, s->st);
     CKL();
-    TRY(copy_out(s, px, s->tmp[0], N));
-    TRY(v_out(s, py, s->tmp[1]));
-    TRY(copy_out(s, pz, s->tmp[2], N));
+    if (s->d.channel) TRY(v_out(s, py, s->tmp[1]));  // loses its wall plane
+    TRY(cb.finish());
     return sync(s);
 }
 
@@ -2620,14 +2731,26 @@ int afmib_advection(afmib_solver* s, double* ua, double* va, double* wa, const d
                     const double* w) {
     if (!s || !ua || !va || !wa || !u || !v || !w) return AFMIB_ERR_ARG;
     const long long N = s->N();
-    TRY(copy_in(s, s->tmp[0], u, N));
-    TRY(v_in(s, s->tmp[1], v));
-    TRY(copy_in(s, s->tmp[2], w, N));
-    launch_advect<double, double>(s->d, s->rhs[0], s->rhs[1], s->rhs[2], s->tmp[0], s->tmp[1], s->tmp[2], s->st);
+    CallBufs cb(s);
+    cb.writes(ua, N);
+    cb.writes(va, s->nv_user());
+    cb.writes(wa, N);
+    cb.reads(u, N);
+    cb.reads(v, s->nv_user());
+    cb.reads(w, N);
+    const double *pu, *pv = s->tmp[1], *pw;
+    double *au, *av = s->rhs[1], *aw;
+    TRY(cb.in(u, N, s->tmp[0], &pu));
+    if (s->d.channel) TRY(v_in(s, s->tmp[1], v));
+    else TRY(cb.in(v, N, s->tmp[1], &pv));
+    TRY(cb.in(w, N, s->tmp[2], &pw));
+    cb.out(ua, N, s->rhs[0], &au);
+    if (!s->d.channel) cb.out(va, N, s->rhs[1], &av);
+    cb.out(wa, N, s->rhs[2], &aw);
+    launch_advect<double, double>(s->d, au, av, aw, pu, pv, pw, s->st);
     CKL();
-    TRY(copy_out(s, ua, s->rhs[0], N));
-    TRY(v_out(s, va, s->rhs[1]));
-    TRY(copy_out(s, wa, s->rhs[2], N));
+    if (s->d.channel) TRY(v_out(s, va, s->rhs[1]));
+    TRY(cb.finish());
     return sync(s);
 }
 
@@ -2642,36 +2765,59 @@ int afmib_mg_solve(afmib_solver* s, double* rhs, int* cycles) {
 
 int afmib_lap_apply(afmib_solver* s, double* y, const double* x) {
     if (!s || !y || !x) return AFMIB_ERR_ARG;
-    TRY(copy_in(s, s->tmp[0], x, s->N()));
-    launch_lap_apply<double>(s->d, s->tmp[1], s->tmp[0], s->st);
+    CallBufs cb(s);
+    cb.writes(y, s->N());
+    cb.reads(x, s->N());
+    const double* in;
+    double* out;
+    TRY(cb.in(x, s->N(), s->tmp[0], &in));
+    cb.out(y, s->N(), s->tmp[1], &out);
+    launch_lap_apply<double>(s->d, out, in, s->st);
     CKL();
-    TRY(copy_out(s, y, s->tmp[1], s->N()));
+    TRY(cb.finish());
     return sync(s);
 }
 
 int afmib_helm_apply(afmib_solver* s, int comp, double scale, double* y, const double* x) {
     if (!s || !y || !x || comp < 0 || comp > 2) return AFMIB_ERR_ARG;
-    if (comp == 1) TRY(v_in(s, s->tmp[0], x));
-    else TRY(copy_in(s, s->tmp[0], x, s->N()));
-    launch_helm_apply<double>(s->d, comp, scale, s->tmp[1], s->tmp[0], s->st);
+    const bool wall = s->d.channel && comp == 1;  // v goes through its padded layout
+    CallBufs cb(s);
+    cb.writes(y, s->N());
+    cb.reads(x, s->N());
+    const double* in = s->tmp[0];
+    double* out = s->tmp[1];
+    if (wall) {
+        TRY(v_in(s, s->tmp[0], x));
+    } else {
+        TRY(cb.in(x, s->N(), s->tmp[0], &in));
+        cb.out(y, s->N(), s->tmp[1], &out);
+    }
+    launch_helm_apply<double>(s->d, comp, scale, out, in, s->st);
     CKL();
-    if (comp == 1) TRY(v_out(s, y, s->tmp[1]));
-    else TRY(copy_out(s, y, s->tmp[1], s->N()));
+    if (wall) TRY(v_out(s, y, s->tmp[1]));
+    TRY(cb.finish());
     return sync(s);
 }
 
 int afmib_helmholtz_cg(afmib_solver* s, int comp, double scale, double* x, const double* b, int* iters) {
     if (!s || !x || !b || comp < 0 || comp > 2) return AFMIB_ERR_ARG;
-    if (comp == 1) {
+    const bool wall = s->d.channel && comp == 1;
+    CallBufs cb(s);
+    cb.writes(x, s->N());
+    cb.reads(b, s->N());
+    double* px = s->tmp[0];
+    const double* pb = s->tmp[1];
+    if (wall) {
         TRY(v_in(s, s->tmp[0], x));
         TRY(v_in(s, s->tmp[1], b));
     } else {
-        TRY(copy_in(s, s->tmp[0], x, s->N()));
-        TRY(copy_in(s, s->tmp[1], b, s->N()));
+        cb.out(x, s->N(), s->tmp[0], &px);
+        if (px != x) TRY(copy_in(s, px, x, s->N()));
+        TRY(cb.in(b, s->N(), s->tmp[1], &pb));
     }
-    const int rc = cg_solve_batch(s, 1, &comp, scale, &s->tmp[0], &s->tmp[1], iters);
-    if (comp == 1) TRY(v_out(s, x, s->tmp[0]));
-    else TRY(copy_out(s, x, s->tmp[0], s->N()));
+    const int rc = cg_solve_batch(s, 1, &comp, scale, &px, &pb, iters);
+    if (wall) TRY(v_out(s, x, s->tmp[0]));
+    TRY(cb.finish());
     TRY(sync(s));
     return rc;
 }
@@ -2681,10 +2827,16 @@ int afmib_restrict(afmib_solver* s, double* coarse, const double* fine) {
     const Dims& d = s->d;
     if (!is_even(d.nx) || !is_even(d.ny) || !(d.nz == 1 || is_even(d.nz))) return s->fail(AFMIB_ERR_ARG, "odd extent");
     const long long nc = s->N() / (d.nz == 1 ? 4 : 8);
-    TRY(copy_in(s, s->tmp[0], fine, s->N()));
-    launch_restrict<double>(d, s->tmp[1], s->tmp[0], s->st);
+    CallBufs cb(s);
+    cb.writes(coarse, nc);
+    cb.reads(fine, s->N());
+    const double* in;
+    double* out;
+    TRY(cb.in(fine, s->N(), s->tmp[0], &in));
+    cb.out(coarse, nc, s->tmp[1], &out);
+    launch_restrict<double>(d, out, in, s->st);
     CKL();
-    TRY(copy_out(s, coarse, s->tmp[1], nc));
+    TRY(cb.finish());
     return sync(s);
 }
 
@@ -2692,10 +2844,17 @@ int afmib_prolong(afmib_solver* s, double* fine, const double* coarse) {
     if (!s || !coarse || !fine) return AFMIB_ERR_ARG;
     const Dims& d = s->d;
     if (!is_even(d.nx) || !is_even(d.ny) || !(d.nz == 1 || is_even(d.nz))) return s->fail(AFMIB_ERR_ARG, "odd extent");
-    TRY(copy_in(s, s->tmp[0], coarse, s->N() / (d.nz == 1 ? 4 : 8)));
-    launch_prolong_assign<double>(d, s->tmp[1], s->tmp[0], s->st);
+    const long long nc = s->N() / (d.nz == 1 ? 4 : 8);
+    CallBufs cb(s);
+    cb.writes(fine, s->N());
+    cb.reads(coarse, nc);
+    const double* in;
+    double* out;
+    TRY(cb.in(coarse, nc, s->tmp[0], &in));
+    cb.out(fine, s->N(), s->tmp[1], &out);
+    launch_prolong_assign<double>(d, out, in, s->st);
     CKL();
-    TRY(copy_out(s, fine, s->tmp[1], s->N()));
+    TRY(cb.finish());
     return sync(s);
 }
 
@@ -2706,17 +2865,29 @@ int afmib_spread(afmib_solver* s, int M, const double* X, const double* F, const
     const int keepM = s->M;
     TRY(marker_alloc(s, M, 0));
     s->M = M;
-    TRY(copy_in(s, s->Xh, X, 3 * (long long)M));
-    TRY(copy_in(s, s->G, F, 3 * (long long)M));
-    if (vol) TRY(copy_in(s, s->U1, vol, M));
+    const long long N = s->N(), m3 = 3 * (long long)M;
+    CallBufs cb(s);
+    cb.reads(X, m3);
+    cb.reads(F, m3);
+    cb.reads(vol, M);
+    cb.writes(fx, N);
+    cb.writes(fy, s->nv_user());
+    cb.writes(fz, N);
+    const double *pX, *pF, *pV = nullptr;
+    double *ox, *oy = s->tmp[1], *oz;
+    TRY(cb.in(X, m3, s->Xh, &pX));
+    TRY(cb.in(F, m3, s->G, &pF));
+    if (vol) TRY(cb.in(vol, M, s->U1, &pV));
+    cb.out(fx, N, s->tmp[0], &ox);
+    if (!s->d.channel) cb.out(fy, N, s->tmp[1], &oy);
+    cb.out(fz, N, s->tmp[2], &oz);
     CK(cudaMemsetAsync(s->dflag, 0, sizeof(int), s->st));
-    TRY(bin_markers(s, s->Xh));
-    TRY(spread_forces(s, vol ? s->U1 : nullptr, s->tmp[0], s->tmp[1], s->tmp[2]));
+    TRY(bin_markers(s, pX));
+    TRY(spread_generic(s, pF, pV, spread_scale(s->d), ox, oy, oz));
     int rc = check_marker_flag(s);
     s->M = keepM;
-    TRY(copy_out(s, fx, s->tmp[0], s->N()));
-    TRY(v_out(s, fy, s->tmp[1]));
-    TRY(copy_out(s, fz, s->tmp[2], s->N()));
+    if (s->d.channel) TRY(v_out(s, fy, s->tmp[1]));
+    TRY(cb.finish());
     TRY(sync(s));
     return rc;
 }
@@ -2728,17 +2899,28 @@ int afmib_interp(afmib_solver* s, int M, const double* X, const double* u, const
     const int keepM = s->M;
     TRY(marker_alloc(s, M, 0));
     s->M = M;
-    TRY(copy_in(s, s->Xh, X, 3 * (long long)M));
-    TRY(copy_in(s, s->tmp[0], u, s->N()));
-    TRY(v_in(s, s->tmp[1], v));
-    TRY(copy_in(s, s->tmp[2], w, s->N()));
+    const long long N = s->N(), m3 = 3 * (long long)M;
+    CallBufs cb(s);
+    cb.reads(X, m3);
+    cb.reads(u, N);
+    cb.reads(v, s->nv_user());
+    cb.reads(w, N);
+    cb.writes(U, m3);
+    const double *pX, *pu, *pv = s->tmp[1], *pw;
+    double* pU;
+    TRY(cb.in(X, m3, s->Xh, &pX));
+    TRY(cb.in(u, N, s->tmp[0], &pu));
+    if (s->d.channel) TRY(v_in(s, s->tmp[1], v));
+    else TRY(cb.in(v, N, s->tmp[1], &pv));
+    TRY(cb.in(w, N, s->tmp[2], &pw));
+    cb.out(U, m3, s->U2, &pU);
     CK(cudaMemsetAsync(s->dflag, 0, sizeof(int), s->st));
-    TRY(bin_markers(s, s->Xh));
-    TRY(interp_markers(s, s->tmp[0], s->tmp[1], s->tmp[2], s->U2));
+    TRY(bin_markers(s, pX));
+    TRY(interp_markers(s, pu, pv, pw, pU));
     CKL();
     int rc = check_marker_flag(s);
     s->M = keepM;
-    TRY(copy_out(s, U, s->U2, 3 * (long long)M));
+    TRY(cb.finish());
     TRY(sync(s));
     return rc;
 }
