@@ -64,7 +64,38 @@ struct Ix2 {
     __device__ __forceinline__ int yp(int y) const { return (y + 1) & my; }
     __device__ __forceinline__ int zm(int z) const { return (z - 1) & mz; }
     __device__ __forceinline__ int zp(int z) const { return (z + 1) & mz; }
+    __device__ __forceinline__ int wz(int z) const { return z & mz; }  // -nz <= z < 2 nz
+    __device__ __forceinline__ int coarse(int x, int y, int z) const { return x | (y << (lx - 1)) | (z << (lxy - 2)); }
 };
+// The same for any extents below 2^31 cells (a solver holds more than 20 arrays of
+// doubles: 2^31 cells would take over 340 GB): 32-bit products, conditional wraps.
+struct IxG {
+    int nx, ny, nz;
+    __host__ __device__ __forceinline__ explicit IxG(const Dims& d) : nx(d.nx), ny(d.ny), nz(d.nz) {}
+    __device__ __forceinline__ int at(int x, int y, int z) const { return x + nx * (y + ny * z); }
+    __device__ __forceinline__ int xm(int x) const { return x == 0 ? nx - 1 : x - 1; }
+    __device__ __forceinline__ int xp(int x) const { return x == nx - 1 ? 0 : x + 1; }
+    __device__ __forceinline__ int ym(int y) const { return y == 0 ? ny - 1 : y - 1; }
+    __device__ __forceinline__ int yp(int y) const { return y == ny - 1 ? 0 : y + 1; }
+    __device__ __forceinline__ int zm(int z) const { return z == 0 ? nz - 1 : z - 1; }
+    __device__ __forceinline__ int zp(int z) const { return z == nz - 1 ? 0 : z + 1; }
+    __device__ __forceinline__ int wz(int z) const { return z < 0 ? z + nz : (z >= nz ? z - nz : z); }
+    __device__ __forceinline__ int coarse(int x, int y, int z) const {
+        return x + (nx >> 1) * (y + (ny >> 1) * z);
+    }
+};
+// One launch with the index type of the grid
+#define AFMIB_IX(d, ...)                         \
+    do {                                         \
+        if (ix2_ok(d)) {                         \
+            typedef Ix2 IX;                      \
+            __VA_ARGS__;                         \
+        } else {                                 \
+            typedef IxG IX;                      \
+            __VA_ARGS__;                         \
+        }                                        \
+    } while (0)
+
 // Block coordinates, walked from the grid's far end when rev. Blocks are
 // dispatched roughly in index order, so a pass over a field larger than L2
 // that runs opposite to the pass before it starts on the rows that pass
@@ -75,8 +106,8 @@ __device__ __forceinline__ uint3 block_at(int rev) {
                : blockIdx;
 }
 
-// Power-of-two kernels apply; AFMIB_IX2=0 keeps the general kernels (read at
-// every launch, so a test can compare both in one process).
+// Power-of-two index arithmetic applies; AFMIB_IX2=0 keeps the general one (read
+// at every launch, so a test can compare both in one process).
 inline bool ix2_ok(const Dims& d) {
     auto p2 = [](int v) { return v > 0 && (v & (v - 1)) == 0; };
     if (const char* e = std::getenv("AFMIB_IX2"))

@@ -147,8 +147,9 @@ template <typename T>
 void launch_helm_jacobi(const Dims& d, int comp, double scale, const T* x, T* xo, const T* b, cudaStream_t s,
                         int rev = 0);
 // One colour of a red-black Gauss-Seidel sweep of (I + scale*Delta) x = b in
-// place (init: from x = 0). Power-of-two extents, nz a multiple of 8;
-// returns false (nothing launched) otherwise.
+// place (init: from x = 0), on the grids of helm_rbgs_ok; returns false (nothing
+// launched) otherwise.
+bool helm_rbgs_ok(const Dims& d);
 template <typename T>
 bool launch_helm_rbgs(const Dims& d, int comp, double scale, int color, int init, T* x, const T* b, cudaStream_t s,
                       int rev = 0);

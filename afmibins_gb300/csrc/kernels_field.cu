@@ -1116,9 +1116,9 @@ __global__ void __launch_bounds__(kRedBlock) k_helm_defect_bfp(Dims d, int comp,
 // diagonal (1 - 6 off in the interior, 1 - 4 off in 2D, 1 - 8 off on the
 // channel u/w wall rows, 1 on the channel v wall plane). x == nullptr starts
 // from zero: x' = b / diag.
-// helm_point_at with Ix2 indexing (power-of-two extents): same terms, same order
-template <typename T>
-__device__ __forceinline__ T helm_point2(const Dims& d, const Ix2& I, int comp, const HelmK<T>& k,
+// helm_point_at with Ix2 or IxG indexing: same terms, same order
+template <typename T, typename IX>
+__device__ __forceinline__ T helm_point2(const Dims& d, const IX& I, int comp, const HelmK<T>& k,
                                          const T* __restrict__ x, int xi, int yi, int zi) {
     const T x0 = x[I.at(xi, yi, zi)];
     const T sx = x[I.at(I.xm(xi), yi, zi)] + x[I.at(I.xp(xi), yi, zi)];
@@ -1145,29 +1145,6 @@ __device__ __forceinline__ T helm_rdiag(const Dims& d, int comp, const HelmK<T>&
         if (comp == 1 && y == 0) return T(1);
     }
     return k.rdiag;
-}
-
-// ZU cells along z per thread, all computed before any is stored (the
-// sweep is out of place, so this only puts ZU cells' loads in flight at once)
-template <typename T, int ZU>
-__global__ void k_helm_jacobi(Dims d, int comp, HelmK<T> k, const T* __restrict__ xv, T* __restrict__ xo,
-                              const T* __restrict__ b) {
-    const int x = blockIdx.x * BX + threadIdx.x, y = blockIdx.y * BY + threadIdx.y, z0 = blockIdx.z * ZU;
-    if (x >= d.nx || y >= d.ny) return;
-    const T rdiag = helm_rdiag(d, comp, k, y);
-    T val[ZU];
-#pragma unroll
-    for (int u = 0; u < ZU; ++u) {
-        const long long i = lin(d, x, y, z0 + u);
-        if (!xv) {
-            val[u] = b[i] * rdiag;
-        } else {
-            const T hx = helm_point_at(d, comp, k, [xv](long long j) { return xv[j]; }, x, y, z0 + u);
-            val[u] = xv[i] + (b[i] - hx) * rdiag;
-        }
-    }
-#pragma unroll
-    for (int u = 0; u < ZU; ++u) xo[lin(d, x, y, z0 + u)] = val[u];
 }
 
 // CG started from zero: r = p = b, n0 = b.b
@@ -1490,17 +1467,17 @@ __global__ void __launch_bounds__(kRedBlock) k_helm_update_df(Dims d, int comp, 
     grid_sum<1>(a, sc, out);
 }
 
-// The same for power-of-two grids with nz % ZU == 0: each thread takes ZU
+// The same for 3D grids with nz % ZU == 0: each thread takes ZU
 // consecutive z cells of one (x, y) column (the column's e values reused from
-// registers, 32-bit shift-composed indices, every load of the batch issued
+// registers, 32-bit indices, every load of the batch issued
 // before the rows are evaluated), blocks walk z batches in steps of grid.z;
 // the same arithmetic per cell, so the same bits.
-template <int ZU, int MINB>
+template <int ZU, int MINB, typename IX>
 __global__ void __launch_bounds__(kRedBlock, MINB) k_helm_update_df2(Dims d, int comp, df2 off, df2 cxa,
                                                               double* __restrict__ x, const float* __restrict__ e,
                                                               float* __restrict__ rh, float* __restrict__ rl,
                                                               RedScratch sc, double* out) {
-    const Ix2 I(d);
+    const IX I(d);
     float acc = 0.f;
     const int xi = blockIdx.x * kRBX + threadIdx.x, yi = blockIdx.y * kRBY + threadIdx.y;
     const bool vwall = d.channel && comp == 1 && yi == 0;
@@ -1514,7 +1491,7 @@ __global__ void __launch_bounds__(kRedBlock, MINB) k_helm_update_df2(Dims d, int
             float col[ZU + 2], ex0[ZU], ex1[ZU], ey0[ZU], ey1[ZU], h[ZU], l[ZU];
             double xv[ZU];
 #pragma unroll
-            for (int u = 0; u < ZU + 2; ++u) col[u] = e[I.at(xi, yi, (z0 + u - 1) & I.mz)];  // z0 - 1 .. z0 + ZU
+            for (int u = 0; u < ZU + 2; ++u) col[u] = e[I.at(xi, yi, I.wz(z0 + u - 1))];  // z0 - 1 .. z0 + ZU
 #pragma unroll
             for (int u = 0; u < ZU; ++u) {
                 const int z = z0 + u, i = I.at(xi, yi, z);
@@ -1553,7 +1530,7 @@ __global__ void __launch_bounds__(kRedBlock, MINB) k_helm_update_df2(Dims d, int
     grid_sum<1>(a, sc, out);
 }
 
-// AFMIB_UPDATE_DF_GENERIC=1: the general kernel on power-of-two grids too
+// AFMIB_UPDATE_DF_GENERIC=1: the one-cell kernel on every grid
 // (read at every launch, so that a test compares both in one process)
 static bool update_df_generic() {
     const char* e = std::getenv("AFMIB_UPDATE_DF_GENERIC");
@@ -1568,12 +1545,12 @@ void launch_helm_update_df(const Dims& d, int comp, double scale, double* x, con
     // and 45.5 for eight (more registers, fewer warps) and 45.5 for the
     // general kernel; registers capped for kUpdateMinBlocks resident blocks
     constexpr int ZU = 2;
-    if (d.nz > 1 && d.nz % ZU == 0 && ix2_ok(d) && !update_df_generic()) {
+    if (d.nz > 1 && d.nz % ZU == 0 && !update_df_generic()) {
         const int gx = (d.nx + kRBX - 1) / kRBX, gy = (d.ny + kRBY - 1) / kRBY;
         int gz = d.nz / ZU;
         if ((long long)gx * gy * gz > kMaxRedBlocks) gz = std::max(1, kMaxRedBlocks / (gx * gy));
-        k_helm_update_df2<ZU, kUpdateMinBlocks><<<dim3(gx, gy, gz), dim3(kRBX, kRBY), 0, s>>>(d, comp, o, c, x, e, rh,
-                                                                                             rl, sc, out);
+        AFMIB_IX(d, (k_helm_update_df2<ZU, kUpdateMinBlocks, IX><<<dim3(gx, gy, gz), dim3(kRBX, kRBY), 0, s>>>(
+                        d, comp, o, c, x, e, rh, rl, sc, out)));
         return;
     }
     k_helm_update_df<<<red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s>>>(d, comp, o, c, x, e, rh, rl, sc, out);
@@ -1641,10 +1618,10 @@ void launch_cgb_direction(const Dims& d, const CgBatch& g, const double* cgs, cu
     if (vec) k_cgb_direction<true><<<grid, kRedBlock, 0, s>>>(N, g, cgs);
     else k_cgb_direction<false><<<grid, kRedBlock, 0, s>>>(N, g, cgs);
 }
-template <typename T, int ZU>
+template <typename T, int ZU, typename IX>
 __global__ void k_helm_jacobi2(Dims d, int comp, HelmK<T> k, const T* __restrict__ xv, T* __restrict__ xo,
                                const T* __restrict__ b, int rev) {
-    const Ix2 I(d);
+    const IX I(d);
     const uint3 B = block_at(rev);
     const int x = B.x * BX + threadIdx.x, y = B.y * BY + threadIdx.y, z0 = B.z * ZU;
     if (x >= d.nx || y >= d.ny) return;
@@ -1665,10 +1642,10 @@ __global__ void k_helm_jacobi2(Dims d, int comp, HelmK<T> k, const T* __restrict
 // colour's cells take b / diag and the other colour's cells are zeroed. For
 // the 7-point operator under red-black ordering the sweep contracts the
 // error as the square of the Jacobi rate.
-template <typename T, int ZU>
+template <typename T, int ZU, typename IX>
 __device__ __forceinline__ void helm_rbgs2_body(Dims d, int comp, const HelmK<T>& k, int color, int init, T* __restrict__ xv,
                                                 const T* __restrict__ b, int rev) {
-    const Ix2 I(d);
+    const IX I(d);
     const uint3 B = block_at(rev);
     const int y = B.y * BY + threadIdx.y, t = B.x * BX + threadIdx.x, z0 = B.z * ZU;
     if (y >= d.ny || 2 * t >= d.nx) return;
@@ -1688,20 +1665,33 @@ __device__ __forceinline__ void helm_rbgs2_body(Dims d, int comp, const HelmK<T>
         if (init) xv[I.at(2 * t + ((y + z0 + u + color + 1) & 1), y, z0 + u)] = T(0);
     }
 }
-template <typename T, int ZU, int MINB>
+template <typename T, int ZU, int MINB, typename IX>
 __global__ void __launch_bounds__(BX * BY, MINB) k_helm_rbgs2b(Dims d, int comp, HelmK<T> k, int color, int init,
                                                               T* __restrict__ xv, const T* __restrict__ b, int rev) {
-    helm_rbgs2_body<T, ZU>(d, comp, k, color, init, xv, b, rev);
+    helm_rbgs2_body<T, ZU, IX>(d, comp, k, color, init, xv, b, rev);
 }
 
+// Red-black order needs every wrap to join the two colours: even extents in the
+// periodic directions (the channel's y has walls; 2D grids keep Jacobi sweeps).
+// On a 96x80x112 grid these sweeps with the interleaved double-float solves take
+// an IB step from 4.57 to 3.88 ms against Jacobi sweeps and FP64 defects, one
+// solve after another.
+bool helm_rbgs_ok(const Dims& d) {
+    return d.nz > 1 && d.nx % 2 == 0 && d.nz % 2 == 0 && (d.channel || d.ny % 2 == 0);
+}
 template <typename T>
 bool launch_helm_rbgs(const Dims& d, int comp, double scale, int color, int init, T* x, const T* b, cudaStream_t s,
                       int rev) {
-    if (!(d.nz % 8 == 0 && d.nx % 2 == 0 && ix2_ok(d))) return false;
-    const dim3 g((d.nx / 2 + BX - 1) / BX, (d.ny + BY - 1) / BY, d.nz / 8);
+    if (!helm_rbgs_ok(d)) return false;
+    const int gx = (d.nx / 2 + BX - 1) / BX, gy = (d.ny + BY - 1) / BY;
+    const dim3 blk(BX, BY);
+    const HelmK<T> k = helm_k<T>(d, scale);
     // registers capped for 6 resident blocks (40 against 48): measured with the
     // multigrid smoother's cap, 50.5 against 50.0 IB steps/s at 256^3
-    k_helm_rbgs2b<T, 8, 6><<<g, dim3(BX, BY), 0, s>>>(d, comp, helm_k<T>(d, scale), color, init, x, b, rev);
+    if (d.nz % 8 == 0)
+        AFMIB_IX(d, (k_helm_rbgs2b<T, 8, 6, IX><<<dim3(gx, gy, d.nz / 8), blk, 0, s>>>(d, comp, k, color, init, x, b, rev)));
+    else
+        AFMIB_IX(d, (k_helm_rbgs2b<T, 2, 6, IX><<<dim3(gx, gy, d.nz / 2), blk, 0, s>>>(d, comp, k, color, init, x, b, rev)));
     return true;
 }
 template bool launch_helm_rbgs<float>(const Dims&, int, double, int, int, float*, const float*, cudaStream_t, int);
@@ -1710,14 +1700,10 @@ template <typename T>
 void launch_helm_jacobi(const Dims& d, int comp, double scale, const T* x, T* xo, const T* b, cudaStream_t s,
                         int rev) {
     const dim3 blk(BX, BY);
-    if (d.nz % 8 == 0 && ix2_ok(d))
-        k_helm_jacobi2<T, 8><<<dim3((d.nx + BX - 1) / BX, (d.ny + BY - 1) / BY, d.nz / 8), blk, 0, s>>>(d, comp, helm_k<T>(d, scale),
-                                                                                                   x, xo, b, rev);
-    else if (d.nz % 8 == 0)
-        k_helm_jacobi<T, 8><<<dim3((d.nx + BX - 1) / BX, (d.ny + BY - 1) / BY, d.nz / 8), blk, 0, s>>>(d, comp, helm_k<T>(d, scale), x,
-                                                                                                  xo, b);
-    else
-        k_helm_jacobi<T, 1><<<grid3(d), blk, 0, s>>>(d, comp, helm_k<T>(d, scale), x, xo, b);
+    const HelmK<T> k = helm_k<T>(d, scale);
+    const dim3 g((d.nx + BX - 1) / BX, (d.ny + BY - 1) / BY, d.nz % 8 == 0 ? d.nz / 8 : d.nz);
+    if (d.nz % 8 == 0) AFMIB_IX(d, (k_helm_jacobi2<T, 8, IX><<<g, blk, 0, s>>>(d, comp, k, x, xo, b, rev)));
+    else AFMIB_IX(d, (k_helm_jacobi2<T, 1, IX><<<g, blk, 0, s>>>(d, comp, k, x, xo, b, rev)));
 }
 template void launch_helm_jacobi<float>(const Dims&, int, double, const float*, float*, const float*, cudaStream_t,
                                         int);

@@ -62,47 +62,64 @@ __device__ __forceinline__ void lap_row(const Dims& d, const T* x, int xi, int y
     }
 }
 
-template <typename T>
+// Neighbour sum and diagonal factor of lap_row with Ix2 or IxG indexing (same
+// terms, same order).
+template <typename T, typename IX>
+__device__ __forceinline__ void lap_row2(const Dims& d, const IX& I, const T* x, int xi, int yi, int zi,
+                                         T& S, int& c) {
+    if (d.nz == 1) {
+        S = x[I.at(I.xm(xi), yi, zi)] + x[I.at(I.xp(xi), yi, zi)];
+        c = 4;
+    } else {
+        S = (x[I.at(I.xm(xi), yi, zi)] + x[I.at(I.xp(xi), yi, zi)]) + (x[I.at(xi, yi, I.zm(zi))] + x[I.at(xi, yi, I.zp(zi))]);
+        c = 6;
+    }
+    if (d.channel) {
+        if (yi > 0) S += x[I.at(xi, yi - 1, zi)]; else --c;
+        if (yi < d.ny - 1) S += x[I.at(xi, yi + 1, zi)]; else --c;
+    } else {
+        S += x[I.at(xi, I.ym(yi), zi)] + x[I.at(xi, I.yp(yi), zi)];
+    }
+}
+
+template <typename T, typename IX>
 __global__ void k_lap(Dims d, LapK<T> k, T* __restrict__ out, const T* __restrict__ in) {
     const int x = blockIdx.x * BX + threadIdx.x, y = blockIdx.y * BY + threadIdx.y, z = blockIdx.z;
     if (x >= d.nx || y >= d.ny) return;
+    const IX I(d);
     T S;
     int c;
-    lap_row(d, in, x, y, z, S, c);
-    out[lin(d, x, y, z)] = k.off * (S - lap_count<T>(c) * in[lin(d, x, y, z)]);
+    lap_row2(d, I, in, x, y, z, S, c);
+    const int i = I.at(x, y, z);
+    out[i] = k.off * (S - lap_count<T>(c) * in[i]);
 }
 
-// r = b - L x at one cell
-template <typename T>
-__device__ __forceinline__ void residual_cell(const Dims& d, const LapK<T>& k, T* r, const T* xv, const T* b, int x,
-                                              int y, int z) {
-    T S;
-    int c;
-    lap_row(d, xv, x, y, z, S, c);
-    const long long i = lin(d, x, y, z);
-    r[i] = b[i] - k.off * (S - lap_count<T>(c) * xv[i]);
-}
-
-template <typename T>
+template <typename T, typename IX>
 __global__ void k_residual(Dims d, LapK<T> k, T* __restrict__ r, const T* __restrict__ xv, const T* __restrict__ b) {
     const int x = blockIdx.x * BX + threadIdx.x, y = blockIdx.y * BY + threadIdx.y, z = blockIdx.z;
     if (x >= d.nx || y >= d.ny) return;
-    residual_cell(d, k, r, xv, b, x, y, z);
+    const IX I(d);
+    T S;
+    int c;
+    lap_row2(d, I, xv, x, y, z, S, c);
+    const int i = I.at(x, y, z);
+    r[i] = b[i] - k.off * (S - lap_count<T>(c) * xv[i]);
 }
 
-template <typename T>
+template <typename T, typename IX>
 __global__ void __launch_bounds__(kRedBlock) k_residual_norm(Dims d, LapK<T> k, T* __restrict__ r,
                                                             const T* __restrict__ xv, const T* __restrict__ b,
                                                             RedScratch sc, double* out) {
     const int xi = blockIdx.x * kRBX + threadIdx.x, yi = blockIdx.y * kRBY + threadIdx.y;
+    const IX I(d);
     T acc = T(0);
     if (xi < d.nx && yi < d.ny)
 #pragma unroll 2
         for (int zi = blockIdx.z; zi < d.nz; zi += gridDim.z) {
             T S;
             int c;
-            lap_row(d, xv, xi, yi, zi, S, c);
-            const long long i = lin(d, xi, yi, zi);
+            lap_row2(d, I, xv, xi, yi, zi, S, c);
+            const int i = I.at(xi, yi, zi);
             const T ri = b[i] - k.off * (S - lap_count<T>(c) * xv[i]);
             r[i] = ri;
             acc += ri * ri;
@@ -230,14 +247,14 @@ __global__ void __launch_bounds__(kRedBlock) k_lap_update_df(Dims d, double* __r
     grid_sum<1>(a, sc, out);
 }
 
-// The same on power-of-two 3D grids, two z cells per thread with every load
+// The same on 3D grids with nz % ZU == 0, two z cells per thread with every load
 // of the pair issued first (as k_helm_update_df2); the same rows, so the
 // same bits.
-template <int ZU, int MINB>
+template <int ZU, int MINB, typename IX>
 __global__ void __launch_bounds__(kRedBlock, MINB) k_lap_update_df2(Dims d, double* __restrict__ x,
                                                              const float* __restrict__ e, float* __restrict__ rh,
                                                              float* __restrict__ rl, RedScratch sc, double* out) {
-    const Ix2 I(d);
+    const IX I(d);
     const int xi = blockIdx.x * kRBX + threadIdx.x, yi = blockIdx.y * kRBY + threadIdx.y;
     const float off = float(d.n) * float(d.n);
     const bool has_ym = !d.channel || yi > 0, has_yp = !d.channel || yi < d.ny - 1;
@@ -250,7 +267,7 @@ __global__ void __launch_bounds__(kRedBlock, MINB) k_lap_update_df2(Dims d, doub
             float col[ZU + 2], ex0[ZU], ex1[ZU], ey0[ZU], ey1[ZU], h[ZU], l[ZU];
             double xv[ZU];
 #pragma unroll
-            for (int u = 0; u < ZU + 2; ++u) col[u] = e[I.at(xi, yi, (z0 + u - 1) & I.mz)];  // z0 - 1 .. z0 + ZU
+            for (int u = 0; u < ZU + 2; ++u) col[u] = e[I.at(xi, yi, I.wz(z0 + u - 1))];  // z0 - 1 .. z0 + ZU
 #pragma unroll
             for (int u = 0; u < ZU; ++u) {
                 const int z = z0 + u, i = I.at(xi, yi, z);
@@ -322,26 +339,21 @@ __global__ void __launch_bounds__(kRedBlock) k_lap_defect_bfp(Dims d, int k2, fl
 }
 
 // One colour of red-black Gauss–Seidel: x_i = (b_i - n^2 S) / (-c n^2).
-template <typename T>
-__device__ __forceinline__ void rbgs_cell(const Dims& d, const LapK<T>& k, T* xv, const T* b, int x, int y, int z,
-                                          T omega) {
-    T S;
-    int c;
-    lap_row(d, xv, x, y, z, S, c);
-    const long long i = lin(d, x, y, z);
-    T v = (S - b[i] * k.inv) * lap_rcount<T>(c);
-    if (omega != T(1)) v = v + (omega - T(1)) * (v - xv[i]);
-    xv[i] = v;
-}
-
 // omega != 1: over-relaxed update x + omega (gs - x); omega == 1 is plain
 // Gauss-Seidel, bit for bit
-template <typename T>
+template <typename T, typename IX>
 __global__ void k_rbgs(Dims d, LapK<T> k, int color, T omega, T* __restrict__ xv, const T* __restrict__ b) {
     const int y = blockIdx.y * BY + threadIdx.y, z = blockIdx.z;
     const int x = 2 * (blockIdx.x * BX + threadIdx.x) + ((y + z + color) & 1);
     if (x >= d.nx || y >= d.ny) return;
-    rbgs_cell(d, k, xv, b, x, y, z, omega);
+    const IX I(d);
+    T S;
+    int c;
+    lap_row2(d, I, xv, x, y, z, S, c);
+    const int i = I.at(x, y, z);
+    T v = (S - b[i] * k.inv) * lap_rcount<T>(c);
+    if (omega != T(1)) v = v + (omega - T(1)) * (v - xv[i]);
+    xv[i] = v;
 }
 
 // Batched forms: each thread takes ZU cells along z of its (x, y) column and
@@ -353,55 +365,10 @@ __global__ void k_rbgs(Dims d, LapK<T> k, int color, T omega, T* __restrict__ xv
 constexpr int kZU = 8;  // z cells per thread of the batched stencil kernels
 constexpr int kZU32 = 4;  // ... of the FP32 red-black colour
 
-template <typename T, int ZU>
-__global__ void k_rbgs_z(Dims d, LapK<T> k, int color, T omega, T* __restrict__ xv, const T* __restrict__ b) {
-    const int y = blockIdx.y * BY + threadIdx.y, t = blockIdx.x * BX + threadIdx.x, z0 = blockIdx.z * ZU;
-    if (y >= d.ny) return;
-    T val[ZU];
-    long long at[ZU];
-#pragma unroll
-    for (int u = 0; u < ZU; ++u) {
-        const int z = z0 + u, x = 2 * t + ((y + z + color) & 1);
-        at[u] = -1;
-        if (x < d.nx) {
-            T S;
-            int c;
-            lap_row(d, xv, x, y, z, S, c);
-            const long long i = lin(d, x, y, z);
-            val[u] = (S - b[i] * k.inv) * lap_rcount<T>(c);
-            if (omega != T(1)) val[u] = val[u] + (omega - T(1)) * (val[u] - xv[i]);
-            at[u] = i;
-        }
-    }
-#pragma unroll
-    for (int u = 0; u < ZU; ++u)
-        if (at[u] >= 0) xv[at[u]] = val[u];
-}
-
-// Neighbour sum and diagonal factor of lap_row with Ix2 indexing (same terms,
-// same order).
-template <typename T>
-__device__ __forceinline__ void lap_row2(const Dims& d, const Ix2& I, const T* x, int xi, int yi, int zi,
-                                         T& S, int& c) {
-    if (d.nz == 1) {
-        S = x[I.at(I.xm(xi), yi, zi)] + x[I.at(I.xp(xi), yi, zi)];
-        c = 4;
-    } else {
-        S = (x[I.at(I.xm(xi), yi, zi)] + x[I.at(I.xp(xi), yi, zi)]) + (x[I.at(xi, yi, I.zm(zi))] + x[I.at(xi, yi, I.zp(zi))]);
-        c = 6;
-    }
-    if (d.channel) {
-        if (yi > 0) S += x[I.at(xi, yi - 1, zi)]; else --c;
-        if (yi < d.ny - 1) S += x[I.at(xi, yi + 1, zi)]; else --c;
-    } else {
-        S += x[I.at(xi, I.ym(yi), zi)] + x[I.at(xi, I.yp(yi), zi)];
-    }
-}
-
-template <typename T, int ZU>
+template <typename T, int ZU, typename IX>
 __device__ __forceinline__ void rbgs_z2_body(Dims d, const LapK<T>& k, int color, T omega, T* __restrict__ xv,
                                              const T* __restrict__ b, int rev) {
-    const Ix2 I(d);
+    const IX I(d);
     const uint3 B = block_at(rev);
     const int y = B.y * BY + threadIdx.y, t = B.x * BX + threadIdx.x, z0 = B.z * ZU;
     if (y >= d.ny || 2 * t >= d.nx) return;
@@ -421,9 +388,9 @@ __device__ __forceinline__ void rbgs_z2_body(Dims d, const LapK<T>& k, int color
 #pragma unroll
     for (int u = 0; u < ZU; ++u) xv[at[u]] = val[u];
 }
-template <typename T, int ZU>
+template <typename T, int ZU, typename IX>
 __global__ void k_rbgs_z2(Dims d, LapK<T> k, int color, T omega, T* __restrict__ xv, const T* __restrict__ b, int rev) {
-    rbgs_z2_body<T, ZU>(d, k, color, omega, xv, b, rev);
+    rbgs_z2_body<T, ZU, IX>(d, k, color, omega, xv, b, rev);
 }
 
 // The first colour (red) of a sweep from x = 0 without reading or clearing x
@@ -432,10 +399,10 @@ __global__ void k_rbgs_z2(Dims d, LapK<T> k, int color, T omega, T* __restrict__
 // not a folded constant) and the update x - 0 the update; the black cell of
 // each pair is written as zero. The same bits as a memset of x followed by
 // the colour launch.
-template <typename T, int ZU, int MINB>
+template <typename T, int ZU, int MINB, typename IX>
 __global__ void __launch_bounds__(BX * BY, MINB) k_rbgs_z2b_init(Dims d, LapK<T> k, T omega, T* __restrict__ xv,
                                                                 const T* __restrict__ b, int rev, T zero) {
-    const Ix2 I(d);
+    const IX I(d);
     const uint3 B = block_at(rev);
     const int y = B.y * BY + threadIdx.y, t = B.x * BX + threadIdx.x, z0 = B.z * ZU;
     if (y >= d.ny || 2 * t >= d.nx) return;
@@ -461,10 +428,10 @@ __global__ void __launch_bounds__(BX * BY, MINB) k_rbgs_z2b_init(Dims d, LapK<T>
         xv[other[u]] = zero;
     }
 }
-template <typename T, int ZU, int MINB>
+template <typename T, int ZU, int MINB, typename IX>
 __global__ void __launch_bounds__(BX * BY, MINB) k_rbgs_z2b(Dims d, LapK<T> k, int color, T omega, T* __restrict__ xv,
                                                            const T* __restrict__ b, int rev) {
-    rbgs_z2_body<T, ZU>(d, k, color, omega, xv, b, rev);
+    rbgs_z2_body<T, ZU, IX>(d, k, color, omega, xv, b, rev);
 }
 
 // The FP32 colour on float pairs: a thread owns the pairs (2t, 2t+1) of its
@@ -536,10 +503,10 @@ __global__ void __launch_bounds__(BX * BY, MINB) k_rbgs_pair(Dims d, int color, 
     for (int u = 0; u < ZU; ++u) xw[pr(y, z0 + u)] = out[u];
 }
 
-template <typename T, int ZU>
+template <typename T, int ZU, typename IX>
 __global__ void k_residual_z2(Dims d, LapK<T> k, T* __restrict__ r, const T* __restrict__ xv, const T* __restrict__ b,
                               int rev) {
-    const Ix2 I(d);
+    const IX I(d);
     const uint3 B = block_at(rev);
     const int x = B.x * BX + threadIdx.x, y = B.y * BY + threadIdx.y, z0 = B.z * ZU;
     if (x >= d.nx || y >= d.ny) return;
@@ -556,42 +523,24 @@ __global__ void k_residual_z2(Dims d, LapK<T> k, T* __restrict__ r, const T* __r
     for (int u = 0; u < ZU; ++u) r[I.at(x, y, z0 + u)] = val[u];
 }
 
-template <typename T, int ZU>
-__global__ void k_residual_z(Dims d, LapK<T> k, T* __restrict__ r, const T* __restrict__ xv, const T* __restrict__ b) {
-    const int x = blockIdx.x * BX + threadIdx.x, y = blockIdx.y * BY + threadIdx.y, z0 = blockIdx.z * ZU;
-    if (x >= d.nx || y >= d.ny) return;
-    T val[ZU];
-#pragma unroll
-    for (int u = 0; u < ZU; ++u) {
-        T S;
-        int c;
-        lap_row(d, xv, x, y, z0 + u, S, c);
-        const long long i = lin(d, x, y, z0 + u);
-        val[u] = b[i] - k.off * (S - lap_count<T>(c) * xv[i]);
-    }
-#pragma unroll
-    for (int u = 0; u < ZU; ++u) r[lin(d, x, y, z0 + u)] = val[u];
-}
-
 // The residual on the red cells alone (restrict_after_sweep): the same
 // expression; the black cells of r are not written. ZU cells along z per thread.
-template <typename T, int ZU, bool P2>
+template <typename T, int ZU, typename IX>
 __global__ void k_residual_red(Dims d, LapK<T> k, T* __restrict__ r, const T* __restrict__ xv, const T* __restrict__ b,
                                int rev) {
-    const Ix2 I(d);
+    const IX I(d);
     const uint3 B = block_at(rev);
     const int t = B.x * BX + threadIdx.x, y = B.y * BY + threadIdx.y, z0 = B.z * ZU;
     if (2 * t >= d.nx || y >= d.ny) return;
     T val[ZU];
-    long long at[ZU];
+    int at[ZU];
 #pragma unroll
     for (int u = 0; u < ZU; ++u) {
         const int z = z0 + u, x = 2 * t + ((y + z) & 1);
         T S;
         int c;
-        if (P2) lap_row2(d, I, xv, x, y, z, S, c);
-        else lap_row(d, xv, x, y, z, S, c);
-        const long long i = P2 ? (long long)I.at(x, y, z) : lin(d, x, y, z);
+        lap_row2(d, I, xv, x, y, z, S, c);
+        const int i = I.at(x, y, z);
         val[u] = b[i] - k.off * (S - lap_count<T>(c) * xv[i]);
         at[u] = i;
     }
@@ -773,55 +722,29 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_rbgs_pipe(Dims d, const T* 
     }
 }
 
-// Full weighting, src/mg/solver.h:153-181: 64 taps (1,3,3,1)^3/512 around the
-// coarse cell (restrict_taps, mg_cells.cuh); y clamps at the channel walls,
-// wraps in periodic mode.
+// Full weighting on 2D (periodic) grids, src/mg/solver.h:153-181: (1,3,3,1)^2/64
+// over 16 taps; the 3D form is restrict_cell2.
 template <typename T, bool RED>
-__device__ __forceinline__ void restrict_cell(const Dims& d, T* coarse, const T* fine, int xc, int yc, int zc) {
-    const int cx = d.nx / 2, cy = d.ny / 2;
-    const int xcf = 2 * xc + 1, ycf = 2 * yc + 1, zcf = 2 * zc + 1;
-    int xs[4], ys[4], zs[4];
+__device__ __forceinline__ void restrict_cell(const Dims& d, T* coarse, const T* fine, int xc, int yc) {
+    int xs[4], ys[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const int dd = k - 2;
-        xs[k] = wrapi(xcf + dd, d.nx);
-        zs[k] = d.nz == 1 ? 0 : wrapi(zcf + dd, d.nz);
-        if (d.channel) {
-            int yy = ycf + (dd > -ycf ? dd : -ycf);
-            ys[k] = yy < d.ny - 1 ? yy : d.ny - 1;
-        } else {
-            ys[k] = wrapi(ycf + dd, d.ny);
-        }
+        xs[k] = wrapi(2 * xc - 1 + k, d.nx);
+        ys[k] = wrapi(2 * yc - 1 + k, d.ny);
     }
-    if (d.nz == 1) {  // 2D (periodic): (1,3,3,1)^2 / 64 over 16 taps
-        auto row = [&](int ky) {
-            return red_row<T>(ys[ky] & 1, [&](int kx) { return fine[lin(d, xs[kx], ys[ky], 0)]; });
-        };
-        coarse[xc + (long long)cx * yc] =
-            (RED ? full4<T>(row(0), row(1), row(2), row(3))
-                 : restrict_plane<T>([&](int ky, int kx) { return fine[lin(d, xs[kx], ys[ky], 0)]; })) *
-            T(1.0 / 64.0);
-        return;
-    }
-    const long long o = xc + (long long)cx * (yc + (long long)cy * zc);
-    if (RED)
-        coarse[o] = restrict_rows<T>([&](int kz, int ky) {
-            return red_row<T>((ys[ky] + zs[kz]) & 1, [&](int kx) { return fine[lin(d, xs[kx], ys[ky], zs[kz])]; });
-        });
-    else
-        coarse[o] = restrict_taps<T>([&](int kz, int ky, int kx) { return fine[lin(d, xs[kx], ys[ky], zs[kz])]; });
+    auto tap = [&](int ky, int kx) { return fine[xs[kx] + d.nx * ys[ky]]; };
+    auto row = [&](int ky) { return red_row<T>(ys[ky] & 1, [&](int kx) { return tap(ky, kx); }); };
+    coarse[xc + (d.nx / 2) * yc] =
+        (RED ? full4<T>(row(0), row(1), row(2), row(3)) : restrict_plane<T>(tap)) * T(1.0 / 64.0);
 }
 
 // zero (optional): the coarse iterate, set to zero at every coarse cell
 template <typename T, bool RED>
 __global__ void k_restrict(Dims d, T* __restrict__ coarse, const T* __restrict__ fine, T* __restrict__ zero) {
-    const int xc = blockIdx.x * BX + threadIdx.x, yc = blockIdx.y * BY + threadIdx.y, zc = blockIdx.z;
+    const int xc = blockIdx.x * BX + threadIdx.x, yc = blockIdx.y * BY + threadIdx.y;
     if (xc >= d.nx / 2 || yc >= d.ny / 2) return;
-    restrict_cell<T, RED>(d, coarse, fine, xc, yc, zc);
-    if (zero) {
-        const long long cx = d.nx / 2, cy = d.ny / 2;
-        zero[d.nz == 1 ? xc + cx * yc : xc + cx * (yc + cy * zc)] = T(0);
-    }
+    restrict_cell<T, RED>(d, coarse, fine, xc, yc);
+    if (zero) zero[xc + (d.nx / 2) * yc] = T(0);
 }
 
 // Trilinear prolongation (27,9,3,1)/64, src/mg/solver.h:71-151 (prolong_plane4,
@@ -859,78 +782,65 @@ __device__ __forceinline__ void prolong_cell_any(const Dims& d, int xc, int yc, 
         }
     }
 }
+// 2D (periodic) grids: bilinear (9,3,3,1)/16 onto the four fine cells
 template <typename T, bool ADD, bool BLACK>
-__device__ __forceinline__ void prolong_cell(const Dims& d, T* fine, const T* coarse, int xc, int yc, int zc) {
-    const int cx = d.nx / 2, cy = d.ny / 2, cz = d.nz / 2;
-    const int xn = (xc + 1) % cx, yn = (yc + 1) % cy;
+__device__ __forceinline__ void prolong_cell(const Dims& d, T* fine, const T* coarse, int xc, int yc) {
+    const int cx = d.nx / 2, cy = d.ny / 2;
+    const int xn = xc + 1 == cx ? 0 : xc + 1, yn = yc + 1 == cy ? 0 : yc + 1;
     const int xf[2] = {2 * xc + 1, (2 * xc + 2) % d.nx}, yf[2] = {2 * yc + 1, (2 * yc + 2) % d.ny};
-    if (d.nz == 1) {
-        // 2D (periodic): bilinear (9,3,3,1)/16 onto the four fine cells
-        auto C2 = [&](int a, int b) { return coarse[a + (long long)cx * b]; };
-        const T bl = C2(xc, yc), br = C2(xn, yc), ul = C2(xc, yn), ur = C2(xn, yn);
-        prolong_row2(bl, br, ul, ur, black_col(BLACK, 0, 1),
-                     [&](int rx, T v, T s) { prolong_put<T, ADD>(fine, lin(d, xf[rx], yf[0], 0), v, s); });
-        prolong_row2(ul, ur, bl, br, black_col(BLACK, 1, 1),
-                     [&](int rx, T v, T s) { prolong_put<T, ADD>(fine, lin(d, xf[rx], yf[1], 0), v, s); });
-        return;
-    }
-    const int zf[2] = {2 * zc + 1, (2 * zc + 2) % d.nz};
-    prolong_cell_any<T, BLACK>(
-        d, xc, yc, zc, xn, yn, (zc + 1) % cz, xf, yf, zf,
-        [&](int a, int b, int c) { return coarse[a + (long long)cx * (b + (long long)cy * c)]; },
-        [&](int a, int b, int c, T v, T s) { prolong_put<T, ADD>(fine, lin(d, a, b, c), v, s); });
+    auto C2 = [&](int a, int b) { return coarse[a + cx * b]; };
+    const T bl = C2(xc, yc), br = C2(xn, yc), ul = C2(xc, yn), ur = C2(xn, yn);
+    prolong_row2(bl, br, ul, ur, black_col(BLACK, 0, 1),
+                 [&](int rx, T v, T s) { prolong_put<T, ADD>(fine, xf[rx] + d.nx * yf[0], v, s); });
+    prolong_row2(ul, ur, bl, br, black_col(BLACK, 1, 1),
+                 [&](int rx, T v, T s) { prolong_put<T, ADD>(fine, xf[rx] + d.nx * yf[1], v, s); });
 }
 
-// restrict_cell / prolong_cell for 3D power-of-two levels with Ix2 indexing
-// (the same arithmetic)
-template <typename T, bool RED>
-__device__ __forceinline__ void restrict_cell2(const Dims& d, const Ix2& I, T* coarse, const T* fine, int xc, int yc,
+// 3D levels with Ix2 or IxG indexing. Restriction: 64 taps (1,3,3,1)^3/512 around
+// the coarse cell (restrict_taps, mg_cells.cuh); y clamps at the channel walls,
+// wraps in periodic mode.
+template <typename T, bool RED, typename IX>
+__device__ __forceinline__ void restrict_cell2(const Dims& d, const IX& I, T* coarse, const T* fine, int xc, int yc,
                                                int zc) {
-    const int xcf = 2 * xc + 1, ycf = 2 * yc + 1, zcf = 2 * zc + 1;
-    int xs[4], yo[4], zo[4];
-    // parity of row ky's y (clamped at channel walls) plus plane kz's z
-    auto odd = [&](int kz, int ky) { return (((yo[ky] >> I.lx) + (zo[kz] >> I.lxy)) & 1) != 0; };
+    int xs[4], ys[4], zs[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const int dd = k - 2;
-        xs[k] = (xcf + dd) & I.mx;
-        zo[k] = ((zcf + dd) & I.mz) << I.lxy;
-        if (d.channel) {
-            int yy = ycf + (dd > -ycf ? dd : -ycf);
-            yo[k] = (yy < d.ny - 1 ? yy : d.ny - 1) << I.lx;
-        } else {
-            yo[k] = ((ycf + dd) & I.my) << I.lx;
-        }
+        const int x = 2 * xc - 1 + k, y = 2 * yc - 1 + k;
+        xs[k] = k == 0 ? I.xm(2 * xc) : (k == 3 ? I.xp(2 * xc + 1) : x);
+        zs[k] = I.wz(2 * zc - 1 + k);
+        if (d.channel) ys[k] = y < 0 ? 0 : (y > d.ny - 1 ? d.ny - 1 : y);
+        else ys[k] = k == 0 ? I.ym(2 * yc) : (k == 3 ? I.yp(2 * yc + 1) : y);
     }
-    const int o = xc | (yc << (I.lx - 1)) | (zc << (I.lxy - 2));
+    const int o = I.coarse(xc, yc, zc);
     if (RED)
         coarse[o] = restrict_rows<T>([&](int kz, int ky) {
-            return red_row<T>(odd(kz, ky), [&](int kx) { return fine[xs[kx] | yo[ky] | zo[kz]]; });
+            // the row's y comes clamped at channel walls
+            return red_row<T>(((ys[ky] + zs[kz]) & 1) != 0, [&](int kx) { return fine[I.at(xs[kx], ys[ky], zs[kz])]; });
         });
     else
-        coarse[o] = restrict_taps<T>([&](int kz, int ky, int kx) { return fine[xs[kx] | yo[ky] | zo[kz]]; });
+        coarse[o] = restrict_taps<T>([&](int kz, int ky, int kx) { return fine[I.at(xs[kx], ys[ky], zs[kz])]; });
 }
 
-template <typename T, bool RED>
+template <typename T, bool RED, typename IX>
 __global__ void k_restrict2(Dims d, T* __restrict__ coarse, const T* __restrict__ fine, int rev,
                             T* __restrict__ zero) {
-    const Ix2 I(d);
+    const IX I(d);
     const uint3 B = block_at(rev);
     const int xc = B.x * BX + threadIdx.x, yc = B.y * BY + threadIdx.y, zc = B.z;
     if (xc >= d.nx / 2 || yc >= d.ny / 2) return;
     restrict_cell2<T, RED>(d, I, coarse, fine, xc, yc, zc);
-    if (zero) zero[xc | (yc << (I.lx - 1)) | (zc << (I.lxy - 2))] = T(0);
+    if (zero) zero[I.coarse(xc, yc, zc)] = T(0);
 }
 
-template <typename T, bool ADD, bool BLACK>
-__device__ __forceinline__ void prolong_cell2(const Dims& d, const Ix2& I, T* fine, const T* coarse, int xc, int yc,
+template <typename T, bool ADD, bool BLACK, typename IX>
+__device__ __forceinline__ void prolong_cell2(const Dims& d, const IX& I, T* fine, const T* coarse, int xc, int yc,
                                               int zc) {
-    const int cx = d.nx / 2, cy = d.ny / 2, cz = d.nz / 2, lcx = I.lx - 1, lcxy = I.lxy - 2;
-    const int xf[2] = {2 * xc + 1, (2 * xc + 2) & I.mx}, yf[2] = {2 * yc + 1, (2 * yc + 2) & I.my},
-              zf[2] = {2 * zc + 1, (2 * zc + 2) & I.mz};
+    const int cx = d.nx / 2, cy = d.ny / 2, cz = d.nz / 2;
+    const int xf[2] = {2 * xc + 1, I.xp(2 * xc + 1)}, yf[2] = {2 * yc + 1, I.yp(2 * yc + 1)},
+              zf[2] = {2 * zc + 1, I.zp(2 * zc + 1)};
     prolong_cell_any<T, BLACK>(
-        d, xc, yc, zc, (xc + 1) & (cx - 1), (yc + 1) & (cy - 1), (zc + 1) & (cz - 1), xf, yf, zf,
-        [&](int a, int b, int c) { return coarse[a | (b << lcx) | (c << lcxy)]; },
+        d, xc, yc, zc, xc + 1 == cx ? 0 : xc + 1, yc + 1 == cy ? 0 : yc + 1, zc + 1 == cz ? 0 : zc + 1, xf, yf, zf,
+        [&](int a, int b, int c) { return coarse[I.coarse(a, b, c)]; },
         [&](int a, int b, int c, T v, T s) { prolong_put<T, ADD>(fine, I.at(a, b, c), v, s); });
 }
 
@@ -1019,9 +929,9 @@ __global__ void __launch_bounds__(RR_THREADS) k_resid_restrict2(Dims d, T* __res
     }
 }
 
-template <typename T, bool ADD, bool BLACK>
+template <typename T, bool ADD, bool BLACK, typename IX>
 __global__ void k_prolong2(Dims d, T* __restrict__ fine, const T* __restrict__ coarse, int rev) {
-    const Ix2 I(d);
+    const IX I(d);
     const uint3 B = block_at(rev);
     const int xc = B.x * BX + threadIdx.x, yc = B.y * BY + threadIdx.y, zc = B.z;
     if (xc >= d.nx / 2 || yc >= d.ny / 2) return;
@@ -1030,9 +940,9 @@ __global__ void k_prolong2(Dims d, T* __restrict__ fine, const T* __restrict__ c
 
 template <typename T, bool ADD, bool BLACK>
 __global__ void k_prolong(Dims d, T* __restrict__ fine, const T* __restrict__ coarse) {
-    const int xc = blockIdx.x * BX + threadIdx.x, yc = blockIdx.y * BY + threadIdx.y, zc = blockIdx.z;
+    const int xc = blockIdx.x * BX + threadIdx.x, yc = blockIdx.y * BY + threadIdx.y;
     if (xc >= d.nx / 2 || yc >= d.ny / 2) return;
-    prolong_cell<T, ADD, BLACK>(d, fine, coarse, xc, yc, zc);
+    prolong_cell<T, ADD, BLACK>(d, fine, coarse, xc, yc);
 }
 
 // Column-marching transfers for 3D power-of-two levels whose coarse x extent
@@ -1619,31 +1529,30 @@ int batch_min_nx() {
 
 template <typename T>
 void launch_lap_apply(const Dims& d, T* y, const T* x, cudaStream_t s) {
-    k_lap<T><<<grid3(d), dim3(BX, BY), 0, s>>>(d, lap_k<T>(d), y, x);
+    AFMIB_IX(d, (k_lap<T, IX><<<grid3(d), dim3(BX, BY), 0, s>>>(d, lap_k<T>(d), y, x)));
 }
 template <typename T>
 void launch_residual(const Dims& d, T* r, const T* x, const T* b, RedScratch* sc, double* out, cudaStream_t s, int rev) {
-    if (sc && out)
-        k_residual_norm<T><<<red_grid3(d.nx, d.ny, d.nz, red_target<T>()), dim3(kRBX, kRBY), 0, s>>>(d, lap_k<T>(d), r, x, b, *sc, out);
-    else if (d.nz % kZU == 0 && d.nx >= batch_min_nx() && ix2_ok(d))
-        k_residual_z2<T, kZU><<<dim3((d.nx + BX - 1) / BX, (d.ny + BY - 1) / BY, d.nz / kZU), dim3(BX, BY), 0, s>>>(
-            d, lap_k<T>(d), r, x, b, rev);
-    else if (d.nz % kZU == 0 && d.nx >= batch_min_nx())
-        k_residual_z<T, kZU><<<dim3((d.nx + BX - 1) / BX, (d.ny + BY - 1) / BY, d.nz / kZU), dim3(BX, BY), 0, s>>>(
-            d, lap_k<T>(d), r, x, b);
-    else
-        k_residual<T><<<grid3(d), dim3(BX, BY), 0, s>>>(d, lap_k<T>(d), r, x, b);
+    const LapK<T> k = lap_k<T>(d);
+    if (sc && out) {
+        const dim3 g = red_grid3(d.nx, d.ny, d.nz, red_target<T>());
+        AFMIB_IX(d, (k_residual_norm<T, IX><<<g, dim3(kRBX, kRBY), 0, s>>>(d, k, r, x, b, *sc, out)));
+    } else if (d.nz % kZU == 0 && d.nx >= batch_min_nx()) {
+        const dim3 g((d.nx + BX - 1) / BX, (d.ny + BY - 1) / BY, d.nz / kZU);
+        AFMIB_IX(d, (k_residual_z2<T, kZU, IX><<<g, dim3(BX, BY), 0, s>>>(d, k, r, x, b, rev)));
+    } else {
+        AFMIB_IX(d, (k_residual<T, IX><<<grid3(d), dim3(BX, BY), 0, s>>>(d, k, r, x, b)));
+    }
 }
 template <typename T>
 void launch_residual_red(const Dims& d, T* r, const T* x, const T* b, cudaStream_t s, int rev) {
     constexpr int ZU = 4;
     const int gx = (d.nx / 2 + BX - 1) / BX, gy = (d.ny + BY - 1) / BY;
     const LapK<T> k = lap_k<T>(d);
-    const bool batch = d.nz % ZU == 0 && d.nx >= batch_min_nx(), p2 = ix2_ok(d);
-    if (batch && p2) k_residual_red<T, ZU, true><<<dim3(gx, gy, d.nz / ZU), dim3(BX, BY), 0, s>>>(d, k, r, x, b, rev);
-    else if (batch) k_residual_red<T, ZU, false><<<dim3(gx, gy, d.nz / ZU), dim3(BX, BY), 0, s>>>(d, k, r, x, b, rev);
-    else if (p2) k_residual_red<T, 1, true><<<dim3(gx, gy, d.nz), dim3(BX, BY), 0, s>>>(d, k, r, x, b, rev);
-    else k_residual_red<T, 1, false><<<dim3(gx, gy, d.nz), dim3(BX, BY), 0, s>>>(d, k, r, x, b, rev);
+    if (d.nz % ZU == 0 && d.nx >= batch_min_nx())
+        AFMIB_IX(d, (k_residual_red<T, ZU, IX><<<dim3(gx, gy, d.nz / ZU), dim3(BX, BY), 0, s>>>(d, k, r, x, b, rev)));
+    else
+        AFMIB_IX(d, (k_residual_red<T, 1, IX><<<dim3(gx, gy, d.nz), dim3(BX, BY), 0, s>>>(d, k, r, x, b, rev)));
 }
 // The pair kernel is opt-in (AFMIB_RBGS_PAIR=1, read at every launch): at
 // 256^3 its colour launches took 39.5 us against 29.9 for the scalar kernel
@@ -1655,7 +1564,7 @@ constexpr int kPairZU = 4, kPairMinB = 4;
 bool rbgs_pair_ok(const Dims& d) {
     const char* e = std::getenv("AFMIB_RBGS_PAIR");
     if (!(e && e[0] == '1')) return false;
-    return d.nz > 1 && d.nx >= 2 * BX && d.ny % BY == 0 && d.nz % kPairZU == 0;
+    return d.nz > 1 && d.nx >= 2 * BX && d.ny % BY == 0 && d.nz % kPairZU == 0 && ix2_ok(d);
 }
 
 // First colour of a sweep from x = 0 (x's contents ignored and overwritten):
@@ -1667,10 +1576,10 @@ void launch_rbgs_from_zero(const Dims& d, T* x, const T* b, cudaStream_t s, doub
     const char* e = std::getenv("AFMIB_INIT_SWEEP");
     const bool off = e && e[0] == '0';
     if (d.nx < kOmegaMinNx) omega = 1.0;
-    if (!off && sizeof(T) == sizeof(float) && d.nz % kZU == 0 && d.nz % kZU32 == 0 && d.nx >= batch_min_nx() &&
-        ix2_ok(d) && !rbgs_pair_ok(d)) {
+    if (!off && sizeof(T) == sizeof(float) && d.nz % kZU32 == 0 && d.nx >= batch_min_nx() && !rbgs_pair_ok(d)) {
         const dim3 g((d.nx / 2 + BX - 1) / BX, (d.ny + BY - 1) / BY, d.nz / kZU32);
-        k_rbgs_z2b_init<T, kZU32, 6><<<g, dim3(BX, BY), 0, s>>>(d, lap_k<T>(d), T(omega), x, b, rev, T(0));
+        AFMIB_IX(d, (k_rbgs_z2b_init<T, kZU32, 6, IX><<<g, dim3(BX, BY), 0, s>>>(d, lap_k<T>(d), T(omega), x, b, rev,
+                                                                               T(0))));
         return;
     }
     cudaMemsetAsync(x, 0, (size_t)d.ncell() * sizeof(T), s);
@@ -1680,33 +1589,30 @@ void launch_rbgs_from_zero(const Dims& d, T* x, const T* b, cudaStream_t s, doub
 template <typename T>
 void launch_rbgs(const Dims& d, int color, T* x, const T* b, cudaStream_t s, double omega, int rev) {
     if (d.nx < kOmegaMinNx) omega = 1.0;
-    if (d.nz % kZU == 0 && d.nx >= batch_min_nx()) {
-        dim3 g((d.nx / 2 + BX - 1) / BX, (d.ny + BY - 1) / BY, d.nz / kZU);
-        if (ix2_ok(d)) {
-            // FP32 on float pairs (opt-in, AFMIB_RBGS_PAIR=1)
-            if (sizeof(T) == sizeof(float) && rbgs_pair_ok(d)) {
-                const dim3 gp(d.nx / 2 / BX, d.ny / BY, d.nz / kPairZU);
-                k_rbgs_pair<kPairZU, kPairMinB><<<gp, dim3(BX, BY), 0, s>>>(d, color, float(omega), (float*)x,
-                                                                           (const float*)b, rev);
-                return;
-            }
-            // FP32: kZU32 z cells per thread, registers capped for 6 resident
-            // blocks (50.5 against 50.0 IB steps/s at 256^3 for eight cells
-            // and 6 blocks against none; four cells: 29.5 against 30.0 us per
-            // 256^3 colour, 61.1 against 60.8 steps/s; 16: spills, two:
-            // 32.7 us; four cells with 8 blocks: the same as 6)
-            if (sizeof(T) == sizeof(float) && d.nz % kZU32 == 0) {
-                const dim3 g4(g.x, g.y, d.nz / kZU32);
-                k_rbgs_z2b<T, kZU32, 6><<<g4, dim3(BX, BY), 0, s>>>(d, lap_k<T>(d), color, T(omega), x, b, rev);
-            }
-            else
-                k_rbgs_z2<T, kZU><<<g, dim3(BX, BY), 0, s>>>(d, lap_k<T>(d), color, T(omega), x, b, rev);
+    const LapK<T> k = lap_k<T>(d);
+    const int gx = (d.nx / 2 + BX - 1) / BX, gy = (d.ny + BY - 1) / BY;
+    const dim3 blk(BX, BY);
+    constexpr bool f32 = sizeof(T) == sizeof(float);
+    if (d.nx >= batch_min_nx() && d.nz % (f32 ? kZU32 : kZU) == 0) {
+        // FP32 on float pairs (opt-in, AFMIB_RBGS_PAIR=1)
+        if (f32 && rbgs_pair_ok(d)) {
+            const dim3 gp(d.nx / 2 / BX, d.ny / BY, d.nz / kPairZU);
+            k_rbgs_pair<kPairZU, kPairMinB><<<gp, blk, 0, s>>>(d, color, float(omega), (float*)x, (const float*)b, rev);
+            return;
         }
-        else k_rbgs_z<T, kZU><<<g, dim3(BX, BY), 0, s>>>(d, lap_k<T>(d), color, T(omega), x, b);
+        // FP32: kZU32 z cells per thread, registers capped for 6 resident
+        // blocks (50.5 against 50.0 IB steps/s at 256^3 for eight cells
+        // and 6 blocks against none; four cells: 29.5 against 30.0 us per
+        // 256^3 colour, 61.1 against 60.8 steps/s; 16: spills, two:
+        // 32.7 us; four cells with 8 blocks: the same as 6)
+        if (f32)
+            AFMIB_IX(d, (k_rbgs_z2b<T, kZU32, 6, IX><<<dim3(gx, gy, d.nz / kZU32), blk, 0, s>>>(d, k, color, T(omega), x,
+                                                                                              b, rev)));
+        else
+            AFMIB_IX(d, (k_rbgs_z2<T, kZU, IX><<<dim3(gx, gy, d.nz / kZU), blk, 0, s>>>(d, k, color, T(omega), x, b, rev)));
         return;
     }
-    dim3 g((d.nx / 2 + BX - 1) / BX, (d.ny + BY - 1) / BY, d.nz);
-    k_rbgs<T><<<g, dim3(BX, BY), 0, s>>>(d, lap_k<T>(d), color, T(omega), x, b);
+    AFMIB_IX(d, (k_rbgs<T, IX><<<dim3(gx, gy, d.nz), blk, 0, s>>>(d, k, color, T(omega), x, b)));
 }
 namespace {
 int log2_exact(int v) {
@@ -1833,9 +1739,9 @@ void launch_restrict(const Dims& d, T* coarse, const T* fine, cudaStream_t s, in
         }
     }
     dim3 g((d.nx / 2 + BX - 1) / BX, (d.ny / 2 + BY - 1) / BY, d.nz == 1 ? 1 : d.nz / 2);
-    if (d.nz > 1 && d.nx >= 2 && d.ny >= 2 && ix2_ok(d))
-        red ? k_restrict2<T, true><<<g, dim3(BX, BY), 0, s>>>(d, coarse, fine, rev, zero)
-            : k_restrict2<T, false><<<g, dim3(BX, BY), 0, s>>>(d, coarse, fine, rev, zero);
+    if (d.nz > 1)
+        AFMIB_IX(d, (red ? k_restrict2<T, true, IX><<<g, dim3(BX, BY), 0, s>>>(d, coarse, fine, rev, zero)
+                         : k_restrict2<T, false, IX><<<g, dim3(BX, BY), 0, s>>>(d, coarse, fine, rev, zero)));
     else
         red ? k_restrict<T, true><<<g, dim3(BX, BY), 0, s>>>(d, coarse, fine, zero)
             : k_restrict<T, false><<<g, dim3(BX, BY), 0, s>>>(d, coarse, fine, zero);
@@ -1945,9 +1851,9 @@ void launch_prolong_add(const Dims& d, T* fine, const T* coarse, cudaStream_t s,
         }
     }
     dim3 g((d.nx / 2 + BX - 1) / BX, (d.ny / 2 + BY - 1) / BY, d.nz == 1 ? 1 : d.nz / 2);
-    if (d.nz > 1 && d.nx >= 2 && d.ny >= 2 && ix2_ok(d))
-        black ? k_prolong2<T, true, true><<<g, dim3(BX, BY), 0, s>>>(d, fine, coarse, rev)
-              : k_prolong2<T, true, false><<<g, dim3(BX, BY), 0, s>>>(d, fine, coarse, rev);
+    if (d.nz > 1)
+        AFMIB_IX(d, (black ? k_prolong2<T, true, true, IX><<<g, dim3(BX, BY), 0, s>>>(d, fine, coarse, rev)
+                           : k_prolong2<T, true, false, IX><<<g, dim3(BX, BY), 0, s>>>(d, fine, coarse, rev)));
     else
         black ? k_prolong<T, true, true><<<g, dim3(BX, BY), 0, s>>>(d, fine, coarse)
               : k_prolong<T, true, false><<<g, dim3(BX, BY), 0, s>>>(d, fine, coarse);
@@ -1955,7 +1861,8 @@ void launch_prolong_add(const Dims& d, T* fine, const T* coarse, cudaStream_t s,
 template <typename T>
 void launch_prolong_assign(const Dims& d, T* fine, const T* coarse, cudaStream_t s) {
     dim3 g((d.nx / 2 + BX - 1) / BX, (d.ny / 2 + BY - 1) / BY, d.nz == 1 ? 1 : d.nz / 2);
-    k_prolong<T, false, false><<<g, dim3(BX, BY), 0, s>>>(d, fine, coarse);
+    if (d.nz > 1) AFMIB_IX(d, (k_prolong2<T, false, false, IX><<<g, dim3(BX, BY), 0, s>>>(d, fine, coarse, 0)));
+    else k_prolong<T, false, false><<<g, dim3(BX, BY), 0, s>>>(d, fine, coarse);
 }
 template <typename TD>
 void launch_lap_defect(const Dims& d, TD* r, const double* x, const double* b, RedScratch sc, double* out, cudaStream_t s,
@@ -1971,11 +1878,12 @@ void launch_lap_update_df(const Dims& d, double* x, const float* e, float* rh, f
                           cudaStream_t s) {
     constexpr int ZU = 2;
     const char* g = std::getenv("AFMIB_UPDATE_DF_GENERIC");
-    if (d.nz > 1 && d.nz % ZU == 0 && ix2_ok(d) && !(g && g[0] == '1')) {
+    if (d.nz > 1 && d.nz % ZU == 0 && !(g && g[0] == '1')) {
         const int gx = (d.nx + kRBX - 1) / kRBX, gy = (d.ny + kRBY - 1) / kRBY;
         int gz = d.nz / ZU;
         if ((long long)gx * gy * gz > kMaxRedBlocks) gz = std::max(1, kMaxRedBlocks / (gx * gy));
-        k_lap_update_df2<ZU, kUpdateMinBlocks><<<dim3(gx, gy, gz), dim3(kRBX, kRBY), 0, s>>>(d, x, e, rh, rl, sc, out);
+        AFMIB_IX(d, (k_lap_update_df2<ZU, kUpdateMinBlocks, IX><<<dim3(gx, gy, gz), dim3(kRBX, kRBY), 0, s>>>(
+                        d, x, e, rh, rl, sc, out)));
         return;
     }
     k_lap_update_df<<<red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s>>>(d, x, e, rh, rl, sc, out);

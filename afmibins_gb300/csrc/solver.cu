@@ -1051,7 +1051,7 @@ int helm_solve_mixed(afmib_solver* s, int comp, double scale, double* x, const d
 bool helm_overlap_ok(afmib_solver* s, double scale) {
     const Dims& d = s->d;
     return s->helm_overlap && s->aux && s->hi && s->gs_inner && !s->bfp_defects &&
-           gs_sweeps(d, scale, s->cfg.inner_tol) > 0 && d.nz % 8 == 0 && d.nx % 2 == 0 && ix2_ok(d);
+           gs_sweeps(d, scale, s->cfg.inner_tol) > 0 && helm_rbgs_ok(d);
 }
 
 template <typename F>
