@@ -146,12 +146,13 @@ void launch_cgb_direction(const Dims& d, const CgBatch& g, const double* cgs, cu
 template <typename T>
 void launch_helm_jacobi(const Dims& d, int comp, double scale, const T* x, T* xo, const T* b, cudaStream_t s,
                         int rev = 0);
-// One colour of a red-black Gauss-Seidel sweep of (I + scale*Delta) x = b in
-// place (init: from x = 0), on the grids of helm_rbgs_ok; returns false (nothing
-// launched) otherwise.
+// Red-black Gauss-Seidel for (I + scale*Delta) x = b on the grids of helm_rbgs_ok:
+// a whole sweep from x = 0 (x's contents ignored), and one colour in place.
 bool helm_rbgs_ok(const Dims& d);
 template <typename T>
-bool launch_helm_rbgs(const Dims& d, int comp, double scale, int color, int init, T* x, const T* b, cudaStream_t s,
+void launch_helm_rbgs_first(const Dims& d, int comp, double scale, T* x, const T* b, cudaStream_t s, int rev = 0);
+template <typename T>
+void launch_helm_rbgs(const Dims& d, int comp, double scale, int color, T* x, const T* b, cudaStream_t s,
                       int rev = 0);
 // p' = beta p + r formed on the fly (out of place into pn), q = H p', p'.q and alpha
 template <typename T>
@@ -213,13 +214,13 @@ void launch_helm_defect_bfp(const Dims& d, int comp, double scale, const double*
 // One red (color 0) or black (color 1) Gauss-Seidel half sweep; omega:
 // over-relaxation x + omega (gs - x) on levels with nx >= 64 (1 below).
 // rev (here and in the residual, transfer and Jacobi launchers): blocks in
-// reverse order (block_at, common.cuh) on the batched power-of-two kernels.
+// reverse order (block_at, common.cuh) on the batched kernels.
 template <typename T>
 void launch_rbgs(const Dims& d, int color, T* x, const T* b, cudaStream_t s, double omega = 1.0, int rev = 0);
-// The red colour of a sweep from x = 0 (x's contents ignored, both colours
-// written): the same bits as zeroing x and launch_rbgs(color 0).
+// Both colours from x = 0 (x's contents ignored): the same bits as zeroing x and
+// launch_rbgs of color 0 and of color 1.
 template <typename T>
-void launch_rbgs_from_zero(const Dims& d, T* x, const T* b, cudaStream_t s, double omega = 1.0, int rev = 0);
+void launch_rbgs_first(const Dims& d, T* x, const T* b, cudaStream_t s, double omega = 1.0, int rev = 0);
 // One full red+black sweep per launch, out of place (xin -> xout), z-marching
 // blocks fed by bulk asynchronous row copies; equals the two per-colour
 // launches cell for cell. FY == 0: level not eligible (small, 2D, or rows not
@@ -265,11 +266,9 @@ void launch_vcycle_tail(const TailLevels<T>& a, cudaStream_t s);
 void vcycle_tail_attributes();
 template <typename T>
 void launch_rbgs_pipe(const Dims& d, const PipeCfg& c, const T* xin, T* xout, const T* b, int* err, cudaStream_t s);
-// Full-weighting restriction, src/mg/solver.h:153-181 (d = fine dims); zero
-// (optional): the coarse iterate, set to zero in the same pass.
+// Full-weighting restriction, src/mg/solver.h:153-181 (d = fine dims)
 template <typename T>
-void launch_restrict(const Dims& d, T* coarse, const T* fine, cudaStream_t s, int rev = 0, T* zero = nullptr,
-                     bool red = false);
+void launch_restrict(const Dims& d, T* coarse, const T* fine, cudaStream_t s, int rev = 0, bool red = false);
 // r = b - L x on the red cells only; launch_restrict with red reads those and
 // takes the black ones as zero (restrict_after_sweep, mg_cells.cuh)
 template <typename T>
@@ -279,17 +278,15 @@ void launch_residual_red(const Dims& d, T* r, const T* x, const T* b, cudaStream
 // (prolong_before_sweep)
 template <typename T>
 void launch_prolong_add(const Dims& d, T* fine, const T* coarse, cudaStream_t s, int rev = 0, bool black = false);
-// coarse_b = restriction of (b - L x), coarse_x = 0, in one pass (the
-// residual stays in shared memory), for the levels resid_restrict_fused_ok
+// coarse_b = restriction of (b - L x) in one pass (the residual stays in shared memory), for the levels resid_restrict_fused_ok
 // takes: by default FP32 3D power-of-two levels with nx >= 256 (the column
 // kernel); AFMIB_RESID_RESTRICT=1 the ring kernel, =0 none
-bool resid_restrict_fused_ok(const Dims& d, size_t elem, const void* x, const void* b, const void* cb,
-                             const void* cx);
+bool resid_restrict_fused_ok(const Dims& d, size_t elem, const void* x, const void* b, const void* cb);
 // shared-memory opt-ins of the multigrid kernels (once per device, before
 // any launch or stream capture)
 void mg_kernel_attributes();
 template <typename T>
-void launch_resid_restrict(const Dims& d, T* coarse_b, T* coarse_x, const T* x, const T* b, cudaStream_t s,
+void launch_resid_restrict(const Dims& d, T* coarse_b, const T* x, const T* b, cudaStream_t s,
                            int rev = 0, bool red = false);
 // Prolongation that assigns (for the op-level API).
 template <typename T>

@@ -1638,12 +1638,10 @@ __global__ void k_helm_jacobi2(Dims d, int comp, HelmK<T> k, const T* __restrict
 
 // One colour of a red-black Gauss-Seidel sweep of the FP32 inner Helmholtz
 // solve, in place: x += (b - H x) / diag at the colour's cells (the other
-// colour's values are the latest). With init the sweep starts from x = 0: the
-// colour's cells take b / diag and the other colour's cells are zeroed. For
-// the 7-point operator under red-black ordering the sweep contracts the
-// error as the square of the Jacobi rate.
+// colour's values are the latest). For the 7-point operator under red-black
+// ordering the sweep contracts the error as the square of the Jacobi rate.
 template <typename T, int ZU, typename IX>
-__device__ __forceinline__ void helm_rbgs2_body(Dims d, int comp, const HelmK<T>& k, int color, int init, T* __restrict__ xv,
+__device__ __forceinline__ void helm_rbgs2_body(Dims d, int comp, const HelmK<T>& k, int color, T* __restrict__ xv,
                                                 const T* __restrict__ b, int rev) {
     const IX I(d);
     const uint3 B = block_at(rev);
@@ -1654,21 +1652,61 @@ __device__ __forceinline__ void helm_rbgs2_body(Dims d, int comp, const HelmK<T>
     int at[ZU];
 #pragma unroll
     for (int u = 0; u < ZU; ++u) {
-        const int z = z0 + u, x = 2 * t + ((y + z + color) & 1);
-        const int i = I.at(x, y, z);
-        val[u] = init ? b[i] * rdiag : xv[i] + (b[i] - helm_point2(d, I, comp, k, xv, x, y, z)) * rdiag;
+        const int x = 2 * t + ((y + z0 + u + color) & 1), i = I.at(x, y, z0 + u);
+        val[u] = xv[i] + (b[i] - helm_point2(d, I, comp, k, xv, x, y, z0 + u)) * rdiag;
         at[u] = i;
     }
 #pragma unroll
-    for (int u = 0; u < ZU; ++u) {
-        xv[at[u]] = val[u];
-        if (init) xv[I.at(2 * t + ((y + z0 + u + color + 1) & 1), y, z0 + u)] = T(0);
-    }
+    for (int u = 0; u < ZU; ++u) xv[at[u]] = val[u];
 }
 template <typename T, int ZU, int MINB, typename IX>
-__global__ void __launch_bounds__(BX * BY, MINB) k_helm_rbgs2b(Dims d, int comp, HelmK<T> k, int color, int init,
-                                                              T* __restrict__ xv, const T* __restrict__ b, int rev) {
-    helm_rbgs2_body<T, ZU, IX>(d, comp, k, color, init, xv, b, rev);
+__global__ void __launch_bounds__(BX * BY, MINB) k_helm_rbgs2b(Dims d, int comp, HelmK<T> k, int color, T* __restrict__ xv,
+                                                              const T* __restrict__ b, int rev) {
+    helm_rbgs2_body<T, ZU, IX>(d, comp, k, color, xv, b, rev);
+}
+
+// A whole sweep from x = 0 in one pass: b is read, x written. A red cell takes
+// b / diag; the reds that a black cell sums are formed from b on the fly. A thread
+// owns the pairs (2t, 2t+1) of its (y, z) column, one red and one black cell each:
+// of the black cell's six reds one is the pair's own, the two along z are the own
+// reds of the pairs above and below, and the other three are formed again.
+// Bytes bound: 2 words a cell against 4.5 for a red launch that also clears the
+// black cells and a black one.
+template <typename T, int ZU, int MINB, typename IX>
+__global__ void __launch_bounds__(BX * BY, MINB) k_helm_first(Dims d, int comp, HelmK<T> k, T* __restrict__ xv,
+                                                             const T* __restrict__ b, int rev) {
+    const IX I(d);
+    const uint3 B = block_at(rev);
+    const int y = B.y * BY + threadIdx.y, t = B.x * BX + threadIdx.x, z0 = B.z * ZU;
+    if (y >= d.ny || 2 * t >= d.nx) return;
+    const int ylo = I.ym(y), yhi = I.yp(y);
+    const T rd = helm_rdiag(d, comp, k, y), rlo = helm_rdiag(d, comp, k, ylo), rhi = helm_rdiag(d, comp, k, yhi);
+    const bool cell_rows = d.channel && comp != 1, fixed = d.channel && comp == 1 && y == 0;
+    T red[ZU + 2];
+#pragma unroll
+    for (int u = 0; u < ZU + 2; ++u) {
+        const int z = z0 + u - 1;
+        red[u] = b[I.at(2 * t + ((y + z) & 1), y, I.wz(z))] * rd;
+    }
+    T val[ZU];
+#pragma unroll
+    for (int u = 0; u < ZU; ++u) {
+        const int z = z0 + u, p = (y + z) & 1, x = 2 * t + 1 - p;
+        const T sx = red[u + 1] + b[I.at(p ? I.xm(2 * t) : I.xp(2 * t + 1), y, z)] * rd;
+        const T sz = red[u] + red[u + 2];
+        const T lo = b[I.at(x, ylo, z)] * rlo, hi = b[I.at(x, yhi, z)] * rhi;
+        T hx;  // H x at x = 0 here (helm_point2's forms)
+        if (cell_rows && (y == 0 || y == d.ny - 1)) hx = k.off * (sx + sz) + k.offw * (y == 0 ? hi : lo);
+        else if (cell_rows) hx = k.off * (sx + sz) + k.off * (lo + hi);
+        else hx = fixed ? T(0) : k.off * (sx + (lo + hi) + sz);
+        val[u] = (b[I.at(x, y, z)] - hx) * rd;
+    }
+#pragma unroll
+    for (int u = 0; u < ZU; ++u) {
+        const int z = z0 + u, p = (y + z) & 1;
+        xv[I.at(2 * t + p, y, z)] = red[u + 1];
+        xv[I.at(2 * t + 1 - p, y, z)] = val[u];
+    }
 }
 
 // Red-black order needs every wrap to join the two colours: even extents in the
@@ -1680,21 +1718,35 @@ bool helm_rbgs_ok(const Dims& d) {
     return d.nz > 1 && d.nx % 2 == 0 && d.nz % 2 == 0 && (d.channel || d.ny % 2 == 0);
 }
 template <typename T>
-bool launch_helm_rbgs(const Dims& d, int comp, double scale, int color, int init, T* x, const T* b, cudaStream_t s,
-                      int rev) {
-    if (!helm_rbgs_ok(d)) return false;
+void launch_helm_rbgs_first(const Dims& d, int comp, double scale, T* x, const T* b, cudaStream_t s, int rev) {
+    const char* e = std::getenv("AFMIB_INIT_SWEEP");  // 0: a memset and the two colours
+    if (e && e[0] == '0') {
+        cudaMemsetAsync(x, 0, (size_t)d.ncell() * sizeof(T), s);
+        for (int color = 0; color < 2; ++color) launch_helm_rbgs<T>(d, comp, scale, color, x, b, s, rev);
+        return;
+    }
+    const int gx = (d.nx / 2 + BX - 1) / BX, gy = (d.ny + BY - 1) / BY;
+    const HelmK<T> k = helm_k<T>(d, scale);
+    if (d.nz % 4 == 0)
+        AFMIB_IX(d, (k_helm_first<T, 4, 6, IX><<<dim3(gx, gy, d.nz / 4), dim3(BX, BY), 0, s>>>(d, comp, k, x, b, rev)));
+    else
+        AFMIB_IX(d, (k_helm_first<T, 2, 6, IX><<<dim3(gx, gy, d.nz / 2), dim3(BX, BY), 0, s>>>(d, comp, k, x, b, rev)));
+}
+template void launch_helm_rbgs_first<float>(const Dims&, int, double, float*, const float*, cudaStream_t, int);
+
+template <typename T>
+void launch_helm_rbgs(const Dims& d, int comp, double scale, int color, T* x, const T* b, cudaStream_t s, int rev) {
     const int gx = (d.nx / 2 + BX - 1) / BX, gy = (d.ny + BY - 1) / BY;
     const dim3 blk(BX, BY);
     const HelmK<T> k = helm_k<T>(d, scale);
     // registers capped for 6 resident blocks (40 against 48): measured with the
     // multigrid smoother's cap, 50.5 against 50.0 IB steps/s at 256^3
     if (d.nz % 8 == 0)
-        AFMIB_IX(d, (k_helm_rbgs2b<T, 8, 6, IX><<<dim3(gx, gy, d.nz / 8), blk, 0, s>>>(d, comp, k, color, init, x, b, rev)));
+        AFMIB_IX(d, (k_helm_rbgs2b<T, 8, 6, IX><<<dim3(gx, gy, d.nz / 8), blk, 0, s>>>(d, comp, k, color, x, b, rev)));
     else
-        AFMIB_IX(d, (k_helm_rbgs2b<T, 2, 6, IX><<<dim3(gx, gy, d.nz / 2), blk, 0, s>>>(d, comp, k, color, init, x, b, rev)));
-    return true;
+        AFMIB_IX(d, (k_helm_rbgs2b<T, 2, 6, IX><<<dim3(gx, gy, d.nz / 2), blk, 0, s>>>(d, comp, k, color, x, b, rev)));
 }
-template bool launch_helm_rbgs<float>(const Dims&, int, double, int, int, float*, const float*, cudaStream_t, int);
+template void launch_helm_rbgs<float>(const Dims&, int, double, int, float*, const float*, cudaStream_t, int);
 
 template <typename T>
 void launch_helm_jacobi(const Dims& d, int comp, double scale, const T* x, T* xo, const T* b, cudaStream_t s,

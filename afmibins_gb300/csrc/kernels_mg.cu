@@ -393,39 +393,67 @@ __global__ void k_rbgs_z2(Dims d, LapK<T> k, int color, T omega, T* __restrict__
     rbgs_z2_body<T, ZU, IX>(d, k, color, omega, xv, b, rev);
 }
 
-// The first colour (red) of a sweep from x = 0 without reading or clearing x
-// first: every neighbour is zero, so the neighbour sum lap_row2 forms is the
-// zero `zero` (a kernel argument, so that the arithmetic is rbgs_z2_body's,
-// not a folded constant) and the update x - 0 the update; the black cell of
-// each pair is written as zero. The same bits as a memset of x followed by
-// the colour launch.
+// A whole sweep from x = 0 in one pass: b is read, x written, x never read. A red
+// cell's update has the neighbour sum zero, so the reds that a black cell sums are
+// formed from b on the fly. A thread owns the pairs (2t, 2t+1) of its (y, z)
+// column, one red and one black cell each; of the black cell's six reds one is the
+// pair's own, the two along z are the own reds of the pairs above and below, and
+// the other three are formed again (a fifth load each of b, from L1). `zero` is a
+// kernel argument, so that the arithmetic is rbgs_z2_body's and not a folded
+// constant: the same bits as a memset of x and the two colours. With the viscous
+// solves' first sweeps in the same form: IB steps of the mixed form at 256^3 16.20
+// -> 15.77 ms, at 96x80x112 3.88 -> 3.74; FP64 steps unchanged (13.8 ms at 128^3:
+// the reds formed again cost the FP64 pipe what the launch saves).
 template <typename T, int ZU, int MINB, typename IX>
-__global__ void __launch_bounds__(BX * BY, MINB) k_rbgs_z2b_init(Dims d, LapK<T> k, T omega, T* __restrict__ xv,
-                                                                const T* __restrict__ b, int rev, T zero) {
+__global__ void __launch_bounds__(BX * BY, MINB) k_rbgs_first(Dims d, LapK<T> k, T omega, T* __restrict__ xv,
+                                                             const T* __restrict__ b, int rev, T zero) {
     const IX I(d);
     const uint3 B = block_at(rev);
     const int y = B.y * BY + threadIdx.y, t = B.x * BX + threadIdx.x, z0 = B.z * ZU;
     if (y >= d.ny || 2 * t >= d.nx) return;
+    const bool flat = d.nz == 1;
+    auto count = [&](int yy) {
+        int c = flat ? 4 : 6;
+        if (d.channel) {
+            if (!(yy > 0)) --c;
+            if (!(yy < d.ny - 1)) --c;
+        }
+        return c;
+    };
+    auto update = [&](T S, int i, int c) {
+        T v = (S - b[i] * k.inv) * lap_rcount<T>(c);
+        if (omega != T(1)) v = v + (omega - T(1)) * (v - zero);
+        return v;
+    };
+    const int c = count(y);
+    const bool lo = !d.channel || y > 0, hi = !d.channel || y < d.ny - 1;
+    const int ylo = I.ym(y), yhi = I.yp(y), clo = count(ylo), chi = count(yhi);
+    // own reds of planes z0 - 1 ... z0 + ZU
+    T red[ZU + 2];
+#pragma unroll
+    for (int u = 0; u < ZU + 2; ++u) {
+        const int z = z0 + u - 1;
+        red[u] = flat && u != 1 ? zero : update(zero, I.at(2 * t + ((y + z) & 1), y, I.wz(z)), c);
+    }
     T val[ZU];
-    int at[ZU], other[ZU];
 #pragma unroll
     for (int u = 0; u < ZU; ++u) {
-        const int z = z0 + u, p = (y + z) & 1, x = 2 * t + p;
-        int c = d.nz == 1 ? 4 : 6;
+        const int z = z0 + u, p = (y + z) & 1, x = 2 * t + 1 - p;
+        T S = red[u + 1] + update(zero, I.at(p ? I.xm(2 * t) : I.xp(2 * t + 1), y, z), c);
+        if (!flat) S = S + (red[u] + red[u + 2]);
         if (d.channel) {
-            if (!(y > 0)) --c;
-            if (!(y < d.ny - 1)) --c;
+            if (lo) S += update(zero, I.at(x, ylo, z), clo);
+            if (hi) S += update(zero, I.at(x, yhi, z), chi);
+        } else {
+            S += update(zero, I.at(x, ylo, z), clo) + update(zero, I.at(x, yhi, z), chi);
         }
-        const int i = I.at(x, y, z);
-        val[u] = (zero - b[i] * k.inv) * lap_rcount<T>(c);
-        if (omega != T(1)) val[u] = val[u] + (omega - T(1)) * (val[u] - zero);
-        at[u] = i;
-        other[u] = I.at(2 * t + 1 - p, y, z);
+        val[u] = update(S, I.at(x, y, z), c);
     }
 #pragma unroll
     for (int u = 0; u < ZU; ++u) {
-        xv[at[u]] = val[u];
-        xv[other[u]] = zero;
+        const int z = z0 + u, p = (y + z) & 1;
+        xv[I.at(2 * t + p, y, z)] = red[u + 1];
+        xv[I.at(2 * t + 1 - p, y, z)] = val[u];
     }
 }
 template <typename T, int ZU, int MINB, typename IX>
@@ -738,13 +766,11 @@ __device__ __forceinline__ void restrict_cell(const Dims& d, T* coarse, const T*
         (RED ? full4<T>(row(0), row(1), row(2), row(3)) : restrict_plane<T>(tap)) * T(1.0 / 64.0);
 }
 
-// zero (optional): the coarse iterate, set to zero at every coarse cell
 template <typename T, bool RED>
-__global__ void k_restrict(Dims d, T* __restrict__ coarse, const T* __restrict__ fine, T* __restrict__ zero) {
+__global__ void k_restrict(Dims d, T* __restrict__ coarse, const T* __restrict__ fine) {
     const int xc = blockIdx.x * BX + threadIdx.x, yc = blockIdx.y * BY + threadIdx.y;
     if (xc >= d.nx / 2 || yc >= d.ny / 2) return;
     restrict_cell<T, RED>(d, coarse, fine, xc, yc);
-    if (zero) zero[xc + (d.nx / 2) * yc] = T(0);
 }
 
 // Trilinear prolongation (27,9,3,1)/64, src/mg/solver.h:71-151 (prolong_plane4,
@@ -822,14 +848,12 @@ __device__ __forceinline__ void restrict_cell2(const Dims& d, const IX& I, T* co
 }
 
 template <typename T, bool RED, typename IX>
-__global__ void k_restrict2(Dims d, T* __restrict__ coarse, const T* __restrict__ fine, int rev,
-                            T* __restrict__ zero) {
+__global__ void k_restrict2(Dims d, T* __restrict__ coarse, const T* __restrict__ fine, int rev) {
     const IX I(d);
     const uint3 B = block_at(rev);
     const int xc = B.x * BX + threadIdx.x, yc = B.y * BY + threadIdx.y, zc = B.z;
     if (xc >= d.nx / 2 || yc >= d.ny / 2) return;
     restrict_cell2<T, RED>(d, I, coarse, fine, xc, yc, zc);
-    if (zero) zero[I.coarse(xc, yc, zc)] = T(0);
 }
 
 template <typename T, bool ADD, bool BLACK, typename IX>
@@ -844,8 +868,7 @@ __device__ __forceinline__ void prolong_cell2(const Dims& d, const IX& I, T* fin
         [&](int a, int b, int c, T v, T s) { prolong_put<T, ADD>(fine, I.at(a, b, c), v, s); });
 }
 
-// Fine-level residual fused with the full-weighting restriction and the
-// zeroing of the coarse iterate. A block takes RR_T x RR_T coarse columns
+// Fine-level residual fused with the full-weighting restriction. A block takes RR_T x RR_T coarse columns
 // and RR_CZ coarse planes; r = b - L x of its fine tile (2 RR_T + 2 cells a
 // side: the taps reach one fine cell beyond the tile's own) is formed in
 // shared memory, one fine plane at a time, in a ring of the four planes the
@@ -862,7 +885,7 @@ constexpr int RR_RS = 40, RR_ODD = 20;
 __device__ __forceinline__ int rr_at(int jy, int jx) { return jy * RR_RS + (jx & 1) * RR_ODD + (jx >> 1); }
 
 template <typename T, int RR_CZ>
-__global__ void __launch_bounds__(RR_THREADS) k_resid_restrict2(Dims d, T* __restrict__ cb, T* __restrict__ cx,
+__global__ void __launch_bounds__(RR_THREADS) k_resid_restrict2(Dims d, T* __restrict__ cb,
                                                                const T* __restrict__ xv, const T* __restrict__ b,
                                                                int rev, bool red) {
     __shared__ T ring[4][RR_F * RR_RS];
@@ -924,7 +947,6 @@ __global__ void __launch_bounds__(RR_THREADS) k_resid_restrict2(Dims d, T* __res
             [&](int kz, int ky, int kx) { return ring[(2 * zc - 1 + kz) & 3][row[ky] * RR_RS + col[kx]]; });
         const int o = xc | (yc << (I.lx - 1)) | (zc << (I.lxy - 2));
         cb[o] = acc;
-        cx[o] = T(0);
         __syncthreads();  // the next fills overwrite the two oldest planes
     }
 }
@@ -1013,8 +1035,7 @@ __device__ __forceinline__ void quad_get(const T* p, T (&v)[16 / sizeof(T)]) {
 
 template <typename T, int CZ>
 __global__ void __launch_bounds__(32 * kTrBY) k_restrict_cols(Dims d, T* __restrict__ coarse,
-                                                              const T* __restrict__ fine, int rev,
-                                                              T* __restrict__ zero) {
+                                                              const T* __restrict__ fine, int rev) {
     using TT = TrTile<T>;
     constexpr int CE = TT::CE, M = CE / 2;  // M coarse cells per lane
     constexpr int NP = 2 * CZ + 2;          // fine planes of the block
@@ -1100,10 +1121,8 @@ __global__ void __launch_bounds__(32 * kTrBY) k_restrict_cols(Dims d, T* __restr
         const int o = co | ((zc0 + k) << (I.lxy - 2));
         if constexpr (M == 2) {
             *reinterpret_cast<float2*>(coarse + o) = make_float2(acc[0], acc[1]);
-            if (zero) *reinterpret_cast<float2*>(zero + o) = make_float2(0.f, 0.f);
         } else {
             coarse[o] = acc[0];
-            if (zero) zero[o] = T(0);
         }
 #pragma unroll
         for (int m = 0; m < M; ++m) {
@@ -1140,7 +1159,6 @@ constexpr size_t kRrSmem = sizeof(float) * ((size_t)kRrX * kRrXRows * kRrXW + (s
 
 template <int CZ, bool CH>
 __global__ void __launch_bounds__(32 * kTrBY, 2) k_resid_restrict_cols(Dims d, float* __restrict__ cb,
-                                                                    float* __restrict__ cxz,
                                                                     const float* __restrict__ xv,
                                                                     const float* __restrict__ bv, int rev) {
     constexpr int NP = 2 * CZ + 2;  // fine planes restricted (residuals formed)
@@ -1310,7 +1328,6 @@ __global__ void __launch_bounds__(32 * kTrBY, 2) k_resid_restrict_cols(Dims d, f
             const float a0 = full4<float>(p[0][0], p[1][0], p[2][0], p[3][0]) * float(1.0 / 512.0);
             const float a1 = full4<float>(p[0][1], p[1][1], p[2][1], p[3][1]) * float(1.0 / 512.0);
             *reinterpret_cast<float2*>(cb + o) = make_float2(a0, a1);
-            *reinterpret_cast<float2*>(cxz + o) = make_float2(0.f, 0.f);
         }
     }
     pipe::wait_pending<0>();
@@ -1567,23 +1584,28 @@ bool rbgs_pair_ok(const Dims& d) {
     return d.nz > 1 && d.nx >= 2 * BX && d.ny % BY == 0 && d.nz % kPairZU == 0 && ix2_ok(d);
 }
 
-// First colour of a sweep from x = 0 (x's contents ignored and overwritten):
-// the FP32 batched kernel's own form (k_rbgs_z2b_init), elsewhere a memset of
-// x and the red colour. AFMIB_INIT_SWEEP=0 takes the memset everywhere (read
-// at every launch, so that a test can compare both in one process).
+// A sweep from x = 0 (x's contents ignored and overwritten). AFMIB_INIT_SWEEP=0: a
+// memset of x and the two colours (read at every launch, so that a test can compare
+// both in one process).
 template <typename T>
-void launch_rbgs_from_zero(const Dims& d, T* x, const T* b, cudaStream_t s, double omega, int rev) {
+void launch_rbgs_first(const Dims& d, T* x, const T* b, cudaStream_t s, double omega, int rev) {
     const char* e = std::getenv("AFMIB_INIT_SWEEP");
-    const bool off = e && e[0] == '0';
-    if (d.nx < kOmegaMinNx) omega = 1.0;
-    if (!off && sizeof(T) == sizeof(float) && d.nz % kZU32 == 0 && d.nx >= batch_min_nx() && !rbgs_pair_ok(d)) {
-        const dim3 g((d.nx / 2 + BX - 1) / BX, (d.ny + BY - 1) / BY, d.nz / kZU32);
-        AFMIB_IX(d, (k_rbgs_z2b_init<T, kZU32, 6, IX><<<g, dim3(BX, BY), 0, s>>>(d, lap_k<T>(d), T(omega), x, b, rev,
-                                                                               T(0))));
+    if ((e && e[0] == '0') || d.nx % 2) {
+        cudaMemsetAsync(x, 0, (size_t)d.ncell() * sizeof(T), s);
+        launch_rbgs<T>(d, 0, x, b, s, omega, rev);
+        launch_rbgs<T>(d, 1, x, b, s, omega, rev);
         return;
     }
-    cudaMemsetAsync(x, 0, (size_t)d.ncell() * sizeof(T), s);
-    launch_rbgs<T>(d, 0, x, b, s, omega, rev);
+    if (d.nx < kOmegaMinNx) omega = 1.0;
+    constexpr int ZU = 4, MINB = sizeof(T) == sizeof(float) ? 6 : 4;
+    const int gx = (d.nx / 2 + BX - 1) / BX, gy = (d.ny + BY - 1) / BY;
+    const LapK<T> k = lap_k<T>(d);
+    if (d.nz % ZU == 0 && d.nx >= batch_min_nx())
+        AFMIB_IX(d, (k_rbgs_first<T, ZU, MINB, IX><<<dim3(gx, gy, d.nz / ZU), dim3(BX, BY), 0, s>>>(d, k, T(omega), x, b,
+                                                                                                 rev, T(0))));
+    else
+        AFMIB_IX(d, (k_rbgs_first<T, 1, MINB, IX><<<dim3(gx, gy, d.nz), dim3(BX, BY), 0, s>>>(d, k, T(omega), x, b, rev,
+                                                                                           T(0))));
 }
 
 template <typename T>
@@ -1725,26 +1747,25 @@ inline dim3 transfer_grid(const Dims& d, int planes, int bx = 32) {
 }
 
 template <typename T>
-void launch_restrict(const Dims& d, T* coarse, const T* fine, cudaStream_t s, int rev, T* zero, bool red) {
+void launch_restrict(const Dims& d, T* coarse, const T* fine, cudaStream_t s, int rev, bool red) {
     if constexpr (sizeof(T) == sizeof(float)) {
-        if (!red && transfer_cols_ok(d, fine, coarse) && (d.nx / 2) % TrTile<T>::CX == 0 &&
-            (reinterpret_cast<uintptr_t>(zero) & 15) == 0) {
+        if (!red && transfer_cols_ok(d, fine, coarse) && (d.nx / 2) % TrTile<T>::CX == 0) {
             const int z = transfer_planes(d, TrTile<T>::CX);
             const dim3 g = transfer_grid(d, z, TrTile<T>::CX), b(32, kTrBY);
-            if (z == 8) k_restrict_cols<T, 8><<<g, b, 0, s>>>(d, coarse, fine, rev, zero);
-            else if (z == 4) k_restrict_cols<T, 4><<<g, b, 0, s>>>(d, coarse, fine, rev, zero);
-            else if (z == 2) k_restrict_cols<T, 2><<<g, b, 0, s>>>(d, coarse, fine, rev, zero);
-            else k_restrict_cols<T, 1><<<g, b, 0, s>>>(d, coarse, fine, rev, zero);
+            if (z == 8) k_restrict_cols<T, 8><<<g, b, 0, s>>>(d, coarse, fine, rev);
+            else if (z == 4) k_restrict_cols<T, 4><<<g, b, 0, s>>>(d, coarse, fine, rev);
+            else if (z == 2) k_restrict_cols<T, 2><<<g, b, 0, s>>>(d, coarse, fine, rev);
+            else k_restrict_cols<T, 1><<<g, b, 0, s>>>(d, coarse, fine, rev);
             return;
         }
     }
     dim3 g((d.nx / 2 + BX - 1) / BX, (d.ny / 2 + BY - 1) / BY, d.nz == 1 ? 1 : d.nz / 2);
     if (d.nz > 1)
-        AFMIB_IX(d, (red ? k_restrict2<T, true, IX><<<g, dim3(BX, BY), 0, s>>>(d, coarse, fine, rev, zero)
-                         : k_restrict2<T, false, IX><<<g, dim3(BX, BY), 0, s>>>(d, coarse, fine, rev, zero)));
+        AFMIB_IX(d, (red ? k_restrict2<T, true, IX><<<g, dim3(BX, BY), 0, s>>>(d, coarse, fine, rev)
+                         : k_restrict2<T, false, IX><<<g, dim3(BX, BY), 0, s>>>(d, coarse, fine, rev)));
     else
-        red ? k_restrict<T, true><<<g, dim3(BX, BY), 0, s>>>(d, coarse, fine, zero)
-            : k_restrict<T, false><<<g, dim3(BX, BY), 0, s>>>(d, coarse, fine, zero);
+        red ? k_restrict<T, true><<<g, dim3(BX, BY), 0, s>>>(d, coarse, fine)
+            : k_restrict<T, false><<<g, dim3(BX, BY), 0, s>>>(d, coarse, fine);
 }
 // Fine-level residual and restriction in one pass. AFMIB_RESID_RESTRICT
 // (read at every call, so that a test can compare the paths in one process):
@@ -1754,7 +1775,7 @@ void launch_restrict(const Dims& d, T* coarse, const T* fine, cudaStream_t s, in
 // (k_resid_restrict2) on levels with nx >= AFMIB_RESID_RESTRICT_MIN_NX
 // (default 256; on smaller levels its grid of 2 RR_T x 2 RR_T fine columns
 // per block leaves SMs idle); "0": the residual and restriction kernels.
-static int rr_mode(const Dims& d, size_t elem, const void* x, const void* b, const void* cb, const void* cx) {
+static int rr_mode(const Dims& d, size_t elem, const void* x, const void* b, const void* cb) {
     const char* e = std::getenv("AFMIB_RESID_RESTRICT");
     const char m = e ? e[0] : '2';
     if (m == '1') {
@@ -1766,14 +1787,13 @@ static int rr_mode(const Dims& d, size_t elem, const void* x, const void* b, con
     const char* mn = std::getenv("AFMIB_RR_COLS_MIN_NX");
     const int min_nx = mn ? std::atoi(mn) : 256;
     const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(b) |
-                           reinterpret_cast<uintptr_t>(cb) | reinterpret_cast<uintptr_t>(cx)) & 15) == 0;
+                           reinterpret_cast<uintptr_t>(cb)) & 15) == 0;
     return d.nz > 1 && d.nx >= min_nx && ix2_ok(d) && (d.nx / 2) % 64 == 0 && (d.ny / 2) % kTrBY == 0 && aligned
                ? 2
                : 0;
 }
-bool resid_restrict_fused_ok(const Dims& d, size_t elem, const void* x, const void* b, const void* cb,
-                             const void* cx) {
-    return rr_mode(d, elem, x, b, cb, cx) != 0;
+bool resid_restrict_fused_ok(const Dims& d, size_t elem, const void* x, const void* b, const void* cb) {
+    return rr_mode(d, elem, x, b, cb) != 0;
 }
 
 void mg_kernel_attributes() {
@@ -1789,10 +1809,10 @@ void mg_kernel_attributes() {
 }
 
 template <typename T>
-void launch_resid_restrict(const Dims& d, T* coarse_b, T* coarse_x, const T* x, const T* b, cudaStream_t s, int rev,
+void launch_resid_restrict(const Dims& d, T* coarse_b, const T* x, const T* b, cudaStream_t s, int rev,
                            bool red) {
     if constexpr (sizeof(T) == sizeof(float)) {
-        if (rr_mode(d, sizeof(T), x, b, coarse_b, coarse_x) == 2) {
+        if (rr_mode(d, sizeof(T), x, b, coarse_b) == 2) {
             // coarse planes per block: the largest of 8, 4, 2 that leaves at least
             // AFMIB_RR_MIN_BLOCKS (default 512) blocks (two resident per SM)
             const char* e = std::getenv("AFMIB_RR_MIN_BLOCKS");
@@ -1807,13 +1827,12 @@ void launch_resid_restrict(const Dims& d, T* coarse_b, T* coarse_x, const T* x, 
                 }
             const dim3 g(d.nx / 2 / 64, d.ny / 2 / kTrBY, cz / z), blk(32, kTrBY);
             float* cbf = reinterpret_cast<float*>(coarse_b);
-            float* cxf = reinterpret_cast<float*>(coarse_x);
             const float* xf = reinterpret_cast<const float*>(x);
             const float* bf = reinterpret_cast<const float*>(b);
 #define AFMIB_RR_COLS(CZV)                                                                            \
     do {                                                                                              \
-        if (d.channel) k_resid_restrict_cols<CZV, true><<<g, blk, kRrSmem, s>>>(d, cbf, cxf, xf, bf, rev); \
-        else k_resid_restrict_cols<CZV, false><<<g, blk, kRrSmem, s>>>(d, cbf, cxf, xf, bf, rev);         \
+        if (d.channel) k_resid_restrict_cols<CZV, true><<<g, blk, kRrSmem, s>>>(d, cbf, xf, bf, rev); \
+        else k_resid_restrict_cols<CZV, false><<<g, blk, kRrSmem, s>>>(d, cbf, xf, bf, rev);         \
     } while (0)
             if (z == 8) AFMIB_RR_COLS(8);
             else if (z == 4) AFMIB_RR_COLS(4);
@@ -1828,10 +1847,10 @@ void launch_resid_restrict(const Dims& d, T* coarse_b, T* coarse_x, const T* x, 
     const int cols = (d.nx / 2 / RR_T) * (d.ny / 2 / RR_T), cz = d.nz / 2;
     if (cz % 8 == 0 && cols * (cz / 8) >= 2 * 152)
         k_resid_restrict2<T, 8><<<dim3(d.nx / 2 / RR_T, d.ny / 2 / RR_T, cz / 8), RR_THREADS, 0, s>>>(
-            d, coarse_b, coarse_x, x, b, rev, red);
+            d, coarse_b, x, b, rev, red);
     else
         k_resid_restrict2<T, 2><<<dim3(d.nx / 2 / RR_T, d.ny / 2 / RR_T, cz / 2), RR_THREADS, 0, s>>>(
-            d, coarse_b, coarse_x, x, b, rev, red);
+            d, coarse_b, x, b, rev, red);
 }
 
 template <typename T>
@@ -1909,12 +1928,12 @@ void launch_coarse_solve(const Dims& d, T* x, T* b, T* r, T* p, T* q, double tol
     template void launch_residual<T>(const Dims&, T*, const T*, const T*, RedScratch*, double*, cudaStream_t, int); \
     template void launch_residual_red<T>(const Dims&, T*, const T*, const T*, cudaStream_t, int);                  \
     template void launch_rbgs<T>(const Dims&, int, T*, const T*, cudaStream_t, double, int);                        \
-    template void launch_rbgs_from_zero<T>(const Dims&, T*, const T*, cudaStream_t, double, int);                  \
+    template void launch_rbgs_first<T>(const Dims&, T*, const T*, cudaStream_t, double, int);                      \
     template PipeCfg rbgs_pipe_cfg<T>(const Dims&);                                                      \
     template void launch_rbgs_pipe<T>(const Dims&, const PipeCfg&, const T*, T*, const T*, int*, cudaStream_t); \
-    template void launch_restrict<T>(const Dims&, T*, const T*, cudaStream_t, int, T*, bool);               \
+    template void launch_restrict<T>(const Dims&, T*, const T*, cudaStream_t, int, bool);                   \
     template void launch_prolong_add<T>(const Dims&, T*, const T*, cudaStream_t, int, bool);                \
-    template void launch_resid_restrict<T>(const Dims&, T*, T*, const T*, const T*, cudaStream_t, int, bool); \
+    template void launch_resid_restrict<T>(const Dims&, T*, const T*, const T*, cudaStream_t, int, bool); \
     template void launch_prolong_assign<T>(const Dims&, T*, const T*, cudaStream_t);                     \
     template void launch_coarse_solve<T>(const Dims&, T*, T*, T*, T*, T*, double, int, int*, cudaStream_t);
 

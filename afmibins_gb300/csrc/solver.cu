@@ -603,8 +603,7 @@ int pass_dir(afmib_solver* s, const Dims& d, size_t elem) {
     return s->pass_rev;
 }
 
-// from_zero: x starts at zero and its contents are not (the first colour
-// writes both colours: launch_rbgs_from_zero)
+// from_zero: x starts at zero and its contents are not (launch_rbgs_first)
 template <typename T>
 int smooth(afmib_solver* s, MGLevelT<T>& L, int sweeps, bool from_zero = false) {
     const double Ns = (double)L.d.ncell() * sizeof(T);
@@ -631,9 +630,11 @@ int smooth(afmib_solver* s, MGLevelT<T>& L, int sweeps, bool from_zero = false) 
     }
     for (; j < sweeps; ++j) {
         if (from_zero && j == 0) {
-            ProfScope ps(s, id, 1.5 * Ns);
-            launch_rbgs_from_zero<T>(L.d, L.x, L.b, s->st, omega, pass_dir(s, L.d, sizeof(T)));
-        } else {
+            ProfScope ps(s, id, 2 * Ns);
+            launch_rbgs_first<T>(L.d, L.x, L.b, s->st, omega, pass_dir(s, L.d, sizeof(T)));
+            continue;
+        }
+        {
             ProfScope ps(s, id, 1.5 * Ns);
             launch_rbgs<T>(L.d, 0, L.x, L.b, s->st, omega, pass_dir(s, L.d, sizeof(T)));
         }
@@ -723,10 +724,10 @@ int vcycle(afmib_solver* s, size_t l, bool x_zero = false) {
     const bool red = restrict_after_sweep(L.d, sizeof(T), nu1);
     TRY(smooth(s, L, nu1, x_zero));
     MGLevelT<T>& C = lv[l + 1];
-    if (resid_restrict_fused_ok(L.d, sizeof(T), L.x, L.b, C.b, C.x)) {
-        // x, b read; coarse b and x written (the fine residual stays on chip)
-        ProfScope ps(s, fine ? P_RESID_RESTRICT0 : P_RESID_RESTRICT, 2 * Ns + 2 * Ns / 8);
-        launch_resid_restrict<T>(L.d, C.b, C.x, L.x, L.b, s->st, pass_dir(s, L.d, sizeof(T)), red);
+    if (resid_restrict_fused_ok(L.d, sizeof(T), L.x, L.b, C.b)) {
+        // x, b read; coarse b written (the fine residual stays on chip)
+        ProfScope ps(s, fine ? P_RESID_RESTRICT0 : P_RESID_RESTRICT, 2 * Ns + Ns / 8);
+        launch_resid_restrict<T>(L.d, C.b, L.x, L.b, s->st, pass_dir(s, L.d, sizeof(T)), red);
     } else {
         {
             ProfScope ps(s, fine ? P_RESID0 : P_RESID, 3 * Ns);
@@ -734,13 +735,12 @@ int vcycle(afmib_solver* s, size_t l, bool x_zero = false) {
             else launch_residual<T>(L.d, L.r, L.x, L.b, nullptr, nullptr, s->st, pass_dir(s, L.d, sizeof(T)));
         }
         {
-            // the coarse iterate starts from zero: set in the same pass
-            ProfScope ps(s, fine ? P_RESTRICT0 : P_RESTRICT, Ns + Ns / 8 + Ns / 8);
-            launch_restrict<T>(L.d, C.b, L.r, s->st, pass_dir(s, L.d, sizeof(T)), C.x, red);
+            ProfScope ps(s, fine ? P_RESTRICT0 : P_RESTRICT, Ns + Ns / 8);
+            launch_restrict<T>(L.d, C.b, L.r, s->st, pass_dir(s, L.d, sizeof(T)), red);
         }
     }
     CKL();
-    TRY(vcycle<T>(s, l + 1));
+    TRY(vcycle<T>(s, l + 1, true));
     {
         ProfScope ps(s, fine ? P_PROLONG0 : P_PROLONG, 2 * Ns + Ns / 8);
         launch_prolong_add<T>(L.d, L.x, C.x, s->st, pass_dir(s, L.d, sizeof(T)),
@@ -966,18 +966,20 @@ int gs_sweeps(const Dims& d, double scale, double rel_tol) {
     return sweeps >= 1 && sweeps <= 10 ? sweeps : -1;
 }
 
-// FP32 inner solve by red-black Gauss-Seidel sweeps in place on e32 from
-// zero; false when the grid does not take the kernel (nothing launched)
-bool gs_inner32(afmib_solver* s, int comp, double scale, int sweeps) {
-    const long long N = s->N();
-    for (int j = 0; j < sweeps; ++j)
+// FP32 inner solve by red-black Gauss-Seidel sweeps on e32 from zero, launched on
+// q; walk() gives each launch's block order
+template <typename F>
+void gs_inner32(afmib_solver* s, int comp, double scale, int sweeps, const float* b, cudaStream_t q, F walk) {
+    const double Ns = (double)s->N() * sizeof(float);
+    {
+        ProfScope ps(s, P_JACOBI, 2 * Ns, 1, q);
+        launch_helm_rbgs_first<float>(s->d, comp, scale, s->e32, b, q, walk());
+    }
+    for (int j = 1; j < sweeps; ++j)
         for (int color = 0; color < 2; ++color) {
-            ProfScope ps(s, P_JACOBI, (double)N * 4 * 1.5);
-            if (!launch_helm_rbgs<float>(s->d, comp, scale, color, j == 0 && color == 0, s->e32, s->d32, s->st,
-                                         pass_dir(s, s->d, sizeof(float))))
-                return false;
+            ProfScope ps(s, P_JACOBI, 1.5 * Ns, 1, q);
+            launch_helm_rbgs<float>(s->d, comp, scale, color, s->e32, b, q, walk());
         }
-    return true;
 }
 
 // FP32 inner solve by fixed Jacobi sweeps: e32 = H^-1 d32 to rel_tol
@@ -1016,7 +1018,8 @@ int helm_solve_mixed(afmib_solver* s, int comp, double scale, double* x, const d
         if (outer >= s->cfg.max_mg_cycles) return s->fail(AFMIB_ERR_NOCONV, "defect-correction cap reached (Helmholtz)");
         const int gsw = s->gs_inner ? gs_sweeps(s->d, scale, s->cfg.inner_tol) : -1;
         const int sweeps = s->jacobi_inner ? jacobi_sweeps(s->d, scale, s->cfg.inner_tol) : -1;
-        if (gsw > 0 && gs_inner32(s, comp, scale, gsw)) {
+        if (gsw > 0 && helm_rbgs_ok(s->d)) {
+            gs_inner32(s, comp, scale, gsw, s->d32, s->st, [&] { return pass_dir(s, s->d, sizeof(float)); });
         } else if (sweeps > 0) {
             TRY(jacobi_inner32(s, comp, scale, sweeps));
         } else {
@@ -1094,14 +1097,8 @@ int helm_solve3_mixed(afmib_solver* s, double scale, double* const x[3], const d
             break;
         }
         CK(cudaStreamWaitEvent(s->aux, s->ev_def[c], 0));
-        int rev = 1;  // the defect's walk ended at the last z planes
-        for (int j = 0; j < gsw; ++j)
-            for (int color = 0; color < 2; ++color) {
-                ProfScope ps(s, P_JACOBI, (double)N * 4 * 1.5, 1, s->aux);
-                launch_helm_rbgs<float>(d, c, scale, color, j == 0 && color == 0, s->e32, s->d32c[c], s->aux,
-                                        big ? rev : 0);
-                rev ^= 1;
-            }
+        int rev = 0;  // the defect's walk ended at the last z planes
+        gs_inner32(s, c, scale, gsw, s->d32c[c], s->aux, [&] { return big ? rev ^= 1 : 0; });
         if (df) {
             ProfScope ps(s, P_HELM_UPDATE, (double)N * (8 + 4 + 8 + 8 + 8 + 4), 1, s->aux);
             launch_helm_update_df(d, c, scale, x[c], s->e32, s->d32c[c], s->rlo[c], s->red2, s->scal + 12 + c,
