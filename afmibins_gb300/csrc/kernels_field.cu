@@ -5,6 +5,7 @@
 // output array.
 #include "dfloat.cuh"
 #include "kernels.h"
+#include "mg_cells.cuh"
 #include <algorithm>
 #include <cmath>
 
@@ -1669,7 +1670,8 @@ __global__ void __launch_bounds__(BX * BY, MINB) k_helm_rbgs2b(Dims d, int comp,
 // b / diag; the reds that a black cell sums are formed from b on the fly. A thread
 // owns the pairs (2t, 2t+1) of its (y, z) column, one red and one black cell each:
 // of the black cell's six reds one is the pair's own, the two along z are the own
-// reds of the pairs above and below, and the other three are formed again.
+// reds of the pairs above and below, and the other three are formed again. The same
+// bits as a memset of x and the two colours.
 // Bytes bound: 2 words a cell against 4.5 for a red launch that also clears the
 // black cells and a black one.
 template <typename T, int ZU, int MINB, typename IX>
@@ -1686,20 +1688,21 @@ __global__ void __launch_bounds__(BX * BY, MINB) k_helm_first(Dims d, int comp, 
 #pragma unroll
     for (int u = 0; u < ZU + 2; ++u) {
         const int z = z0 + u - 1;
-        red[u] = b[I.at(2 * t + ((y + z) & 1), y, I.wz(z))] * rd;
+        red[u] = mul_t(b[I.at(2 * t + ((y + z) & 1), y, I.wz(z))], rd);
     }
     T val[ZU];
 #pragma unroll
     for (int u = 0; u < ZU; ++u) {
         const int z = z0 + u, p = (y + z) & 1, x = 2 * t + 1 - p;
-        const T sx = red[u + 1] + b[I.at(p ? I.xm(2 * t) : I.xp(2 * t + 1), y, z)] * rd;
+        const T sx = red[u + 1] + mul_t(b[I.at(p ? I.xm(2 * t) : I.xp(2 * t + 1), y, z)], rd);
         const T sz = red[u] + red[u + 2];
-        const T lo = b[I.at(x, ylo, z)] * rlo, hi = b[I.at(x, yhi, z)] * rhi;
-        T hx;  // H x at x = 0 here (helm_point2's forms)
-        if (cell_rows && (y == 0 || y == d.ny - 1)) hx = k.off * (sx + sz) + k.offw * (y == 0 ? hi : lo);
-        else if (cell_rows) hx = k.off * (sx + sz) + k.off * (lo + hi);
-        else hx = fixed ? T(0) : k.off * (sx + (lo + hi) + sz);
-        val[u] = (b[I.at(x, y, z)] - hx) * rd;
+        const T lo = mul_t(b[I.at(x, ylo, z)], rlo), hi = mul_t(b[I.at(x, yhi, z)], rhi);
+        // H x at x = 0 here: helm_point2's forms, with the roundings of its products
+        T hx;
+        if (cell_rows && (y == 0 || y == d.ny - 1)) hx = fma_t(k.off, sx + sz, mul_t(k.offw, y == 0 ? hi : lo));
+        else if (cell_rows) hx = fma_t(k.off, sx + sz, mul_t(k.off, lo + hi));
+        else hx = fixed ? T(0) : mul_t(k.off, sx + (lo + hi) + sz);
+        val[u] = mul_t(b[I.at(x, y, z)] - hx, rd);
     }
 #pragma unroll
     for (int u = 0; u < ZU; ++u) {

@@ -31,6 +31,26 @@ inline bool prolong_before_sweep(const Dims& d, size_t elem, int nu2) { return r
 __device__ __forceinline__ float fma_t(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ double fma_t(double a, double b, double c) { return fma(a, b, c); }
 
+__device__ __forceinline__ float mul_t(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_t(double a, double b) { return __dmul_rn(a, b); }
+
+// Gauss-Seidel value (S - b / n^2) / c. The product is rounded here: where the
+// value is a term of another sum the compiler would fuse it into that addition,
+// and a value formed twice would not have the same bits.
+template <typename T>
+__device__ __forceinline__ T gs_value(T S, T b, T inv, T rc) {
+    return mul_t(fma_t(-b, inv, S), rc);
+}
+
+// FP32 sweeps may be over-relaxed, FP64 ones are plain: the test and the two
+// operations, left to the compiler, were executed and selected from, three of ten
+// FP64 instructions per cell.
+template <typename T>
+__device__ __forceinline__ T over_relaxed(T v, T old, T omega) {
+    if (sizeof(T) == sizeof(float) && omega != T(1)) v = v + (omega - T(1)) * (v - old);
+    return v;
+}
+
 // f0 + 3 f1 + 3 f2 + f3
 template <typename T>
 __device__ __forceinline__ T full4(T f0, T f1, T f2, T f3) {
