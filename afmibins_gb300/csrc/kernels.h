@@ -212,7 +212,7 @@ bool launch_lap_defect_bfp(const Dims& d, float* r, const double* x, const doubl
 void launch_helm_defect_bfp(const Dims& d, int comp, double scale, const double* x, const double* b, float* r,
                             RedScratch sc, double* out, cudaStream_t s);
 // One red (color 0) or black (color 1) Gauss-Seidel half sweep; omega:
-// over-relaxation x + omega (gs - x) on levels with nx >= 64 (1 below).
+// over-relaxation x + omega (gs - x) on FP32 levels with nx >= 64 (1 below, and in FP64).
 // rev (here and in the residual, transfer and Jacobi launchers): blocks in
 // reverse order (block_at, common.cuh) on the batched kernels.
 template <typename T>
@@ -240,12 +240,17 @@ PipeCfg rbgs_pipe_cfg(const Dims& d);
 // solve alone. Only the first level's x and b are global arrays.
 constexpr int kMaxTailLevels = 12;
 constexpr long long kTailCells = 32768;  // largest level (cells) the tail takes
+// Level on which coarsening stops, solved by its inverse matrix: 3000 clocks of the
+// tail for 4^3 cells, against 13000 in FP32 and 26000 in FP64 for smoothed levels of
+// 4^3 and 2^3 cells (8^2 and below: 25000).
+constexpr long long kDirectCells = 64;
 constexpr int kMaxBasis = 256;           // largest coarsest-level extent of the direct solve
 // Orthonormal eigenvectors (row k: mode k, row 0 the constant) and
 // eigenvalues (of the second difference, times n^-2) of the coarsest
 // Laplacian per axis; on a 2D grid vz, lz belong to y and vy, ly are 1, 0.
 struct TailBasis {
     const double *vx = nullptr, *vy = nullptr, *vz = nullptr, *lx = nullptr, *ly = nullptr, *lz = nullptr;
+    const double* inverse = nullptr;  // of levels of at most kDirectCells cells, the constant mode dropped
 };
 template <typename T>
 struct TailLevels {

@@ -352,8 +352,7 @@ __global__ void k_rbgs(Dims d, LapK<T> k, int color, T omega, T* __restrict__ xv
     lap_row2(d, I, xv, x, y, z, S, c);
     const int i = I.at(x, y, z);
     T v = (S - b[i] * k.inv) * lap_rcount<T>(c);
-    if (omega != T(1)) v = v + (omega - T(1)) * (v - xv[i]);
-    xv[i] = v;
+    xv[i] = sizeof(T) == sizeof(float) ? over_relaxed(v, xv[i], omega) : v;
 }
 
 // Batched forms: each thread takes ZU cells along z of its (x, y) column and
@@ -382,7 +381,7 @@ __device__ __forceinline__ void rbgs_z2_body(Dims d, const LapK<T>& k, int color
         lap_row2(d, I, xv, x, y, z, S, c);
         const int i = I.at(x, y, z);
         val[u] = (S - b[i] * k.inv) * lap_rcount<T>(c);
-        if (omega != T(1)) val[u] = val[u] + (omega - T(1)) * (val[u] - xv[i]);
+        if (sizeof(T) == sizeof(float)) val[u] = over_relaxed(val[u], xv[i], omega);
         at[u] = i;
     }
 #pragma unroll
@@ -400,7 +399,8 @@ __global__ void k_rbgs_z2(Dims d, LapK<T> k, int color, T omega, T* __restrict__
 // pair's own, the two along z are the own reds of the pairs above and below, and
 // the other three are formed again (a fifth load each of b, from L1). `zero` is a
 // kernel argument, so that the arithmetic is rbgs_z2_body's and not a folded
-// constant: the same bits as a memset of x and the two colours. With the viscous
+// constant (nor its products fused: gs_value): the same bits as a memset of x and
+// the two colours. With the viscous
 // solves' first sweeps in the same form: IB steps of the mixed form at 256^3 16.20
 // -> 15.77 ms, at 96x80x112 3.88 -> 3.74; FP64 steps unchanged (13.8 ms at 128^3:
 // the reds formed again cost the FP64 pipe what the launch saves).
@@ -421,9 +421,8 @@ __global__ void __launch_bounds__(BX * BY, MINB) k_rbgs_first(Dims d, LapK<T> k,
         return c;
     };
     auto update = [&](T S, int i, int c) {
-        T v = (S - b[i] * k.inv) * lap_rcount<T>(c);
-        if (omega != T(1)) v = v + (omega - T(1)) * (v - zero);
-        return v;
+        T v = gs_value(S, b[i], k.inv, lap_rcount<T>(c));
+        return over_relaxed(v, zero, omega);
     };
     const int c = count(y);
     const bool lo = !d.channel || y > 0, hi = !d.channel || y < d.ny - 1;

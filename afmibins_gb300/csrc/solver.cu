@@ -2041,8 +2041,31 @@ int setup_basis(afmib_solver* s) {
         all.insert(all.end(), V.begin(), V.end());
         all.insert(all.end(), E.begin(), E.end());
     }
+    // the inverse of a small level (rows padded to 16 bytes in all by an even count)
+    const size_t nc = (size_t)d.ncell(), inv0 = all.size() + (all.size() & 1);
+    const bool dense = nc > 1 && nc <= kDirectCells && nc % 2 == 0;
+    if (dense) {
+        all.resize(inv0 + nc * nc, 0.0);
+        const size_t sx = ext[0], sxy = sx * ext[1];
+        std::vector<double> W(nc);  // row of G: V^T diag(1 / lambda) V e_j, mode by mode
+        const double n2 = (double)d.n * (double)d.n;
+        for (size_t k = 1; k < nc; ++k) {
+            const size_t k0 = k % sx, k1 = k / sx % ext[1], k2 = k / sxy;
+            const double lam = n2 * ((all[off[0] + sx * sx + k0] + all[off[1] + (size_t)ext[1] * ext[1] + k1]) +
+                                     all[off[2] + (size_t)ext[2] * ext[2] + k2]);
+            for (size_t i = 0; i < nc; ++i)
+                W[i] = all[off[0] + k0 * sx + i % sx] * all[off[1] + k1 * ext[1] + i / sx % ext[1]] *
+                       all[off[2] + k2 * ext[2] + i / sxy];
+            for (size_t j = 0; j < nc; ++j) {
+                const double c = W[j] / lam;
+                double* row = all.data() + inv0 + j * nc;
+                for (size_t i = 0; i < nc; ++i) row[i] += c * W[i];
+            }
+        }
+    }
     double* dev = nullptr;
     TRY(dalloc(s, &dev, all.size()));
+    if (dense) s->basis.inverse = dev + inv0;
     CK(cudaMemcpyAsync(dev, all.data(), all.size() * sizeof(double), cudaMemcpyHostToDevice, s->st));
     CK(cudaStreamSynchronize(s->st));  // the host copy goes
     for (int a = 0; a < 3; ++a) {
@@ -2184,7 +2207,7 @@ int create(afmib_solver* s, const afmib_config* c, void* stream) {
         // 2D grids (nz == 1) coarsen x and y only
         const bool flat = t.nz == 1;
         while (is_even(t.nx) && is_even(t.ny) && (flat || is_even(t.nz)) && t.nx >= 2 && t.ny >= 2 &&
-               (flat || t.nz >= 2)) {
+               (flat || t.nz >= 2) && t.ncell() > kDirectCells) {
             t.nx /= 2; t.ny /= 2; if (!flat) t.nz /= 2; t.n /= 2;
             ++levels;
             if (t.nx == 1 || t.ny == 1 || (!flat && t.nz == 1)) break;

@@ -56,7 +56,8 @@ typedef struct afmib_config {
     int n;              /* cells per unit length, 0 -> nx (geometry::n) */
     int bc;             /* AFMIB_BC_CHANNEL: the reference's walls in y; AFMIB_BC_PERIODIC */
     int precision;      /* AFMIB_FP64 (drop-in) or AFMIB_MIXED (FP32 inner, FP64 outer) */
-    int mg_levels;      /* coarsenings of the pressure multigrid; 0 -> until a dimension is odd */
+    int mg_levels;      /* coarsenings of the pressure multigrid; 0 -> until a dimension is odd or a level
+                           has at most 64 cells (solved directly) */
     int nu1, nu2;       /* smoothing sweeps of the FP64 V-cycles, 0 -> 2 (src/ns/projection.h:44);
                            the mixed form's FP32 inner cycles run their own V(2,1)
                            with red-black over-relaxation 1.25 on levels >= 64 */
