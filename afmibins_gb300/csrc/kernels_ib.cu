@@ -249,6 +249,106 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const unsigned* __res
     }
 }
 
+// The same order for up to RS_SMALL pairs in one launch of one block, with the
+// tile ranges: the nine launches of three passes and the bins' memsets took 65 us
+// at a few thousand markers, launch after launch. The pairs stay in shared memory
+// (the values as 16 bits: they are positions); a warp owns a contiguous run of them
+// and counts its digits in a column of its own, so that a rank is the warp's count
+// so far plus the rank among the equal digits of the row, and the order is stable.
+constexpr int RSS_THREADS = 1024, RSS_ITEMS = 16, RS_SMALL = RSS_THREADS * RSS_ITEMS, RSS_COLS = RSS_THREADS / 32 + 1;
+
+// ITEMS rows of 32 pairs per warp
+template <int ITEMS>
+__global__ void __launch_bounds__(RSS_THREADS, 1) k_sort_small(unsigned* __restrict__ kio, int* __restrict__ vio, int n,
+                                                              int bits, int cells_per_tile, int ntiles,
+                                                              int* __restrict__ tstart, int* __restrict__ tend,
+                                                              int* __restrict__ counts) {
+    extern __shared__ unsigned rss_smem[];
+    unsigned* sk = rss_smem;                           // [ITEMS * RSS_THREADS]
+    unsigned* cnt = sk + RSS_THREADS * ITEMS;          // [256][RSS_COLS]
+    unsigned* wsum = cnt + 256 * RSS_COLS;             // [32]
+    unsigned short* sv = (unsigned short*)(wsum + 32);  // [ITEMS * RSS_THREADS]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, i0 = warp * (32 * ITEMS) + lane;
+    const unsigned lt = (1u << lane) - 1u;
+    for (int t = tid; t < ntiles; t += RSS_THREADS) tstart[t] = tend[t] = 0;
+    if (tid < 2) counts[tid] = 0;
+    unsigned key[ITEMS], vp[ITEMS];  // vp: value, and position from bit 16
+#pragma unroll
+    for (int r = 0; r < ITEMS; ++r) {
+        const int i = i0 + 32 * r;
+        key[r] = i < n ? kio[i] : 0xffffffffu;  // the padding stays behind equal digits
+        vp[r] = i < n ? (unsigned)vio[i] : 0u;
+    }
+    for (int shift = 0; shift < bits; shift += 8) {
+        if (shift > 0) {
+#pragma unroll
+            for (int r = 0; r < ITEMS; ++r) {
+                key[r] = sk[i0 + 32 * r];
+                vp[r] = sv[i0 + 32 * r];
+            }
+        }
+        for (int i = tid; i < 256 * RSS_COLS; i += RSS_THREADS) cnt[i] = 0;
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < ITEMS; ++r) {
+            const unsigned dig = (key[r] >> shift) & 255u, peers = __match_any_sync(0xffffffffu, dig);
+            unsigned* c = cnt + dig * RSS_COLS + warp;
+            const unsigned before = *c;
+            __syncwarp();
+            if (lane == __ffs(peers) - 1) *c = before + __popc(peers);
+            __syncwarp();
+            vp[r] |= (before + __popc(peers & lt)) << 16;
+        }
+        __syncthreads();
+        // exclusive scan by digit, then warp: a thread has eight columns of a digit
+        unsigned* c = cnt + (tid >> 2) * RSS_COLS + (tid & 3) * 8;
+        unsigned s = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const unsigned v = c[k];
+            c[k] = s;
+            s += v;
+        }
+        unsigned inc = s;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned v = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += v;
+        }
+        if (lane == 31) wsum[warp] = inc;
+        __syncthreads();
+        if (warp == 0) {
+            const unsigned w = wsum[lane];
+            unsigned x = w;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned v = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += v;
+            }
+            wsum[lane] = x - w;
+        }
+        __syncthreads();
+        const unsigned base = wsum[warp] + inc - s;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) c[k] += base;
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < ITEMS; ++r) {
+            const unsigned pos = cnt[((key[r] >> shift) & 255u) * RSS_COLS + warp] + (vp[r] >> 16);
+            sk[pos] = key[r];
+            sv[pos] = (unsigned short)vp[r];
+        }
+        __syncthreads();
+    }
+    for (int p = tid; p < n; p += RSS_THREADS) {
+        const unsigned k = sk[p], t = k / (unsigned)cells_per_tile;
+        kio[p] = k;
+        vio[p] = sv[p];
+        if (p == 0 || sk[p - 1] / (unsigned)cells_per_tile != t) tstart[t] = p;
+        if (p == n - 1 || sk[p + 1] / (unsigned)cells_per_tile != t) tend[t] = p + 1;
+    }
+}
+
 // tile ranges of the sorted keys: tstart/tend zeroed beforehand
 __global__ void k_tile_ranges(const unsigned* __restrict__ keys, int M, int cells_per_tile, int* __restrict__ tstart,
                               int* __restrict__ tend) {
@@ -259,58 +359,61 @@ __global__ void k_tile_ranges(const unsigned* __restrict__ keys, int M, int cell
     if (p == M - 1 || keys[p + 1] / (unsigned)cells_per_tile != t) tend[t] = p + 1;
 }
 
-// Per tile: slot of each occupied tile (or -1) and the list of output tiles
-// whose (TS+4)^3 neighbourhood holds a marker. Slots are handed out by an
-// atomic counter; a slot only names storage, so its value never reaches a result.
-__global__ void k_active_tiles(int ntx, int nty, int ntz, int channel, const int* __restrict__ tstart,
-                               const int* __restrict__ tend, int* __restrict__ list, int* __restrict__ count,
-                               int* __restrict__ slot, int* __restrict__ occ, int* __restrict__ occ_count) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= ntx * nty * ntz) return;
-    if (tend[t] > tstart[t]) {
-        const int sl = atomicAdd(occ_count, 1);
-        slot[t] = sl;
-        occ[sl] = t;
-    } else {
-        slot[t] = -1;
-    }
-    const int tx = t % ntx, ty = (t / ntx) % nty, tz = t / (ntx * nty);
-    bool any = false;
-    for (int dz = -1; dz <= 1 && !any; ++dz)
-        for (int dy = -1; dy <= 1 && !any; ++dy) {
-            int yy = ty + dy;
-            if (channel && (yy < 0 || yy >= nty)) continue;
-            yy = wrapi(yy, nty);
-            for (int dx = -1; dx <= 1 && !any; ++dx) {
-                const int n = wrapi(tx + dx, ntx) + ntx * (yy + nty * wrapi(tz + dz, ntz));
-                if (tend[n] > tstart[n]) any = true;
+// Per tile: the slot of each occupied tile (or -1) with its cell-start table
+// (ctab[slot][c] = first sorted position of local cell c, c = TS^3 the tile's end,
+// by binary search in the tile's sorted key range), and the list of output tiles
+// whose (TS+4)^3 neighbourhood holds a marker. Slots are handed out by an atomic
+// counter; a slot only names storage, so its value never reaches a result. A block
+// takes 16 tiles at a time: a warp each looks at the neighbours, then all threads
+// fill the tables of the occupied ones.
+constexpr int kTileWarps = 16;
+template <int TS, int TZ>
+__global__ void __launch_bounds__(32 * kTileWarps) k_tiles(int ntx, int nty, int ntz, int channel,
+                                                          const unsigned* __restrict__ keys,
+                                                          const int* __restrict__ tstart, const int* __restrict__ tend,
+                                                          int* __restrict__ list, int* __restrict__ count,
+                                                          int* __restrict__ slot, int* __restrict__ ctab) {
+    constexpr int C = TS * TS * TZ;
+    __shared__ int s_slot[kTileWarps];
+    const int nt = ntx * nty * ntz, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int t0 = blockIdx.x * kTileWarps; t0 < nt; t0 += gridDim.x * kTileWarps) {
+        const int t = t0 + warp;
+        if (t < nt) {
+            const int tx = t % ntx, ty = (t / ntx) % nty, tz = t / (ntx * nty);
+            bool any = false;
+            if (lane < 27) {
+                const int yy = ty + lane / 3 % 3 - 1;
+                if (!channel || (yy >= 0 && yy < nty)) {
+                    const int n = wrapi(tx + lane % 3 - 1, ntx) + ntx * (wrapi(yy, nty) + nty * wrapi(tz + lane / 9 - 1, ntz));
+                    any = tend[n] > tstart[n];
+                }
+            }
+            const unsigned vote = __ballot_sync(0xffffffffu, any);
+            if (lane == 0) {
+                const int sl = (vote >> 13) & 1u ? atomicAdd(count + 1, 1) : -1;  // lane 13: the tile itself
+                slot[t] = s_slot[warp] = sl;
+                if (vote) list[atomicAdd(count, 1)] = t;
+            }
+        } else if (lane == 0) {
+            s_slot[warp] = -1;
+        }
+        __syncthreads();
+        for (int w = 0; w < kTileWarps; ++w) {
+            const int sl = s_slot[w];
+            if (sl < 0) continue;
+            const int a = tstart[t0 + w], b = tend[t0 + w];
+            int* row = ctab + (size_t)sl * (C + 1);
+            for (int c = threadIdx.x; c <= C; c += 32 * kTileWarps) {
+                const unsigned key = (unsigned)(t0 + w) * C + c;
+                int lo = a, hi = b;
+                while (lo < hi) {
+                    const int mid = (lo + hi) >> 1;
+                    if (keys[mid] < key) lo = mid + 1; else hi = mid;
+                }
+                row[c] = lo;
             }
         }
-    if (any) list[atomicAdd(count, 1)] = t;
-}
-
-// Cell-start table of every occupied tile: ctab[slot][c] = first sorted
-// position of local cell c (c = TS^3 holds the tile's end), by binary search
-// in the tile's sorted key range.
-template <int TS, int TZ>
-__global__ void __launch_bounds__(TS * TS * TZ) k_cell_table(const unsigned* __restrict__ keys,
-                                                            const int* __restrict__ tstart, const int* __restrict__ tend,
-                                                            const int* __restrict__ occ, const int* __restrict__ occ_count,
-                                                            int* __restrict__ ctab) {
-    constexpr int C = TS * TS * TZ;
-    const int nocc = *occ_count;
-    for (int li = blockIdx.x; li < nocc; li += gridDim.x) {
-        const int t = occ[li];
-        const int a = tstart[t], b = tend[t];
-        const unsigned key = (unsigned)t * C + threadIdx.x;
-        int lo = a, hi = b;
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (keys[mid] < key) lo = mid + 1; else hi = mid;
-        }
-        int* row = ctab + (size_t)li * (C + 1);
-        row[threadIdx.x] = lo;
-        if (threadIdx.x == 0) row[C] = b;
+        __syncthreads();
     }
 }
 
@@ -828,25 +931,37 @@ void radix_sort_pairs(unsigned* keys, int* vals, unsigned* keys_alt, int* vals_a
     *vals_out = va;
 }
 
+// One block up to RS_SMALL markers: 8.5, 20 and 30 us for 512, 5120 and 7500 of them
+// with the tile ranges, against 30, 59 and 60 us in passes over all SMs plus 10 for
+// the ranges and their memsets. At 20000 a block would take longer than the passes.
+bool sort_bins_small_ok(int n) { return n > 0 && n <= RS_SMALL; }
+void sort_bins_small(unsigned* keys, int* vals, int n, int bits, int cells_per_tile, int ntiles, int* tstart, int* tend,
+                     int* counts, cudaStream_t s) {
+    auto launch = [&](auto* kernel, int items) {
+        const size_t smem = sizeof(unsigned) * ((size_t)RSS_THREADS * items + 256 * RSS_COLS + 32) +
+                            sizeof(unsigned short) * (size_t)RSS_THREADS * items;
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        kernel<<<1, RSS_THREADS, smem, s>>>(keys, vals, n, bits, cells_per_tile, ntiles, tstart, tend, counts);
+    };
+    if (n <= 2 * RSS_THREADS) launch(k_sort_small<2>, 2);
+    else if (n <= 8 * RSS_THREADS) launch(k_sort_small<8>, 8);
+    else launch(k_sort_small<RSS_ITEMS>, RSS_ITEMS);
+}
+
 void launch_tile_ranges(const unsigned* keys, int M, int cells_per_tile, int* tstart, int* tend, cudaStream_t s) {
     if (M > 0) k_tile_ranges<<<(M + 255) / 256, 256, 0, s>>>(keys, M, cells_per_tile, tstart, tend);
 }
 
-void launch_active_tiles(int ntx, int nty, int ntz, int channel, const int* tstart, const int* tend, int* list,
-                         int* count, int* slot, int* occ, int* occ_count, cudaStream_t s) {
-    const int nt = ntx * nty * ntz;
-    k_active_tiles<<<(nt + 255) / 256, 256, 0, s>>>(ntx, nty, ntz, channel, tstart, tend, list, count, slot, occ,
-                                                    occ_count);
-}
-
-void launch_cell_table(int TS, int TZ, const unsigned* keys, const int* tstart, const int* tend, const int* occ,
-                       const int* occ_count, int max_occ, int* ctab, cudaStream_t s) {
-    int blocks = max_occ < 152 * 8 ? max_occ : 152 * 8;
-    if (blocks < 1) blocks = 1;
-    if (TS == 8 && TZ == 8) k_cell_table<8, 8><<<blocks, 512, 0, s>>>(keys, tstart, tend, occ, occ_count, ctab);
-    else if (TS == 4 && TZ == 4) k_cell_table<4, 4><<<blocks, 64, 0, s>>>(keys, tstart, tend, occ, occ_count, ctab);
-    else if (TS == 8) k_cell_table<8, 1><<<blocks, 64, 0, s>>>(keys, tstart, tend, occ, occ_count, ctab);
-    else k_cell_table<4, 1><<<blocks, 16, 0, s>>>(keys, tstart, tend, occ, occ_count, ctab);
+void launch_tiles(int TS, int TZ, int ntx, int nty, int ntz, int channel, const unsigned* keys, const int* tstart,
+                  const int* tend, int* list, int* count, int* slot, int* ctab, cudaStream_t s) {
+    const int nt = ntx * nty * ntz, blocks = std::max(1, std::min((nt + kTileWarps - 1) / kTileWarps, 152 * 4));
+    auto launch = [&](auto* kernel) {
+        kernel<<<blocks, 32 * kTileWarps, 0, s>>>(ntx, nty, ntz, channel, keys, tstart, tend, list, count, slot, ctab);
+    };
+    if (TS == 8 && TZ == 8) launch(k_tiles<8, 8>);
+    else if (TS == 4 && TZ == 4) launch(k_tiles<4, 4>);
+    else if (TS == 8) launch(k_tiles<8, 1>);
+    else launch(k_tiles<4, 1>);
 }
 
 template <typename T, int TS, int TZ, typename TC>

@@ -41,13 +41,15 @@ void radix_sort_pairs(unsigned* keys, int* vals, unsigned* keys_alt, int* vals_a
                       unsigned** keys_out, int** vals_out, cudaStream_t s);
 
 void launch_tile_ranges(const unsigned* keys, int M, int cells_per_tile, int* tstart, int* tend, cudaStream_t s);
-// slot[t] = storage slot of occupied tile t (or -1), occ[slot] = t; list of
-// output tiles with a marker in their 3^3-tile neighbourhood.
-void launch_active_tiles(int ntx, int nty, int ntz, int channel, const int* tstart, const int* tend, int* list,
-                         int* count, int* slot, int* occ, int* occ_count, cudaStream_t s);
-// ctab[slot][c]: first sorted position of local cell c of each occupied tile
-void launch_cell_table(int TS, int TZ, const unsigned* keys, const int* tstart, const int* tend, const int* occ,
-                       const int* occ_count, int max_occ, int* ctab, cudaStream_t s);
+// The sorted pairs (in place) and the tile ranges, counts[0..1] zeroed, in one launch
+// for the marker counts that sort_bins_small_ok takes
+bool sort_bins_small_ok(int n);
+void sort_bins_small(unsigned* keys, int* vals, int n, int bits, int cells_per_tile, int ntiles, int* tstart, int* tend,
+                     int* counts, cudaStream_t s);
+// Tiles near markers (list, count[0]) and the occupied tiles' slots (count[1]) and
+// cell-start tables; count zeroed beforehand
+void launch_tiles(int TS, int TZ, int ntx, int nty, int ntz, int channel, const unsigned* keys, const int* tstart,
+                  const int* tend, int* list, int* count, int* slot, int* ctab, cudaStream_t s);
 
 // f_c(face) = scale * sum_k (phi/n)^3 * vol_k * G_c,k over the active tiles
 // (faces of the other tiles, and of active tiles whose neighbourhood holds no

@@ -231,7 +231,7 @@ struct afmib_solver {
     int tile_cells() const { return TS * TS * TZ; }
     // tcount: [0] active output tiles, [1] occupied tiles, [2] the spreading's tile counter
     int *tstart = nullptr, *tend = nullptr, *tlist = nullptr, *tcount = nullptr;
-    int *tslot = nullptr, *tocc = nullptr, *ctab = nullptr;
+    int *tslot = nullptr, *ctab = nullptr;
     int ctab_cap = 0;  // occupied tiles the cell table can hold
     MarkerW<double> mw{};
     MarkerW<float> mw32{};
@@ -1497,23 +1497,25 @@ int bin_markers(afmib_solver* s, const double* P, bool fp32 = false, bool df_wei
         ProfScope ps(s, P_PREP, (double)M * (24 + 4 + 4 + 12 + 6 + 24 * 8));
         launch_marker_prep<double>(s->d, s->TS, M, P, s->keys, s->vals, s->mw, s->dflag, s->st, df_weights);
     }
-    unsigned* ko;
-    int* vo;
-    {
-        ProfScope ps(s, P_SORT, (double)passes * M * 16, 3 * passes);
+    unsigned* ko = s->keys;
+    int* vo = s->vals;
+    const int C = s->tile_cells();
+    if (sort_bins_small_ok(M)) {
+        ProfScope ps(s, P_SORT, (double)M * 16 + 2.0 * s->ntiles * 4);
+        sort_bins_small(s->keys, s->vals, M, key_bits(s), C, s->ntiles, s->tstart, s->tend, s->tcount, s->st);
+    } else {
+        ProfScope ps(s, P_SORT, (double)passes * M * 16, 3 * passes + 1);
         radix_sort_pairs(s->keys, s->vals, s->keys2, s->vals2, M, key_bits(s), s->hist, &ko, &vo, s->st);
+        CK(cudaMemsetAsync(s->tstart, 0, s->ntiles * sizeof(int), s->st));
+        CK(cudaMemsetAsync(s->tend, 0, s->ntiles * sizeof(int), s->st));
+        CK(cudaMemsetAsync(s->tcount, 0, 2 * sizeof(int), s->st));
+        launch_tile_ranges(ko, M, C, s->tstart, s->tend, s->st);
     }
     s->perm = vo;
-    CK(cudaMemsetAsync(s->tstart, 0, s->ntiles * sizeof(int), s->st));
-    CK(cudaMemsetAsync(s->tend, 0, s->ntiles * sizeof(int), s->st));
-    CK(cudaMemsetAsync(s->tcount, 0, 2 * sizeof(int), s->st));
     {
-        const int C = s->tile_cells();
-        ProfScope ps(s, P_TILES, (double)M * 4 + 5.0 * s->ntiles * 4 + (double)std::min(M, s->ntiles) * (C + 1) * 4, 3);
-        launch_tile_ranges(ko, M, C, s->tstart, s->tend, s->st);
-        launch_active_tiles(s->ntx, s->nty, s->ntz, s->d.channel, s->tstart, s->tend, s->tlist, s->tcount, s->tslot,
-                            s->tocc, s->tcount + 1, s->st);
-        launch_cell_table(s->TS, s->TZ, ko, s->tstart, s->tend, s->tocc, s->tcount + 1, s->ctab_cap, s->ctab, s->st);
+        ProfScope ps(s, P_TILES, (double)M * 4 + 5.0 * s->ntiles * 4 + (double)std::min(M, s->ntiles) * (C + 1) * 4);
+        launch_tiles(s->TS, s->TZ, s->ntx, s->nty, s->ntz, s->d.channel, ko, s->tstart, s->tend, s->tlist, s->tcount,
+                     s->tslot, s->ctab, s->st);
     }
     CKL();
     return AFMIB_OK;
@@ -2008,7 +2010,6 @@ int setup_tiles(afmib_solver* s) {
     TRY(dalloc(s, &s->tlist, s->ntiles));
     TRY(dalloc(s, &s->tcount, 3));
     TRY(dalloc(s, &s->tslot, s->ntiles));
-    TRY(dalloc(s, &s->tocc, s->ntiles));
     return AFMIB_OK;
 }
 
