@@ -263,6 +263,17 @@ struct TailLevels {
     TailBasis basis;
     int* status;  // receives 3 where the coarsest right-hand side is not finite
 };
+// One step of the solve loop on the device: sets the loop's condition to whether
+// another V-cycle is wanted (RMS of the residual above tol and finite, fewer than
+// max cycles) and counts it; the tests of the host's loop.
+struct MgCheck {
+    const double* sum;  // of the squared residual
+    double n, tol;
+    int max;
+    int* cycles;
+};
+cudaError_t add_mg_check(cudaGraph_t g, cudaGraphConditionalHandle h, MgCheck c, cudaGraphNode_t* node);  // the first
+void launch_mg_check(cudaGraphConditionalHandle h, MgCheck c, cudaStream_t s);                           // in the loop
 template <typename T>
 bool vcycle_tail_ok(const TailLevels<T>& a);
 template <typename T>

@@ -1532,6 +1532,24 @@ __global__ void __launch_bounds__(kRedBlock) k_coarse_cg(Dims d, T* __restrict__
 
 }  // namespace
 
+__global__ void k_mg_check(cudaGraphConditionalHandle h, MgCheck c, int first) {
+    const double rms = sqrt(*c.sum) / sqrt(c.n);
+    const int done = first ? 0 : *c.cycles + 1;  // after the cycle before this check
+    *c.cycles = done;
+    cudaGraphSetConditional(h, isfinite(rms) && rms > c.tol && done < c.max ? 1u : 0u);
+}
+cudaError_t add_mg_check(cudaGraph_t g, cudaGraphConditionalHandle h, MgCheck c, cudaGraphNode_t* node) {
+    int first = 1;
+    void* args[] = {&h, &c, &first};
+    cudaKernelNodeParams p = {};
+    p.func = (void*)k_mg_check;
+    p.gridDim = dim3(1);
+    p.blockDim = dim3(1);
+    p.kernelParams = args;
+    return cudaGraphAddKernelNode(node, g, nullptr, 0, &p);
+}
+void launch_mg_check(cudaGraphConditionalHandle h, MgCheck c, cudaStream_t s) { k_mg_check<<<1, 1, 0, s>>>(h, c, 0); }
+
 // smallest level (x extent) on which the smoother and residual take the
 // batched z-column kernels (AFMIB_BATCH_MIN_NX; one cell per thread below:
 // at 64^3 the batched grid is 64 blocks, and the one-cell kernels measured

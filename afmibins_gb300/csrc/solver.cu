@@ -200,6 +200,7 @@ struct afmib_solver {
     int pass_rev = 0;
     cudaGraphExec_t vg64 = nullptr, vg32[kMaxInnerCycles + 1] = {};
     long long vg64_launches = 0, vg32_launches[kMaxInnerCycles + 1] = {};
+    bool mg_loop = true;  // vg64: the whole solve loop, decided on the device (false: not supported)
     bool spread64 = false, interp64 = false;  // mixed form: IB transfers in FP64
     // warm start of each projection from the potential of the previous
     // projection of the same sub-step type (0: BE, 1: CN); off in the FP64
@@ -795,13 +796,52 @@ void drop_graphs(afmib_solver* s) {
     }
 }
 
-// one FP64 V-cycle on level 0 (graph replay when possible)
-int vcycle64_top(afmib_solver* s) {
-    if (s->prof || !s->use_graphs) return vcycle<double>(s, 0);
-    if (!s->vg64) TRY(capture_graph(s, &s->vg64, &s->vg64_launches, [&]() { return vcycle<double>(s, 0); }));
-    CK(cudaGraphLaunch(s->vg64, s->st));
-    s->stats.kernel_launches += s->vg64_launches;
-    return AFMIB_OK;
+// The FP64 solve loop from the residual's squared norm in scal[9] on, as one graph:
+// while the device finds the residual above the tolerance, a V-cycle and the next
+// residual (launch_mg_check; dflag[4]: cycles). A cycle with
+// the norm read by the host cost 12 us more. False where the driver refuses it.
+bool build_mg_loop(afmib_solver* s) {
+    MGLevel& L = s->lv[0];
+    cudaGraph_t g = nullptr;
+    if (cudaGraphCreate(&g, 0) != cudaSuccess) return false;
+    cudaGraphConditionalHandle h;
+    cudaGraphNode_t first, loop;
+    cudaGraphNodeParams np = {};
+    bool ok = cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault) == cudaSuccess;
+    const MgCheck check{s->scal + 9, (double)L.d.ncell(), s->cfg.tol, s->cfg.max_mg_cycles, s->dflag + 4};
+    ok = ok && add_mg_check(g, h, check, &first) == cudaSuccess;
+    if (ok) {
+        np.type = cudaGraphNodeTypeConditional;
+        np.conditional.handle = h;
+        np.conditional.type = cudaGraphCondTypeWhile;
+        np.conditional.size = 1;
+#if CUDART_VERSION >= 13000
+        ok = cudaGraphAddNode(&loop, g, &first, nullptr, 1, &np) == cudaSuccess;
+#else
+        ok = cudaGraphAddNode(&loop, g, &first, 1, &np) == cudaSuccess;
+#endif
+    }
+    if (ok) {
+        const long long l0 = s->stats.kernel_launches;
+        ok = cudaStreamBeginCaptureToGraph(s->st, np.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                           cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+        if (ok) {
+            ok = vcycle<double>(s, 0) == AFMIB_OK;
+            launch_residual<double>(L.d, L.r, L.x, L.b, &s->red, s->scal + 9, s->st);
+            launch_mg_check(h, check, s->st);
+            cudaGraph_t body = nullptr;
+            ok = cudaStreamEndCapture(s->st, &body) == cudaSuccess && ok;
+        }
+        s->vg64_launches = s->stats.kernel_launches - l0 + 2;
+        s->stats.kernel_launches = l0;
+    }
+    ok = ok && cudaGraphInstantiate(&s->vg64, g, 0) == cudaSuccess;
+    cudaGraphDestroy(g);
+    if (!ok) {
+        s->vg64 = nullptr;
+        cudaGetLastError();
+    }
+    return ok;
 }
 
 // the FP32 inner solve of one defect-correction step: x32 = 0, ncyc
@@ -862,20 +902,34 @@ int mg_solve(afmib_solver* s, int* cycles) {
     if (s->lv.size() == 1) {
         TRY(vcycle<double>(s, 0));
     } else {
-        for (;;) {
-            {
-                ProfScope ps(s, P_RESID_NORM, 3 * Ns);
-                launch_residual<double>(L.d, L.r, L.x, L.b, &s->red, s->scal + 9, s->st);
-            }
+        auto resid = [&]() -> int {
+            ProfScope ps(s, P_RESID_NORM, 3 * Ns);
+            launch_residual<double>(L.d, L.r, L.x, L.b, &s->red, s->scal + 9, s->st);
             CKL();
+            return AFMIB_OK;
+        };
+        if (s->mg_loop && s->use_graphs && !s->prof && !s->vg64) s->mg_loop = build_mg_loop(s);
+        const bool graph = s->vg64 && s->use_graphs && !s->prof;
+        TRY(resid());
+        if (graph) {
+            CK(cudaGraphLaunch(s->vg64, s->st));
+            CK(cudaMemcpyAsync(s->hflag + 4, s->dflag + 4, sizeof(int), cudaMemcpyDeviceToHost, s->st));
+        }
+        for (;;) {
             TRY(read_scalars(s, 9, 1));
             const double rms = std::sqrt(s->hscal[9]) / std::sqrt((double)N);
             s->stats.last_mg_rms = rms;
+            if (graph) {
+                c = s->hflag[4];
+                s->stats.kernel_launches += 1 + c * s->vg64_launches;
+            }
             if (!std::isfinite(rms)) { status = s->fail(AFMIB_ERR_NAN, "multigrid residual is not finite"); break; }
             if (rms <= s->cfg.tol) break;
             if (c >= s->cfg.max_mg_cycles) { status = s->fail(AFMIB_ERR_NOCONV, "multigrid cycle cap reached"); break; }
-            TRY(vcycle64_top(s));
+            if (graph) { status = s->fail(AFMIB_ERR_CUDA, "multigrid loop ended early"); break; }
+            TRY(vcycle<double>(s, 0));
             ++c;
+            TRY(resid());
         }
     }
     CK(cudaMemcpyAsync(s->hflag + 1, s->dflag + 1, sizeof(int), cudaMemcpyDeviceToHost, s->st));
@@ -2048,15 +2102,17 @@ int setup_basis(afmib_solver* s) {
     if (dense) {
         all.resize(inv0 + nc * nc, 0.0);
         const size_t sx = ext[0], sxy = sx * ext[1];
-        std::vector<double> W(nc);  // row of G: V^T diag(1 / lambda) V e_j, mode by mode
+        std::vector<double> W(nc);  // V^T diag(1 / lambda) V, mode by mode
         const double n2 = (double)d.n * (double)d.n;
         for (size_t k = 1; k < nc; ++k) {
             const size_t k0 = k % sx, k1 = k / sx % ext[1], k2 = k / sxy;
             const double lam = n2 * ((all[off[0] + sx * sx + k0] + all[off[1] + (size_t)ext[1] * ext[1] + k1]) +
                                      all[off[2] + (size_t)ext[2] * ext[2] + k2]);
-            for (size_t i = 0; i < nc; ++i)
-                W[i] = all[off[0] + k0 * sx + i % sx] * all[off[1] + k1 * ext[1] + i / sx % ext[1]] *
-                       all[off[2] + k2 * ext[2] + i / sxy];
+            const double *wx = &all[off[0] + k0 * sx], *wy = &all[off[1] + k1 * ext[1]], *wz = &all[off[2] + k2 * ext[2]];
+            double* w = W.data();
+            for (int z = 0; z < ext[2]; ++z)
+                for (int y = 0; y < ext[1]; ++y)
+                    for (int x = 0; x < ext[0]; ++x) *w++ = wx[x] * wy[y] * wz[z];
             for (size_t j = 0; j < nc; ++j) {
                 const double c = W[j] / lam;
                 double* row = all.data() + inv0 + j * nc;
@@ -2185,14 +2241,14 @@ int create(afmib_solver* s, const afmib_config* c, void* stream) {
     TRY(dalloc(s, &s->red.partial, (size_t)kMaxRedBlocks * kMaxRedVals));
     TRY(dalloc(s, &s->red.ticket, kMaxRedVals));
     TRY(dalloc(s, &s->scal, 24));
-    TRY(dalloc(s, &s->dflag, 4));
+    TRY(dalloc(s, &s->dflag, 8));
     // one pinned block (an allocation takes about 100 us): scalars, the CG's scalars, flags
     constexpr int kHostScal = 24, kHostCg = 2 * 3 * kCgScalars;
-    CK(cudaMallocHost((void**)&s->hscal, (kHostScal + kHostCg) * sizeof(double) + 4 * sizeof(int)));
+    CK(cudaMallocHost((void**)&s->hscal, (kHostScal + kHostCg) * sizeof(double) + 8 * sizeof(int)));
     s->hcg = s->hscal + kHostScal;
     s->hflag = (int*)(s->hcg + kHostCg);
     CK(cudaMemsetAsync(s->red.ticket, 0, kMaxRedVals * sizeof(unsigned), s->st));
-    CK(cudaMemsetAsync(s->dflag, 0, 4 * sizeof(int), s->st));
+    CK(cudaMemsetAsync(s->dflag, 0, 8 * sizeof(int), s->st));
     CK(cudaMemsetAsync(s->walls, 0, 4 * s->nxz() * sizeof(double), s->st));
     CK(cudaMemsetAsync(s->wallgrad, 0, 8 * s->nxz() * sizeof(double), s->st));
     CK(cudaMemsetAsync(s->u, 0, N * sizeof(double), s->st));
