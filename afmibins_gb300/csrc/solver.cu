@@ -273,7 +273,7 @@ struct afmib_solver {
 
 namespace {
 
-constexpr size_t kArenaMost = 64 << 10, kArenaChunk = 1 << 20;
+constexpr size_t kArenaMost = 2 << 20, kArenaChunk = 1 << 20;  // a chunk takes at least 16 of the buffer it is cut for
 
 #define CK(call)                                                                              \
     do {                                                                                      \
@@ -302,10 +302,11 @@ int dalloc(afmib_solver* s, T** p, size_t count) {
     if (s->creating && bytes <= kArenaMost) {
         const size_t need = (bytes + 255) & ~(size_t)255;
         if (s->arena_left < need) {
-            CK(cudaMalloc(&q, kArenaChunk));
+            const size_t chunk = std::max(kArenaChunk, 16 * need);
+            CK(cudaMalloc(&q, chunk));
             s->allocs.push_back(q);
             s->arena = (char*)q;
-            s->arena_left = kArenaChunk;
+            s->arena_left = chunk;
         }
         *p = (T*)s->arena;
         s->arena += need;
