@@ -306,40 +306,55 @@ __global__ void k_div(Dims d, T* __restrict__ out, const T* __restrict__ u, cons
     out[i] = T(d.n) * ((u[lin(d, xp1(d, x), y, z)] - u[i]) + dv + (w[lin(d, x, y, zp1(d, z))] - w[i]));
 }
 
-// Mixed form: k_div in double-float on the FP32 pipe (GB300's FP64 pipe
-// bounds the FP64 kernel: 81% busy, ncu). The FP64 face velocities are split
-// by integer operations (df_split, 2^-46 relative), the differences and sums
-// are pairs in k_div's order, and the value goes back to FP64 with one
-// addition. out_sum[0]: the sum of the written values (the pressure solve's
+// Mixed form: k_div with its work shared between the FP64 pipe, which bounds the
+// FP64 kernel (81% busy, ncu), and the FP32 and integer pipes: u's difference is an
+// FP64 subtraction and split after it, v's and w's faces are split into double-float
+// pairs by integer operations (df_split, 2^-46 relative; w's once per face of the
+// batch) and subtracted as pairs, the sums are pairs in k_div's order, and the value
+// goes back to FP64 with one addition. 191 us at 256^3 with the batch's loads first,
+// against 205 with no FP64 difference, 193 with two, 214 with three, 232 in FP64, and
+// 235 cell by cell. out_sum[0]: the sum of the written values (the pressure solve's
 // mean removal), each thread's pair sum reduced in a fixed order.
+template <int ZU, typename IX>
 __global__ void __launch_bounds__(kRedBlock) k_div_df(Dims d, double* __restrict__ out, const double* __restrict__ u,
                                                      const double* __restrict__ v, const double* __restrict__ w,
                                                      const double* __restrict__ top,
                                                      const double* __restrict__ bottom, RedScratch sc,
                                                      double* out_sum) {
+    const IX I(d);
     const int x = blockIdx.x * kRBX + threadIdx.x, y = blockIdx.y * kRBY + threadIdx.y;
     const df2 nn = {float(d.n), 0.f};
-    const df2 zero = {0.f, 0.f};
-    df2 acc = zero;
+    df2 acc = {0.f, 0.f};
     if (x < d.nx && y < d.ny)
-        for (int z = blockIdx.z; z < d.nz; z += gridDim.z) {
-            const long long i = lin(d, x, y, z);
-            df2 dv;
-            if (d.channel) {
-                const long long ixz = x + (long long)d.nx * z;
-                const df2 tv = top ? df_split(top[ixz]) : zero, bv = bottom ? df_split(bottom[ixz]) : zero;
-                if (d.ny == 1) dv = df_add(tv, df_neg(bv));
-                else if (y == 0) dv = df_add(df_split(v[lin(d, x, 1, z)]), df_neg(bv));
-                else if (y == d.ny - 1) dv = df_add(tv, df_neg(df_split(v[i])));
-                else dv = df_add(df_split(v[lin(d, x, y + 1, z)]), df_neg(df_split(v[i])));
-            } else {
-                dv = df_add(df_split(v[lin(d, x, yp1(d, y), z)]), df_neg(df_split(v[i])));
+        for (int zb = blockIdx.z; zb < d.nz / ZU; zb += gridDim.z) {
+            // every load of the batch first
+            const int z0 = zb * ZU;
+            double u0[ZU], u1[ZU], v0[ZU], v1[ZU], wz[ZU + 1];
+#pragma unroll
+            for (int k = 0; k < ZU; ++k) {
+                const int z = z0 + k, i = I.at(x, y, z);
+                u0[k] = u[i];
+                u1[k] = u[I.at(I.xp(x), y, z)];
+                if (d.channel) {
+                    const int ixz = x + d.nx * z;
+                    v1[k] = y < d.ny - 1 ? v[I.at(x, y + 1, z)] : (top ? top[ixz] : 0.0);
+                    v0[k] = y > 0 ? v[i] : (bottom ? bottom[ixz] : 0.0);
+                } else {
+                    v1[k] = v[I.at(x, I.yp(y), z)];
+                    v0[k] = v[i];
+                }
+                wz[k] = w[i];
             }
-            const df2 du = df_add(df_split(u[lin(d, xp1(d, x), y, z)]), df_neg(df_split(u[i])));
-            const df2 dw = df_add(df_split(w[lin(d, x, y, zp1(d, z))]), df_neg(df_split(w[i])));
-            const df2 r = df_mul(nn, df_add(df_add(du, dv), dw));
-            out[i] = f32_to_f64(r.hi) + f32_to_f64(r.lo);
-            acc = df_add(acc, r);
+            wz[ZU] = w[I.at(x, y, I.wz(z0 + ZU))];
+#pragma unroll
+            for (int k = 0; k < ZU; ++k) {
+                const df2 du = df_split(u1[k] - u0[k]);
+                const df2 dv = df_add(df_split(v1[k]), df_neg(df_split(v0[k])));
+                const df2 dw = df_add(df_split(wz[k + 1]), df_neg(df_split(wz[k])));
+                const df2 r = df_mul(nn, df_add(df_add(du, dv), dw));
+                out[I.at(x, y, z0 + k)] = f32_to_f64(r.hi) + f32_to_f64(r.lo);
+                acc = df_add(acc, r);
+            }
         }
     double a[1] = {f32_to_f64(acc.hi) + f32_to_f64(acc.lo)};
     grid_sum<1>(a, sc, out_sum);
@@ -1285,7 +1300,12 @@ void launch_div(const Dims& d, T* out, const T* u, const T* v, const T* w, const
 }
 void launch_div_df(const Dims& d, double* out, const double* u, const double* v, const double* w, const double* top,
                    const double* bottom, RedScratch sc, double* out_sum, cudaStream_t s) {
-    k_div_df<<<red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s>>>(d, out, u, v, w, top, bottom, sc, out_sum);
+    const dim3 blk(kRBX, kRBY);
+    if (d.nz % 2 == 0)
+        AFMIB_IX(d, (k_div_df<2, IX><<<red_grid3(d.nx, d.ny, d.nz / 2), blk, 0, s>>>(d, out, u, v, w, top, bottom, sc,
+                                                                                  out_sum)));
+    else
+        AFMIB_IX(d, (k_div_df<1, IX><<<red_grid3(d.nx, d.ny, d.nz), blk, 0, s>>>(d, out, u, v, w, top, bottom, sc, out_sum)));
 }
 template <typename T>
 void launch_grad(const Dims& d, T* px, T* py, T* pz, const T* p, cudaStream_t s) {
