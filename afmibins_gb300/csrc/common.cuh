@@ -84,6 +84,27 @@ struct IxG {
         return x + (nx >> 1) * (y + (ny >> 1) * z);
     }
 };
+// A launch that may be set up while the kernel before it in the stream or graph
+// runs (programmatic dependent launch, no early trigger): 0.2 us less per kernel of
+// 1.3 in a graph of small ones (an early trigger: 0.1 less, and slower from 10^6
+// threads on). The kernel calls wait_launch() before its first access to memory
+// that another one writes or reads; that returns when the kernel before has ended
+// and its writes are visible, and at once where there is none to wait for.
+__device__ __forceinline__ void wait_launch() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename... P, typename... A>
+inline void launch_dep(dim3 grid, dim3 block, size_t smem, cudaStream_t s, void (*kernel)(P...), A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, P(args)...);  // errors reach the caller's cudaGetLastError
+}
 // One launch with the index type of the grid
 #define AFMIB_IX(d, ...)                         \
     do {                                         \

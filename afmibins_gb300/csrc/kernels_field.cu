@@ -933,6 +933,7 @@ __global__ void k_cg_direction(long long N, T* __restrict__ p, const T* __restri
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kRedBlock) k_cgb_init(Dims d, CgBatch g, HelmK<double> k, int gz, double tol,
                                                        RedScratch sc, double* cgs) {
+    wait_launch();
     const int c = blockIdx.z / gz, zb = blockIdx.z - c * gz;
     const int xi = blockIdx.x * kRBX + threadIdx.x, yi = blockIdx.y * kRBY + threadIdx.y;
     const double *x = g.x[c], *b = g.b[c];
@@ -959,6 +960,7 @@ __global__ void __launch_bounds__(kRedBlock) k_cgb_init(Dims d, CgBatch g, HelmK
 
 __global__ void __launch_bounds__(kRedBlock) k_cgb_apply(Dims d, CgBatch g, HelmK<double> k, int gz, RedScratch sc,
                                                         double* cgs) {
+    wait_launch();
     const int c = blockIdx.z / gz, zb = blockIdx.z - c * gz;
     double* s = cgs + kCgScalars * c;
     if (s[5] != 0.0) return;
@@ -983,6 +985,7 @@ __global__ void __launch_bounds__(kRedBlock) k_cgb_apply(Dims d, CgBatch g, Helm
 
 template <bool VEC>
 __global__ void __launch_bounds__(kRedBlock) k_cgb_update(long long N, CgBatch g, double tol, RedScratch sc, double* cgs) {
+    wait_launch();
     const int c = blockIdx.y;
     double* s = cgs + kCgScalars * c;
     if (s[5] != 0.0) return;  // set below only once every block of the system has passed here
@@ -1025,6 +1028,7 @@ __global__ void __launch_bounds__(kRedBlock) k_cgb_update(long long N, CgBatch g
 
 template <bool VEC>
 __global__ void __launch_bounds__(kRedBlock) k_cgb_direction(long long N, CgBatch g, const double* cgs) {
+    wait_launch();
     const int c = blockIdx.y;
     const double* s = cgs + kCgScalars * c;
     if (s[5] != 0.0) return;
@@ -1498,6 +1502,7 @@ __global__ void __launch_bounds__(kRedBlock, MINB) k_helm_update_df2(Dims d, int
                                                               double* __restrict__ x, const float* __restrict__ e,
                                                               float* __restrict__ rh, float* __restrict__ rl,
                                                               RedScratch sc, double* out) {
+    wait_launch();
     const IX I(d);
     float acc = 0.f;
     const int xi = blockIdx.x * kRBX + threadIdx.x, yi = blockIdx.y * kRBY + threadIdx.y;
@@ -1570,8 +1575,7 @@ void launch_helm_update_df(const Dims& d, int comp, double scale, double* x, con
         const int gx = (d.nx + kRBX - 1) / kRBX, gy = (d.ny + kRBY - 1) / kRBY;
         int gz = d.nz / ZU;
         if ((long long)gx * gy * gz > kMaxRedBlocks) gz = std::max(1, kMaxRedBlocks / (gx * gy));
-        AFMIB_IX(d, (k_helm_update_df2<ZU, kUpdateMinBlocks, IX><<<dim3(gx, gy, gz), dim3(kRBX, kRBY), 0, s>>>(
-                        d, comp, o, c, x, e, rh, rl, sc, out)));
+        AFMIB_IX(d, (launch_dep(dim3(gx, gy, gz), dim3(kRBX, kRBY), 0, s, k_helm_update_df2<ZU, kUpdateMinBlocks, IX>, d, comp, o, c, x, e, rh, rl, sc, out)));
         return;
     }
     k_helm_update_df<<<red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s>>>(d, comp, o, c, x, e, rh, rl, sc, out);
@@ -1618,26 +1622,26 @@ void launch_cgb_init(const Dims& d, double scale, const CgBatch& g, double tol, 
                      cudaStream_t s) {
     int gz;
     const dim3 grid = cgb_grid(d, g.n, &gz);
-    k_cgb_init<<<grid, dim3(kRBX, kRBY), 0, s>>>(d, g, helm_k<double>(d, scale), gz, tol, sc, cgs);
+    launch_dep(grid, dim3(kRBX, kRBY), 0, s, k_cgb_init, d, g, helm_k<double>(d, scale), gz, tol, sc, cgs);
 }
 void launch_cgb_apply(const Dims& d, double scale, const CgBatch& g, RedScratch sc, double* cgs, cudaStream_t s) {
     int gz;
     const dim3 grid = cgb_grid(d, g.n, &gz);
-    k_cgb_apply<<<grid, dim3(kRBX, kRBY), 0, s>>>(d, g, helm_k<double>(d, scale), gz, sc, cgs);
+    launch_dep(grid, dim3(kRBX, kRBY), 0, s, k_cgb_apply, d, g, helm_k<double>(d, scale), gz, sc, cgs);
 }
 void launch_cgb_update(const Dims& d, const CgBatch& g, double tol, RedScratch sc, double* cgs, cudaStream_t s) {
     const long long N = d.ncell();
     const bool vec = cgb_vec(N, g);
     const dim3 grid(red_blocks(vec ? N / 2 : N, std::max(1, kRedBlocks64 / g.n)), g.n);
-    if (vec) k_cgb_update<true><<<grid, kRedBlock, 0, s>>>(N, g, tol, sc, cgs);
-    else k_cgb_update<false><<<grid, kRedBlock, 0, s>>>(N, g, tol, sc, cgs);
+    if (vec) launch_dep(grid, kRedBlock, 0, s, k_cgb_update<true>, N, g, tol, sc, cgs);
+    else launch_dep(grid, kRedBlock, 0, s, k_cgb_update<false>, N, g, tol, sc, cgs);
 }
 void launch_cgb_direction(const Dims& d, const CgBatch& g, const double* cgs, cudaStream_t s) {
     const long long N = d.ncell();
     const bool vec = cgb_vec(N, g);
     const dim3 grid(red_blocks(vec ? N / 2 : N, std::max(1, kRedWaveBlocks / g.n)), g.n);
-    if (vec) k_cgb_direction<true><<<grid, kRedBlock, 0, s>>>(N, g, cgs);
-    else k_cgb_direction<false><<<grid, kRedBlock, 0, s>>>(N, g, cgs);
+    if (vec) launch_dep(grid, kRedBlock, 0, s, k_cgb_direction<true>, N, g, cgs);
+    else launch_dep(grid, kRedBlock, 0, s, k_cgb_direction<false>, N, g, cgs);
 }
 template <typename T, int ZU, typename IX>
 __global__ void k_helm_jacobi2(Dims d, int comp, HelmK<T> k, const T* __restrict__ xv, T* __restrict__ xo,
@@ -1683,6 +1687,7 @@ __device__ __forceinline__ void helm_rbgs2_body(Dims d, int comp, const HelmK<T>
 template <typename T, int ZU, int MINB, typename IX>
 __global__ void __launch_bounds__(BX * BY, MINB) k_helm_rbgs2b(Dims d, int comp, HelmK<T> k, int color, T* __restrict__ xv,
                                                               const T* __restrict__ b, int rev) {
+    wait_launch();
     helm_rbgs2_body<T, ZU, IX>(d, comp, k, color, xv, b, rev);
 }
 
@@ -1697,6 +1702,7 @@ __global__ void __launch_bounds__(BX * BY, MINB) k_helm_rbgs2b(Dims d, int comp,
 template <typename T, int ZU, int MINB, typename IX>
 __global__ void __launch_bounds__(BX * BY, MINB) k_helm_first(Dims d, int comp, HelmK<T> k, T* __restrict__ xv,
                                                              const T* __restrict__ b, int rev) {
+    wait_launch();
     const IX I(d);
     const uint3 B = block_at(rev);
     const int y = B.y * BY + threadIdx.y, t = B.x * BX + threadIdx.x, z0 = B.z * ZU;
@@ -1751,9 +1757,9 @@ void launch_helm_rbgs_first(const Dims& d, int comp, double scale, T* x, const T
     const int gx = (d.nx / 2 + BX - 1) / BX, gy = (d.ny + BY - 1) / BY;
     const HelmK<T> k = helm_k<T>(d, scale);
     if (d.nz % 4 == 0)
-        AFMIB_IX(d, (k_helm_first<T, 4, 6, IX><<<dim3(gx, gy, d.nz / 4), dim3(BX, BY), 0, s>>>(d, comp, k, x, b, rev)));
+        AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz / 4), dim3(BX, BY), 0, s, k_helm_first<T, 4, 6, IX>, d, comp, k, x, b, rev)));
     else
-        AFMIB_IX(d, (k_helm_first<T, 2, 6, IX><<<dim3(gx, gy, d.nz / 2), dim3(BX, BY), 0, s>>>(d, comp, k, x, b, rev)));
+        AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz / 2), dim3(BX, BY), 0, s, k_helm_first<T, 2, 6, IX>, d, comp, k, x, b, rev)));
 }
 template void launch_helm_rbgs_first<float>(const Dims&, int, double, float*, const float*, cudaStream_t, int);
 
@@ -1765,9 +1771,9 @@ void launch_helm_rbgs(const Dims& d, int comp, double scale, int color, T* x, co
     // registers capped for 6 resident blocks (40 against 48): measured with the
     // multigrid smoother's cap, 50.5 against 50.0 IB steps/s at 256^3
     if (d.nz % 8 == 0)
-        AFMIB_IX(d, (k_helm_rbgs2b<T, 8, 6, IX><<<dim3(gx, gy, d.nz / 8), blk, 0, s>>>(d, comp, k, color, x, b, rev)));
+        AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz / 8), blk, 0, s, k_helm_rbgs2b<T, 8, 6, IX>, d, comp, k, color, x, b, rev)));
     else
-        AFMIB_IX(d, (k_helm_rbgs2b<T, 2, 6, IX><<<dim3(gx, gy, d.nz / 2), blk, 0, s>>>(d, comp, k, color, x, b, rev)));
+        AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz / 2), blk, 0, s, k_helm_rbgs2b<T, 2, 6, IX>, d, comp, k, color, x, b, rev)));
 }
 template void launch_helm_rbgs<float>(const Dims&, int, double, int, float*, const float*, cudaStream_t, int);
 

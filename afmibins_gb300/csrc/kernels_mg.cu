@@ -96,6 +96,7 @@ __global__ void k_lap(Dims d, LapK<T> k, T* __restrict__ out, const T* __restric
 
 template <typename T, typename IX>
 __global__ void k_residual(Dims d, LapK<T> k, T* __restrict__ r, const T* __restrict__ xv, const T* __restrict__ b) {
+    wait_launch();
     const int x = blockIdx.x * BX + threadIdx.x, y = blockIdx.y * BY + threadIdx.y, z = blockIdx.z;
     if (x >= d.nx || y >= d.ny) return;
     const IX I(d);
@@ -110,6 +111,7 @@ template <typename T, typename IX>
 __global__ void __launch_bounds__(kRedBlock) k_residual_norm(Dims d, LapK<T> k, T* __restrict__ r,
                                                             const T* __restrict__ xv, const T* __restrict__ b,
                                                             RedScratch sc, double* out) {
+    wait_launch();
     const int xi = blockIdx.x * kRBX + threadIdx.x, yi = blockIdx.y * kRBY + threadIdx.y;
     const IX I(d);
     T acc = T(0);
@@ -263,6 +265,7 @@ template <int ZU, int MINB, typename IX>
 __global__ void __launch_bounds__(kRedBlock, MINB) k_lap_update_df2(Dims d, double* __restrict__ x,
                                                              const float* __restrict__ e, float* __restrict__ rh,
                                                              float* __restrict__ rl, RedScratch sc, double* out) {
+    wait_launch();
     const IX I(d);
     const int xi = blockIdx.x * kRBX + threadIdx.x, yi = blockIdx.y * kRBY + threadIdx.y;
     const float off = float(d.n) * float(d.n);
@@ -352,6 +355,7 @@ __global__ void __launch_bounds__(kRedBlock) k_lap_defect_bfp(Dims d, int k2, fl
 // Gauss-Seidel, bit for bit
 template <typename T, typename IX>
 __global__ void k_rbgs(Dims d, LapK<T> k, int color, T omega, T* __restrict__ xv, const T* __restrict__ b) {
+    wait_launch();
     const int y = blockIdx.y * BY + threadIdx.y, z = blockIdx.z;
     const int x = 2 * (blockIdx.x * BX + threadIdx.x) + ((y + z + color) & 1);
     if (x >= d.nx || y >= d.ny) return;
@@ -399,6 +403,7 @@ __device__ __forceinline__ void rbgs_z2_body(Dims d, const LapK<T>& k, int color
 }
 template <typename T, int ZU, typename IX>
 __global__ void k_rbgs_z2(Dims d, LapK<T> k, int color, T omega, T* __restrict__ xv, const T* __restrict__ b, int rev) {
+    wait_launch();
     rbgs_z2_body<T, ZU, IX>(d, k, color, omega, xv, b, rev);
 }
 
@@ -417,6 +422,7 @@ __global__ void k_rbgs_z2(Dims d, LapK<T> k, int color, T omega, T* __restrict__
 template <typename T, int ZU, int MINB, typename IX>
 __global__ void __launch_bounds__(BX * BY, MINB) k_rbgs_first(Dims d, LapK<T> k, T omega, T* __restrict__ xv,
                                                              const T* __restrict__ b, int rev, T zero) {
+    wait_launch();
     const IX I(d);
     const uint3 B = block_at(rev);
     const int y = B.y * BY + threadIdx.y, t = B.x * BX + threadIdx.x, z0 = B.z * ZU;
@@ -468,6 +474,7 @@ __global__ void __launch_bounds__(BX * BY, MINB) k_rbgs_first(Dims d, LapK<T> k,
 template <typename T, int ZU, int MINB, typename IX>
 __global__ void __launch_bounds__(BX * BY, MINB) k_rbgs_z2b(Dims d, LapK<T> k, int color, T omega, T* __restrict__ xv,
                                                            const T* __restrict__ b, int rev) {
+    wait_launch();
     rbgs_z2_body<T, ZU, IX>(d, k, color, omega, xv, b, rev);
 }
 
@@ -543,6 +550,7 @@ __global__ void __launch_bounds__(BX * BY, MINB) k_rbgs_pair(Dims d, int color, 
 template <typename T, int ZU, typename IX>
 __global__ void k_residual_z2(Dims d, LapK<T> k, T* __restrict__ r, const T* __restrict__ xv, const T* __restrict__ b,
                               int rev) {
+    wait_launch();
     const IX I(d);
     const uint3 B = block_at(rev);
     const int x = B.x * BX + threadIdx.x, y = B.y * BY + threadIdx.y, z0 = B.z * ZU;
@@ -565,6 +573,7 @@ __global__ void k_residual_z2(Dims d, LapK<T> k, T* __restrict__ r, const T* __r
 template <typename T, int ZU, typename IX>
 __global__ void k_residual_red(Dims d, LapK<T> k, T* __restrict__ r, const T* __restrict__ xv, const T* __restrict__ b,
                                int rev) {
+    wait_launch();
     const IX I(d);
     const uint3 B = block_at(rev);
     const int t = B.x * BX + threadIdx.x, y = B.y * BY + threadIdx.y, z0 = B.z * ZU;
@@ -777,6 +786,7 @@ __device__ __forceinline__ void restrict_cell(const Dims& d, T* coarse, const T*
 
 template <typename T, bool RED>
 __global__ void k_restrict(Dims d, T* __restrict__ coarse, const T* __restrict__ fine) {
+    wait_launch();
     const int xc = blockIdx.x * BX + threadIdx.x, yc = blockIdx.y * BY + threadIdx.y;
     if (xc >= d.nx / 2 || yc >= d.ny / 2) return;
     restrict_cell<T, RED>(d, coarse, fine, xc, yc);
@@ -858,6 +868,7 @@ __device__ __forceinline__ void restrict_cell2(const Dims& d, const IX& I, T* co
 
 template <typename T, bool RED, typename IX>
 __global__ void k_restrict2(Dims d, T* __restrict__ coarse, const T* __restrict__ fine, int rev) {
+    wait_launch();
     const IX I(d);
     const uint3 B = block_at(rev);
     const int xc = B.x * BX + threadIdx.x, yc = B.y * BY + threadIdx.y, zc = B.z;
@@ -962,6 +973,7 @@ __global__ void __launch_bounds__(RR_THREADS) k_resid_restrict2(Dims d, T* __res
 
 template <typename T, bool ADD, bool BLACK, typename IX>
 __global__ void k_prolong2(Dims d, T* __restrict__ fine, const T* __restrict__ coarse, int rev) {
+    wait_launch();
     const IX I(d);
     const uint3 B = block_at(rev);
     const int xc = B.x * BX + threadIdx.x, yc = B.y * BY + threadIdx.y, zc = B.z;
@@ -971,6 +983,7 @@ __global__ void k_prolong2(Dims d, T* __restrict__ fine, const T* __restrict__ c
 
 template <typename T, bool ADD, bool BLACK>
 __global__ void k_prolong(Dims d, T* __restrict__ fine, const T* __restrict__ coarse) {
+    wait_launch();
     const int xc = blockIdx.x * BX + threadIdx.x, yc = blockIdx.y * BY + threadIdx.y;
     if (xc >= d.nx / 2 || yc >= d.ny / 2) return;
     prolong_cell<T, ADD, BLACK>(d, fine, coarse, xc, yc);
@@ -1045,6 +1058,7 @@ __device__ __forceinline__ void quad_get(const T* p, T (&v)[16 / sizeof(T)]) {
 template <typename T, int CZ>
 __global__ void __launch_bounds__(32 * kTrBY) k_restrict_cols(Dims d, T* __restrict__ coarse,
                                                               const T* __restrict__ fine, int rev) {
+    wait_launch();
     using TT = TrTile<T>;
     constexpr int CE = TT::CE, M = CE / 2;  // M coarse cells per lane
     constexpr int NP = 2 * CZ + 2;          // fine planes of the block
@@ -1170,6 +1184,7 @@ template <int CZ, bool CH>
 __global__ void __launch_bounds__(32 * kTrBY, 2) k_resid_restrict_cols(Dims d, float* __restrict__ cb,
                                                                     const float* __restrict__ xv,
                                                                     const float* __restrict__ bv, int rev) {
+    wait_launch();
     constexpr int NP = 2 * CZ + 2;  // fine planes restricted (residuals formed)
     constexpr int NI = NP + 2;      // staged items: x planes 2 zc0 - 2 .. 2 zc0 + 2 CZ + 1
     constexpr int XCH = (kRrXRows * 36 + 32 * kTrBY - 1) / (32 * kTrBY);
@@ -1369,6 +1384,7 @@ struct ProTile {
 template <typename T, int RZ>
 __global__ void __launch_bounds__(32 * kTrBY) k_prolong_cols(Dims d, T* __restrict__ fine,
                                                              const T* __restrict__ coarse, int rev) {
+    wait_launch();
     using P2 = typename Pair<T>::type;
     using PT = ProTile<T>;
     constexpr int CE = PT::CE;
@@ -1542,6 +1558,7 @@ __global__ void __launch_bounds__(kRedBlock) k_coarse_cg(Dims d, T* __restrict__
 }  // namespace
 
 __global__ void k_mg_check(cudaGraphConditionalHandle h, MgCheck c, int first) {
+    wait_launch();
     const double rms = sqrt(*c.sum) / sqrt(c.n);
     const int done = first ? 0 : *c.cycles + 1;  // after the cycle before this check
     *c.cycles = done;
@@ -1557,7 +1574,7 @@ cudaError_t add_mg_check(cudaGraph_t g, cudaGraphConditionalHandle h, MgCheck c,
     p.kernelParams = args;
     return cudaGraphAddKernelNode(node, g, nullptr, 0, &p);
 }
-void launch_mg_check(cudaGraphConditionalHandle h, MgCheck c, cudaStream_t s) { k_mg_check<<<1, 1, 0, s>>>(h, c, 0); }
+void launch_mg_check(cudaGraphConditionalHandle h, MgCheck c, cudaStream_t s) { launch_dep(1, 1, 0, s, k_mg_check, h, c, 0); }
 
 // smallest level (x extent) on which the smoother and residual take the
 // batched z-column kernels (AFMIB_BATCH_MIN_NX; one cell per thread below:
@@ -1580,12 +1597,12 @@ void launch_residual(const Dims& d, T* r, const T* x, const T* b, RedScratch* sc
     const LapK<T> k = lap_k<T>(d);
     if (sc && out) {
         const dim3 g = red_grid3(d.nx, d.ny, d.nz, red_target<T>());
-        AFMIB_IX(d, (k_residual_norm<T, IX><<<g, dim3(kRBX, kRBY), 0, s>>>(d, k, r, x, b, *sc, out)));
+        AFMIB_IX(d, (launch_dep(g, dim3(kRBX, kRBY), 0, s, k_residual_norm<T, IX>, d, k, r, x, b, *sc, out)));
     } else if (d.nz % kZU == 0 && d.nx >= batch_min_nx()) {
         const dim3 g((d.nx + BX - 1) / BX, (d.ny + BY - 1) / BY, d.nz / kZU);
-        AFMIB_IX(d, (k_residual_z2<T, kZU, IX><<<g, dim3(BX, BY), 0, s>>>(d, k, r, x, b, rev)));
+        AFMIB_IX(d, (launch_dep(g, dim3(BX, BY), 0, s, k_residual_z2<T, kZU, IX>, d, k, r, x, b, rev)));
     } else {
-        AFMIB_IX(d, (k_residual<T, IX><<<grid3(d), dim3(BX, BY), 0, s>>>(d, k, r, x, b)));
+        AFMIB_IX(d, (launch_dep(grid3(d), dim3(BX, BY), 0, s, k_residual<T, IX>, d, k, r, x, b)));
     }
 }
 template <typename T>
@@ -1594,9 +1611,9 @@ void launch_residual_red(const Dims& d, T* r, const T* x, const T* b, cudaStream
     const int gx = (d.nx / 2 + BX - 1) / BX, gy = (d.ny + BY - 1) / BY;
     const LapK<T> k = lap_k<T>(d);
     if (d.nz % ZU == 0 && d.nx >= batch_min_nx())
-        AFMIB_IX(d, (k_residual_red<T, ZU, IX><<<dim3(gx, gy, d.nz / ZU), dim3(BX, BY), 0, s>>>(d, k, r, x, b, rev)));
+        AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz / ZU), dim3(BX, BY), 0, s, k_residual_red<T, ZU, IX>, d, k, r, x, b, rev)));
     else
-        AFMIB_IX(d, (k_residual_red<T, 1, IX><<<dim3(gx, gy, d.nz), dim3(BX, BY), 0, s>>>(d, k, r, x, b, rev)));
+        AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz), dim3(BX, BY), 0, s, k_residual_red<T, 1, IX>, d, k, r, x, b, rev)));
 }
 // The pair kernel is opt-in (AFMIB_RBGS_PAIR=1, read at every launch): at
 // 256^3 its colour launches took 39.5 us against 29.9 for the scalar kernel
@@ -1628,11 +1645,9 @@ void launch_rbgs_first(const Dims& d, T* x, const T* b, cudaStream_t s, double o
     const int gx = (d.nx / 2 + BX - 1) / BX, gy = (d.ny + BY - 1) / BY;
     const LapK<T> k = lap_k<T>(d);
     if (d.nz % ZU == 0 && d.nx >= batch_min_nx())
-        AFMIB_IX(d, (k_rbgs_first<T, ZU, MINB, IX><<<dim3(gx, gy, d.nz / ZU), dim3(BX, BY), 0, s>>>(d, k, T(omega), x, b,
-                                                                                                 rev, T(0))));
+        AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz / ZU), dim3(BX, BY), 0, s, k_rbgs_first<T, ZU, MINB, IX>, d, k, T(omega), x, b, rev, T(0))));
     else
-        AFMIB_IX(d, (k_rbgs_first<T, 1, MINB, IX><<<dim3(gx, gy, d.nz), dim3(BX, BY), 0, s>>>(d, k, T(omega), x, b, rev,
-                                                                                           T(0))));
+        AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz), dim3(BX, BY), 0, s, k_rbgs_first<T, 1, MINB, IX>, d, k, T(omega), x, b, rev, T(0))));
 }
 
 template <typename T>
@@ -1655,13 +1670,12 @@ void launch_rbgs(const Dims& d, int color, T* x, const T* b, cudaStream_t s, dou
         // 256^3 colour, 61.1 against 60.8 steps/s; 16: spills, two:
         // 32.7 us; four cells with 8 blocks: the same as 6)
         if (f32)
-            AFMIB_IX(d, (k_rbgs_z2b<T, kZU32, 6, IX><<<dim3(gx, gy, d.nz / kZU32), blk, 0, s>>>(d, k, color, T(omega), x,
-                                                                                              b, rev)));
+            AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz / kZU32), blk, 0, s, k_rbgs_z2b<T, kZU32, 6, IX>, d, k, color, T(omega), x, b, rev)));
         else
-            AFMIB_IX(d, (k_rbgs_z2<T, kZU64, IX><<<dim3(gx, gy, d.nz / kZU64), blk, 0, s>>>(d, k, color, T(omega), x, b, rev)));
+            AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz / kZU64), blk, 0, s, k_rbgs_z2<T, kZU64, IX>, d, k, color, T(omega), x, b, rev)));
         return;
     }
-    AFMIB_IX(d, (k_rbgs<T, IX><<<dim3(gx, gy, d.nz), blk, 0, s>>>(d, k, color, T(omega), x, b)));
+    AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz), blk, 0, s, k_rbgs<T, IX>, d, k, color, T(omega), x, b)));
 }
 namespace {
 int log2_exact(int v) {
@@ -1779,20 +1793,20 @@ void launch_restrict(const Dims& d, T* coarse, const T* fine, cudaStream_t s, in
         if (!red && transfer_cols_ok(d, fine, coarse) && (d.nx / 2) % TrTile<T>::CX == 0) {
             const int z = transfer_planes(d, TrTile<T>::CX);
             const dim3 g = transfer_grid(d, z, TrTile<T>::CX), b(32, kTrBY);
-            if (z == 8) k_restrict_cols<T, 8><<<g, b, 0, s>>>(d, coarse, fine, rev);
-            else if (z == 4) k_restrict_cols<T, 4><<<g, b, 0, s>>>(d, coarse, fine, rev);
-            else if (z == 2) k_restrict_cols<T, 2><<<g, b, 0, s>>>(d, coarse, fine, rev);
-            else k_restrict_cols<T, 1><<<g, b, 0, s>>>(d, coarse, fine, rev);
+            if (z == 8) launch_dep(g, b, 0, s, k_restrict_cols<T, 8>, d, coarse, fine, rev);
+            else if (z == 4) launch_dep(g, b, 0, s, k_restrict_cols<T, 4>, d, coarse, fine, rev);
+            else if (z == 2) launch_dep(g, b, 0, s, k_restrict_cols<T, 2>, d, coarse, fine, rev);
+            else launch_dep(g, b, 0, s, k_restrict_cols<T, 1>, d, coarse, fine, rev);
             return;
         }
     }
     dim3 g((d.nx / 2 + BX - 1) / BX, (d.ny / 2 + BY - 1) / BY, d.nz == 1 ? 1 : d.nz / 2);
     if (d.nz > 1)
-        AFMIB_IX(d, (red ? k_restrict2<T, true, IX><<<g, dim3(BX, BY), 0, s>>>(d, coarse, fine, rev)
-                         : k_restrict2<T, false, IX><<<g, dim3(BX, BY), 0, s>>>(d, coarse, fine, rev)));
+        AFMIB_IX(d, (red ? launch_dep(g, dim3(BX, BY), 0, s, k_restrict2<T, true, IX>, d, coarse, fine, rev)
+                         : launch_dep(g, dim3(BX, BY), 0, s, k_restrict2<T, false, IX>, d, coarse, fine, rev)));
     else
-        red ? k_restrict<T, true><<<g, dim3(BX, BY), 0, s>>>(d, coarse, fine)
-            : k_restrict<T, false><<<g, dim3(BX, BY), 0, s>>>(d, coarse, fine);
+        red ? launch_dep(g, dim3(BX, BY), 0, s, k_restrict<T, true>, d, coarse, fine)
+            : launch_dep(g, dim3(BX, BY), 0, s, k_restrict<T, false>, d, coarse, fine);
 }
 // Fine-level residual and restriction in one pass. AFMIB_RESID_RESTRICT
 // (read at every call, so that a test can compare the paths in one process):
@@ -1858,8 +1872,8 @@ void launch_resid_restrict(const Dims& d, T* coarse_b, const T* x, const T* b, c
             const float* bf = reinterpret_cast<const float*>(b);
 #define AFMIB_RR_COLS(CZV)                                                                            \
     do {                                                                                              \
-        if (d.channel) k_resid_restrict_cols<CZV, true><<<g, blk, kRrSmem, s>>>(d, cbf, xf, bf, rev); \
-        else k_resid_restrict_cols<CZV, false><<<g, blk, kRrSmem, s>>>(d, cbf, xf, bf, rev);         \
+        if (d.channel) launch_dep(g, blk, kRrSmem, s, k_resid_restrict_cols<CZV, true>, d, cbf, xf, bf, rev); \
+        else launch_dep(g, blk, kRrSmem, s, k_resid_restrict_cols<CZV, false>, d, cbf, xf, bf, rev);         \
     } while (0)
             if (z == 8) AFMIB_RR_COLS(8);
             else if (z == 4) AFMIB_RR_COLS(4);
@@ -1889,26 +1903,26 @@ void launch_prolong_add(const Dims& d, T* fine, const T* coarse, cudaStream_t s,
             int z = std::min(transfer_planes(d), e ? std::max(1, std::atoi(e)) : 8);
             while (z & (z - 1)) z &= z - 1;  // a power of two, so a divisor of the plane count
             const dim3 g = transfer_grid(d, z), b(32, kTrBY);
-            if (z == 8) k_prolong_cols<T, 8><<<g, b, 0, s>>>(d, fine, coarse, rev);
-            else if (z == 4) k_prolong_cols<T, 4><<<g, b, 0, s>>>(d, fine, coarse, rev);
-            else if (z == 2) k_prolong_cols<T, 2><<<g, b, 0, s>>>(d, fine, coarse, rev);
-            else k_prolong_cols<T, 1><<<g, b, 0, s>>>(d, fine, coarse, rev);
+            if (z == 8) launch_dep(g, b, 0, s, k_prolong_cols<T, 8>, d, fine, coarse, rev);
+            else if (z == 4) launch_dep(g, b, 0, s, k_prolong_cols<T, 4>, d, fine, coarse, rev);
+            else if (z == 2) launch_dep(g, b, 0, s, k_prolong_cols<T, 2>, d, fine, coarse, rev);
+            else launch_dep(g, b, 0, s, k_prolong_cols<T, 1>, d, fine, coarse, rev);
             return;
         }
     }
     dim3 g((d.nx / 2 + BX - 1) / BX, (d.ny / 2 + BY - 1) / BY, d.nz == 1 ? 1 : d.nz / 2);
     if (d.nz > 1)
-        AFMIB_IX(d, (black ? k_prolong2<T, true, true, IX><<<g, dim3(BX, BY), 0, s>>>(d, fine, coarse, rev)
-                           : k_prolong2<T, true, false, IX><<<g, dim3(BX, BY), 0, s>>>(d, fine, coarse, rev)));
+        AFMIB_IX(d, (black ? launch_dep(g, dim3(BX, BY), 0, s, k_prolong2<T, true, true, IX>, d, fine, coarse, rev)
+                           : launch_dep(g, dim3(BX, BY), 0, s, k_prolong2<T, true, false, IX>, d, fine, coarse, rev)));
     else
-        black ? k_prolong<T, true, true><<<g, dim3(BX, BY), 0, s>>>(d, fine, coarse)
-              : k_prolong<T, true, false><<<g, dim3(BX, BY), 0, s>>>(d, fine, coarse);
+        black ? launch_dep(g, dim3(BX, BY), 0, s, k_prolong<T, true, true>, d, fine, coarse)
+              : launch_dep(g, dim3(BX, BY), 0, s, k_prolong<T, true, false>, d, fine, coarse);
 }
 template <typename T>
 void launch_prolong_assign(const Dims& d, T* fine, const T* coarse, cudaStream_t s) {
     dim3 g((d.nx / 2 + BX - 1) / BX, (d.ny / 2 + BY - 1) / BY, d.nz == 1 ? 1 : d.nz / 2);
-    if (d.nz > 1) AFMIB_IX(d, (k_prolong2<T, false, false, IX><<<g, dim3(BX, BY), 0, s>>>(d, fine, coarse, 0)));
-    else k_prolong<T, false, false><<<g, dim3(BX, BY), 0, s>>>(d, fine, coarse);
+    if (d.nz > 1) AFMIB_IX(d, (launch_dep(g, dim3(BX, BY), 0, s, k_prolong2<T, false, false, IX>, d, fine, coarse, 0)));
+    else launch_dep(g, dim3(BX, BY), 0, s, k_prolong<T, false, false>, d, fine, coarse);
 }
 template <typename TD>
 void launch_lap_defect(const Dims& d, TD* r, const double* x, const double* b, RedScratch sc, double* out, cudaStream_t s,
@@ -1933,8 +1947,7 @@ void launch_lap_update_df(const Dims& d, double* x, const float* e, float* rh, f
         const int gx = (d.nx + kRBX - 1) / kRBX, gy = (d.ny + kRBY - 1) / kRBY;
         int gz = d.nz / ZU;
         if ((long long)gx * gy * gz > kMaxRedBlocks) gz = std::max(1, kMaxRedBlocks / (gx * gy));
-        AFMIB_IX(d, (k_lap_update_df2<ZU, kUpdateMinBlocks, IX><<<dim3(gx, gy, gz), dim3(kRBX, kRBY), 0, s>>>(
-                        d, x, e, rh, rl, sc, out)));
+        AFMIB_IX(d, (launch_dep(dim3(gx, gy, gz), dim3(kRBX, kRBY), 0, s, k_lap_update_df2<ZU, kUpdateMinBlocks, IX>, d, x, e, rh, rl, sc, out)));
         return;
     }
     k_lap_update_df<<<red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s>>>(d, x, e, rh, rl, sc, out);

@@ -524,6 +524,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_mg_tail(const __grid_consta
         if (L.nc > 1) cl.sync();
         else __syncthreads();
     };
+    wait_launch();
     {
         const TailLv<T>& L = args.lv[0];
         int z0;
@@ -847,13 +848,15 @@ void launch_vcycle_tail(const TailLevels<T>& a, cudaStream_t s) {
     cfg.blockDim = dim3(most > kTailThreads / 2 ? kTailThreads : kTailThreads / 2);
     cfg.dynamicSmemBytes = bytes;
     cfg.stream = s;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = cs;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // launch_dep
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     // errors reach the caller's cudaGetLastError
     if (a.flat) cudaLaunchKernelEx(&cfg, k_mg_tail<T, true, false>, g);
     else if (g.channel) cudaLaunchKernelEx(&cfg, k_mg_tail<T, false, true>, g);
