@@ -50,6 +50,7 @@ __global__ void k_advect_adjoint(Dims d, double* __restrict__ ou, double* __rest
                                  const double* __restrict__ u, const double* __restrict__ v, const double* __restrict__ w,
                                  const double* __restrict__ lu, const double* __restrict__ lv,
                                  const double* __restrict__ lw, int acc) {
+    wait_launch();
     const int x = blockIdx.x * BX + threadIdx.x, y = blockIdx.y * BY + threadIdx.y, z = blockIdx.z;
     if (x >= d.nx || y >= d.ny) return;
     const Ix I{d};
@@ -109,6 +110,7 @@ __device__ __forceinline__ void weights4(double s, double off, int& base, double
 __global__ void k_marker_grad(Dims d, int M, const double* __restrict__ X, const double* __restrict__ g,
                               const double* __restrict__ Fu, const double* __restrict__ Fv,
                               const double* __restrict__ Fw, double scale, double* __restrict__ gX) {
+    wait_launch();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= M) return;
     const int ext[3] = {d.nx, d.ny, d.nz};
@@ -145,6 +147,7 @@ __global__ void k_marker_grad(Dims d, int M, const double* __restrict__ X, const
 __global__ void k_springs_adjoint(int M, const double* __restrict__ X, const int* __restrict__ ns,
                                   const int* __restrict__ ni, double kspring, const double* __restrict__ lamG,
                                   double* __restrict__ gX, double* __restrict__ dk_part) {
+    wait_launch();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= M) return;
     double kx[3] = {0, 0, 0}, kt[3] = {0, 0, 0};
@@ -165,6 +168,7 @@ __global__ void k_springs_adjoint(int M, const double* __restrict__ X, const int
 // symmetric), in two passes through Z = L lamG (stored like lamG).
 __global__ void k_lap_soa(int M, const double* __restrict__ lam, const int* __restrict__ ns,
                           const int* __restrict__ ni, double* __restrict__ Z) {
+    wait_launch();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= M) return;
     for (int a = 0; a < 3; ++a) {
@@ -176,6 +180,7 @@ __global__ void k_lap_soa(int M, const double* __restrict__ lam, const int* __re
 }
 __global__ void k_bend_adjoint(int M, const double* __restrict__ Z, const int* __restrict__ ns,
                                const int* __restrict__ ni, double kb, double* __restrict__ gX) {
+    wait_launch();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= M) return;
     for (int a = 0; a < 3; ++a) {
@@ -191,24 +196,24 @@ __global__ void k_bend_adjoint(int M, const double* __restrict__ Z, const int* _
 void launch_bending_adjoint(int M, const int* ns, const int* ni, double kb, const double* lamG, double* Z, double* gX,
                             cudaStream_t s) {
     if (M <= 0) return;
-    k_lap_soa<<<(M + 255) / 256, 256, 0, s>>>(M, lamG, ns, ni, Z);
-    k_bend_adjoint<<<(M + 255) / 256, 256, 0, s>>>(M, Z, ns, ni, kb, gX);
+    launch_dep((M + 255) / 256, 256, 0, s, k_lap_soa, M, lamG, ns, ni, Z);
+    launch_dep((M + 255) / 256, 256, 0, s, k_bend_adjoint, M, Z, ns, ni, kb, gX);
 }
 
 void launch_advect_adjoint(const Dims& d, double* ou, double* ov, double* ow, const double* u, const double* v,
                            const double* w, const double* lu, const double* lv, const double* lw, int acc,
                            cudaStream_t s) {
-    k_advect_adjoint<<<grid3(d), dim3(BX, BY), 0, s>>>(d, ou, ov, ow, u, v, w, lu, lv, lw, acc);
+    launch_dep(grid3(d), dim3(BX, BY), 0, s, k_advect_adjoint, d, ou, ov, ow, u, v, w, lu, lv, lw, acc);
 }
 
 void launch_marker_grad(const Dims& d, int M, const double* X, const double* g, const double* Fu, const double* Fv,
                         const double* Fw, double scale, double* gX, cudaStream_t s) {
-    if (M > 0) k_marker_grad<<<(M + 127) / 128, 128, 0, s>>>(d, M, X, g, Fu, Fv, Fw, scale, gX);
+    if (M > 0) launch_dep((M + 127) / 128, 128, 0, s, k_marker_grad, d, M, X, g, Fu, Fv, Fw, scale, gX);
 }
 
 void launch_springs_adjoint(int M, const double* X, const int* ns, const int* ni, double kspring, const double* lamG,
                             double* gX, double* dk_part, cudaStream_t s) {
-    if (M > 0) k_springs_adjoint<<<(M + 255) / 256, 256, 0, s>>>(M, X, ns, ni, kspring, lamG, gX, dk_part);
+    if (M > 0) launch_dep((M + 255) / 256, 256, 0, s, k_springs_adjoint, M, X, ns, ni, kspring, lamG, gX, dk_part);
 }
 
 }  // namespace afmib
@@ -217,12 +222,14 @@ namespace afmib {
 namespace {
 // soa[c*M + k] = c0 * aos[3k + c]
 __global__ void k_aos_to_soa(int M, const double* __restrict__ aos, double* __restrict__ soa, double c0) {
+    wait_launch();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= M) return;
     for (int c = 0; c < 3; ++c) soa[(size_t)c * M + k] = c0 * aos[3 * k + c];
 }
 // aos[3k + c] += c0 * soa[c*M + k]
 __global__ void k_soa_add_aos(int M, const double* __restrict__ soa, double* __restrict__ aos, double c0) {
+    wait_launch();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= M) return;
     for (int c = 0; c < 3; ++c) aos[3 * k + c] += c0 * soa[(size_t)c * M + k];
@@ -230,9 +237,9 @@ __global__ void k_soa_add_aos(int M, const double* __restrict__ soa, double* __r
 }  // namespace
 
 void launch_aos_to_soa(int M, const double* aos, double* soa, double c0, cudaStream_t s) {
-    if (M > 0) k_aos_to_soa<<<(M + 255) / 256, 256, 0, s>>>(M, aos, soa, c0);
+    if (M > 0) launch_dep((M + 255) / 256, 256, 0, s, k_aos_to_soa, M, aos, soa, c0);
 }
 void launch_soa_add_aos(int M, const double* soa, double* aos, double c0, cudaStream_t s) {
-    if (M > 0) k_soa_add_aos<<<(M + 255) / 256, 256, 0, s>>>(M, soa, aos, c0);
+    if (M > 0) launch_dep((M + 255) / 256, 256, 0, s, k_soa_add_aos, M, soa, aos, c0);
 }
 }  // namespace afmib

@@ -41,6 +41,7 @@ template <typename TI, typename T, bool P2>
 __global__ void __launch_bounds__(BX * BY, P2 ? 6 : 4) k_advect(Dims d, T* __restrict__ ua, T* __restrict__ va,
                                                                  T* __restrict__ wa, const TI* __restrict__ ui,
                                                                  const TI* __restrict__ vi, const TI* __restrict__ wi) {
+    wait_launch();
     AFMIB_XYZ
     // loads in the storage type TI, arithmetic in T (FP32 for the mixed form)
     struct Ld {
@@ -107,6 +108,7 @@ __global__ void __launch_bounds__(kAdvMaxNx) k_advect_rows(Dims d, int by, int z
                                                           double* __restrict__ va, double* __restrict__ wa,
                                                           const double* __restrict__ u, const double* __restrict__ v,
                                                           const double* __restrict__ w) {
+    wait_launch();
     extern __shared__ double sh[];  // [2][3][kAdvRows][threads]: uu, uv, uw of every thread's cells
     const int nt = blockDim.x, t = threadIdx.x;
     const int x = t % d.nx, ty = t / d.nx;
@@ -234,6 +236,7 @@ __global__ void __launch_bounds__(BX * BY, P2 ? 4 : 3) k_advect_df(Dims d, float
                                                                    const float* __restrict__ vl,
                                                                    const float* __restrict__ wh,
                                                                    const float* __restrict__ wl) {
+    wait_launch();
     AFMIB_XYZ
     const Ix2 I(d);
     auto lin = [&](int xx, int yy, int zz) -> long long {
@@ -290,6 +293,7 @@ __global__ void __launch_bounds__(BX * BY, P2 ? 4 : 3) k_advect_df(Dims d, float
 template <typename T>
 __global__ void k_div(Dims d, T* __restrict__ out, const T* __restrict__ u, const T* __restrict__ v,
                       const T* __restrict__ w, const T* __restrict__ top, const T* __restrict__ bottom) {
+    wait_launch();
     AFMIB_XYZ
     const long long i = lin(d, x, y, z);
     T dv;
@@ -321,6 +325,7 @@ __global__ void __launch_bounds__(kRedBlock) k_div_df(Dims d, double* __restrict
                                                      const double* __restrict__ top,
                                                      const double* __restrict__ bottom, RedScratch sc,
                                                      double* out_sum) {
+    wait_launch();
     const IX I(d);
     const int x = blockIdx.x * kRBX + threadIdx.x, y = blockIdx.y * kRBY + threadIdx.y;
     const df2 nn = {float(d.n), 0.f};
@@ -363,6 +368,7 @@ __global__ void __launch_bounds__(kRedBlock) k_div_df(Dims d, double* __restrict
 // Gradient, src/alg/grad.h:29-44.
 template <typename T>
 __global__ void k_grad(Dims d, T* __restrict__ px, T* __restrict__ py, T* __restrict__ pz, const T* __restrict__ p) {
+    wait_launch();
     AFMIB_XYZ
     const long long i = lin(d, x, y, z);
     const T n = T(d.n), p0 = p[i];
@@ -378,6 +384,7 @@ __global__ void k_grad_sub(Dims d, T* __restrict__ u, T* __restrict__ v, T* __re
                            T* __restrict__ wg, float* __restrict__ u32, float* __restrict__ v32,
                            float* __restrict__ w32, int round_shadow, float* __restrict__ u32l,
                            float* __restrict__ v32l, float* __restrict__ w32l) {
+    wait_launch();
     AFMIB_XYZ
     const long long i = lin(d, x, y, z);
     const T n = T(d.n), p0 = p[i];
@@ -427,6 +434,7 @@ __global__ void k_grad_sub(Dims d, T* __restrict__ u, T* __restrict__ v, T* __re
 // nx*min(ny, nz) wall entries and the w corrections read the x-gradient rows.
 // corrected: every nx*nz entry, the w corrections from the z-gradient rows.
 __global__ void k_wall_update(Dims d, double* __restrict__ walls, const double* __restrict__ wg, int corrected) {
+    wait_launch();
     const long long nxz = (long long)d.nx * d.nz;
     const long long cnt = corrected ? nxz : (long long)d.nx * (d.ny < d.nz ? d.ny : d.nz);
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < cnt; i += (long long)gridDim.x * blockDim.x) {
@@ -497,6 +505,7 @@ __device__ __forceinline__ T helm_point(const Dims& d, int comp, const HelmK<T>&
 
 template <typename T>
 __global__ void k_helm_apply(Dims d, int comp, HelmK<T> k, T* __restrict__ out, const T* __restrict__ in) {
+    wait_launch();
     AFMIB_XYZ
     out[lin(d, x, y, z)] = helm_point(d, comp, k, in, x, y, z);
 }
@@ -507,6 +516,7 @@ __global__ void k_helm_rhs(Dims d, int comp, int be, T* __restrict__ r, const T*
                            const TF* __restrict__ f, const TA* __restrict__ adv, const double* __restrict__ top,
                            const double* __restrict__ bottom, HelmK<T> kp, double s_plus, double s_minus, double hdt,
                            double inv_rho) {
+    wait_launch();
     AFMIB_XYZ
     const long long i = lin(d, x, y, z);
     if (d.channel && comp == 1 && y == 0) { r[i] = T(0); return; }
@@ -589,6 +599,7 @@ __global__ void __launch_bounds__(kRedBlock) k_helm_rhs_be_defect(Dims d, int co
                                                                  RedScratch sc, double* out,
                                                                  float* __restrict__ r_lo, double* __restrict__ uo_out,
                                                                  bool lo_split) {
+    wait_launch();
     float acc = 0.f;
     auto body = [&](int xi, int yi, int zi) {
         const long long i = lin(d, xi, yi, zi);
@@ -637,6 +648,7 @@ __global__ void k_helm_rhs_cn_q(Dims d, int comp, double* __restrict__ r, const 
                                 const double* __restrict__ q, const TF* __restrict__ f, const TA* __restrict__ adv,
                                 const double* __restrict__ top, const double* __restrict__ bottom, double s_plus,
                                 double s_minus, double off, double hdt, double inv_rho) {
+    wait_launch();
     AFMIB_XYZ
     const long long i = lin(d, x, y, z);
     if (d.channel && comp == 1 && y == 0) { r[i] = 0.0; return; }
@@ -667,6 +679,7 @@ __global__ void __launch_bounds__(kRedBlock) k_helm_cn_first(Dims d, int comp, d
                                                             const double* __restrict__ bottom, double s_plus,
                                                             double s_minus, double offd, double hdt, double inv_rho,
                                                             RedScratch sc, double* out) {
+    wait_launch();
     const int xi = blockIdx.x * kRBX + threadIdx.x, yi = blockIdx.y * kRBY + threadIdx.y;
     float acc = 0.f;
     if (xi < d.nx && yi < d.ny)
@@ -764,6 +777,7 @@ __global__ void __launch_bounds__(kRedBlock) k_helm_rhs_be_defect_df(Dims d, int
                                                                     const double* __restrict__ top,
                                                                     const double* __restrict__ bottom, DfCoef c,
                                                                     RedScratch sc, double* out) {
+    wait_launch();
     float acc = 0.f;
     auto body = [&](int xi, int yi, int zi) {
         const long long i = lin(d, xi, yi, zi);
@@ -808,6 +822,7 @@ __global__ void __launch_bounds__(kRedBlock) k_helm_cn_first_df(Dims d, int comp
                                                                const double* __restrict__ top,
                                                                const double* __restrict__ bottom, DfCoef c,
                                                                RedScratch sc, double* out) {
+    wait_launch();
     const int xi = blockIdx.x * kRBX + threadIdx.x, yi = blockIdx.y * kRBY + threadIdx.y;
     float acc = 0.f;
     if (xi < d.nx && yi < d.ny)
@@ -843,6 +858,7 @@ template <typename T>
 __global__ void __launch_bounds__(kRedBlock) k_cg_init(Dims d, int comp, HelmK<T> k, const T* __restrict__ x,
                                                       const T* __restrict__ b, T* __restrict__ r, T* __restrict__ p,
                                                       RedScratch sc, double* cgs) {
+    wait_launch();
     const int xi = blockIdx.x * kRBX + threadIdx.x, yi = blockIdx.y * kRBY + threadIdx.y;
     T acc = T(0);
     if (xi < d.nx && yi < d.ny)
@@ -861,6 +877,7 @@ __global__ void __launch_bounds__(kRedBlock) k_cg_init(Dims d, int comp, HelmK<T
 template <typename T>
 __global__ void __launch_bounds__(kRedBlock) k_cg_apply(Dims d, int comp, HelmK<T> k, const T* __restrict__ p,
                                                        T* __restrict__ q, RedScratch sc, double* cgs) {
+    wait_launch();
     const int xi = blockIdx.x * kRBX + threadIdx.x, yi = blockIdx.y * kRBY + threadIdx.y;
     T acc = T(0);
     if (xi < d.nx && yi < d.ny)
@@ -879,6 +896,7 @@ template <typename T>
 __global__ void __launch_bounds__(kRedBlock) k_cg_update(long long N, T* __restrict__ x, T* __restrict__ r,
                                                         const T* __restrict__ p, const T* __restrict__ q,
                                                         RedScratch sc, double* cgs) {
+    wait_launch();
     const T alpha = T(cgs[4]);
     T part = T(0);
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
@@ -901,6 +919,7 @@ template <typename T>
 __global__ void __launch_bounds__(kRedBlock) k_cg_dir_apply(Dims d, int comp, HelmK<T> k, const T* __restrict__ p,
                                                            const T* __restrict__ r, T* __restrict__ pn,
                                                            T* __restrict__ q, RedScratch sc, double* cgs) {
+    wait_launch();
     const T beta = T(cgs[3]);
     auto P = [p, r, beta](long long i) { return p[i] * beta + r[i]; };
     const int xi = blockIdx.x * kRBX + threadIdx.x, yi = blockIdx.y * kRBY + threadIdx.y;
@@ -921,6 +940,7 @@ __global__ void __launch_bounds__(kRedBlock) k_cg_dir_apply(Dims d, int comp, He
 
 template <typename T>
 __global__ void k_cg_direction(long long N, T* __restrict__ p, const T* __restrict__ r, const double* cgs) {
+    wait_launch();
     const T beta = T(cgs[3]);
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x)
         p[i] = p[i] * beta + r[i];
@@ -1060,6 +1080,7 @@ __global__ void __launch_bounds__(kRedBlock) k_helm_defect(Dims d, int comp, Hel
                                                           const double* __restrict__ b, TD* __restrict__ r,
                                                           RedScratch sc, double* out, float* __restrict__ r_lo,
                                                           bool lo_split) {
+    wait_launch();
     TD acc = TD(0);
     auto body = [&](int xi, int yi, int zi) {
         const long long i = lin(d, xi, yi, zi);
@@ -1091,6 +1112,7 @@ __global__ void __launch_bounds__(kRedBlock) k_helm_defect(Dims d, int comp, Hel
 __global__ void __launch_bounds__(kRedBlock) k_helm_defect_bfp(Dims d, int comp, double s, const double* __restrict__ x,
                                                               const double* __restrict__ b, float* __restrict__ r,
                                                               RedScratch sc, double* out) {
+    wait_launch();
     const int xi = blockIdx.x * kRBX + threadIdx.x, yi = blockIdx.y * kRBY + threadIdx.y;
     const double off = s * (double)d.n * (double)d.n;
     const df2 f1 = df_split(off), f3 = df_split(off / 3.0);
@@ -1172,6 +1194,7 @@ template <typename T>
 __global__ void __launch_bounds__(kRedBlock) k_cg_init_zero(long long N, const T* __restrict__ b, T* __restrict__ x,
                                                            T* __restrict__ r, T* __restrict__ p, RedScratch sc,
                                                            double* cgs) {
+    wait_launch();
     T part = T(0);
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
         const T bi = b[i];
@@ -1186,6 +1209,7 @@ __global__ void __launch_bounds__(kRedBlock) k_cg_init_zero(long long N, const T
 
 template <typename TE>
 __global__ void k_add_correction(long long N, double* __restrict__ x, const TE* __restrict__ e) {
+    wait_launch();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x)
         x[i] = x[i] + cvt<double, TE>(e[i]);
 }
@@ -1193,6 +1217,7 @@ __global__ void k_add_correction(long long N, double* __restrict__ x, const TE* 
 // The same, four cells per thread and iteration with 16-byte accesses
 // (n4 = N / 4; x and e 16-byte aligned)
 __global__ void k_add_correction4(long long n4, double2* __restrict__ x, const float4* __restrict__ e) {
+    wait_launch();
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n4; q += (long long)gridDim.x * blockDim.x) {
         const float4 c = e[q];
         double2 a = x[2 * q], b = x[2 * q + 1];
@@ -1210,6 +1235,7 @@ __global__ void k_add_correction4(long long n4, double2* __restrict__ x, const f
 // ---------------------------------------------------------------------------
 template <typename T, bool SQ>
 __global__ void __launch_bounds__(kRedBlock) k_sum(long long N, const T* __restrict__ x, RedScratch sc, double* out) {
+    wait_launch();
     T part = T(0);
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
         const T e = x[i];
@@ -1221,6 +1247,7 @@ __global__ void __launch_bounds__(kRedBlock) k_sum(long long N, const T* __restr
 
 template <typename T>
 __global__ void k_sub_scalar(long long N, T* __restrict__ x, const double* sum, double scale) {
+    wait_launch();
     const T m = T(sum[0] * scale);
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x)
         x[i] = x[i] - m;
@@ -1228,30 +1255,35 @@ __global__ void k_sub_scalar(long long N, T* __restrict__ x, const double* sum, 
 
 template <typename T>
 __global__ void k_fill(long long N, T* __restrict__ x, T v) {
+    wait_launch();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x)
         x[i] = v;
 }
 
 template <typename T>
 __global__ void k_axpy(long long N, T* __restrict__ y, const T* __restrict__ x, T a) {
+    wait_launch();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x)
         y[i] = y[i] + a * x[i];
 }
 
 template <typename T>
 __global__ void k_lincomb(long long N, T* __restrict__ y, T a, const T* __restrict__ x, T b, const T* __restrict__ z) {
+    wait_launch();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x)
         y[i] = a * x[i] + b * z[i];
 }
 
 template <typename T>
 __global__ void k_scale(long long N, T* __restrict__ x, T a) {
+    wait_launch();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x)
         x[i] = a * x[i];
 }
 
 template <typename TO, typename TI>
 __global__ void k_convert(long long N, TO* __restrict__ o, const TI* __restrict__ in) {
+    wait_launch();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x)
         o[i] = (TO)in[i];
 }
@@ -1285,51 +1317,51 @@ void launch_advect(const Dims& d, T* ua, T* va, T* wa, const TI* u, const TI* v,
                 }
             }
             const size_t smem = sizeof(double) * 2 * 3 * kAdvRows * nt;
-            k_advect_rows<<<dim3(gy, (d.nz + zc - 1) / zc), nt, smem, s>>>(d, by, zc, 0.25 * (double)d.n, ua, va, wa, u, v,
-                                                                         w);
+            launch_dep(dim3(gy, (d.nz + zc - 1) / zc), nt, smem, s, k_advect_rows, d, by, zc, 0.25 * (double)d.n, ua,
+                       va, wa, u, v, w);
             return;
         }
     }
-    if (ix2_ok(d)) k_advect<TI, T, true><<<grid3(d), block3(), 0, s>>>(d, ua, va, wa, u, v, w);
-    else k_advect<TI, T, false><<<grid3(d), block3(), 0, s>>>(d, ua, va, wa, u, v, w);
+    if (ix2_ok(d)) launch_dep(grid3(d), block3(), 0, s, k_advect<TI, T, true>, d, ua, va, wa, u, v, w);
+    else launch_dep(grid3(d), block3(), 0, s, k_advect<TI, T, false>, d, ua, va, wa, u, v, w);
 }
 void launch_advect_df(const Dims& d, float* ua, float* va, float* wa, const float* uh, const float* ul,
                       const float* vh, const float* vl, const float* wh, const float* wl, cudaStream_t s) {
-    if (ix2_ok(d)) k_advect_df<true><<<grid3(d), block3(), 0, s>>>(d, ua, va, wa, uh, ul, vh, vl, wh, wl);
-    else k_advect_df<false><<<grid3(d), block3(), 0, s>>>(d, ua, va, wa, uh, ul, vh, vl, wh, wl);
+    if (ix2_ok(d)) launch_dep(grid3(d), block3(), 0, s, k_advect_df<true>, d, ua, va, wa, uh, ul, vh, vl, wh, wl);
+    else launch_dep(grid3(d), block3(), 0, s, k_advect_df<false>, d, ua, va, wa, uh, ul, vh, vl, wh, wl);
 }
 template <typename T>
 void launch_div(const Dims& d, T* out, const T* u, const T* v, const T* w, const T* top, const T* bottom, cudaStream_t s) {
-    k_div<T><<<grid3(d), block3(), 0, s>>>(d, out, u, v, w, top, bottom);
+    launch_dep(grid3(d), block3(), 0, s, k_div<T>, d, out, u, v, w, top, bottom);
 }
 void launch_div_df(const Dims& d, double* out, const double* u, const double* v, const double* w, const double* top,
                    const double* bottom, RedScratch sc, double* out_sum, cudaStream_t s) {
     const dim3 blk(kRBX, kRBY);
     if (d.nz % 2 == 0)
-        AFMIB_IX(d, (k_div_df<2, IX><<<red_grid3(d.nx, d.ny, d.nz / 2), blk, 0, s>>>(d, out, u, v, w, top, bottom, sc,
-                                                                                  out_sum)));
+        AFMIB_IX(d, (launch_dep(red_grid3(d.nx, d.ny, d.nz / 2), blk, 0, s, k_div_df<2, IX>, d, out, u, v, w, top,
+                                bottom, sc, out_sum)));
     else
-        AFMIB_IX(d, (k_div_df<1, IX><<<red_grid3(d.nx, d.ny, d.nz), blk, 0, s>>>(d, out, u, v, w, top, bottom, sc, out_sum)));
+        AFMIB_IX(d, (launch_dep(red_grid3(d.nx, d.ny, d.nz), blk, 0, s, k_div_df<1, IX>, d, out, u, v, w, top,
+                                bottom, sc, out_sum)));
 }
 template <typename T>
 void launch_grad(const Dims& d, T* px, T* py, T* pz, const T* p, cudaStream_t s) {
-    k_grad<T><<<grid3(d), block3(), 0, s>>>(d, px, py, pz, p);
+    launch_dep(grid3(d), block3(), 0, s, k_grad<T>, d, px, py, pz, p);
 }
 template <typename T>
 void launch_grad_sub(const Dims& d, T* u, T* v, T* w, const T* phi, T* wallgrad, cudaStream_t s, float* u32,
                      float* v32, float* w32, int round_shadow, float* u32l, float* v32l, float* w32l) {
-    k_grad_sub<T><<<grid3(d), block3(), 0, s>>>(d, u, v, w, phi, wallgrad, u32, v32, w32, round_shadow, u32l, v32l,
-                                                w32l);
+    launch_dep(grid3(d), block3(), 0, s, k_grad_sub<T>, d, u, v, w, phi, wallgrad, u32, v32, w32, round_shadow, u32l,
+               v32l, w32l);
 }
 void launch_wall_update(const Dims& d, double* walls, const double* wallgrad, cudaStream_t s, int corrected) {
-    k_wall_update<<<ew_blocks((long long)d.nx * d.nz), 256, 0, s>>>(d, walls, wallgrad, corrected);
+    launch_dep(ew_blocks((long long)d.nx * d.nz), 256, 0, s, k_wall_update, d, walls, wallgrad, corrected);
 }
 template <typename T, typename TF, typename TA>
 void launch_helm_rhs(const Dims& d, int comp, int be, T* r, const T* uold, const TF* f, const TA* adv, const double* top,
                      const double* bottom, double s_plus, double s_minus, double dt, double inv_rho, cudaStream_t s) {
-    k_helm_rhs<T, TF, TA><<<grid3(d), block3(), 0, s>>>(d, comp, be, r, uold, f, adv, top, bottom,
-                                                        helm_k<T>(d, s_plus), s_plus, s_minus,
-                                                        be ? dt / 2 : dt, inv_rho);
+    launch_dep(grid3(d), block3(), 0, s, k_helm_rhs<T, TF, TA>, d, comp, be, r, uold, f, adv, top, bottom,
+               helm_k<T>(d, s_plus), s_plus, s_minus, be ? dt / 2 : dt, inv_rho);
 }
 template <typename TF, typename TA>
 void launch_helm_rhs_be_defect(const Dims& d, int comp, double* b, float* r, double* q, const double* uold,
@@ -1337,9 +1369,9 @@ void launch_helm_rhs_be_defect(const Dims& d, int comp, double* b, float* r, dou
                                double dt, double inv_rho, RedScratch sc, double* out, cudaStream_t s, int walk_blocks,
                                float* r_lo, double* uo_out) {
 #define AFMIB_BE(WALKV, DFRV, GRID)                                                                          \
-    k_helm_rhs_be_defect<TF, TA, WALKV, DFRV><<<GRID, dim3(kRBX, kRBY), 0, s>>>(                             \
-        d, comp, b, r, q, uold, f, adv, top, bottom, helm_k<double>(d, s_minus), s_minus, dt / 2, inv_rho, sc,  \
-        out, r_lo, uo_out, lo_split())
+    launch_dep(GRID, dim3(kRBX, kRBY), 0, s, k_helm_rhs_be_defect<TF, TA, WALKV, DFRV>, d, comp, b, r, q, uold, f, \
+               adv, top, bottom, helm_k<double>(d, s_minus), s_minus, dt / 2, inv_rho, sc, out, r_lo, uo_out, \
+               lo_split())
     if (walk_blocks > 0) {
         if (r_lo) AFMIB_BE(true, true, walk_grid(d, walk_blocks));
         else AFMIB_BE(true, false, walk_grid(d, walk_blocks));
@@ -1368,11 +1400,11 @@ void launch_helm_rhs_be_defect_df(const Dims& d, int comp, float* r, float* r_lo
                                   double* out, cudaStream_t s, int walk_blocks) {
     const DfCoef c = df_coef(d, dt / 2, inv_rho, s_minus * double(d.n) * double(d.n), s_minus);
     if (walk_blocks > 0)
-        k_helm_rhs_be_defect_df<TA, true><<<walk_grid(d, walk_blocks), dim3(kRBX, kRBY), 0, s>>>(
-            d, comp, r, r_lo, q, uo_out, uold, f, adv, top, bottom, c, sc, out);
+        launch_dep(walk_grid(d, walk_blocks), dim3(kRBX, kRBY), 0, s, k_helm_rhs_be_defect_df<TA, true>, d, comp, r,
+                   r_lo, q, uo_out, uold, f, adv, top, bottom, c, sc, out);
     else
-        k_helm_rhs_be_defect_df<TA, false><<<red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s>>>(
-            d, comp, r, r_lo, q, uo_out, uold, f, adv, top, bottom, c, sc, out);
+        launch_dep(red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s, k_helm_rhs_be_defect_df<TA, false>, d, comp,
+                   r, r_lo, q, uo_out, uold, f, adv, top, bottom, c, sc, out);
 }
 template <typename TA>
 void launch_helm_cn_first_df(const Dims& d, int comp, double* x, float* rh, float* rl, const double* uold,
@@ -1380,8 +1412,8 @@ void launch_helm_cn_first_df(const Dims& d, int comp, double* x, float* rh, floa
                              double s_plus, double s_minus, double dt, double inv_rho, RedScratch sc, double* out,
                              cudaStream_t s) {
     const DfCoef c = df_coef(d, dt, inv_rho, (s_plus - s_minus) * double(d.n) * double(d.n), s_plus - s_minus);
-    k_helm_cn_first_df<TA><<<red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s>>>(d, comp, x, rh, rl, uold, q, f, adv,
-                                                                                    top, bottom, c, sc, out);
+    launch_dep(red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s, k_helm_cn_first_df<TA>, d, comp, x, rh, rl, uold,
+               q, f, adv, top, bottom, c, sc, out);
 }
 template void launch_helm_rhs_be_defect_df<float>(const Dims&, int, float*, float*, double*, double*, const double*,
                                                   const double*, const float*, const double*, const double*, double,
@@ -1394,17 +1426,16 @@ template <typename TF, typename TA>
 void launch_helm_rhs_cn_q(const Dims& d, int comp, double* r, const double* uold, const double* q, const TF* f,
                           const TA* adv, const double* top, const double* bottom, double s_plus, double s_minus,
                           double dt, double inv_rho, cudaStream_t s) {
-    k_helm_rhs_cn_q<TF, TA><<<grid3(d), block3(), 0, s>>>(d, comp, r, uold, q, f, adv, top, bottom, s_plus, s_minus,
-                                                          s_plus * double(d.n) * double(d.n), dt,
-                                                          inv_rho);
+    launch_dep(grid3(d), block3(), 0, s, k_helm_rhs_cn_q<TF, TA>, d, comp, r, uold, q, f, adv, top, bottom, s_plus,
+               s_minus, s_plus * double(d.n) * double(d.n), dt, inv_rho);
 }
 template <typename TF, typename TA>
 void launch_helm_cn_first(const Dims& d, int comp, double* x, float* rh, float* rl, const double* uold, const double* q,
                           const TF* f, const TA* adv, const double* top, const double* bottom, double s_plus,
                           double s_minus, double dt, double inv_rho, RedScratch sc, double* out, cudaStream_t s) {
-    k_helm_cn_first<TF, TA><<<red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s>>>(
-        d, comp, x, rh, rl, uold, q, f, adv, top, bottom, s_plus, s_minus,
-        (s_plus - s_minus) * double(d.n) * double(d.n), dt, inv_rho, sc, out);
+    launch_dep(red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s, k_helm_cn_first<TF, TA>, d, comp, x, rh, rl,
+               uold, q, f, adv, top, bottom, s_plus, s_minus, (s_plus - s_minus) * double(d.n) * double(d.n), dt,
+               inv_rho, sc, out);
 }
 template void launch_helm_cn_first<double, float>(const Dims&, int, double*, float*, float*, const double*,
                                                   const double*, const double*, const float*, const double*,
@@ -1433,11 +1464,11 @@ template <typename TD>
 void launch_helm_defect(const Dims& d, int comp, double scale, const double* x, const double* b, TD* r, RedScratch sc,
                         double* out, cudaStream_t s, int walk_blocks, float* r_lo) {
     if (walk_blocks > 0)
-        k_helm_defect<TD, true><<<walk_grid(d, walk_blocks), dim3(kRBX, kRBY), 0, s>>>(
-            d, comp, helm_k<double>(d, scale), x, b, r, sc, out, r_lo, lo_split());
+        launch_dep(walk_grid(d, walk_blocks), dim3(kRBX, kRBY), 0, s, k_helm_defect<TD, true>, d, comp,
+                   helm_k<double>(d, scale), x, b, r, sc, out, r_lo, lo_split());
     else
-        k_helm_defect<TD, false><<<red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s>>>(
-            d, comp, helm_k<double>(d, scale), x, b, r, sc, out, r_lo, lo_split());
+        launch_dep(red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s, k_helm_defect<TD, false>, d, comp,
+                   helm_k<double>(d, scale), x, b, r, sc, out, r_lo, lo_split());
 }
 
 // Mixed form, recursive outer residual of a viscous solve: with the FP32
@@ -1450,6 +1481,7 @@ __global__ void __launch_bounds__(kRedBlock) k_helm_update_df(Dims d, int comp, 
                                                              double* __restrict__ x, const float* __restrict__ e,
                                                              float* __restrict__ rh, float* __restrict__ rl,
                                                              RedScratch sc, double* out) {
+    wait_launch();
     float acc = 0.f;
     const int xi = blockIdx.x * kRBX + threadIdx.x, yi = blockIdx.y * kRBY + threadIdx.y;
     if (xi < d.nx && yi < d.ny)
@@ -1575,36 +1607,40 @@ void launch_helm_update_df(const Dims& d, int comp, double scale, double* x, con
         const int gx = (d.nx + kRBX - 1) / kRBX, gy = (d.ny + kRBY - 1) / kRBY;
         int gz = d.nz / ZU;
         if ((long long)gx * gy * gz > kMaxRedBlocks) gz = std::max(1, kMaxRedBlocks / (gx * gy));
-        AFMIB_IX(d, (launch_dep(dim3(gx, gy, gz), dim3(kRBX, kRBY), 0, s, k_helm_update_df2<ZU, kUpdateMinBlocks, IX>, d, comp, o, c, x, e, rh, rl, sc, out)));
+        AFMIB_IX(d, (launch_dep(dim3(gx, gy, gz), dim3(kRBX, kRBY), 0, s, k_helm_update_df2<ZU, kUpdateMinBlocks,
+                                IX>, d, comp, o, c, x, e, rh, rl, sc, out)));
         return;
     }
-    k_helm_update_df<<<red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s>>>(d, comp, o, c, x, e, rh, rl, sc, out);
+    launch_dep(red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s, k_helm_update_df, d, comp, o, c, x, e, rh, rl,
+               sc, out);
 }
 template <typename T>
 void launch_cg_init_zero(long long n, const T* b, T* x, T* r, T* p, RedScratch sc, double* cgs, cudaStream_t s) {
-    k_cg_init_zero<T><<<red_blocks(n), kRedBlock, 0, s>>>(n, b, x, r, p, sc, cgs);
+    launch_dep(red_blocks(n), kRedBlock, 0, s, k_cg_init_zero<T>, n, b, x, r, p, sc, cgs);
 }
 template <typename TE>
 void launch_add_correction(long long n, double* x, const TE* e, cudaStream_t s) {
     if (sizeof(TE) == 4 && n % 4 == 0 && ((uintptr_t)x % 16) == 0 && ((uintptr_t)e % 16) == 0) {
-        k_add_correction4<<<ew_blocks(n / 4), 256, 0, s>>>(n / 4, reinterpret_cast<double2*>(x),
-                                                          reinterpret_cast<const float4*>(e));
+        launch_dep(ew_blocks(n / 4), 256, 0, s, k_add_correction4, n / 4, reinterpret_cast<double2*>(x),
+                   reinterpret_cast<const float4*>(e));
         return;
     }
-    k_add_correction<TE><<<ew_blocks(n), 256, 0, s>>>(n, x, e);
+    launch_dep(ew_blocks(n), 256, 0, s, k_add_correction<TE>, n, x, e);
 }
 template <typename T>
 void launch_helm_apply(const Dims& d, int comp, double scale, T* y, const T* x, cudaStream_t s) {
-    k_helm_apply<T><<<grid3(d), block3(), 0, s>>>(d, comp, helm_k<T>(d, scale), y, x);
+    launch_dep(grid3(d), block3(), 0, s, k_helm_apply<T>, d, comp, helm_k<T>(d, scale), y, x);
 }
 template <typename T>
 void launch_cg_init(const Dims& d, int comp, double scale, const T* x, const T* b, T* r, T* p, RedScratch sc,
                     double* cgs, cudaStream_t s) {
-    k_cg_init<T><<<red_grid3(d.nx, d.ny, d.nz, red_target<T>()), dim3(kRBX, kRBY), 0, s>>>(d, comp, helm_k<T>(d, scale), x, b, r, p, sc, cgs);
+    launch_dep(red_grid3(d.nx, d.ny, d.nz, red_target<T>()), dim3(kRBX, kRBY), 0, s, k_cg_init<T>, d, comp,
+               helm_k<T>(d, scale), x, b, r, p, sc, cgs);
 }
 template <typename T>
 void launch_cg_apply(const Dims& d, int comp, double scale, const T* p, T* q, RedScratch sc, double* cgs, cudaStream_t s) {
-    k_cg_apply<T><<<red_grid3(d.nx, d.ny, d.nz, red_target<T>()), dim3(kRBX, kRBY), 0, s>>>(d, comp, helm_k<T>(d, scale), p, q, sc, cgs);
+    launch_dep(red_grid3(d.nx, d.ny, d.nz, red_target<T>()), dim3(kRBX, kRBY), 0, s, k_cg_apply<T>, d, comp,
+               helm_k<T>(d, scale), p, q, sc, cgs);
 }
 // the grid of one system, times the systems along z
 static dim3 cgb_grid(const Dims& d, int n, int* gz) {
@@ -1646,6 +1682,7 @@ void launch_cgb_direction(const Dims& d, const CgBatch& g, const double* cgs, cu
 template <typename T, int ZU, typename IX>
 __global__ void k_helm_jacobi2(Dims d, int comp, HelmK<T> k, const T* __restrict__ xv, T* __restrict__ xo,
                                const T* __restrict__ b, int rev) {
+    wait_launch();
     const IX I(d);
     const uint3 B = block_at(rev);
     const int x = B.x * BX + threadIdx.x, y = B.y * BY + threadIdx.y, z0 = B.z * ZU;
@@ -1757,9 +1794,11 @@ void launch_helm_rbgs_first(const Dims& d, int comp, double scale, T* x, const T
     const int gx = (d.nx / 2 + BX - 1) / BX, gy = (d.ny + BY - 1) / BY;
     const HelmK<T> k = helm_k<T>(d, scale);
     if (d.nz % 4 == 0)
-        AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz / 4), dim3(BX, BY), 0, s, k_helm_first<T, 4, 6, IX>, d, comp, k, x, b, rev)));
+        AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz / 4), dim3(BX, BY), 0, s, k_helm_first<T, 4, 6, IX>, d, comp, k, x,
+                                b, rev)));
     else
-        AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz / 2), dim3(BX, BY), 0, s, k_helm_first<T, 2, 6, IX>, d, comp, k, x, b, rev)));
+        AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz / 2), dim3(BX, BY), 0, s, k_helm_first<T, 2, 6, IX>, d, comp, k, x,
+                                b, rev)));
 }
 template void launch_helm_rbgs_first<float>(const Dims&, int, double, float*, const float*, cudaStream_t, int);
 
@@ -1771,9 +1810,11 @@ void launch_helm_rbgs(const Dims& d, int comp, double scale, int color, T* x, co
     // registers capped for 6 resident blocks (40 against 48): measured with the
     // multigrid smoother's cap, 50.5 against 50.0 IB steps/s at 256^3
     if (d.nz % 8 == 0)
-        AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz / 8), blk, 0, s, k_helm_rbgs2b<T, 8, 6, IX>, d, comp, k, color, x, b, rev)));
+        AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz / 8), blk, 0, s, k_helm_rbgs2b<T, 8, 6, IX>, d, comp, k, color, x,
+                                b, rev)));
     else
-        AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz / 2), blk, 0, s, k_helm_rbgs2b<T, 2, 6, IX>, d, comp, k, color, x, b, rev)));
+        AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz / 2), blk, 0, s, k_helm_rbgs2b<T, 2, 6, IX>, d, comp, k, color, x,
+                                b, rev)));
 }
 template void launch_helm_rbgs<float>(const Dims&, int, double, int, float*, const float*, cudaStream_t, int);
 
@@ -1783,8 +1824,8 @@ void launch_helm_jacobi(const Dims& d, int comp, double scale, const T* x, T* xo
     const dim3 blk(BX, BY);
     const HelmK<T> k = helm_k<T>(d, scale);
     const dim3 g((d.nx + BX - 1) / BX, (d.ny + BY - 1) / BY, d.nz % 8 == 0 ? d.nz / 8 : d.nz);
-    if (d.nz % 8 == 0) AFMIB_IX(d, (k_helm_jacobi2<T, 8, IX><<<g, blk, 0, s>>>(d, comp, k, x, xo, b, rev)));
-    else AFMIB_IX(d, (k_helm_jacobi2<T, 1, IX><<<g, blk, 0, s>>>(d, comp, k, x, xo, b, rev)));
+    if (d.nz % 8 == 0) AFMIB_IX(d, (launch_dep(g, blk, 0, s, k_helm_jacobi2<T, 8, IX>, d, comp, k, x, xo, b, rev)));
+    else AFMIB_IX(d, (launch_dep(g, blk, 0, s, k_helm_jacobi2<T, 1, IX>, d, comp, k, x, xo, b, rev)));
 }
 template void launch_helm_jacobi<float>(const Dims&, int, double, const float*, float*, const float*, cudaStream_t,
                                         int);
@@ -1792,53 +1833,55 @@ template void launch_helm_jacobi<float>(const Dims&, int, double, const float*, 
 template <typename T>
 void launch_cg_dir_apply(const Dims& d, int comp, double scale, const T* p, const T* r, T* pn, T* q, RedScratch sc,
                          double* cgs, cudaStream_t s) {
-    k_cg_dir_apply<T><<<red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s>>>(d, comp, helm_k<T>(d, scale), p, r, pn, q, sc, cgs);
+    launch_dep(red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s, k_cg_dir_apply<T>, d, comp, helm_k<T>(d, scale),
+               p, r, pn, q, sc, cgs);
 }
 template <typename T>
 void launch_cg_update(long long n, T* x, T* r, const T* p, const T* q, RedScratch sc, double* cgs, cudaStream_t s) {
-    k_cg_update<T><<<red_blocks(n, red_target<T>()), kRedBlock, 0, s>>>(n, x, r, p, q, sc, cgs);
+    launch_dep(red_blocks(n, red_target<T>()), kRedBlock, 0, s, k_cg_update<T>, n, x, r, p, q, sc, cgs);
 }
 template <typename T>
 void launch_cg_direction(long long n, T* p, const T* r, const double* cgs, cudaStream_t s) {
-    k_cg_direction<T><<<ew_blocks(n), 256, 0, s>>>(n, p, r, cgs);
+    launch_dep(ew_blocks(n), 256, 0, s, k_cg_direction<T>, n, p, r, cgs);
 }
 template <typename T>
 void launch_sum(long long n, const T* x, RedScratch sc, double* out, cudaStream_t s) {
-    k_sum<T, false><<<red_blocks(n, red_target<T>()), kRedBlock, 0, s>>>(n, x, sc, out);
+    launch_dep(red_blocks(n, red_target<T>()), kRedBlock, 0, s, k_sum<T, false>, n, x, sc, out);
 }
 template <typename T>
 void launch_sumsq(long long n, const T* x, RedScratch sc, double* out, cudaStream_t s) {
-    k_sum<T, true><<<red_blocks(n, red_target<T>()), kRedBlock, 0, s>>>(n, x, sc, out);
+    launch_dep(red_blocks(n, red_target<T>()), kRedBlock, 0, s, k_sum<T, true>, n, x, sc, out);
 }
 template <typename T>
 void launch_sub_scalar_scaled(long long n, T* x, const double* sum, double scale, cudaStream_t s) {
-    k_sub_scalar<T><<<ew_blocks(n), 256, 0, s>>>(n, x, sum, scale);
+    launch_dep(ew_blocks(n), 256, 0, s, k_sub_scalar<T>, n, x, sum, scale);
 }
 template <typename T>
 void launch_fill(long long n, T* x, T value, cudaStream_t s) {
-    k_fill<T><<<ew_blocks(n), 256, 0, s>>>(n, x, value);
+    launch_dep(ew_blocks(n), 256, 0, s, k_fill<T>, n, x, value);
 }
 template <typename T>
 void launch_axpy(long long n, T* y, const T* x, T a, cudaStream_t s) {
-    k_axpy<T><<<ew_blocks(n), 256, 0, s>>>(n, y, x, a);
+    launch_dep(ew_blocks(n), 256, 0, s, k_axpy<T>, n, y, x, a);
 }
 template <typename T>
 void launch_scale(long long n, T* x, T a, cudaStream_t s) {
-    k_scale<T><<<ew_blocks(n), 256, 0, s>>>(n, x, a);
+    launch_dep(ew_blocks(n), 256, 0, s, k_scale<T>, n, x, a);
 }
 template <typename T>
 void launch_lincomb(long long n, T* y, T a, const T* x, T b, const T* z, cudaStream_t s) {
-    k_lincomb<T><<<ew_blocks(n), 256, 0, s>>>(n, y, a, x, b, z);
+    launch_dep(ew_blocks(n), 256, 0, s, k_lincomb<T>, n, y, a, x, b, z);
 }
 template <typename TO, typename TI>
 void launch_convert(long long n, TO* out, const TI* in, cudaStream_t s) {
-    k_convert<TO, TI><<<ew_blocks(n), 256, 0, s>>>(n, out, in);
+    launch_dep(ew_blocks(n), 256, 0, s, k_convert<TO, TI>, n, out, in);
 }
 
 // FP32 shadow of an FP64 velocity field (and, with lo, the rest of its
 // pair), as k_grad_sub writes it
 __global__ void k_shadow(long long N, float* __restrict__ o, const double* __restrict__ in, int round_shadow,
                          float* __restrict__ lo) {
+    wait_launch();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
         if (lo) {
             const df2 p = df_split_round(in[i]);
@@ -1850,7 +1893,7 @@ __global__ void k_shadow(long long N, float* __restrict__ o, const double* __res
     }
 }
 void launch_shadow(long long n, float* out, const double* in, cudaStream_t s, int round_shadow, float* lo) {
-    k_shadow<<<ew_blocks(n), 256, 0, s>>>(n, out, in, round_shadow, lo);
+    launch_dep(ew_blocks(n), 256, 0, s, k_shadow, n, out, in, round_shadow, lo);
 }
 
 #define AFMIB_INST(T)                                                                                          \
@@ -1891,7 +1934,8 @@ template void launch_helm_rhs<double, double, float>(const Dims&, int, int, doub
                                                      double, double, cudaStream_t);
 void launch_helm_defect_bfp(const Dims& d, int comp, double scale, const double* x, const double* b, float* r,
                             RedScratch sc, double* out, cudaStream_t s) {
-    k_helm_defect_bfp<<<red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s>>>(d, comp, scale, x, b, r, sc, out);
+    launch_dep(red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s, k_helm_defect_bfp, d, comp, scale, x, b, r, sc,
+               out);
 }
 template void launch_helm_defect<float>(const Dims&, int, double, const double*, const double*, float*, RedScratch,
                                         double*, cudaStream_t, int, float*);

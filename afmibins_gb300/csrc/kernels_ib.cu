@@ -41,6 +41,7 @@ __device__ __forceinline__ float sinpi_cospi(float x, float* c) {
 template <typename T>
 __global__ void k_springs(int M, const double* __restrict__ X, const int* __restrict__ ns, const int* __restrict__ ni,
                           double k, T* __restrict__ G) {
+    wait_launch();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= M) return;
     const double xi = X[3 * i], yi = X[3 * i + 1], zi = X[3 * i + 2];
@@ -60,6 +61,7 @@ __global__ void k_springs(int M, const double* __restrict__ X, const int* __rest
 // like X: Y_i = sum_{j in N(i)} (X_j - X_i)
 __global__ void k_lap_aos(int M, const double* __restrict__ X, const int* __restrict__ ns, const int* __restrict__ ni,
                           double* __restrict__ Y) {
+    wait_launch();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= M) return;
     const double xi = X[3 * i], yi = X[3 * i + 1], zi = X[3 * i + 2];
@@ -81,6 +83,7 @@ __global__ void k_lap_aos(int M, const double* __restrict__ X, const int* __rest
 template <typename T>
 __global__ void k_spring_bend(int M, const double* __restrict__ Y, const int* __restrict__ ns,
                               const int* __restrict__ ni, double ks, double kb, T* __restrict__ G) {
+    wait_launch();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= M) return;
     const double yi[3] = {Y[3 * i], Y[3 * i + 1], Y[3 * i + 2]};
@@ -101,6 +104,7 @@ __global__ void k_spring_bend(int M, const double* __restrict__ Y, const int* __
 template <typename T, bool DF>
 __global__ void k_marker_prep(Dims d, int TS, int M, const double* __restrict__ X, unsigned* __restrict__ keys,
                               int* __restrict__ vals, MarkerW<T> mw, int* __restrict__ flag) {
+    wait_launch();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= M) return;
     const int ext[3] = {d.nx, d.ny, d.nz};
@@ -172,6 +176,7 @@ constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
 
 __global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const unsigned* __restrict__ keys, int n, int shift,
                                                         unsigned* __restrict__ hist, int nblk) {
+    wait_launch();
     __shared__ unsigned cnt[256];
     cnt[threadIdx.x] = 0;
     __syncthreads();
@@ -188,6 +193,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const unsigned* __restri
 // totals go behind them (hist[256 nblk + digit]) and the scatter scans those 256.
 // (One block over all of it took 15 us per pass at 200,000 markers and 100 at 10^6.)
 __global__ void __launch_bounds__(RS_THREADS) k_rs_scan(unsigned* __restrict__ hist, int nblk) {
+    wait_launch();
     const int dig = blockIdx.x * (RS_THREADS / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     unsigned* row = hist + (size_t)dig * nblk;
     unsigned run = 0;
@@ -216,6 +222,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_scan(unsigned* __restrict__ h
 __global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const unsigned* __restrict__ kin, const int* __restrict__ vin,
                                                            unsigned* __restrict__ kout, int* __restrict__ vout, int n,
                                                            int shift, const unsigned* __restrict__ hist, int nblk) {
+    wait_launch();
     constexpr int W = RS_THREADS / 32;
     __shared__ unsigned cnt[256][W + 1];
     __shared__ unsigned wsum[W];
@@ -285,6 +292,7 @@ __global__ void __launch_bounds__(RSS_THREADS, 1) k_sort_small(unsigned* __restr
                                                               int bits, int cells_per_tile, int ntiles,
                                                               int* __restrict__ tstart, int* __restrict__ tend,
                                                               int* __restrict__ counts) {
+    wait_launch();
     extern __shared__ unsigned rss_smem[];
     unsigned* sk = rss_smem;                           // [ITEMS * RSS_THREADS]
     unsigned* cnt = sk + RSS_THREADS * ITEMS;          // [256][RSS_COLS]
@@ -374,6 +382,7 @@ __global__ void __launch_bounds__(RSS_THREADS, 1) k_sort_small(unsigned* __restr
 // tile ranges of the sorted keys: tstart/tend zeroed beforehand
 __global__ void k_tile_ranges(const unsigned* __restrict__ keys, int M, int cells_per_tile, int* __restrict__ tstart,
                               int* __restrict__ tend) {
+    wait_launch();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= M) return;
     const unsigned t = keys[p] / (unsigned)cells_per_tile;
@@ -396,6 +405,7 @@ __global__ void __launch_bounds__(32 * kTileWarps) k_tiles(int ntx, int nty, int
                                                           const int* __restrict__ tstart, const int* __restrict__ tend,
                                                           int* __restrict__ list, int* __restrict__ count,
                                                           int* __restrict__ slot, int* __restrict__ ctab) {
+    wait_launch();
     constexpr int C = TS * TS * TZ;
     __shared__ int s_slot[kTileWarps];
     __shared__ unsigned s_key[kTileKeys];
@@ -553,6 +563,7 @@ __global__ void __launch_bounds__(32 * kSpreadWarps, kSpreadBlocks)
                    const double* __restrict__ vol, double scale, const int* __restrict__ slot,
                    const int* __restrict__ ctab, const int* __restrict__ list, const int* __restrict__ count, int cap,
                    T* __restrict__ fu, T* __restrict__ fv, T* __restrict__ fw, int* __restrict__ next_item) {
+    wait_launch();
     // 3D: TZ == TS, the neighbourhood grows by 2 cells per side along every
     // axis. 2D (TZ == 1, nz == 1): one plane, no z halo.
     constexpr int NW = kSpreadWarps, NT = 32 * NW, E = TS + 4, EZ = TZ == 1 ? 1 : TS + 4, HZ = TZ == 1 ? 0 : 2;
@@ -776,6 +787,7 @@ __global__ void __launch_bounds__(32 * kSpreadWarps, kSpreadBlocks)
 template <typename T, typename TF>
 __global__ void k_interp(Dims d, int M, const int* __restrict__ perm, MarkerW<T> mw, const TF* __restrict__ u,
                          const TF* __restrict__ v, const TF* __restrict__ w, double* __restrict__ U) {
+    wait_launch();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= M) return;
     const int k = perm ? perm[p] : p;
@@ -834,6 +846,7 @@ __global__ void __launch_bounds__(kInterpDfBlock) k_interp_dfl(Dims d, int M, co
                                                                const float* __restrict__ vl,
                                                                const float* __restrict__ wh,
                                                                const float* __restrict__ wl, double* __restrict__ U) {
+    wait_launch();
     const int p = (blockIdx.x * kInterpDfBlock + threadIdx.x) >> 2;
     const int q = threadIdx.x & 3;
     if (p >= M) return;  // a quad leaves together
@@ -911,6 +924,7 @@ __global__ void __launch_bounds__(kInterpDfBlock) k_interp_dfl(Dims d, int M, co
 // X_out = X_in + c * U  (U component-major)
 __global__ void k_marker_axpy(int M, double* __restrict__ Xo, const double* __restrict__ Xi, const double* __restrict__ U,
                               double c) {
+    wait_launch();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= M) return;
 #pragma unroll
@@ -923,12 +937,12 @@ template <typename T>
 void launch_springs_bending(int M, const double* X, const int* nstart, const int* nidx, double ks, double kb,
                             double* Y, T* G, cudaStream_t s) {
     if (M <= 0) return;
-    k_lap_aos<<<(M + 255) / 256, 256, 0, s>>>(M, X, nstart, nidx, Y);
-    k_spring_bend<T><<<(M + 255) / 256, 256, 0, s>>>(M, Y, nstart, nidx, ks, kb, G);
+    launch_dep((M + 255) / 256, 256, 0, s, k_lap_aos, M, X, nstart, nidx, Y);
+    launch_dep((M + 255) / 256, 256, 0, s, k_spring_bend<T>, M, Y, nstart, nidx, ks, kb, G);
 }
 template <typename T>
 void launch_springs(int M, const double* X, const int* nstart, const int* nidx, double k, T* G, cudaStream_t s) {
-    if (M > 0) k_springs<T><<<(M + 255) / 256, 256, 0, s>>>(M, X, nstart, nidx, k, G);
+    if (M > 0) launch_dep((M + 255) / 256, 256, 0, s, k_springs<T>, M, X, nstart, nidx, k, G);
 }
 
 template <typename T>
@@ -936,9 +950,9 @@ void launch_marker_prep(const Dims& d, int TS, int M, const double* X, unsigned*
                         int* flag, cudaStream_t s, bool df_weights) {
     if (M <= 0) return;
     if (df_weights && sizeof(T) == sizeof(double))
-        k_marker_prep<T, true><<<(M + 255) / 256, 256, 0, s>>>(d, TS, M, X, keys, vals, mw, flag);
+        launch_dep((M + 255) / 256, 256, 0, s, k_marker_prep<T, true>, d, TS, M, X, keys, vals, mw, flag);
     else
-        k_marker_prep<T, false><<<(M + 255) / 256, 256, 0, s>>>(d, TS, M, X, keys, vals, mw, flag);
+        launch_dep((M + 255) / 256, 256, 0, s, k_marker_prep<T, false>, d, TS, M, X, keys, vals, mw, flag);
 }
 
 size_t radix_sort_temp_bytes(int n) {
@@ -954,9 +968,9 @@ void radix_sort_pairs(unsigned* keys, int* vals, unsigned* keys_alt, int* vals_a
     int* va = vals;
     int* vb = vals_alt;
     for (int shift = 0; shift < bits && n > 0; shift += 8) {
-        k_rs_hist<<<nblk, RS_THREADS, 0, s>>>(ka, n, shift, hist, nblk);
-        k_rs_scan<<<256 / (RS_THREADS / 32), RS_THREADS, 0, s>>>(hist, nblk);
-        k_rs_scatter<<<nblk, RS_THREADS, 0, s>>>(ka, va, kb, vb, n, shift, hist, nblk);
+        launch_dep(nblk, RS_THREADS, 0, s, k_rs_hist, ka, n, shift, hist, nblk);
+        launch_dep(256 / (RS_THREADS / 32), RS_THREADS, 0, s, k_rs_scan, hist, nblk);
+        launch_dep(nblk, RS_THREADS, 0, s, k_rs_scatter, ka, va, kb, vb, n, shift, hist, nblk);
         unsigned* tk = ka; ka = kb; kb = tk;
         int* tv = va; va = vb; vb = tv;
     }
@@ -974,7 +988,7 @@ void sort_bins_small(unsigned* keys, int* vals, int n, int bits, int cells_per_t
         const size_t smem = sizeof(unsigned) * ((size_t)RSS_THREADS * items + 256 * RSS_COLS + 32) +
                             sizeof(unsigned short) * (size_t)RSS_THREADS * items;
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        kernel<<<1, RSS_THREADS, smem, s>>>(keys, vals, n, bits, cells_per_tile, ntiles, tstart, tend, counts);
+        launch_dep(1, RSS_THREADS, smem, s, kernel, keys, vals, n, bits, cells_per_tile, ntiles, tstart, tend, counts);
     };
     if (n <= 2 * RSS_THREADS) launch(k_sort_small<2>, 2);
     else if (n <= 8 * RSS_THREADS) launch(k_sort_small<8>, 8);
@@ -982,14 +996,15 @@ void sort_bins_small(unsigned* keys, int* vals, int n, int bits, int cells_per_t
 }
 
 void launch_tile_ranges(const unsigned* keys, int M, int cells_per_tile, int* tstart, int* tend, cudaStream_t s) {
-    if (M > 0) k_tile_ranges<<<(M + 255) / 256, 256, 0, s>>>(keys, M, cells_per_tile, tstart, tend);
+    if (M > 0) launch_dep((M + 255) / 256, 256, 0, s, k_tile_ranges, keys, M, cells_per_tile, tstart, tend);
 }
 
 void launch_tiles(int TS, int TZ, int ntx, int nty, int ntz, int channel, const unsigned* keys, const int* tstart,
                   const int* tend, int* list, int* count, int* slot, int* ctab, cudaStream_t s) {
     const int nt = ntx * nty * ntz, blocks = std::max(1, std::min((nt + kTileWarps - 1) / kTileWarps, 152 * 16));
     auto launch = [&](auto* kernel) {
-        kernel<<<blocks, 32 * kTileWarps, 0, s>>>(ntx, nty, ntz, channel, keys, tstart, tend, list, count, slot, ctab);
+        launch_dep(blocks, 32 * kTileWarps, 0, s, kernel, ntx, nty, ntz, channel, keys, tstart, tend, list, count,
+                   slot, ctab);
     };
     if (TS == 8 && TZ == 8) launch(k_tiles<8, 8>);
     else if (TS == 4 && TZ == 4) launch(k_tiles<4, 4>);
@@ -1005,8 +1020,8 @@ static void spread_launch(const Dims& d, int M, const int* perm, MarkerW<T> mw, 
     const size_t smem = sizeof(TC) * ((size_t)cap * kSpreadVals + (3 * kSpreadWarps + TZ - 1) * TS * TS) + 8 * (size_t)cap;
     cudaFuncSetAttribute(k_spread_tiles<T, TS, TZ, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     const int blocks = std::max(1, std::min(3 * max_tiles, 152 * kSpreadBlocks));
-    k_spread_tiles<T, TS, TZ, TC><<<blocks, 32 * kSpreadWarps, smem, s>>>(d, M, perm, mw, G, vol, scale, slot, ctab,
-                                                                         list, count, cap, fu, fv, fw, next_tile);
+    launch_dep(blocks, 32 * kSpreadWarps, smem, s, k_spread_tiles<T, TS, TZ, TC>, d, M, perm, mw, G, vol, scale,
+               slot, ctab, list, count, cap, fu, fv, fw, next_tile);
 }
 
 template <typename T>
@@ -1033,7 +1048,7 @@ void launch_spread(const Dims& d, int TS, int M, const int* perm, MarkerW<T> mw,
 template <typename T, typename TF>
 void launch_interp(const Dims& d, int M, const int* perm, MarkerW<T> mw, const TF* u, const TF* v, const TF* w, double* U,
                    cudaStream_t s) {
-    if (M > 0) k_interp<T, TF><<<(M + 127) / 128, 128, 0, s>>>(d, M, perm, mw, u, v, w, U);
+    if (M > 0) launch_dep((M + 127) / 128, 128, 0, s, k_interp<T, TF>, d, M, perm, mw, u, v, w, U);
 }
 
 void launch_interp_dfl(const Dims& d, int M, const int* perm, MarkerW<double> mw, const double* u, const double* v,
@@ -1042,14 +1057,15 @@ void launch_interp_dfl(const Dims& d, int M, const int* perm, MarkerW<double> mw
     if (M <= 0) return;
     const int blocks = (int)((4LL * M + kInterpDfBlock - 1) / kInterpDfBlock);
     if (uh && ul && vh && vl && wh && wl)
-        k_interp_dfl<true><<<blocks, kInterpDfBlock, 0, s>>>(d, M, perm, mw, u, v, w, uh, ul, vh, vl, wh, wl, U);
+        launch_dep(blocks, kInterpDfBlock, 0, s, k_interp_dfl<true>, d, M, perm, mw, u, v, w, uh, ul, vh, vl, wh, wl,
+                   U);
     else
-        k_interp_dfl<false><<<blocks, kInterpDfBlock, 0, s>>>(d, M, perm, mw, u, v, w, nullptr, nullptr, nullptr,
-                                                               nullptr, nullptr, nullptr, U);
+        launch_dep(blocks, kInterpDfBlock, 0, s, k_interp_dfl<false>, d, M, perm, mw, u, v, w, nullptr, nullptr,
+                   nullptr, nullptr, nullptr, nullptr, U);
 }
 
 void launch_marker_axpy(int M, double* Xo, const double* Xi, const double* U, double c, cudaStream_t s) {
-    if (M > 0) k_marker_axpy<<<(M + 255) / 256, 256, 0, s>>>(M, Xo, Xi, U, c);
+    if (M > 0) launch_dep((M + 255) / 256, 256, 0, s, k_marker_axpy, M, Xo, Xi, U, c);
 }
 
 #define AFMIB_IB_INST(T)                                                                                        \

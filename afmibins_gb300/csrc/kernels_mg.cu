@@ -84,6 +84,7 @@ __device__ __forceinline__ void lap_row2(const Dims& d, const IX& I, const T* x,
 
 template <typename T, typename IX>
 __global__ void k_lap(Dims d, LapK<T> k, T* __restrict__ out, const T* __restrict__ in) {
+    wait_launch();
     const int x = blockIdx.x * BX + threadIdx.x, y = blockIdx.y * BY + threadIdx.y, z = blockIdx.z;
     if (x >= d.nx || y >= d.ny) return;
     const IX I(d);
@@ -139,6 +140,7 @@ __global__ void __launch_bounds__(kRedBlock) k_lap_defect(Dims d, LapK<double> k
                                                          const double* __restrict__ xv,
                                                          const double* __restrict__ b, RedScratch sc, double* out,
                                                          float* __restrict__ r_lo, bool lo_split) {
+    wait_launch();
     const int xi = blockIdx.x * kRBX + threadIdx.x, yi = blockIdx.y * kRBY + threadIdx.y;
     TD acc = TD(0);
     if (xi < d.nx && yi < d.ny)
@@ -172,6 +174,7 @@ __global__ void __launch_bounds__(kRedBlock) k_lap_defect_df(Dims d, float* __re
                                                             const double* __restrict__ xv,
                                                             const double* __restrict__ b, const double* sum,
                                                             double scale, RedScratch sc, double* out) {
+    wait_launch();
     const IX I(d);
     const int x = blockIdx.x * kRBX + threadIdx.x, y = blockIdx.y * kRBY + threadIdx.y;
     const df2 off = {float(d.n) * float(d.n), 0.f};  // exact for n < 4096
@@ -220,6 +223,7 @@ __global__ void __launch_bounds__(kRedBlock) k_lap_defect_df(Dims d, float* __re
 __global__ void __launch_bounds__(kRedBlock) k_lap_update_df(Dims d, double* __restrict__ x,
                                                             const float* __restrict__ e, float* __restrict__ rh,
                                                             float* __restrict__ rl, RedScratch sc, double* out) {
+    wait_launch();
     const int xi = blockIdx.x * kRBX + threadIdx.x, yi = blockIdx.y * kRBY + threadIdx.y;
     const float off = float(d.n) * float(d.n);
     float acc = 0.f;
@@ -319,6 +323,7 @@ __global__ void __launch_bounds__(kRedBlock, MINB) k_lap_update_df2(Dims d, doub
 __global__ void __launch_bounds__(kRedBlock) k_lap_defect_bfp(Dims d, int k2, float* __restrict__ r,
                                                              const double* __restrict__ xv, const double* __restrict__ b,
                                                              RedScratch sc, double* out) {
+    wait_launch();
     const int xi = blockIdx.x * kRBX + threadIdx.x, yi = blockIdx.y * kRBY + threadIdx.y;
     float acc = 0.f;
     if (xi < d.nx && yi < d.ny)
@@ -492,6 +497,7 @@ __global__ void __launch_bounds__(BX * BY, MINB) k_rbgs_z2b(Dims d, LapK<T> k, i
 template <int ZU, int MINB>
 __global__ void __launch_bounds__(BX * BY, MINB) k_rbgs_pair(Dims d, int color, float omega, float* __restrict__ xv,
                                                             const float* __restrict__ b, int rev) {
+    wait_launch();
     const Ix2 I(d);
     const uint3 B = block_at(rev);
     const int t = B.x * BX + threadIdx.x, y = B.y * BY + threadIdx.y, z0 = B.z * ZU;
@@ -676,6 +682,7 @@ __device__ __forceinline__ void gs_quad(T* row, const T* rowm, const T* rowp, co
 template <typename T, int D, bool CH>
 __global__ void __launch_bounds__(kPipeThreads, 1) k_rbgs_pipe(Dims d, const T* __restrict__ xin, T* __restrict__ xout,
                                                             const T* __restrict__ b, int FY, int ZC, int lnx, int lny) {
+    wait_launch();
     extern __shared__ __align__(128) unsigned char smem[];
     typedef typename Vec4<T>::type V;
     constexpr int R = D + 4;
@@ -908,6 +915,7 @@ template <typename T, int RR_CZ>
 __global__ void __launch_bounds__(RR_THREADS) k_resid_restrict2(Dims d, T* __restrict__ cb,
                                                                const T* __restrict__ xv, const T* __restrict__ b,
                                                                int rev, bool red) {
+    wait_launch();
     __shared__ T ring[4][RR_F * RR_RS];
     const Ix2 I(d);
     const uint3 B = block_at(rev);
@@ -1552,6 +1560,7 @@ template <typename T>
 __global__ void __launch_bounds__(kRedBlock) k_coarse_cg(Dims d, T* __restrict__ xv, T* __restrict__ b, T* __restrict__ r,
                                                         T* __restrict__ p, T* __restrict__ q, double tol, int maxit,
                                                         int* status) {
+    wait_launch();
     coarse_cg_block(d, xv, b, r, p, q, tol, maxit, status);
 }
 
@@ -1574,7 +1583,8 @@ cudaError_t add_mg_check(cudaGraph_t g, cudaGraphConditionalHandle h, MgCheck c,
     p.kernelParams = args;
     return cudaGraphAddKernelNode(node, g, nullptr, 0, &p);
 }
-void launch_mg_check(cudaGraphConditionalHandle h, MgCheck c, cudaStream_t s) { launch_dep(1, 1, 0, s, k_mg_check, h, c, 0); }
+void launch_mg_check(cudaGraphConditionalHandle h, MgCheck c, cudaStream_t s) { launch_dep(1, 1, 0, s, k_mg_check, h,
+        c, 0); }
 
 // smallest level (x extent) on which the smoother and residual take the
 // batched z-column kernels (AFMIB_BATCH_MIN_NX; one cell per thread below:
@@ -1590,7 +1600,7 @@ int batch_min_nx() {
 
 template <typename T>
 void launch_lap_apply(const Dims& d, T* y, const T* x, cudaStream_t s) {
-    AFMIB_IX(d, (k_lap<T, IX><<<grid3(d), dim3(BX, BY), 0, s>>>(d, lap_k<T>(d), y, x)));
+    AFMIB_IX(d, (launch_dep(grid3(d), dim3(BX, BY), 0, s, k_lap<T, IX>, d, lap_k<T>(d), y, x)));
 }
 template <typename T>
 void launch_residual(const Dims& d, T* r, const T* x, const T* b, RedScratch* sc, double* out, cudaStream_t s, int rev) {
@@ -1611,7 +1621,8 @@ void launch_residual_red(const Dims& d, T* r, const T* x, const T* b, cudaStream
     const int gx = (d.nx / 2 + BX - 1) / BX, gy = (d.ny + BY - 1) / BY;
     const LapK<T> k = lap_k<T>(d);
     if (d.nz % ZU == 0 && d.nx >= batch_min_nx())
-        AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz / ZU), dim3(BX, BY), 0, s, k_residual_red<T, ZU, IX>, d, k, r, x, b, rev)));
+        AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz / ZU), dim3(BX, BY), 0, s, k_residual_red<T, ZU, IX>, d, k, r, x,
+                                b, rev)));
     else
         AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz), dim3(BX, BY), 0, s, k_residual_red<T, 1, IX>, d, k, r, x, b, rev)));
 }
@@ -1645,9 +1656,11 @@ void launch_rbgs_first(const Dims& d, T* x, const T* b, cudaStream_t s, double o
     const int gx = (d.nx / 2 + BX - 1) / BX, gy = (d.ny + BY - 1) / BY;
     const LapK<T> k = lap_k<T>(d);
     if (d.nz % ZU == 0 && d.nx >= batch_min_nx())
-        AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz / ZU), dim3(BX, BY), 0, s, k_rbgs_first<T, ZU, MINB, IX>, d, k, T(omega), x, b, rev, T(0))));
+        AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz / ZU), dim3(BX, BY), 0, s, k_rbgs_first<T, ZU, MINB, IX>, d, k,
+                                T(omega), x, b, rev, T(0))));
     else
-        AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz), dim3(BX, BY), 0, s, k_rbgs_first<T, 1, MINB, IX>, d, k, T(omega), x, b, rev, T(0))));
+        AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz), dim3(BX, BY), 0, s, k_rbgs_first<T, 1, MINB, IX>, d, k, T(omega),
+                                x, b, rev, T(0))));
 }
 
 template <typename T>
@@ -1661,7 +1674,8 @@ void launch_rbgs(const Dims& d, int color, T* x, const T* b, cudaStream_t s, dou
         // FP32 on float pairs (opt-in, AFMIB_RBGS_PAIR=1)
         if (f32 && rbgs_pair_ok(d)) {
             const dim3 gp(d.nx / 2 / BX, d.ny / BY, d.nz / kPairZU);
-            k_rbgs_pair<kPairZU, kPairMinB><<<gp, blk, 0, s>>>(d, color, float(omega), (float*)x, (const float*)b, rev);
+            launch_dep(gp, blk, 0, s, k_rbgs_pair<kPairZU, kPairMinB>, d, color, float(omega), (float*)x,
+                       (const float*)b, rev);
             return;
         }
         // FP32: kZU32 z cells per thread, registers capped for 6 resident
@@ -1670,9 +1684,11 @@ void launch_rbgs(const Dims& d, int color, T* x, const T* b, cudaStream_t s, dou
         // 256^3 colour, 61.1 against 60.8 steps/s; 16: spills, two:
         // 32.7 us; four cells with 8 blocks: the same as 6)
         if (f32)
-            AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz / kZU32), blk, 0, s, k_rbgs_z2b<T, kZU32, 6, IX>, d, k, color, T(omega), x, b, rev)));
+            AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz / kZU32), blk, 0, s, k_rbgs_z2b<T, kZU32, 6, IX>, d, k, color,
+                                    T(omega), x, b, rev)));
         else
-            AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz / kZU64), blk, 0, s, k_rbgs_z2<T, kZU64, IX>, d, k, color, T(omega), x, b, rev)));
+            AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz / kZU64), blk, 0, s, k_rbgs_z2<T, kZU64, IX>, d, k, color,
+                                    T(omega), x, b, rev)));
         return;
     }
     AFMIB_IX(d, (launch_dep(dim3(gx, gy, d.nz), blk, 0, s, k_rbgs<T, IX>, d, k, color, T(omega), x, b)));
@@ -1749,11 +1765,15 @@ void launch_rbgs_pipe(const Dims& d, const PipeCfg& c, const T* xin, T* xout, co
     (void)err;  // the copies are cp.async groups: no wait can time out
     const int lnx = log2_exact(d.nx), lny = log2_exact(d.ny);
     if (c.D == 4) {
-        if (d.channel) k_rbgs_pipe<T, 4, true><<<c.grid, kPipeThreads, c.smem, s>>>(d, xin, xout, b, c.FY, c.ZC, lnx, lny);
-        else k_rbgs_pipe<T, 4, false><<<c.grid, kPipeThreads, c.smem, s>>>(d, xin, xout, b, c.FY, c.ZC, lnx, lny);
+        if (d.channel) launch_dep(c.grid, kPipeThreads, c.smem, s, k_rbgs_pipe<T, 4, true>, d, xin, xout, b, c.FY,
+                                  c.ZC, lnx, lny);
+        else launch_dep(c.grid, kPipeThreads, c.smem, s, k_rbgs_pipe<T, 4, false>, d, xin, xout, b, c.FY, c.ZC, lnx,
+                        lny);
     } else {
-        if (d.channel) k_rbgs_pipe<T, 2, true><<<c.grid, kPipeThreads, c.smem, s>>>(d, xin, xout, b, c.FY, c.ZC, lnx, lny);
-        else k_rbgs_pipe<T, 2, false><<<c.grid, kPipeThreads, c.smem, s>>>(d, xin, xout, b, c.FY, c.ZC, lnx, lny);
+        if (d.channel) launch_dep(c.grid, kPipeThreads, c.smem, s, k_rbgs_pipe<T, 2, true>, d, xin, xout, b, c.FY,
+                                  c.ZC, lnx, lny);
+        else launch_dep(c.grid, kPipeThreads, c.smem, s, k_rbgs_pipe<T, 2, false>, d, xin, xout, b, c.FY, c.ZC, lnx,
+                        lny);
     }
 }
 
@@ -1887,11 +1907,11 @@ void launch_resid_restrict(const Dims& d, T* coarse_b, const T* x, const T* b, c
     // blocks per SM, else 2
     const int cols = (d.nx / 2 / RR_T) * (d.ny / 2 / RR_T), cz = d.nz / 2;
     if (cz % 8 == 0 && cols * (cz / 8) >= 2 * 152)
-        k_resid_restrict2<T, 8><<<dim3(d.nx / 2 / RR_T, d.ny / 2 / RR_T, cz / 8), RR_THREADS, 0, s>>>(
-            d, coarse_b, x, b, rev, red);
+        launch_dep(dim3(d.nx / 2 / RR_T, d.ny / 2 / RR_T, cz / 8), RR_THREADS, 0, s, k_resid_restrict2<T, 8>, d,
+                   coarse_b, x, b, rev, red);
     else
-        k_resid_restrict2<T, 2><<<dim3(d.nx / 2 / RR_T, d.ny / 2 / RR_T, cz / 2), RR_THREADS, 0, s>>>(
-            d, coarse_b, x, b, rev, red);
+        launch_dep(dim3(d.nx / 2 / RR_T, d.ny / 2 / RR_T, cz / 2), RR_THREADS, 0, s, k_resid_restrict2<T, 2>, d,
+                   coarse_b, x, b, rev, red);
 }
 
 template <typename T>
@@ -1927,17 +1947,18 @@ void launch_prolong_assign(const Dims& d, T* fine, const T* coarse, cudaStream_t
 template <typename TD>
 void launch_lap_defect(const Dims& d, TD* r, const double* x, const double* b, RedScratch sc, double* out, cudaStream_t s,
                        float* r_lo) {
-    k_lap_defect<TD><<<red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s>>>(d, lap_k<double>(d), r, x, b, sc, out, r_lo,
-                                                                              lo_split());
+    launch_dep(red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s, k_lap_defect<TD>, d, lap_k<double>(d), r, x, b,
+               sc, out, r_lo, lo_split());
 }
 void launch_lap_defect_df(const Dims& d, float* rh, float* rl, const double* x, const double* b, const double* sum,
                           double scale, RedScratch sc, double* out, cudaStream_t s) {
     const dim3 blk(kRBX, kRBY);
     if (d.nz % 2 == 0)
-        AFMIB_IX(d, (k_lap_defect_df<2, IX><<<red_grid3(d.nx, d.ny, d.nz / 2), blk, 0, s>>>(d, rh, rl, x, b, sum, scale, sc,
-                                                                                         out)));
+        AFMIB_IX(d, (launch_dep(red_grid3(d.nx, d.ny, d.nz / 2), blk, 0, s, k_lap_defect_df<2, IX>, d, rh, rl, x, b,
+                                sum, scale, sc, out)));
     else
-        AFMIB_IX(d, (k_lap_defect_df<1, IX><<<red_grid3(d.nx, d.ny, d.nz), blk, 0, s>>>(d, rh, rl, x, b, sum, scale, sc, out)));
+        AFMIB_IX(d, (launch_dep(red_grid3(d.nx, d.ny, d.nz), blk, 0, s, k_lap_defect_df<1, IX>, d, rh, rl, x, b, sum,
+                                scale, sc, out)));
 }
 void launch_lap_update_df(const Dims& d, double* x, const float* e, float* rh, float* rl, RedScratch sc, double* out,
                           cudaStream_t s) {
@@ -1947,17 +1968,18 @@ void launch_lap_update_df(const Dims& d, double* x, const float* e, float* rh, f
         const int gx = (d.nx + kRBX - 1) / kRBX, gy = (d.ny + kRBY - 1) / kRBY;
         int gz = d.nz / ZU;
         if ((long long)gx * gy * gz > kMaxRedBlocks) gz = std::max(1, kMaxRedBlocks / (gx * gy));
-        AFMIB_IX(d, (launch_dep(dim3(gx, gy, gz), dim3(kRBX, kRBY), 0, s, k_lap_update_df2<ZU, kUpdateMinBlocks, IX>, d, x, e, rh, rl, sc, out)));
+        AFMIB_IX(d, (launch_dep(dim3(gx, gy, gz), dim3(kRBX, kRBY), 0, s, k_lap_update_df2<ZU, kUpdateMinBlocks, IX>,
+                                d, x, e, rh, rl, sc, out)));
         return;
     }
-    k_lap_update_df<<<red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s>>>(d, x, e, rh, rl, sc, out);
+    launch_dep(red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s, k_lap_update_df, d, x, e, rh, rl, sc, out);
 }
 bool launch_lap_defect_bfp(const Dims& d, float* r, const double* x, const double* b, RedScratch sc, double* out,
                            cudaStream_t s) {
     int k = 0;
     while ((1 << k) < d.n) ++k;
     if ((1 << k) != d.n || 2 * k > 126) return false;  // n must be a power of two
-    k_lap_defect_bfp<<<red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s>>>(d, 2 * k, r, x, b, sc, out);
+    launch_dep(red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s, k_lap_defect_bfp, d, 2 * k, r, x, b, sc, out);
     return true;
 }
 template void launch_lap_defect<float>(const Dims&, float*, const double*, const double*, RedScratch, double*,
@@ -1965,7 +1987,7 @@ template void launch_lap_defect<float>(const Dims&, float*, const double*, const
 
 template <typename T>
 void launch_coarse_solve(const Dims& d, T* x, T* b, T* r, T* p, T* q, double tol, int maxit, int* status, cudaStream_t s) {
-    k_coarse_cg<T><<<1, kRedBlock, 0, s>>>(d, x, b, r, p, q, tol, maxit, status);
+    launch_dep(1, kRedBlock, 0, s, k_coarse_cg<T>, d, x, b, r, p, q, tol, maxit, status);
 }
 
 #define AFMIB_MG_INST(T)                                                                                 \
