@@ -319,6 +319,19 @@ int dalloc(afmib_solver* s, T** p, size_t count) {
     return AFMIB_OK;
 }
 
+// n fields in one allocation, each aligned as its own would be
+template <typename T>
+int dalloc_fields(afmib_solver* s, T** p, int n, size_t count) {
+    const size_t stride = (count * sizeof(T) + 255) / 256 * 256 / sizeof(T);
+    if (s->creating && count * sizeof(T) <= kArenaMost) {  // cut from the arena one by one
+        for (int k = 0; k < n; ++k) TRY(dalloc(s, &p[k], count));
+        return AFMIB_OK;
+    }
+    TRY(dalloc(s, p, n * stride));
+    for (int k = 1; k < n; ++k) p[k] = p[0] + k * stride;
+    return AFMIB_OK;
+}
+
 bool is_even(int v) { return v % 2 == 0; }
 
 // --- layout conversions between the caller's v (ny-1 interior planes in
@@ -2200,13 +2213,7 @@ int create(afmib_solver* s, const afmib_config* c, void* stream) {
     TRY(dalloc(s, &s->u, N));
     TRY(dalloc(s, &s->v, N));
     TRY(dalloc(s, &s->w, N));
-    for (int k = 0; k < 3; ++k) {
-        TRY(dalloc(s, &s->uo[k], N));
-        TRY(dalloc(s, &s->adv[k], N));
-        TRY(dalloc(s, &s->rhs[k], N));
-        TRY(dalloc(s, &s->f[k], N));
-        TRY(dalloc(s, &s->tmp[k], N));
-    }
+    for (double** q : {s->uo, s->adv, s->rhs, s->f, s->tmp}) TRY(dalloc_fields(s, q, 3, N));
     TRY(dalloc(s, &s->divb, N));
     if (const char* e = std::getenv("AFMIB_FUSED_RHS")) s->fused_rhs = std::string(e) != "0";
     if (const char* e = std::getenv("AFMIB_HELM_OVERLAP")) s->helm_overlap = std::string(e) != "0";
@@ -2232,11 +2239,8 @@ int create(afmib_solver* s, const afmib_config* c, void* stream) {
     }
     TRY(dalloc(s, &s->walls, 4 * s->nxz()));
     TRY(dalloc(s, &s->wallgrad, 8 * s->nxz()));
-    for (int c = 0; c < (s->mixed ? 1 : 3); ++c) {
-        TRY(dalloc(s, &s->cg_r[c], N));
-        TRY(dalloc(s, &s->cg_p[c], N));
-        TRY(dalloc(s, &s->cg_q[c], N));
-    }
+    const int ncg = s->mixed ? 1 : 3;
+    for (double** q : {s->cg_r, s->cg_p, s->cg_q}) TRY(dalloc_fields(s, q, ncg, N));
     TRY(dalloc(s, &s->cgs, 3 * kCgScalars));
     for (auto& e : s->ev_cg) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     TRY(dalloc(s, &s->red.partial, (size_t)kMaxRedBlocks * kMaxRedVals));
