@@ -1810,6 +1810,15 @@ int helm_inverse(afmib_solver* s, double* x, const double* b) {
         const double* const bs[3] = {b, b + N, b + 2 * N};
         return cg_solve_batch(s, 3, comp, s->s_minus(), xs, bs, nullptr);
     }
+    if (helm_overlap_ok(s, s->s_minus())) {
+        double* const xs[3] = {x, x + N, x + 2 * N};
+        const double* const bs[3] = {b, b + N, b + 2 * N};
+        return helm_solve3_mixed(s, s->s_minus(), xs, bs, [&](int c, cudaStream_t hs, float* lo) {
+            ProfScope ps(s, P_HELM_DEFECT, (double)N * (8 + 8 + 4), 1, hs);
+            launch_helm_defect<float>(s->d, c, s->s_minus(), xs[c], bs[c], s->d32c[c], s->red, s->scal + 12 + c, hs,
+                                      s->walk_blocks, lo);
+        });
+    }
     for (int c = 0; c < 3; ++c) {
         TRY(helm_solve_mixed(s, c, s->s_minus(), x + c * N, b + c * N));
     }
