@@ -28,11 +28,12 @@
 // pass waits for its instructions (a variant for two blocks per thread in registers
 // took the 32^3 level's colours from 1000 to 1700 clocks).
 //
-// Measured on GB300 (us per launch, launches back to back): FP32 from 32^3 24.6
-// (38.6 with a phase per half sweep, all taps moved between CTAs and levels down to
-// one cell; 56 with the 32^3 level in launches of its own and one block below it),
-// FP64 from 16^3 23.2 (41.0; 121 in one block), FP64 2D from 128^2 41.8 (63.5),
-// FP32 from 24x20x28 to 6x5x7 23.8 (28.7), a coarsest 15^3 level with the 30^3 above
+// Measured on GB300 (us per launch, launches back to back; about 5 more inside a
+// V-cycle, where its instructions are cold): FP32 from 32^3 21.8 (38.6 with a phase
+// per half sweep, cells decoded in every phase, all taps moved between CTAs and levels
+// down to one cell; 56 with the 32^3 level in launches of its own and one block below
+// it), FP64 from 16^3 20.9 (41.0; 121 in one block), FP64 2D from 128^2 39.4 (63.5),
+// FP32 from 24x20x28 to 6x5x7 20.9 (28.7), a coarsest 15^3 level with the 30^3 above
 // it 31.
 #include <cooperative_groups.h>
 
@@ -680,6 +681,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_mg_tail(const __grid_consta
         }
         smooth_level(l, L.nu2, false, false);
     }
+    cl.barrier_arrive();  // no CTA leaves while another may still read its shared memory
     {
         const TailLv<T>& L = g.lv[0];
         int z0;
@@ -687,7 +689,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_mg_tail(const __grid_consta
         T* gx = g.gx + (size_t)z0 * L.nx * L.ny;
         for (int i = threadIdx.x; i < total; i += blockDim.x) gx[i] = sm[L.ox + i];
     }
-    cl.sync();  // no CTA leaves while another may still read its shared memory
+    cl.barrier_wait();
 }
 
 template <typename T>
