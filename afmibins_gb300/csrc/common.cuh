@@ -84,6 +84,24 @@ struct IxG {
         return x + (nx >> 1) * (y + (ny >> 1) * z);
     }
 };
+// Rows split by colour: the cells with x + y + z even in the row's first half, the
+// others in the second, both by x / 2. A red-black pass reads and writes one colour
+// of a row in contiguous words, where an interleaved row moves every sector for half
+// of its bytes.
+struct Split2 : Ix2 {
+    __host__ __device__ __forceinline__ explicit Split2(const Dims& d) : Ix2(d) {}
+    __device__ __forceinline__ int at(int x, int y, int z) const {
+        return (x >> 1) | (((x ^ y ^ z) & 1) << (lx - 1)) | (y << lx) | (z << lxy);
+    }
+};
+template <typename IX, bool SPLIT>
+struct RowIx {
+    typedef IX type;
+};
+template <>
+struct RowIx<Ix2, true> {
+    typedef Split2 type;
+};
 // A launch that may be set up while the kernel before it in the stream or graph
 // runs (programmatic dependent launch, no early trigger): 0.2 us less per kernel of
 // 1.3 in a graph of small ones (an early trigger: 0.1 less, and slower from 10^6

@@ -199,11 +199,11 @@ void launch_lap_defect(const Dims& d, TD* r, const double* x, const double* b, R
 // Mixed form: the first defect of a pressure solve in double-float,
 // (rh, rl) = (b - sum * scale) - L x (sum null: no mean), out[0] = rh.rh
 void launch_lap_defect_df(const Dims& d, float* rh, float* rl, const double* x, const double* b, const double* sum,
-                          double scale, RedScratch sc, double* out, cudaStream_t s);
+                          double scale, RedScratch sc, double* out, cudaStream_t s, bool split = false);
 // Mixed form: x += e, (rh, rl) -= L e in double-float, out[0] = rh.rh
 // (r_lo of launch_lap_defect starts the pair)
 void launch_lap_update_df(const Dims& d, double* x, const float* e, float* rh, float* rl, RedScratch sc, double* out,
-                          cudaStream_t s);
+                          cudaStream_t s, bool split = false);
 // The mixed form's FP64-state defects evaluated with int64 block arithmetic
 // and float pairs (no FP64 instruction; see dfloat.cuh). The Laplacian form
 // needs n a power of two and returns false (nothing launched) otherwise.
@@ -216,11 +216,13 @@ void launch_helm_defect_bfp(const Dims& d, int comp, double scale, const double*
 // rev (here and in the residual, transfer and Jacobi launchers): blocks in
 // reverse order (block_at, common.cuh) on the batched kernels.
 template <typename T>
-void launch_rbgs(const Dims& d, int color, T* x, const T* b, cudaStream_t s, double omega = 1.0, int rev = 0);
+void launch_rbgs(const Dims& d, int color, T* x, const T* b, cudaStream_t s, double omega = 1.0, int rev = 0,
+                 bool split = false);
 // Both colours from x = 0 (x's contents ignored): the same bits as zeroing x and
 // launch_rbgs of color 0 and of color 1.
 template <typename T>
-void launch_rbgs_first(const Dims& d, T* x, const T* b, cudaStream_t s, double omega = 1.0, int rev = 0);
+void launch_rbgs_first(const Dims& d, T* x, const T* b, cudaStream_t s, double omega = 1.0, int rev = 0,
+                       bool split = false);
 // One full red+black sweep per launch, out of place (xin -> xout), z-marching
 // blocks fed by bulk asynchronous row copies; equals the two per-colour
 // launches cell for cell. FY == 0: level not eligible (small, 2D, or rows not
@@ -293,7 +295,8 @@ void launch_residual_red(const Dims& d, T* r, const T* x, const T* b, cudaStream
 // the black cells only, where the kernel can leave the others out
 // (prolong_before_sweep)
 template <typename T>
-void launch_prolong_add(const Dims& d, T* fine, const T* coarse, cudaStream_t s, int rev = 0, bool black = false);
+void launch_prolong_add(const Dims& d, T* fine, const T* coarse, cudaStream_t s, int rev = 0, bool black = false,
+                        bool split = false);
 // coarse_b = restriction of (b - L x) in one pass (the residual stays in shared memory), for the levels resid_restrict_fused_ok
 // takes: by default FP32 3D power-of-two levels with nx >= 256 (the column
 // kernel); AFMIB_RESID_RESTRICT=1 the ring kernel, =0 none
@@ -301,9 +304,12 @@ bool resid_restrict_fused_ok(const Dims& d, size_t elem, const void* x, const vo
 // shared-memory opt-ins of the multigrid kernels (once per device, before
 // any launch or stream capture)
 void mg_kernel_attributes();
+// split (here, in the sweeps, the prolongation, the first defect and its update): x and b
+// of the FP32 fine level split by colour (Split2, common.cuh), where mg_split_ok
+bool mg_split_ok(const Dims& d, const float* x, const float* b, const float* cb, const float* cx);
 template <typename T>
 void launch_resid_restrict(const Dims& d, T* coarse_b, const T* x, const T* b, cudaStream_t s,
-                           int rev = 0, bool red = false);
+                           int rev = 0, bool red = false, bool split = false);
 // Prolongation that assigns (for the op-level API).
 template <typename T>
 void launch_prolong_assign(const Dims& d, T* fine, const T* coarse, cudaStream_t s);

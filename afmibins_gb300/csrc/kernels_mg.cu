@@ -169,13 +169,14 @@ __global__ void __launch_bounds__(kRedBlock) k_lap_defect(Dims d, LapK<double> k
 // five splits per cell, two z cells' loads first: 178 us at 256^3 (eight splits cell
 // by cell: 282; four cells: 223). The pair is the FP32 defect rh and its rest rl of
 // k_lap_update_df, out[0] = rh.rh.
-template <int ZU, typename IX>
+template <int ZU, typename IX, bool SPLIT>
 __global__ void __launch_bounds__(kRedBlock) k_lap_defect_df(Dims d, float* __restrict__ rh, float* __restrict__ rl,
                                                             const double* __restrict__ xv,
                                                             const double* __restrict__ b, const double* sum,
                                                             double scale, RedScratch sc, double* out) {
     wait_launch();
     const IX I(d);
+    const typename RowIx<IX, SPLIT>::type E(d);  // of rh
     const int x = blockIdx.x * kRBX + threadIdx.x, y = blockIdx.y * kRBY + threadIdx.y;
     const df2 off = {float(d.n) * float(d.n), 0.f};  // exact for n < 4096
     const df2 m = sum ? df_split(sum[0] * scale) : df2{0.f, 0.f};
@@ -206,7 +207,7 @@ __global__ void __launch_bounds__(kRedBlock) k_lap_defect_df(Dims d, float* __re
                 const df2 L = df_mul(off, df_add(S, df_neg(df_mul(df2{c, 0.f}, df_split(col[k + 1])))));
                 const df2 r = df_add(df_add(df_split(bv[k]), df_neg(m)), df_neg(L));
                 const int i = I.at(x, y, z0 + k);
-                rh[i] = r.hi;
+                rh[E.at(x, y, z0 + k)] = r.hi;
                 rl[i] = r.lo;
                 acc += r.hi * r.hi;
             }
@@ -265,12 +266,13 @@ __global__ void __launch_bounds__(kRedBlock) k_lap_update_df(Dims d, double* __r
 // The same on 3D grids with nz % ZU == 0, two z cells per thread with every load
 // of the pair issued first (as k_helm_update_df2); the same rows, so the
 // same bits.
-template <int ZU, int MINB, typename IX>
+template <int ZU, int MINB, typename IX, bool SPLIT>
 __global__ void __launch_bounds__(kRedBlock, MINB) k_lap_update_df2(Dims d, double* __restrict__ x,
                                                              const float* __restrict__ e, float* __restrict__ rh,
                                                              float* __restrict__ rl, RedScratch sc, double* out) {
     wait_launch();
     const IX I(d);
+    const typename RowIx<IX, SPLIT>::type E(d);  // of e and rh
     const int xi = blockIdx.x * kRBX + threadIdx.x, yi = blockIdx.y * kRBY + threadIdx.y;
     const float off = float(d.n) * float(d.n);
     const bool has_ym = !d.channel || yi > 0, has_yp = !d.channel || yi < d.ny - 1;
@@ -283,15 +285,15 @@ __global__ void __launch_bounds__(kRedBlock, MINB) k_lap_update_df2(Dims d, doub
             float col[ZU + 2], ex0[ZU], ex1[ZU], ey0[ZU], ey1[ZU], h[ZU], l[ZU];
             double xv[ZU];
 #pragma unroll
-            for (int u = 0; u < ZU + 2; ++u) col[u] = e[I.at(xi, yi, I.wz(z0 + u - 1))];  // z0 - 1 .. z0 + ZU
+            for (int u = 0; u < ZU + 2; ++u) col[u] = e[E.at(xi, yi, I.wz(z0 + u - 1))];  // z0 - 1 .. z0 + ZU
 #pragma unroll
             for (int u = 0; u < ZU; ++u) {
                 const int z = z0 + u, i = I.at(xi, yi, z);
-                ex0[u] = e[I.at(I.xm(xi), yi, z)];
-                ex1[u] = e[I.at(I.xp(xi), yi, z)];
-                ey0[u] = has_ym ? e[I.at(xi, ym, z)] : 0.f;
-                ey1[u] = has_yp ? e[I.at(xi, yp, z)] : 0.f;
-                h[u] = rh[i];
+                ex0[u] = e[E.at(I.xm(xi), yi, z)];
+                ex1[u] = e[E.at(I.xp(xi), yi, z)];
+                ey0[u] = has_ym ? e[E.at(xi, ym, z)] : 0.f;
+                ey1[u] = has_yp ? e[E.at(xi, yp, z)] : 0.f;
+                h[u] = rh[E.at(xi, yi, z)];
                 l[u] = rl[i];
                 xv[u] = x[i];
             }
@@ -307,7 +309,7 @@ __global__ void __launch_bounds__(kRedBlock, MINB) k_lap_update_df2(Dims d, doub
                 r.hi = h[u];
                 r.lo = l[u];
                 r = df_add(r, df_neg(le));
-                rh[i] = r.hi;
+                rh[E.at(xi, yi, z0 + u)] = r.hi;
                 rl[i] = r.lo;
                 x[i] = xv[u] + cvt<double, float>(e0);
                 acc += r.hi * r.hi;
@@ -424,11 +426,12 @@ __global__ void k_rbgs_z2(Dims d, LapK<T> k, int color, T omega, T* __restrict__
 // solves' first sweeps in the same form: IB steps of the mixed form at 256^3 16.20
 // -> 15.77 ms, at 96x80x112 3.88 -> 3.74; FP64 steps unchanged (13.8 ms at 128^3:
 // the reds formed again cost the FP64 pipe what the launch saves).
-template <typename T, int ZU, int MINB, typename IX>
+template <typename T, int ZU, int MINB, typename IX, bool SPLIT = false>
 __global__ void __launch_bounds__(BX * BY, MINB) k_rbgs_first(Dims d, LapK<T> k, T omega, T* __restrict__ xv,
                                                              const T* __restrict__ b, int rev, T zero) {
     wait_launch();
     const IX I(d);
+    const typename RowIx<IX, SPLIT>::type E(d);
     const uint3 B = block_at(rev);
     const int y = B.y * BY + threadIdx.y, t = B.x * BX + threadIdx.x, z0 = B.z * ZU;
     if (y >= d.ny || 2 * t >= d.nx) return;
@@ -453,29 +456,71 @@ __global__ void __launch_bounds__(BX * BY, MINB) k_rbgs_first(Dims d, LapK<T> k,
 #pragma unroll
     for (int u = 0; u < ZU + 2; ++u) {
         const int z = z0 + u - 1;
-        red[u] = flat && u != 1 ? zero : update(zero, I.at(2 * t + ((y + z) & 1), y, I.wz(z)), c);
+        red[u] = flat && u != 1 ? zero : update(zero, E.at(2 * t + ((y + z) & 1), y, I.wz(z)), c);
     }
     T val[ZU];
 #pragma unroll
     for (int u = 0; u < ZU; ++u) {
         const int z = z0 + u, p = (y + z) & 1, x = 2 * t + 1 - p;
-        T S = red[u + 1] + update(zero, I.at(p ? I.xm(2 * t) : I.xp(2 * t + 1), y, z), c);
+        T S = red[u + 1] + update(zero, E.at(p ? I.xm(2 * t) : I.xp(2 * t + 1), y, z), c);
         if (!flat) S = S + (red[u] + red[u + 2]);
         if (d.channel) {
-            if (lo) S += update(zero, I.at(x, ylo, z), clo);
-            if (hi) S += update(zero, I.at(x, yhi, z), chi);
+            if (lo) S += update(zero, E.at(x, ylo, z), clo);
+            if (hi) S += update(zero, E.at(x, yhi, z), chi);
         } else {
-            S += update(zero, I.at(x, ylo, z), clo) + update(zero, I.at(x, yhi, z), chi);
+            S += update(zero, E.at(x, ylo, z), clo) + update(zero, E.at(x, yhi, z), chi);
         }
-        val[u] = update(S, I.at(x, y, z), c);
+        val[u] = update(S, E.at(x, y, z), c);
     }
 #pragma unroll
     for (int u = 0; u < ZU; ++u) {
         const int z = z0 + u, p = (y + z) & 1;
-        xv[I.at(2 * t + p, y, z)] = red[u + 1];
-        xv[I.at(2 * t + 1 - p, y, z)] = val[u];
+        xv[E.at(2 * t + p, y, z)] = red[u + 1];
+        xv[E.at(2 * t + 1 - p, y, z)] = val[u];
     }
 }
+// One colour with x and b split by colour within each row (Split2): every load and
+// store of a warp is 32 consecutive words, the z neighbours come from the column's
+// registers (mg_split_ok for what it measured).
+template <int ZU, int MINB>
+__global__ void __launch_bounds__(BX * BY, MINB) k_rbgs_split(Dims d, LapK<float> k, int color, float omega,
+                                                             float* __restrict__ xv, const float* __restrict__ b,
+                                                             int rev) {
+    wait_launch();
+    const Ix2 I(d);
+    const uint3 B = block_at(rev);
+    const int y = B.y * BY + threadIdx.y, t = B.x * BX + threadIdx.x, z0 = B.z * ZU, h = d.nx / 2;
+    const bool lo = !d.channel || y > 0, hi = !d.channel || y < d.ny - 1;
+    const int c = 6 - (lo ? 0 : 1) - (hi ? 0 : 1);
+    const int yo = y << I.lx, ym = I.ym(y) << I.lx, yp = I.yp(y) << I.lx;
+    const int other = (1 - color) * h + t, own = color * h + t;
+    float o[ZU + 2], side[ZU], dn[ZU], up[ZU], bv[ZU], old[ZU];
+#pragma unroll
+    for (int u = 0; u < ZU + 2; ++u) o[u] = xv[(I.wz(z0 + u - 1) << I.lxy) + yo + other];
+#pragma unroll
+    for (int u = 0; u < ZU; ++u) {
+        const int zo = (z0 + u) << I.lxy;
+        // the cell is x = 2t + p: beside it the pair's other cell and one of the next or last pair
+        const int p = (y + z0 + u + color) & 1, tn = (p ? t + 1 : t - 1) & (h - 1);
+        side[u] = xv[zo + yo + other - t + tn];
+        dn[u] = lo ? xv[zo + ym + other] : 0.f;
+        up[u] = hi ? xv[zo + yp + other] : 0.f;
+        bv[u] = b[zo + yo + own];
+        old[u] = xv[zo + yo + own];
+    }
+#pragma unroll
+    for (int u = 0; u < ZU; ++u) {
+        float S = (o[u + 1] + side[u]) + (o[u] + o[u + 2]);
+        if (d.channel) {
+            if (lo) S += dn[u];
+            if (hi) S += up[u];
+        } else {
+            S += dn[u] + up[u];
+        }
+        xv[((z0 + u) << I.lxy) + yo + own] = over_relaxed(gs_value(S, bv[u], k.inv, lap_rcount<float>(c)), old[u], omega);
+    }
+}
+
 template <typename T, int ZU, int MINB, typename IX>
 __global__ void __launch_bounds__(BX * BY, MINB) k_rbgs_z2b(Dims d, LapK<T> k, int color, T omega, T* __restrict__ xv,
                                                            const T* __restrict__ b, int rev) {
@@ -1185,10 +1230,14 @@ constexpr int kRrX = 4, kRrB = 4, kRrXRows = 2 * kTrBY + 4;
 constexpr int kRrXW = 144, kRrW = 136;  // floats a staged x row (36 chunks) / b and residual row (34)
 constexpr int kRrTasks = kTrRows * 34;  // residual chunks a plane
 constexpr int kRrPT = (kRrTasks + 32 * kTrBY - 1) / (32 * kTrBY);
-constexpr size_t kRrSmem = sizeof(float) * ((size_t)kRrX * kRrXRows * kRrXW + (size_t)kRrB * kTrRows * kRrW +
+// Split rows (Split2) are staged as 72 even cells, then 72 odd ones, from x = 2 xc0 - 8
+// for x and for b (a colour's half of a row goes to one of the two by the parity of
+// y + z), and read from there by pairs.
+constexpr int kRrBW = 144, kRrHalf = 72;
+constexpr size_t kRrSmem = sizeof(float) * ((size_t)kRrX * kRrXRows * kRrXW + (size_t)kRrB * kTrRows * kRrBW +
                                             (size_t)kTrRows * kRrW);
 
-template <int CZ, bool CH>
+template <int CZ, bool CH, bool SPLIT>
 __global__ void __launch_bounds__(32 * kTrBY, 2) k_resid_restrict_cols(Dims d, float* __restrict__ cb,
                                                                     const float* __restrict__ xv,
                                                                     const float* __restrict__ bv, int rev) {
@@ -1196,11 +1245,12 @@ __global__ void __launch_bounds__(32 * kTrBY, 2) k_resid_restrict_cols(Dims d, f
     constexpr int NP = 2 * CZ + 2;  // fine planes restricted (residuals formed)
     constexpr int NI = NP + 2;      // staged items: x planes 2 zc0 - 2 .. 2 zc0 + 2 CZ + 1
     constexpr int XCH = (kRrXRows * 36 + 32 * kTrBY - 1) / (32 * kTrBY);
-    constexpr int BCH = (kTrRows * 34 + 32 * kTrBY - 1) / (32 * kTrBY);
+    constexpr int BC = SPLIT ? 36 : 34, BW = SPLIT ? kRrBW : kRrW;  // chunks and floats a staged b row
+    constexpr int BCH = (kTrRows * BC + 32 * kTrBY - 1) / (32 * kTrBY);
     extern __shared__ __align__(16) float rr_smem[];
     float* xs = rr_smem;                          // [kRrX][kRrXRows][kRrXW]
-    float* bs = xs + kRrX * kRrXRows * kRrXW;     // [kRrB][kTrRows][kRrW]
-    float* rs = bs + kRrB * kTrRows * kRrW;       // [kTrRows][kRrW]
+    float* bs = xs + kRrX * kRrXRows * kRrXW;     // [kRrB][kTrRows][BW]
+    float* rs = bs + kRrB * kTrRows * BW;         // [kTrRows][kRrW]
     const Ix2 I(d);
     const uint3 B = block_at(rev);
     const int lane = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + lane;
@@ -1212,6 +1262,15 @@ __global__ void __launch_bounds__(32 * kTrBY, 2) k_resid_restrict_cols(Dims d, f
     // this thread's chunks of every x / b plane: source offset within the
     // plane (-1: none), destination offset within the slot
     int xsrc[XCH], xdst[XCH], bsrc[BCH], bdst[BCH];
+    // split rows: chunk k of row y holds four cells of colour k / 18; on a plane of
+    // parity 0 they go to the half h = (y + k / 18) & 1, on the others to 1 - h (bit 0
+    // of the destination, the offsets being multiples of four)
+    auto chunk = [&](int k, int y, int& src, int& dst) {
+        const int h = k / 18, kk = k - 18 * h;
+        src = ((xc0 - 4 + 4 * kk) & (I.mx >> 1)) | (h << (I.lx - 1)) | (y << I.lx);
+        dst = (4 * kk) | ((y + h) & 1);
+    };
+    auto to = [&](int dst, int k) { return SPLIT ? (dst & ~1) + kRrHalf * ((dst + k) & 1) : dst; };
 #pragma unroll
     for (int u = 0; u < XCH; ++u) {
         const int c = tid + u * 32 * kTrBY;
@@ -1219,8 +1278,13 @@ __global__ void __launch_bounds__(32 * kTrBY, 2) k_resid_restrict_cols(Dims d, f
         xdst[u] = 0;
         if (c < kRrXRows * 36) {
             const int j = c / 36, k = c - j * 36;
-            xsrc[u] = ((2 * xc0 - 8 + 4 * k) & I.mx) | (yrow(2 * yc0 - 2 + j) << I.lx);
-            xdst[u] = j * kRrXW + 4 * k;
+            if (SPLIT) {
+                chunk(k, yrow(2 * yc0 - 2 + j), xsrc[u], xdst[u]);
+                xdst[u] += j * kRrXW;
+            } else {
+                xsrc[u] = ((2 * xc0 - 8 + 4 * k) & I.mx) | (yrow(2 * yc0 - 2 + j) << I.lx);
+                xdst[u] = j * kRrXW + 4 * k;
+            }
         }
     }
 #pragma unroll
@@ -1228,10 +1292,15 @@ __global__ void __launch_bounds__(32 * kTrBY, 2) k_resid_restrict_cols(Dims d, f
         const int c = tid + u * 32 * kTrBY;
         bsrc[u] = -1;
         bdst[u] = 0;
-        if (c < kTrRows * 34) {
-            const int j = c / 34, k = c - j * 34;
-            bsrc[u] = ((2 * xc0 - 4 + 4 * k) & I.mx) | (yrow(2 * yc0 - 1 + j) << I.lx);
-            bdst[u] = j * kRrW + 4 * k;
+        if (c < kTrRows * BC) {
+            const int j = c / BC, k = c - j * BC;
+            if (SPLIT) {
+                chunk(k, yrow(2 * yc0 - 1 + j), bsrc[u], bdst[u]);
+                bdst[u] += j * BW;
+            } else {
+                bsrc[u] = ((2 * xc0 - 4 + 4 * k) & I.mx) | (yrow(2 * yc0 - 1 + j) << I.lx);
+                bdst[u] = j * BW + 4 * k;
+            }
         }
     }
     // this thread's residual chunks: residual row jr, chunk k (cells
@@ -1252,8 +1321,8 @@ __global__ void __launch_bounds__(32 * kTrBY, 2) k_resid_restrict_cols(Dims d, f
             const int ye = CH ? (y < 0 ? 0 : (y > d.ny - 1 ? d.ny - 1 : y)) : y;
             const int jx = ye - (2 * yc0 - 2);
             tr[u] = jr * kRrW + 4 * k;
-            tb[u] = jr * kRrW + 4 * k;
-            tx[u] = jx * kRrXW + 4 * k + 4;
+            tb[u] = jr * BW + (SPLIT ? 2 * k + 2 : 4 * k);
+            tx[u] = jx * kRrXW + (SPLIT ? 2 * k + 2 : 4 * k + 4);
             tym[u] = !CH || ye > 0;
             typ[u] = !CH || ye < d.ny - 1;
         }
@@ -1267,13 +1336,13 @@ __global__ void __launch_bounds__(32 * kTrBY, 2) k_resid_restrict_cols(Dims d, f
             const float* xsp = xv + zo;
 #pragma unroll
             for (int u = 0; u < XCH; ++u)
-                if (xsrc[u] >= 0) pipe::cp16(xd + xdst[u], xsp + xsrc[u]);
+                if (xsrc[u] >= 0) pipe::cp16(xd + to(xdst[u], k), xsp + xsrc[u]);
             if (k >= 1 && k <= NP) {
-                float* bd = bs + (k % kRrB) * kTrRows * kRrW;
+                float* bd = bs + (k % kRrB) * kTrRows * BW;
                 const float* bsp = bv + zo;
 #pragma unroll
                 for (int u = 0; u < BCH; ++u)
-                    if (bsrc[u] >= 0) pipe::cp16(bd + bdst[u], bsp + bsrc[u]);
+                    if (bsrc[u] >= 0) pipe::cp16(bd + to(bdst[u], k), bsp + bsrc[u]);
             }
         }
         pipe::commit();
@@ -1295,18 +1364,24 @@ __global__ void __launch_bounds__(32 * kTrBY, 2) k_resid_restrict_cols(Dims d, f
         const float* xc = xs + ((i + 1) % kRrX) * kRrXRows * kRrXW;
         const float* xm = xs + (i % kRrX) * kRrXRows * kRrXW;        // z - 1
         const float* xp = xs + ((i + 2) % kRrX) * kRrXRows * kRrXW;  // z + 1
-        const float* bp = bs + ((i + 1) % kRrB) * kTrRows * kRrW;
+        const float* bp = bs + ((i + 1) % kRrB) * kTrRows * BW;
+        // four cells from x = 2 xc0 - 4 + 4 k
+        auto four = [](const float* p) {
+            if (!SPLIT) return *reinterpret_cast<const float4*>(p);
+            const float2 e = *reinterpret_cast<const float2*>(p), o = *reinterpret_cast<const float2*>(p + kRrHalf);
+            return make_float4(e.x, o.x, e.y, o.y);
+        };
 #pragma unroll
         for (int u = 0; u < kRrPT; ++u) {
             if (tr[u] < 0) break;
             const float* c0 = xc + tx[u];
-            const float4 v = *reinterpret_cast<const float4*>(c0);
-            const float4 vym = *reinterpret_cast<const float4*>(c0 - kRrXW);
-            const float4 vyp = *reinterpret_cast<const float4*>(c0 + kRrXW);
-            const float4 vzm = *reinterpret_cast<const float4*>(xm + tx[u]);
-            const float4 vzp = *reinterpret_cast<const float4*>(xp + tx[u]);
-            const float4 vb = *reinterpret_cast<const float4*>(bp + tb[u]);
-            const float l = c0[-1], r = c0[4];
+            const float4 v = four(c0);
+            const float4 vym = four(c0 - kRrXW);
+            const float4 vyp = four(c0 + kRrXW);
+            const float4 vzm = four(xm + tx[u]);
+            const float4 vzp = four(xp + tx[u]);
+            const float4 vb = four(bp + tb[u]);
+            const float l = SPLIT ? c0[kRrHalf - 1] : c0[-1], r = SPLIT ? c0[2] : c0[4];
             const bool hm = tym[u], hp = typ[u];
             float4 o;
             o.x = cell(v.x, l, v.y, vzm.x, vzp.x, vym.x, vyp.x, vb.x, hm, hp);
@@ -1389,7 +1464,7 @@ struct ProTile {
     static constexpr int STAGE = FROWS * FW + CROWS * CW;
 };
 
-template <typename T, int RZ>
+template <typename T, int RZ, bool SPLIT>
 __global__ void __launch_bounds__(32 * kTrBY) k_prolong_cols(Dims d, T* __restrict__ fine,
                                                              const T* __restrict__ coarse, int rev) {
     wait_launch();
@@ -1416,8 +1491,15 @@ __global__ void __launch_bounds__(32 * kTrBY) k_prolong_cols(Dims d, T* __restri
             for (int c = tid; c < PT::FROWS * (PT::FW / CE); c += 32 * kTrBY) {
                 const int j = c / (PT::FW / CE), k = c - j * (PT::FW / CE);
                 const int jz = j / (2 * kTrBY), jy = j - jz * (2 * kTrBY);
-                pipe::cp16(dst + j * PT::FW + k * CE,
-                           fine + ((2 * t0 + k * CE) | ((2 * s0 + jy) << I.lx) | ((2 * r + jz) << I.lxy)));
+                const int row = ((2 * s0 + jy) << I.lx) | ((2 * r + jz) << I.lxy);
+                if (SPLIT) {  // staged as 32 even cells, then 32 odd ones
+                    constexpr int HC = PT::FW / CE / 2;
+                    const int h = k / HC, kk = k - h * HC;
+                    pipe::cp16(dst + j * PT::FW + ((jy + jz + h) & 1) * 32 + kk * CE,
+                               fine + ((t0 + kk * CE) | (h << (I.lx - 1)) | row));
+                } else {
+                    pipe::cp16(dst + j * PT::FW + k * CE, fine + ((2 * t0 + k * CE) | row));
+                }
             }
             T* cdst = dst + PT::FROWS * PT::FW;
             const T* cpl = coarse + (((r + 1) & (cz - 1)) << lcxy);
@@ -1472,11 +1554,23 @@ __global__ void __launch_bounds__(32 * kTrBY) k_prolong_cols(Dims d, T* __restri
                 for (int i = 0; i < 3; ++i) h[i] = wl ? q[1][i] : near4(q[1][i], q[2 * jy][i]);
                 const T sc1 = wl ? T(1.0 / 16.0) : T(1.0 / 64.0);
                 // fine x = 2t (nearest to t, far t - 1), 2t + 1 (far t + 1)
-                const P2 old = *reinterpret_cast<const P2*>(sf + (jz * 2 * kTrBY + 2 * ty + jy) * PT::FW + 2 * lane);
-                P2 out;
+                const T* sr = sf + (jz * 2 * kTrBY + 2 * ty + jy) * PT::FW;
+                P2 old, out;
+                if (SPLIT) {
+                    old.x = sr[lane];
+                    old.y = sr[32 + lane];
+                } else {
+                    old = *reinterpret_cast<const P2*>(sr + 2 * lane);
+                }
                 out.x = fma_t(near4(h[1], h[0]), sc1, old.x);
                 out.y = fma_t(near4(h[1], h[2]), sc1, old.y);
-                *reinterpret_cast<P2*>(fine + ((2 * t) | ((2 * s + jy) << I.lx) | ((2 * r + jz) << I.lxy))) = out;
+                const int row = ((2 * s + jy) << I.lx) | ((2 * r + jz) << I.lxy), p = (jy + jz) & 1;
+                if (SPLIT) {
+                    fine[t | (p << (I.lx - 1)) | row] = out.x;
+                    fine[t | ((1 - p) << (I.lx - 1)) | row] = out.y;
+                } else {
+                    *reinterpret_cast<P2*>(fine + ((2 * t) | row)) = out;
+                }
             }
         }
 #pragma unroll
@@ -1643,12 +1737,18 @@ bool rbgs_pair_ok(const Dims& d) {
 // memset of x and the two colours (read at every launch, so that a test can compare
 // both in one process).
 template <typename T>
-void launch_rbgs_first(const Dims& d, T* x, const T* b, cudaStream_t s, double omega, int rev) {
+void launch_rbgs_first(const Dims& d, T* x, const T* b, cudaStream_t s, double omega, int rev, bool split) {
+    if constexpr (sizeof(T) == sizeof(float))
+        if (split) {
+            launch_dep(dim3(d.nx / 2 / BX, d.ny / BY, d.nz / 4), dim3(BX, BY), 0, s, k_rbgs_first<T, 4, 6, Ix2, true>, d,
+                       lap_k<T>(d), T(omega), x, b, rev, T(0));
+            return;
+        }
     const char* e = std::getenv("AFMIB_INIT_SWEEP");
     if ((e && e[0] == '0') || d.nx % 2) {
         cudaMemsetAsync(x, 0, (size_t)d.ncell() * sizeof(T), s);
-        launch_rbgs<T>(d, 0, x, b, s, omega, rev);
-        launch_rbgs<T>(d, 1, x, b, s, omega, rev);
+        launch_rbgs<T>(d, 0, x, b, s, omega, rev, false);
+        launch_rbgs<T>(d, 1, x, b, s, omega, rev, false);
         return;
     }
     if (d.nx < kOmegaMinNx) omega = 1.0;
@@ -1664,7 +1764,13 @@ void launch_rbgs_first(const Dims& d, T* x, const T* b, cudaStream_t s, double o
 }
 
 template <typename T>
-void launch_rbgs(const Dims& d, int color, T* x, const T* b, cudaStream_t s, double omega, int rev) {
+void launch_rbgs(const Dims& d, int color, T* x, const T* b, cudaStream_t s, double omega, int rev, bool split) {
+    if constexpr (sizeof(T) == sizeof(float))
+        if (split) {
+            launch_dep(dim3(d.nx / 2 / BX, d.ny / BY, d.nz / 4), dim3(BX, BY), 0, s, k_rbgs_split<4, 6>, d, lap_k<T>(d), color,
+                       float(omega), x, b, rev);
+            return;
+        }
     if (d.nx < kOmegaMinNx) omega = 1.0;
     const LapK<T> k = lap_k<T>(d);
     const int gx = (d.nx / 2 + BX - 1) / BX, gy = (d.ny + BY - 1) / BY;
@@ -1857,23 +1963,46 @@ bool resid_restrict_fused_ok(const Dims& d, size_t elem, const void* x, const vo
     return rr_mode(d, elem, x, b, cb) != 0;
 }
 
+// An FP32 fine level whose iterate and right-hand side are split by colour: every
+// kernel that takes them there has a split form, and the two arrays do not fit in
+// the L2 (126 MB): at 512^3 a colour takes 194 us instead of 243, the fused
+// residual-restriction 469 instead of 404 and the residual update 1139 instead of 996,
+// an IB step 104.4 ms instead of 108.5; at 256^3 26.6 / 29.3, 76 / 65 and 144 / 135 us,
+// no difference in all. AFMIB_SPLIT=0, 1: at no, at every such size.
+bool mg_split_ok(const Dims& d, const float* x, const float* b, const float* cb, const float* cx) {
+    const char* e = std::getenv("AFMIB_SPLIT");
+    if (e ? e[0] == '0' : d.ncell() <= 1ll << 24) return false;
+    const char* i = std::getenv("AFMIB_INIT_SWEEP");
+    const char* g = std::getenv("AFMIB_UPDATE_DF_GENERIC");
+    return !(i && i[0] == '0') && !(g && g[0] == '1') && !rbgs_pair_ok(d) && rr_mode(d, sizeof(float), x, b, cb) == 2 &&
+           transfer_cols_ok(d, x, cx) && d.nz % 4 == 0 && d.ny % BY == 0;
+}
+
 void mg_kernel_attributes() {
     auto set = [](const void* f) { cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRrSmem); };
-    set((const void*)k_resid_restrict_cols<8, false>);
-    set((const void*)k_resid_restrict_cols<4, false>);
-    set((const void*)k_resid_restrict_cols<2, false>);
-    set((const void*)k_resid_restrict_cols<1, false>);
-    set((const void*)k_resid_restrict_cols<8, true>);
-    set((const void*)k_resid_restrict_cols<4, true>);
-    set((const void*)k_resid_restrict_cols<2, true>);
-    set((const void*)k_resid_restrict_cols<1, true>);
+    set((const void*)k_resid_restrict_cols<8, false, false>);
+    set((const void*)k_resid_restrict_cols<8, false, true>);
+    set((const void*)k_resid_restrict_cols<4, false, false>);
+    set((const void*)k_resid_restrict_cols<4, false, true>);
+    set((const void*)k_resid_restrict_cols<2, false, false>);
+    set((const void*)k_resid_restrict_cols<2, false, true>);
+    set((const void*)k_resid_restrict_cols<1, false, false>);
+    set((const void*)k_resid_restrict_cols<1, false, true>);
+    set((const void*)k_resid_restrict_cols<8, true, false>);
+    set((const void*)k_resid_restrict_cols<8, true, true>);
+    set((const void*)k_resid_restrict_cols<4, true, false>);
+    set((const void*)k_resid_restrict_cols<4, true, true>);
+    set((const void*)k_resid_restrict_cols<2, true, false>);
+    set((const void*)k_resid_restrict_cols<2, true, true>);
+    set((const void*)k_resid_restrict_cols<1, true, false>);
+    set((const void*)k_resid_restrict_cols<1, true, true>);
 }
 
 template <typename T>
 void launch_resid_restrict(const Dims& d, T* coarse_b, const T* x, const T* b, cudaStream_t s, int rev,
-                           bool red) {
+                           bool red, bool split) {
     if constexpr (sizeof(T) == sizeof(float)) {
-        if (rr_mode(d, sizeof(T), x, b, coarse_b) == 2) {
+        if (split || rr_mode(d, sizeof(T), x, b, coarse_b) == 2) {
             // coarse planes per block: the largest of 8, 4, 2 that leaves at least
             // AFMIB_RR_MIN_BLOCKS (default 512) blocks (two resident per SM)
             const char* e = std::getenv("AFMIB_RR_MIN_BLOCKS");
@@ -1892,8 +2021,14 @@ void launch_resid_restrict(const Dims& d, T* coarse_b, const T* x, const T* b, c
             const float* bf = reinterpret_cast<const float*>(b);
 #define AFMIB_RR_COLS(CZV)                                                                            \
     do {                                                                                              \
-        if (d.channel) launch_dep(g, blk, kRrSmem, s, k_resid_restrict_cols<CZV, true>, d, cbf, xf, bf, rev); \
-        else launch_dep(g, blk, kRrSmem, s, k_resid_restrict_cols<CZV, false>, d, cbf, xf, bf, rev);         \
+        if (d.channel && split)                                                                       \
+            launch_dep(g, blk, kRrSmem, s, k_resid_restrict_cols<CZV, true, true>, d, cbf, xf, bf, rev); \
+        else if (split)                                                                               \
+            launch_dep(g, blk, kRrSmem, s, k_resid_restrict_cols<CZV, false, true>, d, cbf, xf, bf, rev); \
+        else if (d.channel)                                                                           \
+            launch_dep(g, blk, kRrSmem, s, k_resid_restrict_cols<CZV, true, false>, d, cbf, xf, bf, rev); \
+        else                                                                                          \
+            launch_dep(g, blk, kRrSmem, s, k_resid_restrict_cols<CZV, false, false>, d, cbf, xf, bf, rev); \
     } while (0)
             if (z == 8) AFMIB_RR_COLS(8);
             else if (z == 4) AFMIB_RR_COLS(4);
@@ -1915,18 +2050,18 @@ void launch_resid_restrict(const Dims& d, T* coarse_b, const T* x, const T* b, c
 }
 
 template <typename T>
-void launch_prolong_add(const Dims& d, T* fine, const T* coarse, cudaStream_t s, int rev, bool black) {
+void launch_prolong_add(const Dims& d, T* fine, const T* coarse, cudaStream_t s, int rev, bool black, bool split) {
     if constexpr (sizeof(T) == sizeof(float)) {
-        if (transfer_cols_ok(d, fine, coarse)) {
+        if (split || transfer_cols_ok(d, fine, coarse)) {
             // AFMIB_PROLONG_MAX_PLANES caps the planes per block (a sweep knob)
             const char* e = std::getenv("AFMIB_PROLONG_MAX_PLANES");
             int z = std::min(transfer_planes(d), e ? std::max(1, std::atoi(e)) : 8);
             while (z & (z - 1)) z &= z - 1;  // a power of two, so a divisor of the plane count
             const dim3 g = transfer_grid(d, z), b(32, kTrBY);
-            if (z == 8) launch_dep(g, b, 0, s, k_prolong_cols<T, 8>, d, fine, coarse, rev);
-            else if (z == 4) launch_dep(g, b, 0, s, k_prolong_cols<T, 4>, d, fine, coarse, rev);
-            else if (z == 2) launch_dep(g, b, 0, s, k_prolong_cols<T, 2>, d, fine, coarse, rev);
-            else launch_dep(g, b, 0, s, k_prolong_cols<T, 1>, d, fine, coarse, rev);
+            if (z == 8) launch_dep(g, b, 0, s, split ? k_prolong_cols<T, 8, true> : k_prolong_cols<T, 8, false>, d, fine, coarse, rev);
+            else if (z == 4) launch_dep(g, b, 0, s, split ? k_prolong_cols<T, 4, true> : k_prolong_cols<T, 4, false>, d, fine, coarse, rev);
+            else if (z == 2) launch_dep(g, b, 0, s, split ? k_prolong_cols<T, 2, true> : k_prolong_cols<T, 2, false>, d, fine, coarse, rev);
+            else launch_dep(g, b, 0, s, split ? k_prolong_cols<T, 1, true> : k_prolong_cols<T, 1, false>, d, fine, coarse, rev);
             return;
         }
     }
@@ -1951,24 +2086,34 @@ void launch_lap_defect(const Dims& d, TD* r, const double* x, const double* b, R
                sc, out, r_lo, lo_split());
 }
 void launch_lap_defect_df(const Dims& d, float* rh, float* rl, const double* x, const double* b, const double* sum,
-                          double scale, RedScratch sc, double* out, cudaStream_t s) {
+                          double scale, RedScratch sc, double* out, cudaStream_t s, bool split) {
     const dim3 blk(kRBX, kRBY);
+    if (split) {
+        launch_dep(red_grid3(d.nx, d.ny, d.nz / 2), blk, 0, s, k_lap_defect_df<2, Ix2, true>, d, rh, rl, x, b, sum, scale, sc,
+                   out);
+        return;
+    }
     if (d.nz % 2 == 0)
-        AFMIB_IX(d, (launch_dep(red_grid3(d.nx, d.ny, d.nz / 2), blk, 0, s, k_lap_defect_df<2, IX>, d, rh, rl, x, b,
+        AFMIB_IX(d, (launch_dep(red_grid3(d.nx, d.ny, d.nz / 2), blk, 0, s, k_lap_defect_df<2, IX, false>, d, rh, rl, x, b,
                                 sum, scale, sc, out)));
     else
-        AFMIB_IX(d, (launch_dep(red_grid3(d.nx, d.ny, d.nz), blk, 0, s, k_lap_defect_df<1, IX>, d, rh, rl, x, b, sum,
+        AFMIB_IX(d, (launch_dep(red_grid3(d.nx, d.ny, d.nz), blk, 0, s, k_lap_defect_df<1, IX, false>, d, rh, rl, x, b, sum,
                                 scale, sc, out)));
 }
 void launch_lap_update_df(const Dims& d, double* x, const float* e, float* rh, float* rl, RedScratch sc, double* out,
-                          cudaStream_t s) {
+                          cudaStream_t s, bool split) {
     constexpr int ZU = 2;
     const char* g = std::getenv("AFMIB_UPDATE_DF_GENERIC");
-    if (d.nz > 1 && d.nz % ZU == 0 && !(g && g[0] == '1')) {
+    if (split || (d.nz > 1 && d.nz % ZU == 0 && !(g && g[0] == '1'))) {
         const int gx = (d.nx + kRBX - 1) / kRBX, gy = (d.ny + kRBY - 1) / kRBY;
         int gz = d.nz / ZU;
         if ((long long)gx * gy * gz > kMaxRedBlocks) gz = std::max(1, kMaxRedBlocks / (gx * gy));
-        AFMIB_IX(d, (launch_dep(dim3(gx, gy, gz), dim3(kRBX, kRBY), 0, s, k_lap_update_df2<ZU, kUpdateMinBlocks, IX>,
+        if (split) {
+            launch_dep(dim3(gx, gy, gz), dim3(kRBX, kRBY), 0, s, k_lap_update_df2<ZU, kUpdateMinBlocks, Ix2, true>, d, x, e,
+                       rh, rl, sc, out);
+            return;
+        }
+        AFMIB_IX(d, (launch_dep(dim3(gx, gy, gz), dim3(kRBX, kRBY), 0, s, k_lap_update_df2<ZU, kUpdateMinBlocks, IX, false>,
                                 d, x, e, rh, rl, sc, out)));
         return;
     }
@@ -1994,13 +2139,13 @@ void launch_coarse_solve(const Dims& d, T* x, T* b, T* r, T* p, T* q, double tol
     template void launch_lap_apply<T>(const Dims&, T*, const T*, cudaStream_t);                          \
     template void launch_residual<T>(const Dims&, T*, const T*, const T*, RedScratch*, double*, cudaStream_t, int); \
     template void launch_residual_red<T>(const Dims&, T*, const T*, const T*, cudaStream_t, int);                  \
-    template void launch_rbgs<T>(const Dims&, int, T*, const T*, cudaStream_t, double, int);                        \
-    template void launch_rbgs_first<T>(const Dims&, T*, const T*, cudaStream_t, double, int);                      \
+    template void launch_rbgs<T>(const Dims&, int, T*, const T*, cudaStream_t, double, int, bool);                        \
+    template void launch_rbgs_first<T>(const Dims&, T*, const T*, cudaStream_t, double, int, bool);                      \
     template PipeCfg rbgs_pipe_cfg<T>(const Dims&);                                                      \
     template void launch_rbgs_pipe<T>(const Dims&, const PipeCfg&, const T*, T*, const T*, int*, cudaStream_t); \
     template void launch_restrict<T>(const Dims&, T*, const T*, cudaStream_t, int, bool);                   \
-    template void launch_prolong_add<T>(const Dims&, T*, const T*, cudaStream_t, int, bool);                \
-    template void launch_resid_restrict<T>(const Dims&, T*, const T*, const T*, cudaStream_t, int, bool); \
+    template void launch_prolong_add<T>(const Dims&, T*, const T*, cudaStream_t, int, bool, bool);                \
+    template void launch_resid_restrict<T>(const Dims&, T*, const T*, const T*, cudaStream_t, int, bool, bool); \
     template void launch_prolong_assign<T>(const Dims&, T*, const T*, cudaStream_t);                     \
     template void launch_coarse_solve<T>(const Dims&, T*, T*, T*, T*, T*, double, int, int*, cudaStream_t);
 

@@ -200,6 +200,7 @@ struct afmib_solver {
     int pass_rev = 0;
     cudaGraphExec_t vg64 = nullptr, vg32[kMaxInnerCycles + 1] = {};
     long long vg64_launches = 0, vg32_launches[kMaxInnerCycles + 1] = {};
+    bool split0 = false;  // the FP32 fine level's x and b are split by colour
     bool mg_loop = true;  // vg64: the whole solve loop, decided on the device (false: not supported)
     bool spread64 = false, interp64 = false;  // mixed form: IB transfers in FP64
     // warm start of each projection from the potential of the previous
@@ -620,7 +621,7 @@ int pass_dir(afmib_solver* s, const Dims& d, size_t elem) {
 
 // from_zero: x starts at zero and its contents are not (launch_rbgs_first)
 template <typename T>
-int smooth(afmib_solver* s, MGLevelT<T>& L, int sweeps, bool from_zero = false) {
+int smooth(afmib_solver* s, MGLevelT<T>& L, int sweeps, bool from_zero = false, bool split = false) {
     const double Ns = (double)L.d.ncell() * sizeof(T);
     const int id = L.d.nx == s->d.nx ? P_RBGS0 : P_RBGS;  // finest level kept apart in the profile
     const double omega = sizeof(T) == sizeof(float) ? s->inner_omega : 1.0;
@@ -646,16 +647,16 @@ int smooth(afmib_solver* s, MGLevelT<T>& L, int sweeps, bool from_zero = false) 
     for (; j < sweeps; ++j) {
         if (from_zero && j == 0) {
             ProfScope ps(s, id, 2 * Ns);
-            launch_rbgs_first<T>(L.d, L.x, L.b, s->st, omega, pass_dir(s, L.d, sizeof(T)));
+            launch_rbgs_first<T>(L.d, L.x, L.b, s->st, omega, pass_dir(s, L.d, sizeof(T)), split);
             continue;
         }
         {
             ProfScope ps(s, id, 1.5 * Ns);
-            launch_rbgs<T>(L.d, 0, L.x, L.b, s->st, omega, pass_dir(s, L.d, sizeof(T)));
+            launch_rbgs<T>(L.d, 0, L.x, L.b, s->st, omega, pass_dir(s, L.d, sizeof(T)), split);
         }
         {
             ProfScope ps(s, id, 1.5 * Ns);
-            launch_rbgs<T>(L.d, 1, L.x, L.b, s->st, omega, pass_dir(s, L.d, sizeof(T)));
+            launch_rbgs<T>(L.d, 1, L.x, L.b, s->st, omega, pass_dir(s, L.d, sizeof(T)), split);
         }
     }
     CKL();
@@ -737,12 +738,13 @@ int vcycle(afmib_solver* s, size_t l, bool x_zero = false) {
     const int nu1 = sizeof(T) == sizeof(float) ? (fine ? s->inner_nu1 : s->inner_nu1c) : s->cfg.nu1;
     const int nu2 = sizeof(T) == sizeof(float) ? (fine ? s->inner_nu2 : s->inner_nu2c) : s->cfg.nu2;
     const bool red = restrict_after_sweep(L.d, sizeof(T), nu1);
-    TRY(smooth(s, L, nu1, x_zero));
+    const bool split = fine && sizeof(T) == sizeof(float) && s->split0;
+    TRY(smooth(s, L, nu1, x_zero, split));
     MGLevelT<T>& C = lv[l + 1];
-    if (resid_restrict_fused_ok(L.d, sizeof(T), L.x, L.b, C.b)) {
+    if (split || resid_restrict_fused_ok(L.d, sizeof(T), L.x, L.b, C.b)) {
         // x, b read; coarse b written (the fine residual stays on chip)
         ProfScope ps(s, fine ? P_RESID_RESTRICT0 : P_RESID_RESTRICT, 2 * Ns + Ns / 8);
-        launch_resid_restrict<T>(L.d, C.b, L.x, L.b, s->st, pass_dir(s, L.d, sizeof(T)), red);
+        launch_resid_restrict<T>(L.d, C.b, L.x, L.b, s->st, pass_dir(s, L.d, sizeof(T)), red, split);
     } else {
         {
             ProfScope ps(s, fine ? P_RESID0 : P_RESID, 3 * Ns);
@@ -759,9 +761,9 @@ int vcycle(afmib_solver* s, size_t l, bool x_zero = false) {
     {
         ProfScope ps(s, fine ? P_PROLONG0 : P_PROLONG, 2 * Ns + Ns / 8);
         launch_prolong_add<T>(L.d, L.x, C.x, s->st, pass_dir(s, L.d, sizeof(T)),
-                              prolong_before_sweep(L.d, sizeof(T), nu2));
+                              prolong_before_sweep(L.d, sizeof(T), nu2), split);
     }
-    TRY(smooth(s, L, nu2));
+    TRY(smooth(s, L, nu2, false, split));
     return AFMIB_OK;
 }
 
@@ -876,7 +878,7 @@ int inner_vcycles32(afmib_solver* s, int ncyc) {
             for (int k = 0; k < nc; ++k) TRY(vcycle<float>(s, 0, k == 0));
             if (lap_df_on(s)) {
                 ProfScope ps(s, P_LAP_UPDATE, (double)N * (8 + 4 + 8 + 8 + 8 + 4));
-                launch_lap_update_df(L.d, L.x, L32.x, L32.b, s->plo, s->red, s->scal + 9, s->st);
+                launch_lap_update_df(L.d, L.x, L32.x, L32.b, s->plo, s->red, s->scal + 9, s->st, s->split0);
             } else {
                 ProfScope ps(s, P_CORRECT, (double)N * (8 + 4 + 8));
                 launch_add_correction<float>(N, L.x, L32.x, s->st);
@@ -1237,7 +1239,7 @@ int mg_solve_mixed(afmib_solver* s, int* cycles) {
             ProfScope ps(s, P_LAP_DEFECT, (double)N * (8 + 8 + 4 + (df ? 4 : 0)));
             if (fuse_mean)
                 launch_lap_defect_df(L.d, L32.b, s->plo, L.x, L.b, s->scal + 8, 1.0 / (double)N, s->red, s->scal + 9,
-                                     s->st);
+                                     s->st, s->split0);
             else if (!s->bfp_defects || !launch_lap_defect_bfp(L.d, L32.b, L.x, L.b, s->red, s->scal + 9, s->st))
                 launch_lap_defect<float>(L.d, L32.b, L.x, L.b, s->red, s->scal + 9, s->st, df ? s->plo : nullptr);
         }
@@ -2392,6 +2394,8 @@ int create(afmib_solver* s, const afmib_config* c, void* stream) {
                 s->tail_level32 = (int)l;
         }
     }
+    s->split0 = s->mixed && s->lv32.size() > 1 && s->tail_level32 != 0 && lap_df_on(s) && s->proj_df && !s->pipe_smoother &&
+                s->inner_nu1 > 0 && mg_split_ok(s->d, s->lv32[0].x, s->lv32[0].b, s->lv32[1].b, s->lv32[1].x);
     CK(cudaStreamSynchronize(s->st));
     return AFMIB_OK;
 }
