@@ -14,6 +14,8 @@
 #include <string>
 #include <vector>
 
+#include <cuda.h>  // types; the one driver call is looked up at run time
+
 #include "afmib.h"
 #include "kernels.h"
 #include "kernels_ib.h"
@@ -279,7 +281,10 @@ constexpr size_t kArenaMost = 2 << 20, kArenaChunk = 1 << 20;  // a chunk takes 
 #define CK(call)                                                                              \
     do {                                                                                      \
         cudaError_t e_ = (call);                                                              \
-        if (e_ != cudaSuccess) return s->fail(AFMIB_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
+        if (e_ != cudaSuccess) {                                                              \
+            cudaGetLastError(); /* reported here, not by the next call as well */             \
+            return s->fail(AFMIB_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
+        }                                                                                     \
     } while (0)
 
 #define CKL()                                                                                 \
@@ -373,12 +378,38 @@ int copy_out(afmib_solver* s, double* dst, const double* src, long long n) {
     return AFMIB_OK;
 }
 
+// Whether the n doubles at p lie within one allocation of the current device's own
+// memory (not host, managed or another device's). The copies refuse a buffer that
+// ends before its field does; a kernel on the buffer itself would not notice.
+bool on_device(const void* p, long long n) {
+    typedef CUresult (*Query)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+    static const Query query = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult r;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 7000, cudaEnableDefault, &r) != cudaSuccess)
+            cudaGetLastError();
+        return (Query)f;
+    }();
+    CUpointer_attribute want[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                  CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                  CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    unsigned type = 0, managed = 0;  // 0: not known to the driver
+    int ordinal = -1, dev = -2;
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    void* got[] = {&type, &managed, &ordinal, &start, &size};
+    const CUdeviceptr a = (CUdeviceptr)(uintptr_t)p;
+    return query && query(5, want, got, a) == CUDA_SUCCESS && type == CU_MEMORYTYPE_DEVICE && !managed &&
+           cudaGetDevice(&dev) == cudaSuccess && ordinal == dev && a >= start &&
+           a + (size_t)n * sizeof(double) <= start + size;
+}
+
 // The caller's buffers of a single-operator call: the kernels read and write
-// them in place where they are memory of this device, aligned, and no output
-// overlaps another buffer of the call (then the copies that every other pointer
-// needs would be most of the call: 12 of them for a spread and an
+// them in place where they are whole buffers in memory of this device, aligned, and
+// no output overlaps another buffer of the call (then the copies that every other
+// pointer needs would be most of the call: 12 of them for a spread and an
 // interpolation, 500 MB each way at 256^3); host, managed and other devices'
-// memory goes through the solver's own buffers.
+// memory and buffers of several mappings go through the solver's own buffers.
 struct CallBufs {
     afmib_solver* s;
     struct Range { uintptr_t a, b; bool out; };
@@ -398,13 +429,7 @@ struct CallBufs {
                 if (r.a == a && r.b == b && r.out == out && self++ == 0) continue;  // the buffer itself
                 if (out || r.out) return false;
             }
-        cudaPointerAttributes at{};
-        if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        int dev = -1;
-        return at.type == cudaMemoryTypeDevice && cudaGetDevice(&dev) == cudaSuccess && at.device == dev;
+        return on_device(p, n);
     }
     // p itself, or its values in own
     int in(const double* p, long long n, double* own, const double** use) {
