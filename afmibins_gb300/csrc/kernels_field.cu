@@ -1524,18 +1524,18 @@ __global__ void __launch_bounds__(kRedBlock) k_helm_update_df(Dims d, int comp, 
     grid_sum<1>(a, sc, out);
 }
 
-// The same for 3D grids with nz % ZU == 0: each thread takes ZU
+// The same for power-of-two grids with nz % ZU == 0: each thread takes ZU
 // consecutive z cells of one (x, y) column (the column's e values reused from
-// registers, 32-bit indices, every load of the batch issued
+// registers, 32-bit shift-composed indices, every load of the batch issued
 // before the rows are evaluated), blocks walk z batches in steps of grid.z;
 // the same arithmetic per cell, so the same bits.
-template <int ZU, int MINB, typename IX>
+template <int ZU, int MINB>
 __global__ void __launch_bounds__(kRedBlock, MINB) k_helm_update_df2(Dims d, int comp, df2 off, df2 cxa,
                                                               double* __restrict__ x, const float* __restrict__ e,
                                                               float* __restrict__ rh, float* __restrict__ rl,
                                                               RedScratch sc, double* out) {
     wait_launch();
-    const IX I(d);
+    const Ix2 I(d);
     float acc = 0.f;
     const int xi = blockIdx.x * kRBX + threadIdx.x, yi = blockIdx.y * kRBY + threadIdx.y;
     const bool vwall = d.channel && comp == 1 && yi == 0;
@@ -1588,7 +1588,7 @@ __global__ void __launch_bounds__(kRedBlock, MINB) k_helm_update_df2(Dims d, int
     grid_sum<1>(a, sc, out);
 }
 
-// AFMIB_UPDATE_DF_GENERIC=1: the one-cell kernel on every grid
+// AFMIB_UPDATE_DF_GENERIC=1: the one-cell kernel on power-of-two grids too
 // (read at every launch, so that a test compares both in one process)
 static bool update_df_generic() {
     const char* e = std::getenv("AFMIB_UPDATE_DF_GENERIC");
@@ -1603,12 +1603,12 @@ void launch_helm_update_df(const Dims& d, int comp, double scale, double* x, con
     // and 45.5 for eight (more registers, fewer warps) and 45.5 for the
     // general kernel; registers capped for kUpdateMinBlocks resident blocks
     constexpr int ZU = 2;
-    if (d.nz > 1 && d.nz % ZU == 0 && !update_df_generic()) {
+    if (d.nz > 1 && d.nz % ZU == 0 && ix2_ok(d) && !update_df_generic()) {
         const int gx = (d.nx + kRBX - 1) / kRBX, gy = (d.ny + kRBY - 1) / kRBY;
         int gz = d.nz / ZU;
         if ((long long)gx * gy * gz > kMaxRedBlocks) gz = std::max(1, kMaxRedBlocks / (gx * gy));
-        AFMIB_IX(d, (launch_dep(dim3(gx, gy, gz), dim3(kRBX, kRBY), 0, s, k_helm_update_df2<ZU, kUpdateMinBlocks,
-                                IX>, d, comp, o, c, x, e, rh, rl, sc, out)));
+        launch_dep(dim3(gx, gy, gz), dim3(kRBX, kRBY), 0, s, k_helm_update_df2<ZU, kUpdateMinBlocks>, d, comp, o, c,
+                   x, e, rh, rl, sc, out);
         return;
     }
     launch_dep(red_grid3(d.nx, d.ny, d.nz), dim3(kRBX, kRBY), 0, s, k_helm_update_df, d, comp, o, c, x, e, rh, rl,
@@ -1777,9 +1777,8 @@ __global__ void __launch_bounds__(BX * BY, MINB) k_helm_first(Dims d, int comp, 
 
 // Red-black order needs every wrap to join the two colours: even extents in the
 // periodic directions (the channel's y has walls; 2D grids keep Jacobi sweeps).
-// On a 96x80x112 grid these sweeps with the interleaved double-float solves take
-// an IB step from 4.57 to 3.88 ms against Jacobi sweeps and FP64 defects, one
-// solve after another.
+// On a 96x80x112 grid these sweeps with the interleaved solves take an IB step from
+// 4.57 to 3.88 ms against Jacobi sweeps, one solve after another.
 bool helm_rbgs_ok(const Dims& d) {
     return d.nz > 1 && d.nx % 2 == 0 && d.nz % 2 == 0 && (d.channel || d.ny % 2 == 0);
 }

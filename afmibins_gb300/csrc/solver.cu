@@ -1152,14 +1152,23 @@ bool helm_overlap_ok(afmib_solver* s, double scale) {
            gs_sweeps(d, scale, s->cfg.inner_tol) > 0 && helm_rbgs_ok(d);
 }
 
+// Whether the interleaved solves of a sub-step keep the outer residual as a pair of
+// floats (helm_df): on power-of-two extents, where the pair's update with its shifted
+// indices saves time at the sizes that are bound by memory (256^3: 43.0 -> 45.5 steps/s).
+// Elsewhere, and in the adjoint's solves, FP64 defects after each correction hold 53
+// bits against 47 and cost no more (96x80x112 IB step 3.04 ms against 3.15 with pairs,
+// 64^3 gradient 13.6 ms with either, 48^3 12.5 against 13.0).
+bool helm_pairs_ok(const afmib_solver* s) {
+    return s->helm_df && s->rlo[0] && ix2_ok(s->d) && s->d.nz % 8 == 0;
+}
+
 template <typename F>
-int helm_solve3_mixed(afmib_solver* s, double scale, double* const x[3], const double* const b[3], F first) {
+int helm_solve3_mixed(afmib_solver* s, double scale, double* const x[3], const double* const b[3], bool df, F first) {
     const Dims& d = s->d;
     const long long N = s->N();
     const int gsw = gs_sweeps(d, scale, s->cfg.inner_tol);
     const bool big = s->alternate && (double)N * sizeof(float) >= 32.0 * (1 << 20);
     cudaStream_t hs = s->hi;
-    const bool df = s->helm_df && s->rlo[0];
     auto post = [&](int c, cudaStream_t q) -> int {
         CK(cudaMemcpyAsync(s->hscal + 12 + c, s->scal + 12 + c, sizeof(double), cudaMemcpyDeviceToHost, q));
         CK(cudaEventRecord(s->ev_def[c], q));
@@ -1379,7 +1388,7 @@ int substep(afmib_solver* s) {
         // backward Euler: right-hand side, first defect (x starts at uold),
         // Q(uold) and the copy of uold in one pass per component;
         // Crank-Nicolson: right-hand sides from Q(uold), then the solves
-        const bool ovl = helm_overlap_ok(s, s->s_minus());
+        const bool ovl = helm_overlap_ok(s, s->s_minus()), pairs = ovl && helm_pairs_ok(s);
         auto walls_of = [&](int c, const double** top, const double** bot) {
             *top = (!d.channel || c == 1) ? nullptr : (c == 0 ? ut : wt);
             *bot = (!d.channel || c == 1) ? nullptr : (c == 0 ? ub : wb);
@@ -1402,7 +1411,7 @@ int substep(afmib_solver* s) {
         };
         if (be) {
             if (ovl) {
-                TRY(helm_solve3_mixed(s, s->s_minus(), vel, s->rhs, [&](int c, cudaStream_t hs, float* lo) {
+                TRY(helm_solve3_mixed(s, s->s_minus(), vel, s->rhs, pairs, [&](int c, cudaStream_t hs, float* lo) {
                     be_first(c, s->d32c[c], s->scal + 12 + c, s->walk_blocks_be, hs, lo);
                 }));
             } else {
@@ -1414,7 +1423,7 @@ int substep(afmib_solver* s) {
             }
             s->qo_valid = true;
         } else {
-            const bool cn_first = ovl && s->helm_df && s->rlo[0] && s->qo_valid && s->cn_start_old;
+            const bool cn_first = pairs && s->qo_valid && s->cn_start_old;
             for (int c = 0; c < 3 && !cn_first; ++c) {
                 const double *top, *bot;
                 walls_of(c, &top, &bot);
@@ -1440,7 +1449,7 @@ int substep(afmib_solver* s) {
             }
             CKL();
             if (ovl) {
-                TRY(helm_solve3_mixed(s, s->s_minus(), vel, s->rhs, [&](int c, cudaStream_t hs, float* lo) {
+                TRY(helm_solve3_mixed(s, s->s_minus(), vel, s->rhs, pairs, [&](int c, cudaStream_t hs, float* lo) {
                     if (cn_first) {
                         const double *top, *bot;
                         walls_of(c, &top, &bot);
@@ -1840,10 +1849,10 @@ int helm_inverse(afmib_solver* s, double* x, const double* b) {
     if (helm_overlap_ok(s, s->s_minus())) {
         double* const xs[3] = {x, x + N, x + 2 * N};
         const double* const bs[3] = {b, b + N, b + 2 * N};
-        return helm_solve3_mixed(s, s->s_minus(), xs, bs, [&](int c, cudaStream_t hs, float* lo) {
+        return helm_solve3_mixed(s, s->s_minus(), xs, bs, false, [&](int c, cudaStream_t hs, float*) {
             ProfScope ps(s, P_HELM_DEFECT, (double)N * (8 + 8 + 4), 1, hs);
             launch_helm_defect<float>(s->d, c, s->s_minus(), xs[c], bs[c], s->d32c[c], s->red, s->scal + 12 + c, hs,
-                                      s->walk_blocks, lo);
+                                      s->walk_blocks);
         });
     }
     for (int c = 0; c < 3; ++c) {
