@@ -132,8 +132,9 @@ struct afmib_solver {
     // (AFMIB_CN_START_OLD=0: the current velocity and an FP64 stencil)
     bool cn_start_old = true;
     double *divb = nullptr, *walls = nullptr, *wallgrad = nullptr;
-    // CG vectors (the mixed form solves one system at a time with them), the
-    // batched solve's scalars, their two pinned copies and the copies' events
+    // CG vectors (one system's; a batch's other two work in adv and tmp, which are idle
+    // while a sub-step's or the reverse pass's solves run), the batched solve's scalars,
+    // their two pinned copies and the copies' events
     double *cg_r[3] = {}, *cg_p[3] = {}, *cg_q[3] = {};
     double *cgs = nullptr, *hcg = nullptr;
     cudaEvent_t ev_cg[2] = {};
@@ -541,7 +542,8 @@ int read_scalars(afmib_solver* s, int first, int n) {
 
 // ---------------------------------------------------------------------------
 // CG, src/alg/cg.h:32-56 (absolute 2-norm stop, warm start from x), bounded,
-// on n independent systems at once (CgBatch). The host launches each iteration
+// on n independent systems at once (CgBatch; with more than one, x and b are not adv or
+// tmp, which hold the other systems' vectors). The host launches each iteration
 // before it has read the previous one's norms (a system that has stopped
 // returns at once from every later launch), so the GPU does not wait for the
 // host: one iteration of empty launches at the end instead of a round trip of
@@ -2287,8 +2289,14 @@ int create(afmib_solver* s, const afmib_config* c, void* stream) {
     }
     TRY(dalloc(s, &s->walls, 4 * s->nxz()));
     TRY(dalloc(s, &s->wallgrad, 8 * s->nxz()));
-    const int ncg = s->mixed ? 1 : 3;
-    for (double** q : {s->cg_r, s->cg_p, s->cg_q}) TRY(dalloc_fields(s, q, ncg, N));
+    {
+        double** const cg[3] = {s->cg_r, s->cg_p, s->cg_q};
+        for (int k = 0; k < 3; ++k) {
+            TRY(dalloc(s, &cg[k][0], N));
+            cg[k][1] = s->adv[k];
+            cg[k][2] = s->tmp[k];
+        }
+    }
     TRY(dalloc(s, &s->cgs, 3 * kCgScalars));
     for (auto& e : s->ev_cg) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     TRY(dalloc(s, &s->red.partial, (size_t)kMaxRedBlocks * kMaxRedVals));
