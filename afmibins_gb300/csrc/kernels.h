@@ -257,6 +257,7 @@ struct TailBasis {
 template <typename T>
 struct TailLevels {
     int nlev, flat, x_zero;  // flat: 2D grid; x_zero: x starts at zero, its contents not yet cleared
+    int cluster;             // vcycle_tail_cluster
     Dims d[kMaxTailLevels];
     int nu1[kMaxTailLevels], nu2[kMaxTailLevels];
     double omega;
@@ -280,8 +281,10 @@ template <typename T>
 bool vcycle_tail_ok(const TailLevels<T>& a);
 template <typename T>
 void launch_vcycle_tail(const TailLevels<T>& a, cudaStream_t s);
-// the tail kernels' opt-ins on the current device (before any launch or stream capture)
-void vcycle_tail_attributes();
+// the tail kernels' opt-ins on the current device (before any launch or stream capture),
+// and the CTAs of its clusters: 16 where the device takes a non-portable size, else 8
+// (or fewer), no more than most
+int vcycle_tail_cluster(int most);
 template <typename T>
 void launch_rbgs_pipe(const Dims& d, const PipeCfg& c, const T* xin, T* xout, const T* b, int* err, cudaStream_t s);
 // Full-weighting restriction, src/mg/solver.h:153-181 (d = fine dims)

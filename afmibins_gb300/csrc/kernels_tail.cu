@@ -711,31 +711,23 @@ bool tail_attributes() {
     return ok16;
 }
 
-// CTAs per cluster: 16 where the device takes a non-portable size, else 8, else 1
-int tail_cluster() {
-    static const int cs = [] {
-        const bool ok16 = tail_attributes();
-        for (int c : {16, 8}) {
-            if (c == 16 && !ok16) continue;
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(c);
-            cfg.blockDim = dim3(kTailThreads);
-            cfg.dynamicSmemBytes = kTailSmem;
-            cudaLaunchAttribute at[1];
-            at[0].id = cudaLaunchAttributeClusterDimension;
-            at[0].val.clusterDim.x = c;
-            at[0].val.clusterDim.y = 1;
-            at[0].val.clusterDim.z = 1;
-            cfg.attrs = at;
-            cfg.numAttrs = 1;
-            int n = 0;
-            if (cudaOccupancyMaxActiveClusters(&n, tail_kernel<double>(false, true), &cfg) == cudaSuccess && n > 0)
-                return c;
-            cudaGetLastError();
-        }
-        return 1;
-    }();
-    return cs;
+// whether a cluster of c CTAs with the tail's shared memory fits the current device
+bool cluster_fits(int c) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(c);
+    cfg.blockDim = dim3(kTailThreads);
+    cfg.dynamicSmemBytes = kTailSmem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = c;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, tail_kernel<double>(false, true), &cfg) == cudaSuccess && n > 0) return true;
+    cudaGetLastError();
+    return false;
 }
 
 // Largest level of the tail by element size. FP32: a 32^3 level takes 15 us in
@@ -814,15 +806,14 @@ template <typename T>
 bool vcycle_tail_ok(const TailLevels<T>& a) {
     if (a.nlev < 1 || a.nlev > kMaxTailLevels || !a.basis.vx) return false;
     TailArgs<T> g{};
-    const int cs = tail_cluster();
-    const size_t bytes = tail_layout(a, cs, &g);
+    const size_t bytes = tail_layout(a, a.cluster, &g);
     return bytes > 0 && bytes <= kTailSmem;
 }
 
 template <typename T>
 void launch_vcycle_tail(const TailLevels<T>& a, cudaStream_t s) {
     TailArgs<T> g{};
-    int cs = tail_cluster();
+    int cs = a.cluster;
     size_t bytes = tail_layout(a, cs, &g);
     // one CTA where every level is the first CTA's own
     if (g.lv[0].nc == 1) cs = 1;
@@ -865,7 +856,12 @@ void launch_vcycle_tail(const TailLevels<T>& a, cudaStream_t s) {
     else cudaLaunchKernelEx(&cfg, k_mg_tail<T, false, false>, g);
 }
 
-void vcycle_tail_attributes() { tail_attributes(); }
+int vcycle_tail_cluster(int most) {
+    const bool ok16 = tail_attributes();
+    for (int c : {16, 8, 4, 2})
+        if (c <= most && (c < 16 || ok16) && cluster_fits(c)) return c;
+    return 1;
+}
 
 template bool vcycle_tail_ok<float>(const TailLevels<float>&);
 template bool vcycle_tail_ok<double>(const TailLevels<double>&);

@@ -182,9 +182,9 @@ struct afmib_solver {
     // integer form being instruction-bound at about the FP64 kernels' time)
     bool bfp_defects = false;
     // first multigrid level handled by the V-cycle tail of each hierarchy
-    // (-1: none; AFMIB_MG_TAIL=0), and the eigenbasis of the coarsest level's
-    // direct solve
-    int tail_level = -1, tail_level32 = -1;
+    // (-1: none; AFMIB_MG_TAIL=0), the CTAs of its cluster (at most 16,
+    // AFMIB_MG_TAIL_CLUSTER), and the eigenbasis of the coarsest level's direct solve
+    int tail_level = -1, tail_level32 = -1, tail_cluster = 16;
     TailBasis basis{};
     // mixed form: inner Helmholtz solves by fixed Jacobi sweeps where the
     // operator's diagonal dominance bounds them, as red-black Gauss-Seidel
@@ -700,6 +700,7 @@ TailLevels<T> tail_levels(afmib_solver* s, size_t l, bool x_zero) {
     if (a.nlev > kMaxTailLevels) return a;
     a.flat = s->d.nz == 1;
     a.x_zero = x_zero;
+    a.cluster = s->tail_cluster;
     for (int k = 0; k < a.nlev; ++k) {
         const bool fine = l + k == 0;
         a.d[k] = lv[l + k].d;
@@ -2202,7 +2203,8 @@ int create(afmib_solver* s, const afmib_config* c, void* stream) {
     struct Created { afmib_solver* s; ~Created() { s->creating = false; } } created{s};
     afmib_config& g = s->cfg;
     mg_kernel_attributes();  // before any capture of the V-cycles
-    vcycle_tail_attributes();
+    if (const char* e = std::getenv("AFMIB_MG_TAIL_CLUSTER")) s->tail_cluster = std::max(1, std::atoi(e));
+    s->tail_cluster = vcycle_tail_cluster(s->tail_cluster);
     if (g.n <= 0) g.n = g.nx;
     if (g.nu1 <= 0) g.nu1 = 2;
     if (g.nu2 <= 0) g.nu2 = 2;
