@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const unsigned* __res
 // (the values as 16 bits: they are positions); a warp owns a contiguous run of them
 // and counts its digits in a column of its own, so that a rank is the warp's count
 // so far plus the rank among the equal digits of the row, and the order is stable.
-constexpr int RSS_THREADS = 1024, RSS_ITEMS = 16, RS_SMALL = RSS_THREADS * RSS_ITEMS, RSS_COLS = RSS_THREADS / 32 + 1;
+constexpr int RSS_THREADS = 1024, RSS_ITEMS = 8, RS_SMALL = RSS_THREADS * RSS_ITEMS, RSS_COLS = RSS_THREADS / 32 + 1;
 
 // ITEMS rows of 32 pairs per warp
 template <int ITEMS>
@@ -483,7 +483,10 @@ template <>
 __device__ __forceinline__ double tc_to<double, dfl>(dfl v) { return f32_to_f64(v.v.hi) + f32_to_f64(v.v.lo); }
 
 // Running sum of double-float products: an exact two-sum of the leading words and
-// a plain sum of the trailing ones.
+// a plain sum of the trailing ones. Over the spreading's parts (60 terms at most per
+// half warp, then pair additions) its error is no larger than that of a chain of pair
+// additions: rms of the terms' sum of magnitudes, weights and forces of random sign,
+// 8 terms 1.4e-14 and 1.5e-14, 400 terms 2.9e-15 and 3.0e-15, 6000 7.8e-16 and 1.7e-15.
 struct alignas(8) DfAcc {
     float s, e;  // leading sum (two-summed), trailing sum
 };
@@ -534,7 +537,9 @@ __device__ __forceinline__ df2 dfacc_pair(DfAcc a) {
 // ---------------------------------------------------------------------------
 constexpr int kSpreadWarps = 8;
 constexpr int kSpreadCap = 192;  // FP64 or double-float markers staged at once
-constexpr int kSpreadBlocks = 5;  // blocks per SM
+// Resident blocks per SM that the registers are capped for and the grid counts on; 8^3
+// tiles of FP64 or double-float values take 47 KB of shared memory, which leaves four.
+constexpr int kSpreadBlocks = 5;
 // values staged per marker: 4 x weights, and the products of 4 z and 4 y weights
 // with the force
 constexpr int kSpreadVals = 4 + 16;
@@ -978,10 +983,13 @@ void radix_sort_pairs(unsigned* keys, int* vals, unsigned* keys_alt, int* vals_a
     *vals_out = va;
 }
 
-// One block up to RS_SMALL markers: 8.5, 20 and 30 us for 512, 5120 and 7500 of them
-// with the tile ranges, against 30, 59 and 60 us in passes over all SMs plus 10 for
-// the ranges and their memsets. At 20000 a block would take longer than the passes.
-bool sort_bins_small_ok(int n) { return n > 0 && n <= RS_SMALL; }
+// One block up to RS_SMALL markers and 65536 tiles (it clears the tile ranges too): with
+// the ranges 11.7, 16.7, 26.9 and 36.9 us for 512, 2048, 5120 and 8192 markers on 4096
+// tiles against 32, 41, 42 and 42 in passes over all SMs with the memsets; 14.8, 20.5,
+// 34.8 and 44.3 against 34, 44, 46 and 46 on 32768. At 9000 markers the passes win (45.2
+// against 43.0, 53.4 against 46.8), and the line in tiles is where 8192 markers take as
+// long (65536: 51.9 against 52.4; 131072: 61.7 against 52.6; on 262144 2048 do).
+bool sort_bins_small_ok(int n, int ntiles) { return n > 0 && n <= RS_SMALL && ntiles <= 65536; }
 void sort_bins_small(unsigned* keys, int* vals, int n, int bits, int cells_per_tile, int ntiles, int* tstart, int* tend,
                      int* counts, cudaStream_t s) {
     auto launch = [&](auto* kernel, int items) {
@@ -991,7 +999,6 @@ void sort_bins_small(unsigned* keys, int* vals, int n, int bits, int cells_per_t
         launch_dep(1, RSS_THREADS, smem, s, kernel, keys, vals, n, bits, cells_per_tile, ntiles, tstart, tend, counts);
     };
     if (n <= 2 * RSS_THREADS) launch(k_sort_small<2>, 2);
-    else if (n <= 8 * RSS_THREADS) launch(k_sort_small<8>, 8);
     else launch(k_sort_small<RSS_ITEMS>, RSS_ITEMS);
 }
 

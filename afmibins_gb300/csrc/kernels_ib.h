@@ -42,8 +42,8 @@ void radix_sort_pairs(unsigned* keys, int* vals, unsigned* keys_alt, int* vals_a
 
 void launch_tile_ranges(const unsigned* keys, int M, int cells_per_tile, int* tstart, int* tend, cudaStream_t s);
 // The sorted pairs (in place) and the tile ranges, counts[0..1] zeroed, in one launch
-// for the marker counts that sort_bins_small_ok takes
-bool sort_bins_small_ok(int n);
+// for the counts that sort_bins_small_ok takes
+bool sort_bins_small_ok(int n, int ntiles);
 void sort_bins_small(unsigned* keys, int* vals, int n, int bits, int cells_per_tile, int ntiles, int* tstart, int* tend,
                      int* counts, cudaStream_t s);
 // Tiles near markers (list, count[0]) and the occupied tiles' slots (count[1]) and

@@ -1607,7 +1607,7 @@ int bin_markers(afmib_solver* s, const double* P, bool fp32 = false, bool df_wei
     unsigned* ko = s->keys;
     int* vo = s->vals;
     const int C = s->tile_cells();
-    if (sort_bins_small_ok(M)) {
+    if (sort_bins_small_ok(M, s->ntiles)) {
         ProfScope ps(s, P_SORT, (double)M * 16 + 2.0 * s->ntiles * 4);
         sort_bins_small(s->keys, s->vals, M, key_bits(s), C, s->ntiles, s->tstart, s->tend, s->tcount, s->st);
     } else {
