@@ -1681,9 +1681,11 @@ void launch_mg_check(cudaGraphConditionalHandle h, MgCheck c, cudaStream_t s) { 
         c, 0); }
 
 // smallest level (x extent) on which the smoother and residual take the
-// batched z-column kernels (AFMIB_BATCH_MIN_NX; one cell per thread below:
-// at 64^3 the batched grid is 64 blocks, and the one-cell kernels measured
-// 5% faster over the coarse levels of a 256^3 V-cycle)
+// batched z-column kernels, 4 (FP32) or 2 (FP64) cells per thread
+// (AFMIB_BATCH_MIN_NX; one cell per thread below). With levels from 96 and from 64 on
+// batched, an FP64 channel step at 96x64x64 takes 3.94 and 3.95 ms against 3.83 (its
+// colours 10.4 us against 9.9: too few blocks), a mixed step at 96x80x112 3.21 and 3.22
+// against 3.26 (7.7 us against 8.4), one at 256^3 14.7 in every case.
 int batch_min_nx() {
     static const int v = [] {
         const char* e = std::getenv("AFMIB_BATCH_MIN_NX");
@@ -1888,10 +1890,11 @@ void launch_rbgs_pipe(const Dims& d, const PipeCfg& c, const T* xin, T* xout, co
 // kTrBY | ny / 2 and 16-byte aligned fine and coarse arrays;
 // AFMIB_TRANSFER_COLS=0 keeps the one-cell kernels (read at every launch, so
 // that a test can compare both in one process). FP64 keeps the one-cell
-// kernels: there both transfers are bound by the FP64 pipe (64 dependent FMAs
-// per coarse cell, about 9 FP64 operations per prolonged cell), and the column
-// kernels, with the same operations, measured 296 / 307 against 261 / 278 us
-// per 256^3 launch.
+// kernels, which take half of the cells (restrict_after_sweep,
+// prolong_before_sweep): residual, restriction and prolongation 119, 136 and 111 us
+// per 256^3 launch (21.2, 23.2 and 19.3 at 128^3), against 232, 173 and 193 (35.5,
+// 42.1 and 28.7) with the column kernels, which need every cell of the residual, and
+// 232, 262 and 147 with one-cell kernels on all cells.
 static bool transfer_cols_ok(const Dims& d, const void* fine, const void* coarse) {
     if (const char* e = std::getenv("AFMIB_TRANSFER_COLS"))
         if (e[0] == '0') return false;
@@ -1966,9 +1969,9 @@ bool resid_restrict_fused_ok(const Dims& d, size_t elem, const void* x, const vo
 // An FP32 fine level whose iterate and right-hand side are split by colour: every
 // kernel that takes them there has a split form, and the two arrays do not fit in
 // the L2 (126 MB): at 512^3 a colour takes 194 us instead of 243, the fused
-// residual-restriction 469 instead of 404 and the residual update 1139 instead of 996,
-// an IB step 104.4 ms instead of 108.5; at 256^3 26.6 / 29.3, 76 / 65 and 144 / 135 us,
-// no difference in all. AFMIB_SPLIT=0, 1: at no, at every such size.
+// residual-restriction 469 instead of 404 and the residual update 1145 instead of 997,
+// an IB step 104.6 ms instead of 108.5; at 256^3 26.7 / 29.6, 76 / 65 and 144 / 134 us,
+// a step 14.68 / 14.74 ms. AFMIB_SPLIT=0, 1: at no, at every such size.
 bool mg_split_ok(const Dims& d, const float* x, const float* b, const float* cb, const float* cx) {
     const char* e = std::getenv("AFMIB_SPLIT");
     if (e ? e[0] == '0' : d.ncell() <= 1ll << 24) return false;
