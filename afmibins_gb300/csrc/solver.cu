@@ -1144,7 +1144,8 @@ int helm_solve_mixed(afmib_solver* s, int comp, double scale, double* x, const d
 // behind it. Components are served in the order their defects were queued.
 // Each component goes through exactly the steps of helm_solve_mixed (same
 // defects, corrections and stopping test, bit for bit); only the order of
-// the norms' partial sums differs. first(c) launches component c's first
+// the norms' partial sums differs. With df the defects after the first are the
+// pair's updates on the correction stream instead (helm_pairs_ok). first(c) launches component c's first
 // defect into d32c[c] with its squared norm in scal[12 + c]. Needs the
 // Gauss-Seidel inner solve (helm_overlap_ok). With per-kernel profiling on,
 // each launch is timed by events on its own stream (durations of kernels
